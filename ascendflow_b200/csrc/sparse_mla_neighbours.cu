@@ -16,25 +16,12 @@
 namespace sparse_mla {
 namespace {
 
-constexpr int kSelectThreads = 512;
-constexpr int kSelectWarps = kSelectThreads / 32;
-
 // Monotone map of a finite FP32 value to an unsigned key: larger value, larger key.
 __device__ __forceinline__ uint32_t score_key(float value) {
   const uint32_t bits = __float_as_uint(value);
   return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
 }
 
-// One block per query token (blocks stride over tokens). Candidates are compressed rows
-// [0, min(available, cutoff)): the rows the attention kernel would accept for this token. The
-// min(TopK, candidates) highest scores win, ties going to the lower index; winners are written in
-// ascending index order, the rest of the 512 entries is -1.
-//
-// More candidates than TopK: an MSB-first radix select over the keys (four 8-bit digits, one
-// histogram per warp, one addition per warp and bin, so that the exponent digit's few hot bins
-// do not serialise anything)
-// finds the key of the TopK-th highest score and how many entries equal to it are taken; one more
-// pass in index order writes the winners through a block-wide prefix count.
 struct SelectParams {
   const float* scores;       // [T, span]
   const int32_t* cu;         // [B + 1]
@@ -45,140 +32,458 @@ struct SelectParams {
   int64_t span;
 };
 
+// The request of a token, found by a whole warp: 32 probes of cu_seqlens_q per step, so that 128
+// requests take two dependent loads and not seven.
+__device__ __forceinline__ int request_of(const int32_t* cu, int batches, int token, int lane) {
+  int lo = 0, hi = batches;  // invariant: cu[lo] <= token < cu[hi]
+  while (hi - lo > 1) {
+    const int step = (hi - lo + 31) >> 5;
+    const int probe = lo + lane * step;
+    const bool below = probe < hi && __ldg(cu + probe) <= token;
+    lo += (31 - __clz(__ballot_sync(0xffffffffu, below))) * step;  // lane 0 probes cu[lo]: always set
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
 // Completed compressed rows a token may see: min(C, cutoff), with the attention operator's
 // cutoff = max(0, C R + r - n + j + 1) / R (examples/sparse_attention/attention.py:339-341).
-__device__ __forceinline__ int visible_compressed_rows(const SelectParams& p, int token) {
-  int lo = 0, hi = p.batches;  // invariant: cu[lo] <= token < cu[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(p.cu + mid) <= token) lo = mid; else hi = mid;
-  }
-  const int begin = __ldg(p.cu + lo), count = __ldg(p.cu + lo + 1) - begin;
-  const int available = __ldg(p.seq_cmp + lo);
-  const int completed = available * p.ratio + __ldg(p.residual + lo);
+// Called by whole warps.
+__device__ __forceinline__ int visible_compressed_rows(const SelectParams& p, int token, int lane) {
+  const int request = request_of(p.cu, p.batches, token, lane);
+  const int begin = __ldg(p.cu + request), count = __ldg(p.cu + request + 1) - begin;
+  const int available = __ldg(p.seq_cmp + request);
+  const int completed = available * p.ratio + __ldg(p.residual + request);
   return min(available, max(0, completed - count + (token - begin) + 1) / p.ratio);
 }
 
-// Four consecutive scores per thread and step (16-byte loads, two in flight); `span` is a
-// multiple of four, so every row starts on a 16-byte boundary.
+// Four consecutive scores as keys (one 16-byte load); `span` is a multiple of four, so every row
+// starts on a 16-byte boundary and a load may run past `candidates` but never past the row.
 __device__ __forceinline__ void load_keys(const float* row, int i, int candidates, uint32_t (&key)[4], bool (&valid)[4]) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (i < candidates) v = __ldg(reinterpret_cast<const float4*>(row + i));  // may run past `candidates`, never past the row
+  if (i < candidates) v = __ldg(reinterpret_cast<const float4*>(row + i));
   key[0] = score_key(v.x); key[1] = score_key(v.y); key[2] = score_key(v.z); key[3] = score_key(v.w);
 #pragma unroll
   for (int e = 0; e < 4; ++e) valid[e] = i + e < candidates;
 }
 
-__global__ void __launch_bounds__(kSelectThreads) topk_select_kernel(const SelectParams p) {
-  __shared__ unsigned histogram[kSelectWarps][256];
-  __shared__ unsigned totals[256];
-  __shared__ unsigned long long warp_count[kSelectWarps], base_count;
-  __shared__ unsigned prefix_key, wanted;
+constexpr int kSelectBins = 256;
+constexpr int kSelectWindow = 65536;  // row positions covered by the bitmap of winners at a time
+
+// Shared memory of one selecting block.
+template <int kThreads, int kCapacity>
+struct SelectShared {
+  uint2 list[kCapacity];               // candidates: row position, score
+  __align__(16) unsigned bitmap[kSelectWindow / 32];
+  unsigned short place[kSelectWindow / 32];  // winners before each word of the bitmap
+  unsigned histogram[kSelectBins];
+  unsigned warp_sum[kThreads / 32];
+  unsigned count, low, high;           // candidates listed; extremes of what is being binned
+  unsigned bin, before, in_bin;        // result of find_bin
+  unsigned few_count;                  // entries in `few`
+  unsigned long long few[32], limit;   // the threshold bin's entries; the last winner
+};
+
+// Start `bytes` (a multiple of 16) at a 16-byte aligned address on their way to L2.
+__device__ __forceinline__ void prefetch_l2(const void* at, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(at), "r"(bytes));
+}
+
+// Inclusive prefix sum over a warp.
+__device__ __forceinline__ unsigned warp_scan(unsigned value, int lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned up = __shfl_up_sync(0xffffffffu, value, d);
+    if (lane >= d) value += up;
+  }
+  return value;
+}
+
+// The bin in which the running count over the histogram reaches `wanted`, what lies before it and
+// what it holds (s.bin stays as it was if the whole histogram holds fewer). Clears the histogram.
+// Called by the whole block after a barrier; ends with one.
+template <typename Shared>
+__device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kStep = kSelectThreads * 4;
-  constexpr int kInFlight = 2;  // 16-byte loads in flight per thread in the counting passes (four: slower)
-  for (int token = blockIdx.x; token < p.tokens; token += gridDim.x) {
-    const int candidates = int(min((int64_t)visible_compressed_rows(p, token), p.span));
-    const int take = min(kTopK, candidates);
-    int32_t* list = p.out + (size_t)token * kTopK;
-    const float* row = p.scores + (size_t)token * p.span;
-    __syncthreads();  // the shared words of the previous token are no longer read
-    if (candidates <= kTopK) {
-      for (int i = threadIdx.x; i < kTopK; i += blockDim.x) list[i] = i < candidates ? i : -1;
-      continue;
-    }
-    // ---- radix select: key of the take-th highest score ------------------------------------
-    if (threadIdx.x == 0) { prefix_key = 0; wanted = unsigned(take); }
-    for (int digit = 3; digit >= 0; --digit) {
-      const int shift = digit * 8;
-      for (int i = threadIdx.x; i < kSelectWarps * 256; i += blockDim.x) (&histogram[0][0])[i] = 0;
-      __syncthreads();
-      const unsigned prefix = prefix_key;
-      const unsigned mask = digit == 3 ? 0u : (0xffffffffu << (shift + 8));
-      // Lanes that fall into the same bin (most of them, for the exponent digit) add once,
-      // through their lowest lane.
-      for (int first = 0; first < candidates; first += kInFlight * kStep) {
-        uint32_t key[kInFlight][4];
-        bool valid[kInFlight][4];
-#pragma unroll
-        for (int h = 0; h < kInFlight; ++h) load_keys(row, first + h * kStep + threadIdx.x * 4, candidates, key[h], valid[h]);
-#pragma unroll
-        for (int h = 0; h < kInFlight; ++h)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const bool counted = valid[h][e] && (key[h][e] & mask) == prefix;
-            // from the second digit on, most warps hold no entry with the prefix: nothing to vote on
-            if (__ballot_sync(0xffffffffu, counted) == 0u) continue;
-            const unsigned bin = counted ? (key[h][e] >> shift) & 255u : 256u;
-            const unsigned peers = __match_any_sync(0xffffffffu, bin);
-            if (counted && lane == __ffs(peers) - 1) atomicAdd(&histogram[warp][bin], unsigned(__popc(peers)));
-          }
-      }
-      __syncthreads();
-      if (threadIdx.x < 256) {
-        unsigned sum = 0;
-#pragma unroll
-        for (int w = 0; w < kSelectWarps; ++w) sum += histogram[w][threadIdx.x];
-        totals[threadIdx.x] = sum;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {  // walk down from the highest bin until `wanted` entries are covered
-        unsigned above = 0;
-        int bin = 255;
-        while (bin > 0 && above + totals[bin] < wanted) above += totals[bin--];
-        prefix_key = prefix | (unsigned(bin) << shift);
-        wanted -= above;  // entries still to take among those that share the longer prefix
-      }
-      __syncthreads();
-    }
-    const unsigned threshold = prefix_key, equal_taken = wanted;  // wanted >= 1
-    // ---- winners in index order -------------------------------------------------------------
-    // Counts are packed: entries above the threshold in the low half, entries equal to it in the
-    // high half of a 64-bit word.
-    if (threadIdx.x == 0) base_count = 0;
+  unsigned mine = 0, scan = 0;
+  if (threadIdx.x < kSelectBins) {
+    mine = s.histogram[threadIdx.x];
+    s.histogram[threadIdx.x] = 0;
+    scan = warp_scan(mine, lane);
+    if (lane == 31) s.warp_sum[warp] = scan;
+  }
+  __syncthreads();
+  if (threadIdx.x < kSelectBins) {
+    unsigned before = scan - mine;
+    for (int w = 0; w < warp; ++w) before += s.warp_sum[w];
+    if (before < wanted && wanted <= before + mine) { s.bin = threadIdx.x; s.before = before; s.in_bin = mine; }
+  }
+  __syncthreads();
+}
+
+// The selection for any row, whatever its scores: an MSB-first radix select over the keys (four
+// 8-bit digits, one histogram per warp, one addition per warp and bin) finds the key of the
+// TopK-th highest score and how many entries equal to it are taken; one more pass in index order
+// writes the winners through a block-wide prefix count. Reads the row five times. Used where the
+// listed candidates of `topk_select_kernel` turn out to be too few or too many (masses of equal
+// scores, or scores whose sample says little about the row). Called by the whole block.
+template <int kThreads>
+__device__ __noinline__ void select_row_by_digits(const float* row, int candidates, int32_t* list, unsigned (*histogram)[256],
+                                                  unsigned* totals) {
+  __shared__ unsigned long long warp_count[kThreads / 32], base_count;
+  __shared__ unsigned prefix_key, wanted;
+  constexpr int kWarps = kThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kStep = kThreads * 4;
+  if (threadIdx.x == 0) { prefix_key = 0; wanted = kTopK; }
+  for (int digit = 3; digit >= 0; --digit) {
+    const int shift = digit * 8;
+    for (int i = threadIdx.x; i < kWarps * 256; i += kThreads) (&histogram[0][0])[i] = 0;
     __syncthreads();
+    const unsigned prefix = prefix_key;
+    const unsigned mask = digit == 3 ? 0u : (0xffffffffu << (shift + 8));
     for (int first = 0; first < candidates; first += kStep) {
-      const int i = first + threadIdx.x * 4;
       uint32_t key[4];
       bool valid[4];
-      load_keys(row, i, candidates, key, valid);
-      unsigned long long mine = 0;
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (valid[e]) mine += key[e] > threshold ? 1ull : (key[e] == threshold ? (1ull << 32) : 0ull);
-      unsigned long long scan = mine;  // inclusive scan over the warp
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long up = __shfl_up_sync(0xffffffffu, scan, d);
-        if (lane >= d) scan += up;
-      }
-      if (lane == 31) warp_count[warp] = scan;
-      __syncthreads();
-      unsigned long long before = base_count + scan - mine;
-      for (int w = 0; w < warp; ++w) before += warp_count[w];
-      unsigned greater_before = unsigned(before), equal_before = unsigned(before >> 32);
-      // An entry equal to the threshold is a winner while fewer than `equal_taken` such entries
-      // precede it; every winner's position is the number of winners before it.
+      load_keys(row, first + threadIdx.x * 4, candidates, key, valid);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        if (!valid[e]) continue;
-        if (key[e] > threshold) {
-          list[greater_before + min(equal_before, equal_taken)] = i + e;
-          ++greater_before;
-        } else if (key[e] == threshold) {
-          if (equal_before < equal_taken) list[greater_before + equal_before] = i + e;
-          ++equal_before;
-        }
+        const bool counted = valid[e] && (key[e] & mask) == prefix;
+        // from the second digit on, most warps hold no entry with the prefix: nothing to vote on
+        if (__ballot_sync(0xffffffffu, counted) == 0u) continue;
+        // Lanes that fall into the same bin (most of them, for the exponent digit) add once,
+        // through their lowest lane.
+        const unsigned bin = counted ? (key[e] >> shift) & 255u : 256u;
+        const unsigned peers = __match_any_sync(0xffffffffu, bin);
+        if (counted && lane == __ffs(peers) - 1) atomicAdd(&histogram[warp][bin], unsigned(__popc(peers)));
       }
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+      unsigned sum = 0;
+      for (int w = 0; w < kWarps; ++w) sum += histogram[w][threadIdx.x];
+      totals[threadIdx.x] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // walk down from the highest bin until `wanted` entries are covered
+      unsigned above = 0;
+      int bin = 255;
+      while (bin > 0 && above + totals[bin] < wanted) above += totals[bin--];
+      prefix_key = prefix | (unsigned(bin) << shift);
+      wanted -= above;  // entries still to take among those that share the longer prefix
+    }
+    __syncthreads();
+  }
+  const unsigned threshold = prefix_key, equal_taken = wanted;  // wanted >= 1
+  // Counts are packed: entries above the threshold in the low half, entries equal to it in the
+  // high half of a 64-bit word.
+  if (threadIdx.x == 0) base_count = 0;
+  __syncthreads();
+  for (int first = 0; first < candidates; first += kStep) {
+    const int i = first + threadIdx.x * 4;
+    uint32_t key[4];
+    bool valid[4];
+    load_keys(row, i, candidates, key, valid);
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (valid[e]) mine += key[e] > threshold ? 1ull : (key[e] == threshold ? (1ull << 32) : 0ull);
+    unsigned long long scan = mine;  // inclusive scan over the warp
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, scan, d);
+      if (lane >= d) scan += up;
+    }
+    if (lane == 31) warp_count[warp] = scan;
+    __syncthreads();
+    unsigned long long before = base_count + scan - mine;
+    for (int w = 0; w < warp; ++w) before += warp_count[w];
+    unsigned greater_before = unsigned(before), equal_before = unsigned(before >> 32);
+    // An entry equal to the threshold is a winner while fewer than `equal_taken` such entries
+    // precede it; every winner's position is the number of winners before it.
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!valid[e]) continue;
+      if (key[e] > threshold) {
+        list[greater_before + min(equal_before, equal_taken)] = i + e;
+        ++greater_before;
+      } else if (key[e] == threshold) {
+        if (equal_before < equal_taken) list[greater_before + equal_before] = i + e;
+        ++equal_before;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long add = 0;
+      for (int w = 0; w < kWarps; ++w) add += warp_count[w];
+      base_count += add;
+    }
+    __syncthreads();
+  }
+}
+
+// One block per query token. Candidates are compressed rows [0, min(available, cutoff)): the rows
+// the attention kernel would accept for this token. The min(TopK, candidates) highest scores win,
+// ties going to the lower index; winners are written in ascending index order, the rest of the 512
+// entries is -1.
+//
+// Bound by memory: the row is streamed once. A strided sample (one or two thousand scores, eight
+// to a sector) gives a floor that about twice TopK scores lie above; the stream lists what reaches
+// the floor (two instructions per score, next to nothing listed), and the exact selection runs on
+// that short list in shared memory: a histogram of the keys' distances from the highest, 256
+// bins, normally once; the few entries of the threshold's bin are ranked by comparison; a bitmap
+// of winning positions gives the output order. The list holds every score that reaches the
+// floor, so the result is exact whenever the list has at least TopK entries and did not
+// overflow; otherwise (hardly ever, unless most of the row is equal) `select_row_by_digits`.
+template <int kThreads, int kCapacity, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
+  using Shared = SelectShared<kThreads, kCapacity>;
+  extern __shared__ __align__(16) unsigned char select_smem[];
+  Shared& s = *reinterpret_cast<Shared*>(select_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int token = blockIdx.x;
+  const int candidates = int(min((int64_t)visible_compressed_rows(p, token, lane), p.span));
+  int32_t* list = p.out + (size_t)token * kTopK;
+  const float* row = p.scores + (size_t)token * p.span;
+  if (candidates <= kTopK) {
+    for (int i = threadIdx.x; i < kTopK; i += kThreads) list[i] = i < candidates ? i : -1;
+    return;
+  }
+  for (int i = threadIdx.x * 4; i < min(candidates + 31, kSelectWindow) / 32; i += kThreads * 4)
+    *reinterpret_cast<uint4*>(&s.bitmap[i]) = make_uint4(0, 0, 0, 0);
+  if (threadIdx.x < kSelectBins) s.histogram[threadIdx.x] = 0;
+  if (threadIdx.x == 0) { s.count = s.few_count = 0; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
+  __syncthreads();
+
+  // ---- floor ----------------------------------------------------------------------------------
+  unsigned floor_key = 0;  // short rows: everything is listed
+  if (candidates > kCapacity) {
+    constexpr int kMostQuads = 2;  // sampled 16-byte quads per thread, at most; two neighbouring threads share a sector
+    const int quads = candidates >= 160 * kThreads ? 2 : 1, sampled = quads * kThreads;
+    const unsigned row_pairs = unsigned(candidates) >> 3;
+    uint32_t key[4 * kMostQuads];
+#pragma unroll
+    for (int q = 0; q < kMostQuads; ++q) {
+      if (q < quads) {
+        const unsigned pair = (q * kThreads + threadIdx.x) >> 1;
+        const unsigned at = unsigned((unsigned long long)pair * row_pairs / unsigned(sampled / 2)) * 2 + (threadIdx.x & 1);
+        const float4 v = __ldg(reinterpret_cast<const float4*>(row) + at);
+        key[4 * q + 0] = score_key(v.x); key[4 * q + 1] = score_key(v.y);
+        key[4 * q + 2] = score_key(v.z); key[4 * q + 3] = score_key(v.w);
+      } else {
+        key[4 * q + 0] = key[4 * q + 1] = key[4 * q + 2] = key[4 * q + 3] = 0;
+      }
+    }
+    // The row's head on its way to L2 (behind the sample) while the floor is found.
+    if (threadIdx.x == 0) prefetch_l2(row, min(unsigned(candidates) * 4u & ~15u, 65536u));
+    // Only the sample's upper end matters: its maximum, and the lowest of the maxima of four
+    // threads each, above which lie at least kThreads / 4 samples (about four times as many).
+    unsigned best = 0;
+#pragma unroll
+    for (int e = 0; e < 4 * kMostQuads; ++e) best = max(best, key[e]);
+    best = max(best, __shfl_xor_sync(0xffffffffu, best, 1));
+    best = max(best, __shfl_xor_sync(0xffffffffu, best, 2));
+    const unsigned warp_low = __reduce_min_sync(0xffffffffu, best), warp_high = __reduce_max_sync(0xffffffffu, best);
+    if (lane == 0) { atomicMin(&s.low, warp_low); atomicMax(&s.high, warp_high); }
+    __syncthreads();
+    // Samples expected among the TopK best, and five standard deviations of that count on top:
+    // the floor lies below the TopK-th best score in all but a few rows in a hundred thousand.
+    const float expected = float(kTopK) * float(4 * sampled) / float(candidates);
+    unsigned wanted = unsigned(expected + 5.f * sqrtf(expected) + 2.f), lower = s.low, upper = s.high;
+    while (true) {  // normally once; again inside a bin that holds too many (a sample of both signs, say)
+      const int shift = max(0, 24 - __clz(int(upper - lower)));  // 256 bins over [lower, upper]
+#pragma unroll
+      for (int e = 0; e < 4 * kMostQuads; ++e)
+        if (key[e] >= lower && key[e] <= upper) atomicAdd(&s.histogram[(upper - key[e]) >> shift], 1u);
       __syncthreads();
-      if (threadIdx.x == 0) {
-        unsigned long long add = 0;
-        for (int w = 0; w < kSelectWarps; ++w) add += warp_count[w];
-        base_count += add;
+      find_bin(s, wanted);
+      if (s.bin == kSelectBins) break;  // fewer samples than wanted: all of them
+      const unsigned depth = ((s.bin + 1) << shift) - 1;
+      lower = depth >= upper - lower ? lower : upper - depth;
+      if (s.in_bin <= 32 || shift == 0) break;
+      upper -= s.bin << shift;
+      wanted -= s.before;
+    }
+    floor_key = lower;
+  }
+
+  // ---- one pass over the row --------------------------------------------------------------------
+  // Scores that reach the floor are listed in any order. (Subnormals are flushed in what follows:
+  // a floor among them would not tell them and the zeros apart.)
+  const float floor_value = floor_key == 0 ? -INFINITY : __uint_as_float(floor_key & 0x80000000u ? floor_key ^ 0x80000000u : ~floor_key);
+  if ((__float_as_uint(floor_value) & 0x7f800000u) == 0) {
+    select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
+    return;
+  }
+  constexpr int kInFlight = 4;  // 16-byte loads in flight per thread
+  const unsigned end = unsigned(candidates);  // unsigned: a step may reach past INT32_MAX
+  for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kInFlight * 4 * kThreads) {
+    float4 v[kInFlight];
+#pragma unroll
+    for (int h = 0; h < kInFlight; ++h) {
+      const unsigned i = first + h * kThreads * 4;
+      v[h] = i < end ? __ldcs(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // The sign of score - floor, shifted in: bit 15 - (4 h + e) is clear where the score reaches it.
+    unsigned below = 0;
+#pragma unroll
+    for (int h = 0; h < kInFlight; ++h) {
+      below = __funnelshift_l(__float_as_uint(v[h].x - floor_value), below, 1);
+      below = __funnelshift_l(__float_as_uint(v[h].y - floor_value), below, 1);
+      below = __funnelshift_l(__float_as_uint(v[h].z - floor_value), below, 1);
+      below = __funnelshift_l(__float_as_uint(v[h].w - floor_value), below, 1);
+    }
+    unsigned hits = ~below & 0xffffu;
+    if (first + (kInFlight - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
+#pragma unroll
+      for (int h = 0; h < kInFlight; ++h) {
+        const unsigned i = first + h * kThreads * 4, left = i < end ? min(end - i, 4u) : 0u;
+        hits &= ~((15u >> left) << (4 * (kInFlight - 1 - h)));
       }
+    }
+    if (hits == 0) continue;
+    unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+    if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
+#pragma unroll
+    for (int h = 0; h < kInFlight; ++h) {
+      const float values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (hits >> (4 * (kInFlight - 1 - h) + 3 - e) & 1) s.list[at++] = make_uint2(first + h * kThreads * 4 + e, __float_as_uint(values[e]));
+    }
+  }
+  __syncthreads();
+  const int listed = int(s.count);
+  if (listed < kTopK || listed > kCapacity) {
+    select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
+    return;
+  }
+
+  // ---- the TopK best of the list ----------------------------------------------------------------
+  // Ordered by (distance of the key from the highest, row position): smaller is better, all
+  // distinct. First the distance, then (more than 32 equal scores at the threshold) the position.
+  // "The highest" is the sample's, and what lies above it counts as distance 0, until the
+  // threshold turns out to lie there.
+  unsigned top = s.high, bottom = floor_key;
+  bool exact = false;
+  auto find_extremes = [&]() {
+    unsigned low = 0xffffffffu, high = 0;
+    for (int i = threadIdx.x; i < listed; i += kThreads) {
+      const unsigned key = score_key(__uint_as_float(s.list[i].y));
+      low = min(low, key);
+      high = max(high, key);
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    if (lane == 0) { atomicMin(&s.low, low); atomicMax(&s.high, high); }
+    __syncthreads();
+    top = s.high;
+    bottom = s.low;
+    exact = true;
+  };
+  if (floor_key == 0) find_extremes();  // nothing was sampled
+  unsigned wanted = kTopK;
+  int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
+  unsigned prefix = 0;  // leading bits found so far
+  unsigned ties = 0xffffffffu;  // distance of the threshold, once the position decides
+  while (true) {
+    for (int i = threadIdx.x; i < listed; i += kThreads) {
+      const uint2 entry = s.list[i];
+      const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
+      const unsigned value = ties == 0xffffffffu ? distance : entry.x;
+      if ((unsigned long long)value >> above == prefix && (ties == 0xffffffffu || distance == ties))
+        atomicAdd(&s.histogram[value >> shift & (kSelectBins - 1)], 1u);
+    }
+    __syncthreads();
+    find_bin(s, wanted);
+    prefix = prefix << (above - shift) | s.bin;
+    if (prefix == 0 && !exact) {
+      find_extremes();
+      above = 32 - __clz(int(top - bottom));
+      shift = max(0, above - 8);
+      continue;
+    }
+    wanted -= s.before;
+    if (s.in_bin <= 32) break;
+    above = shift;
+    if (shift == 0) {  // (positions are distinct: only for the distance)
+      ties = prefix;
+      prefix = 0;
+      above = 32 - __clz(candidates - 1);
+    }
+    shift = max(0, above - 8);
+  }
+  // The threshold bin's entries side by side: the wanted-th smallest of them is the last winner.
+  for (int i = threadIdx.x; i < listed; i += kThreads) {
+    const uint2 entry = s.list[i];
+    const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
+    if (ties == 0xffffffffu ? distance >> shift == prefix : distance == ties && entry.x >> shift == prefix)
+      s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~key << 32 | entry.x;
+  }
+  __syncthreads();
+  if (threadIdx.x < s.few_count) {
+    unsigned before = 0;
+    for (unsigned i = 0; i < s.few_count; ++i) before += s.few[i] < s.few[threadIdx.x];
+    if (before + 1 == wanted) s.limit = s.few[threadIdx.x];
+  }
+  __syncthreads();
+  const unsigned long long limit = s.limit;
+
+  // ---- winners in index order ---------------------------------------------------------------------
+  // A bitmap of winning positions and the number of winners before each of its words: every winner
+  // finds its place in the output by itself.
+  unsigned written = 0;
+  for (int window = 0; window < candidates; window += kSelectWindow) {
+    if (window > 0) {
+      for (int i = threadIdx.x; i < kSelectWindow / 32; i += kThreads) s.bitmap[i] = 0;
       __syncthreads();
     }
-    for (int i = take + threadIdx.x; i < kTopK; i += blockDim.x) list[i] = -1;
+    unsigned winners = 0;  // of this thread's entries (ten at most)
+    static_assert(kCapacity <= 32 * kThreads, "a bit per entry of a thread");
+    for (int i = threadIdx.x, bit = 0; i < listed; i += kThreads, ++bit) {
+      const uint2 entry = s.list[i];
+      const unsigned index = entry.x - window;
+      if (index < kSelectWindow && ((unsigned long long)~score_key(__uint_as_float(entry.y)) << 32 | entry.x) <= limit) {
+        atomicOr(&s.bitmap[index >> 5], 1u << (index & 31));
+        winners |= 1u << bit;
+      }
+    }
+    __syncthreads();
+    const int words = (min(candidates - window, kSelectWindow) + 31) / 32;
+    // Eight words (32 bytes) per thread: threads beyond the words have none.
+    static_assert(kSelectWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
+    const int first = threadIdx.x * 8;
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    if (first < words) a = *reinterpret_cast<const uint4*>(&s.bitmap[first]);
+    if (first + 4 < words) b = *reinterpret_cast<const uint4*>(&s.bitmap[first + 4]);
+    const unsigned counts[8] = {unsigned(__popc(a.x)), unsigned(__popc(a.y)), unsigned(__popc(a.z)), unsigned(__popc(a.w)),
+                                unsigned(__popc(b.x)), unsigned(__popc(b.y)), unsigned(__popc(b.z)), unsigned(__popc(b.w))};
+    unsigned mine = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine += counts[i];
+    const unsigned scan = warp_scan(mine, lane);
+    if (lane == 31) s.warp_sum[warp] = scan;
+    __syncthreads();
+    unsigned at = written + scan - mine;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) at += s.warp_sum[w];
+      written += s.warp_sum[w];
+    }
+    if (first < words) {
+      unsigned packed[4];  // a count is at most 512: two to a word
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        packed[i] = at | (at + counts[2 * i]) << 16;
+        at += counts[2 * i] + counts[2 * i + 1];
+      }
+      *reinterpret_cast<uint4*>(&s.place[first]) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+    __syncthreads();
+    for (; winners != 0; winners &= winners - 1) {
+      const unsigned position = s.list[(__ffs(winners) - 1) * kThreads + threadIdx.x].x, index = position - window;
+      list[s.place[index >> 5] + __popc(s.bitmap[index >> 5] & ((1u << (index & 31)) - 1))] = position;
+    }
+    __syncthreads();  // the bitmap and the sums are free again
   }
 }
 
@@ -211,6 +516,23 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
+template <int kThreads, int kCapacity, int kBlocks>
+int launch_select(const SelectParams& p, cudaStream_t stream) {
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks>;
+  constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity>));
+  // A per-device setting: plain words written with the same value by whoever gets there first.
+  static bool configured[64] = {false};
+  int device = 0;
+  if (cudaError_t error = cudaGetDevice(&device)) return int(error);
+  if (device < 0 || device >= 64) return -1;
+  if (!configured[device]) {
+    if (cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return int(error);
+    configured[device] = true;
+  }
+  kernel<<<p.tokens, kThreads, bytes, stream>>>(p);
+  return int(cudaGetLastError());
+}
+
 }  // namespace
 }  // namespace sparse_mla
 
@@ -233,9 +555,11 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   p.span = SPAN;
   int device = 0, multiprocessors = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
-  const int64_t cap = int64_t(multiprocessors) * 4;
-  topk_select_kernel<<<int(T < cap ? T : cap), kSelectThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  return int(cudaGetLastError());
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Few tokens, or rows whose list of candidates would not fit the small blocks: one large block per
+  // SM and token. Otherwise small blocks, eight to an SM, whose phases overlap.
+  if (T < 2 * multiprocessors || SPAN > 131072) return launch_select<1024, 8192, 1>(p, s);
+  return launch_select<256, 2560, 6>(p, s);
 }
 
 int launch_sparse_mla_cache_append(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,

@@ -131,6 +131,47 @@ def test_gpu_selection_over_long_rows(max_seq, ratio):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tokens,visible", [
+    # 256-thread blocks: TopK, the candidate list (2560), one step of the stream (4096), the sample's
+    # sizes, the window of winners (65536), each with its neighbours
+    (320, (1, 4, 511, 512, 513, 2559, 2560, 2561, 4095, 4097, 16383, 32769, 65535, 65536, 65537, 70001)),
+    # 1024-thread blocks: the list (8192) and one step (16384)
+    (19, (512, 513, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
+])
+def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
+    """One token per request, every row length in turn; continuous, 8-bit-mantissa, offset and
+    clustered scores in turn (what a sample of the row says about it differs)."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    rng = np.random.default_rng(tokens)
+    policy = O.make_policy(tokens, tokens, ratio=1, max_seq=131072, blocks=8)
+    lengths = np.array([visible[i % len(visible)] for i in range(tokens)], dtype=np.int32)
+    data = {
+        "cu_seqlens_q": np.arange(tokens + 1, dtype=np.int32),
+        "seqused_ori_kv": lengths, "seqused_cmp_kv": lengths,
+        "cmp_residual_kv": np.zeros(tokens, dtype=np.int32),
+    }
+    span = -(-max(visible) // 4) * 4
+    scores = rng.normal(size=(tokens, span)).astype(np.float32)
+    for token in range(tokens):
+        kind = (token // len(visible) + token) % 4
+        if kind == 1:
+            scores[token] = (scores[token].view(np.uint32) & 0xFFFF0000).view(np.float32)
+        elif kind == 2:
+            scores[token] += 1000.0
+        elif kind == 3:  # the winners side by side, between the places a sample looks at
+            first = int(rng.integers(0, max(1, lengths[token] - 600)))
+            scores[token, first:first + 600] += 50.0
+    expected = O.select_topk_indices(scores, data, policy)
+    device = {k: torch.from_numpy(v).cuda() for k, v in data.items()}
+    actual = neighbours.topk_indices(torch.from_numpy(scores).cuda(), device["cu_seqlens_q"], device["seqused_cmp_kv"],
+                                     device["cmp_residual_kv"], ratio=1)
+    assert np.array_equal(actual.cpu().numpy(), expected)
+
+
+@pytest.mark.gpu
 def test_gpu_selection_feeds_the_attention_call():
     """Scores -> indices on the device -> attention, against the oracle fed with the oracle's selection."""
     import torch
