@@ -63,6 +63,49 @@ def build_library(force=False, verbose=False):
     return LIBRARY
 
 
+HOST_SOURCE = PACKAGE / "csrc" / "host_calls.cpp"
+HOST_LIBRARY = PACKAGE / "lib" / "_host_calls.so"
+HOST_STAMP = HOST_LIBRARY.with_suffix(".stamp")
+
+
+def _host_command():
+    """How the native host side is compiled: a CPython module against this interpreter's torch."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    flags = ["-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    includes = [f"-I{path}" for path in (*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"])]
+    libraries = [f"-L{path}" for path in cpp_extension.library_paths("cuda")]
+    return [os.environ.get("CXX", "g++"), *flags, *includes, "-o", str(HOST_LIBRARY), str(HOST_SOURCE), *libraries,
+            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lcudart"]
+
+
+def _host_identity():
+    import sys
+
+    import torch
+
+    digest = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    for path in (HOST_SOURCE, ROOT / "include" / "sparse_mla.h"):
+        digest.update(path.read_bytes())
+    return digest.hexdigest()
+
+
+def build_host_library(force=False):
+    """Compile the native host side when its source, the header or torch changed; return its path."""
+    identity = _host_identity()
+    if not force and HOST_LIBRARY.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text() == identity:
+        return HOST_LIBRARY
+    HOST_LIBRARY.parent.mkdir(parents=True, exist_ok=True)
+    result = subprocess.run(_host_command(), capture_output=True, text=True)
+    require(result.returncode == 0, "building the native host side failed:\n" + result.stderr[-4000:], kind=ErrorKind.RESOURCE)
+    HOST_STAMP.write_text(identity)
+    return HOST_LIBRARY
+
+
 def is_current():
     """True when the built library matches the sources and flags it would be built from now."""
     return LIBRARY.exists() and STAMP.exists() and STAMP.read_text() == _identity()

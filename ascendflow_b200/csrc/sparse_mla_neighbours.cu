@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
 // i.e. to row `position % rows_per_page` of page `table[b][position / rows_per_page]`.
 __global__ void cache_append_kernel(const char* new_rows, char* cache, const int32_t* table, const int32_t* cu,
                                     const int32_t* lengths, int batches, int tokens, int pages, int blocks,
-                                    int page_rows, int32_t* status) {
+                                    int page_rows, int32_t* status, volatile int32_t* flag) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; token < tokens; token += warps) {
@@ -506,7 +506,11 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
     const int column = position / page_rows;
     const int page = position >= 0 && column < pages ? __ldg(table + (size_t)lo * pages + column) : -1;
     if (position < 0 || (unsigned)page >= (unsigned)blocks) {  // nowhere to put it: reported, not written
-      if (lane == 0 && atomicCAS(status, kStatusOk, kStatusBadPage) == kStatusOk) { status[1] = token; status[2] = position; }
+      if (lane == 0 && atomicCAS(status, kStatusOk, kStatusBadPage) == kStatusOk) {
+        status[1] = token;
+        status[2] = position;
+        if (flag != nullptr) *flag = 1;
+      }
       continue;
     }
     const uint4* source = reinterpret_cast<const uint4*>(new_rows + (size_t)token * kRowBytes);
@@ -562,21 +566,28 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   return launch_select<256, 2560, 6>(p, s);
 }
 
+int launch_sparse_mla_cache_append_flagged(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,
+                                           void* arg_cu_seqlens_q, void* arg_seqused_kv, void* status_words, void* flag,
+                                           int64_t B, int64_t T, int64_t PAGES, int64_t BLOCKS, int64_t PAGE_ROWS) {
+  if (B <= 0 || T <= 0 || PAGES <= 0 || BLOCKS < 0 || status_words == nullptr) return -1;
+  if (PAGE_ROWS != 64 && PAGE_ROWS != 128) return -1;
+  if (B > INT32_MAX || T > INT32_MAX || PAGES > INT32_MAX || BLOCKS > INT32_MAX / kPage) return -1;
+  const int64_t blocks = (T + 7) / 8;  // eight warps = eight rows per block
+  cache_append_kernel<<<int(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const char*>(arg_new_rows), static_cast<char*>(arg_cache), static_cast<const int32_t*>(arg_block_table),
+      static_cast<const int32_t*>(arg_cu_seqlens_q), static_cast<const int32_t*>(arg_seqused_kv), int(B), int(T), int(PAGES),
+      int(BLOCKS), int(PAGE_ROWS), static_cast<int32_t*>(status_words), static_cast<volatile int32_t*>(flag));
+  return int(cudaGetLastError());
+}
+
 int launch_sparse_mla_cache_append(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,
                                    void* arg_cu_seqlens_q, void* arg_seqused_kv, void* npu_workspace, int64_t B,
                                    int64_t T, int64_t PAGES, int64_t BLOCKS, int64_t PAGE_ROWS) {
-  if (B <= 0 || T <= 0 || PAGES <= 0 || BLOCKS < 0 || npu_workspace == nullptr) return -1;
-  if (PAGE_ROWS != 64 && PAGE_ROWS != 128) return -1;
-  if (B > INT32_MAX || T > INT32_MAX || PAGES > INT32_MAX || BLOCKS > INT32_MAX / kPage) return -1;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int status = int(cudaMemsetAsync(npu_workspace, 0, kWorkspaceBytes, s))) return status;
-  const int64_t blocks = (T + 7) / 8;  // eight warps = eight rows per block
-  cache_append_kernel<<<int(blocks), 256, 0, s>>>(
-      static_cast<const char*>(arg_new_rows), static_cast<char*>(arg_cache), static_cast<const int32_t*>(arg_block_table),
-      static_cast<const int32_t*>(arg_cu_seqlens_q), static_cast<const int32_t*>(arg_seqused_kv), int(B), int(T), int(PAGES),
-      int(BLOCKS), int(PAGE_ROWS),
-      reinterpret_cast<int32_t*>(static_cast<char*>(npu_workspace) + kWorkspaceStatusOffset));
-  return int(cudaGetLastError());
+  if (npu_workspace == nullptr || B <= 0 || T <= 0) return -1;
+  if (int status = int(cudaMemsetAsync(npu_workspace, 0, kWorkspaceBytes, static_cast<cudaStream_t>(stream)))) return status;
+  return launch_sparse_mla_cache_append_flagged(stream, arg_new_rows, arg_cache, arg_block_table, arg_cu_seqlens_q, arg_seqused_kv,
+                                                static_cast<char*>(npu_workspace) + kWorkspaceStatusOffset, nullptr, B, T, PAGES,
+                                                BLOCKS, PAGE_ROWS);
 }
 
 }  // extern "C"

@@ -13,6 +13,7 @@ import ctypes as ct
 
 import torch
 
+from . import host
 from .build import library_path
 from .diagnostics import require
 from .runtime.torch import _library
@@ -43,6 +44,10 @@ def _raise_on(status):
 
 def topk_indices(scores, cu_seqlens_q, seqused_cmp_kv, cmp_residual_kv, *, ratio=2, out=None):
     """`cmp_sparse_indices` `[T, 1, 512]` int32 from index scores `[T, SPAN]` float32."""
+    selected = host.calls.topk_indices(scores, cu_seqlens_q, seqused_cmp_kv, cmp_residual_kv, ratio, out)
+    if selected is not None:
+        return selected
+    # refused by the native side, or the first call: the checks below say why
     _check(scores, torch.float32, "scores")
     for name, tensor in (("cu_seqlens_q", cu_seqlens_q), ("seqused_cmp_kv", seqused_cmp_kv),
                          ("cmp_residual_kv", cmp_residual_kv)):
@@ -56,6 +61,7 @@ def topk_indices(scores, cu_seqlens_q, seqused_cmp_kv, cmp_residual_kv, *, ratio
     _check(out, torch.int32, "cmp_sparse_indices")
     require(tuple(out.shape) == (tokens, 1, 512), "cmp_sparse_indices must be [T, 1, 512]")
     launch = _entry("launch_sparse_mla_topk_indices", 6, 4)
+    host.connect()
     stream = torch.cuda.current_stream(scores.device).cuda_stream
     _raise_on(launch(stream, scores.data_ptr(), cu_seqlens_q.data_ptr(), seqused_cmp_kv.data_ptr(),
                      cmp_residual_kv.data_ptr(), out.data_ptr(), batches, tokens, span, 128 // ratio))
@@ -68,6 +74,10 @@ def cache_append(new_rows, cache, block_table, cu_seqlens_q, seqused_kv):
     `seqused_kv` counts the new rows, as it does for the attention call that follows. Returns the
     status block (word 0: 0 ok, 1 a row had no legal page), which synchronises the stream.
     """
+    status = host.calls.cache_append(new_rows, cache, block_table, cu_seqlens_q, seqused_kv)
+    if status is not None:
+        return status
+    # refused by the native side, or the first call: the checks below say why
     require(new_rows.is_cuda and cache.is_cuda and new_rows.dtype == cache.dtype
             and new_rows.dtype in (torch.bfloat16, torch.float16), "rows and cache must be 16-bit CUDA tensors of one dtype")
     require(new_rows.is_contiguous() and cache.is_contiguous(), "rows and cache must be contiguous")
@@ -78,6 +88,7 @@ def cache_append(new_rows, cache, block_table, cu_seqlens_q, seqused_kv):
     library = _library(library_path()) if "library" not in _entry_points else _entry_points["library"]
     _entry_points["library"] = library
     launch = _entry("launch_sparse_mla_cache_append", 7, 5)
+    host.connect()
     workspace = torch.empty(1024, dtype=torch.uint8, device=cache.device)
     stream = torch.cuda.current_stream(cache.device).cuda_stream
     _raise_on(launch(stream, new_rows.data_ptr(), cache.data_ptr(), block_table.data_ptr(), cu_seqlens_q.data_ptr(),

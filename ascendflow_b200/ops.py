@@ -6,12 +6,17 @@ same names, layouts and dtypes, the output passed explicitly
 (`docs/guide/runtime.md:88-89` of the reference). It launches on torch's current
 CUDA stream through the C ABI. There is no CPU or eager fallback: a missing
 library or a non-CUDA tensor raises.
+
+A call normally stays in native code (`host.py`): checks, status block and launch in about three
+microseconds. What that refuses, and the first call of a process, goes through the Python front end
+(`runtime/`), which words the errors.
 """
 
 from __future__ import annotations
 
 import torch
 
+from . import host
 from .runtime.torch import TorchRuntime
 
 TENSORS = (
@@ -29,6 +34,7 @@ def runtime():
     if _runtime is None or _runtime._closed:
         _runtime = TorchRuntime(torch)
         _kernels.clear()
+        host.calls.release_workspaces()
     return _runtime
 
 
@@ -39,28 +45,30 @@ def kernel(name="sparse_mla"):
     return _kernels[name]
 
 
+def _checked(*tensors):
+    """The call through the Python front end."""
+    host.connect()
+    kernel("sparse_mla_f16" if tensors[0].dtype == torch.float16 else "sparse_mla")(*tensors)
+
+
 def sparse_mla(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block_table,
                cu_seqlens_q, seqused_ori_kv, seqused_cmp_kv, cmp_residual_kv, ori_topk_length,
                sinks, attention_out):
     """Run sparse MLA attention into `attention_out` on the current stream; returns it."""
-    name = "sparse_mla_f16" if q.dtype == torch.float16 else "sparse_mla"
-    kernel(name)(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block_table,
+    if not _launch(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block_table,
+                   cu_seqlens_q, seqused_ori_kv, seqused_cmp_kv, cmp_residual_kv, ori_topk_length,
+                   sinks, attention_out):
+        _checked(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block_table,
                  cu_seqlens_q, seqused_ori_kv, seqused_cmp_kv, cmp_residual_kv, ori_topk_length,
                  sinks, attention_out)
     return attention_out
 
 
-@torch.library.custom_op("ascendflow_b200::sparse_mla", mutates_args=("attention_out",),
-                         device_types="cuda")
-def _sparse_mla_op(q: torch.Tensor, ori_kv: torch.Tensor, cmp_kv: torch.Tensor,
-                   cmp_sparse_indices: torch.Tensor, ori_block_table: torch.Tensor,
-                   cmp_block_table: torch.Tensor, cu_seqlens_q: torch.Tensor,
-                   seqused_ori_kv: torch.Tensor, seqused_cmp_kv: torch.Tensor,
-                   cmp_residual_kv: torch.Tensor, ori_topk_length: torch.Tensor,
-                   sinks: torch.Tensor, attention_out: torch.Tensor) -> None:
-    sparse_mla(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block_table,
-               cu_seqlens_q, seqused_ori_kv, seqused_cmp_kv, cmp_residual_kv, ori_topk_length,
-               sinks, attention_out)
+# `torch.ops.ascendflow_b200.sparse_mla` is registered by the native module when it is loaded: no
+# result, `attention_out` mutated, CUDA only, no gradient. Tracing needs nothing computed.
+_launch = host.calls.sparse_mla
+host.set_fallback(_checked)
+torch.library.register_fake("ascendflow_b200::sparse_mla", lambda *tensors: None)
 
 
 def resolve_rows(cmp_sparse_indices, ori_block_table, cmp_block_table, cu_seqlens_q,

@@ -214,6 +214,15 @@ int launch_sparse_mla_cache_append(void* stream, void* arg_new_rows, void* arg_c
                                    void* npu_workspace, int64_t B, int64_t T, int64_t PAGES,
                                    int64_t BLOCKS, int64_t PAGE_ROWS);
 
+/* The same without the memset in front: `status_words` (device, SPARSE_MLA_STATUS_WORDS int32) must be
+ * zero on entry and stays zero unless a row has no legal page; the kernel then also stores 1 to
+ * `flag` (device address of mapped host memory, or NULL), so that a caller who waits for the stream
+ * anyway sees on the host whether there is a status to fetch. */
+int launch_sparse_mla_cache_append_flagged(void* stream, void* arg_new_rows, void* arg_cache,
+                                           void* arg_block_table, void* arg_cu_seqlens_q, void* arg_seqused_kv,
+                                           void* status_words, void* flag, int64_t B, int64_t T, int64_t PAGES,
+                                           int64_t BLOCKS, int64_t PAGE_ROWS);
+
 /* Self-test of the bounded on-chip wait (no counterpart in the reference, whose synchronisation
  * is proven at compile time): one warp waits on a barrier nobody signals; after `limit_cycles`
  * SM clocks (<= 2^31) it gives up, writes SPARSE_MLA_STATUS_WAIT_EXPIRED to the status block of

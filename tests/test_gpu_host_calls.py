@@ -1,0 +1,100 @@
+"""The native host side against the Python front end: same results for what it accepts, the front end's
+errors for what it does not, on streams and threads."""
+
+import numpy as np
+import pytest
+
+from oracle import sparse_mla_oracle as O
+from tests import support as S
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def call():
+    policy = O.make_policy(4, 16, max_seq=4096, blocks=128)
+    return S.to_device(O.validation_inputs(policy, "mixed"), policy)[0]
+
+
+def arguments(tensors, **changed):
+    return [changed.get(name, tensors[name]) for name in S.TENSOR_ORDER]
+
+
+@pytest.mark.parametrize("entry", ["function", "op"])
+@pytest.mark.parametrize("name,change,message", [
+    ("q", lambda t: t.float(), "dtype differs"),
+    ("sinks", lambda t: t[:32], "shape differs"),
+    ("cmp_kv", lambda t: t[:, :32].contiguous(), "contract differs"),
+    ("cu_seqlens_q", lambda t: t.cpu(), "CUDA tensor"),
+    ("ori_topk_length", lambda t: t.view(-1), "rank differs"),
+    ("attention_out", None, "disjoint"),
+    ("cmp_sparse_indices", lambda t: t.repeat(1, 1, 2)[:, :, ::2], "contiguous"),
+])
+def test_refused_arguments_raise_the_front_ends_error(call, entry, name, change, message):
+    import torch
+
+    from ascendflow_b200 import ops
+    from ascendflow_b200.diagnostics import CompileError
+
+    ops.sparse_mla(*arguments(call))  # the entry points are connected
+    wrong = arguments(call, **{name: call["q"] if change is None else change(call[name])})
+    with pytest.raises(CompileError, match=message):
+        (ops.sparse_mla if entry == "function" else torch.ops.ascendflow_b200.sparse_mla)(*wrong)
+
+
+def test_streams_and_threads_get_the_same_output(call):
+    import threading
+
+    import torch
+
+    from ascendflow_b200 import ops
+
+    binding = ops.kernel().bind(*arguments(call))
+    binding()
+    torch.cuda.synchronize()
+    expected = call["attention_out"].clone()
+    outputs = {}
+
+    def work(key):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            mine = torch.empty_like(call["attention_out"])
+            for _ in range(20):
+                torch.ops.ascendflow_b200.sparse_mla(*arguments(call, attention_out=mine))
+        stream.synchronize()
+        outputs[key] = mine
+
+    threads = [threading.Thread(target=work, args=(key,)) for key in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert all(torch.equal(outputs[key], expected) for key in range(4))
+
+
+def test_op_counts_as_a_mutation_and_has_no_gradient(call):
+    import torch
+
+    out = torch.empty_like(call["attention_out"])
+    version = out._version
+    torch.ops.ascendflow_b200.sparse_mla(*arguments(call, attention_out=out))
+    assert out._version == version + 1
+    q = call["q"].clone().requires_grad_()
+    torch.ops.ascendflow_b200.sparse_mla(*arguments(call, q=q, attention_out=out))
+    with pytest.raises(RuntimeError):
+        out.sum().backward()
+
+
+def test_append_reports_a_bad_page_once_and_is_clean_afterwards():
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    cache = torch.zeros((4, 128, 1, 512), dtype=torch.bfloat16, device="cuda")
+    rows = torch.ones((3, 512), dtype=torch.bfloat16, device="cuda")
+    cu = torch.tensor([0, 3], dtype=torch.int32, device="cuda")
+    table = torch.tensor([[0, 1, 2, 3]], dtype=torch.int32, device="cuda")
+    for length, code in ((3, 0), (514, 1), (512, 0)):
+        status = neighbours.cache_append(rows, cache, table, cu, torch.tensor([length], dtype=torch.int32, device="cuda"))
+        assert status[0] == code and len(status) == 8
+        if code:
+            assert status[1:3] in ((1, 512), (2, 513))
+    assert np.array_equal(cache.view(512, 512)[:, 0].float().cpu().numpy().nonzero()[0], [0, 1, 2, 509, 510, 511])
