@@ -12,6 +12,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
+#include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -35,12 +36,12 @@ constexpr int kTensors = SPARSE_MLA_TENSORS;
 using Tensors = std::array<const at::Tensor*, kTensors>;
 enum Argument { kQ, kOriKv, kCmpKv, kIndices, kOriTable, kCmpTable, kCu, kSeqOri, kSeqCmp, kResidual, kTopkLength, kSinks, kOut };
 
-using LaunchAttention = decltype(&launch_sparse_mla);
+using LaunchAttention = decltype(&launch_sparse_mla_kept_status);
 using LaunchSelect = decltype(&launch_sparse_mla_topk_indices);
 using LaunchAppend = decltype(&launch_sparse_mla_cache_append_flagged);
 
 // Entry points of the kernel library (loaded, and its hash verified, by the Python side).
-LaunchAttention launch_bf16 = nullptr, launch_f16 = nullptr;
+LaunchAttention launch_attention = nullptr;
 LaunchSelect launch_select = nullptr;
 LaunchAppend launch_append = nullptr;
 PyObject* checked_attention = nullptr;  // the Python front end's call, for arguments refused here
@@ -96,7 +97,7 @@ bool accepted(const Tensors& t, int device, Sizes* s) {
   return true;
 }
 
-// One status block per device and stream, kept. At most kMostWorkspaces of them: a program that makes
+// One status block per device and stream, kept (and zero: no call clears it). At most kMostWorkspaces of them: a program that makes
 // streams without end gets the oldest one's memory back for the newest (the allocator holds freed
 // memory until its stream is done with it).
 constexpr size_t kWorkspaceBytes = 1024, kMostWorkspaces = 64;
@@ -113,7 +114,7 @@ at::Tensor workspace_for(const c10::cuda::CUDAStream& stream) {
   std::lock_guard<std::mutex> lock(workspace_mutex);
   for (const Workspace& w : *workspaces)
     if (w.device == stream.device_index() && w.stream == stream.stream()) return w.memory;
-  at::Tensor memory = at::empty({int64_t(kWorkspaceBytes)}, at::TensorOptions(at::kByte).device(at::kCUDA, stream.device_index()));
+  at::Tensor memory = at::zeros({int64_t(kWorkspaceBytes)}, at::TensorOptions(at::kByte).device(at::kCUDA, stream.device_index()));
   c10::cuda::CUDACachingAllocator::recordStream(memory.storage().data_ptr(), stream);
   if (workspaces->size() >= kMostWorkspaces) workspaces->erase(workspaces->begin());
   workspaces->push_back({stream.device_index(), stream.stream(), memory});
@@ -123,7 +124,7 @@ at::Tensor workspace_for(const c10::cuda::CUDAStream& stream) {
 // Launches an accepted call on the current stream. -1000: not accepted, nothing enqueued.
 constexpr int kRefused = -1000;
 int attention(const Tensors& t) {
-  if (launch_bf16 == nullptr) return kRefused;
+  if (launch_attention == nullptr) return kRefused;
   const c10::DeviceIndex device = c10::cuda::current_device();
   Sizes s;
   if (!accepted(t, device, &s)) return kRefused;
@@ -134,9 +135,8 @@ int attention(const Tensors& t) {
   void* p[kTensors];
   for (int i = 0; i < kTensors; ++i) p[i] = const_cast<void*>(t[i]->const_data_ptr());
   const at::Tensor workspace = workspace_for(stream);
-  const LaunchAttention launch = t[kQ]->scalar_type() == at::kHalf ? launch_f16 : launch_bf16;
-  return launch(stream.stream(), p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], p[11], p[12],
-                workspace.mutable_data_ptr(), s.batches, s.tokens, s.pages, s.ori_blocks, s.cmp_blocks, s.cmp_page);
+  return launch_attention(stream.stream(), t[kQ]->scalar_type() == at::kHalf, p, workspace.mutable_data_ptr(), s.batches, s.tokens,
+                          s.pages, s.ori_blocks, s.cmp_blocks, s.cmp_page);
 }
 
 // ---- the registered op -----------------------------------------------------------------------------
@@ -341,14 +341,12 @@ PyObject* call_append(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
   END_HANDLE_TH_ERRORS
 }
 
-// (launch_sparse_mla, launch_sparse_mla_f16, ..._topk_indices, ..._cache_append_flagged: addresses; the
-// front end's call)
+// (launch_sparse_mla_kept_status, ..._topk_indices, ..._cache_append_flagged: addresses; the front end's call)
 PyObject* configure(PyObject*, PyObject* arguments) {
-  unsigned long long bf16, f16, select, append;
+  unsigned long long attention, select, append;
   PyObject* fallback;
-  if (!PyArg_ParseTuple(arguments, "KKKKO", &bf16, &f16, &select, &append, &fallback)) return nullptr;
-  launch_bf16 = reinterpret_cast<LaunchAttention>(bf16);
-  launch_f16 = reinterpret_cast<LaunchAttention>(f16);
+  if (!PyArg_ParseTuple(arguments, "KKKO", &attention, &select, &append, &fallback)) return nullptr;
+  launch_attention = reinterpret_cast<LaunchAttention>(attention);
   launch_select = reinterpret_cast<LaunchSelect>(select);
   launch_append = reinterpret_cast<LaunchAppend>(append);
   Py_XSETREF(checked_attention, Py_NewRef(fallback));

@@ -234,6 +234,16 @@ int launch_sparse_mla_f16(void* stream, void* arg_q, void* arg_ori_kv, void* arg
   return umma::launch<0>(p, s, multiprocessors());
 }
 
+int launch_sparse_mla_kept_status(void* stream, int64_t f16, void* const* tensors, void* npu_workspace, int64_t B,
+                                  int64_t T, int64_t PAGES, int64_t ORI_BLOCKS, int64_t CMP_BLOCKS, int64_t CMP_PAGE) {
+  Params p;
+  if (!fill(p, tensors[0], tensors[1], tensors[2], tensors[3], tensors[4], tensors[5], tensors[6], tensors[7], tensors[8],
+            tensors[9], tensors[10], tensors[11], tensors[12], npu_workspace, B, T, PAGES, ORI_BLOCKS, CMP_BLOCKS, CMP_PAGE))
+    return -1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return f16 != 0 ? umma::launch<0>(p, s, multiprocessors()) : umma::launch<1>(p, s, multiprocessors());
+}
+
 // The portable-instruction BF16 kernel under its own name: the cross-check of the tcgen05 kernel.
 int launch_sparse_mla_warp_mma(void* stream, void* arg_q, void* arg_ori_kv, void* arg_cmp_kv,
                                void* arg_cmp_sparse_indices, void* arg_ori_block_table,

@@ -12,6 +12,7 @@
 
 #include "../../include/sparse_mla.h"
 #include "sparse_mla_common.cuh"
+#include "tcgen05_ptx.cuh"
 
 namespace sparse_mla {
 namespace {
@@ -242,6 +243,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   Shared& s = *reinterpret_cast<Shared*>(select_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int token = blockIdx.x;
+  sm100::wait_for_predecessor();
+  sm100::let_successor_start();
   const int candidates = int(min((int64_t)visible_compressed_rows(p, token, lane), p.span));
   int32_t* list = p.out + (size_t)token * kTopK;
   const float* row = p.scores + (size_t)token * p.span;
@@ -533,8 +536,7 @@ int launch_select(const SelectParams& p, cudaStream_t stream) {
     if (cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return int(error);
     configured[device] = true;
   }
-  kernel<<<p.tokens, kThreads, bytes, stream>>>(p);
-  return int(cudaGetLastError());
+  return int(sm100::launch_overlapped(kernel, p.tokens, kThreads, bytes, stream, p));
 }
 
 }  // namespace

@@ -92,8 +92,8 @@ constexpr uint32_t kHalfLanes = 16u << 16;                   // lane offset of t
 struct TokenInfo {
   int token;
   int chunks;                 // live chunks of this token
+  uint2 live[kMaxChunks];     // per live chunk, in order: live bits of its rows 0-31 and 32-63
   unsigned char chunk[kMaxChunks];
-  unsigned live[kSlots / 32]; // bit l of word i: slot 32 i + l is live
 };
 static_assert(sizeof(TokenInfo) <= 128, "the info area holds two 128-byte entries");
 
@@ -146,23 +146,20 @@ struct Shared {
 // share most of their window rows in L2 while different blocks read different windows at any one
 // time. Every role of a block walks the same sequence.
 struct TokenWalk {
-  int block, grid, group, tokens, k;
+  unsigned start, within, group, stride, tokens;  // start < tokens + stride < 2^32
   __device__ __forceinline__ explicit TokenWalk(const Params& p)
-      : block(blockIdx.x), grid(gridDim.x), group(p.token_group), tokens(p.tokens), k(0) {}
+      : start(blockIdx.x * p.token_group), within(0), group(p.token_group), stride(gridDim.x * p.token_group), tokens(p.tokens) {}
   __device__ __forceinline__ int next() {  // next token of this block, or -1 when done
-    while (true) {
-      const int round = k / group;
-      if ((long long)round * grid * group >= tokens) return -1;
-      const long long token = ((long long)round * grid + block) * group + k % group;
-      ++k;
-      if (token < tokens) return int(token);
-    }
+    if (within == group) { start += stride; within = 0; }
+    const unsigned token = start + within;
+    if (token >= tokens) return -1;  // (and so is every later one)
+    ++within;
+    return int(token);
   }
   __device__ __forceinline__ int peek() const { TokenWalk copy = *this; return copy.next(); }
   __device__ __forceinline__ int count() const {  // how many tokens next() hands out in all
-    const int per_round = grid * group;  // at most the SM count times eight
-    const int rounds = tokens / per_round, rest = tokens - rounds * per_round - block * group;
-    return rounds * group + (rest < 0 ? 0 : (rest > group ? group : rest));
+    const unsigned rounds = tokens / stride, rest = tokens - rounds * stride, mine = blockIdx.x * group;
+    return int(rounds * group + (rest <= mine ? 0 : min(rest - mine, group)));
   }
 };
 
@@ -184,26 +181,31 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 
-// Warp-cooperative form of `token_geometry`: the request search probes 32 positions of
-// cu_seqlens_q per step instead of one, and every other per-token scalar is loaded before the
-// search so that the loads overlap (a cold block starts with this chain on its critical path).
+// Warp-cooperative form of `token_geometry`. A cold block starts with this chain of dependent
+// loads on its critical path (700 cycles and more each), so the request search probes 32 positions
+// of cu_seqlens_q per step, and in its last step (the only one for up to 32 requests) every lane
+// loads all scalars of its candidate along with the probe.
 __device__ __forceinline__ TokenGeometry token_geometry_warp(const Params& p, int token, int lane) {
   const int requested = __ldg(p.topk_len + token);
   int lo = 0, hi = p.batches;  // invariant: cu[lo] <= token < cu[hi]
-  while (hi - lo > 1) {
+  while (hi - lo > 32) {
     const int step = (hi - lo + 31) >> 5;
     const int probe = lo + lane * step;
     const bool below = probe < hi && __ldg(p.cu + probe) <= token;
     const unsigned mask = __ballot_sync(0xffffffffu, below);  // lane 0 probes cu[lo]: always set
-    const int last = 31 - __clz(mask);
-    lo += last * step;
+    lo += (31 - __clz(mask)) * step;
     hi = min(hi, lo + step);
   }
-  TokenGeometry g;
-  g.batch = lo;
-  const int begin = __ldg(p.cu + lo), end = __ldg(p.cu + lo + 1);
-  const int length = __ldg(p.seq_ori + lo), available = __ldg(p.seq_cmp + lo), residual = __ldg(p.residual + lo);
+  const int mine = min(lo + lane, hi - 1);
+  const int my_begin = __ldg(p.cu + mine), my_end = __ldg(p.cu + mine + 1);
+  const int my_length = __ldg(p.seq_ori + mine), my_available = __ldg(p.seq_cmp + mine), my_residual = __ldg(p.residual + mine);
+  const int found = 31 - __clz(__ballot_sync(0xffffffffu, lo + lane < hi && my_begin <= token));
+  const int begin = __shfl_sync(0xffffffffu, my_begin, found), end = __shfl_sync(0xffffffffu, my_end, found);
+  const int length = __shfl_sync(0xffffffffu, my_length, found), available = __shfl_sync(0xffffffffu, my_available, found);
+  const int residual = __shfl_sync(0xffffffffu, my_residual, found);
   const int count = end - begin, offset = token - begin;
+  TokenGeometry g;
+  g.batch = lo + found;
   g.right = max(0, length - count + offset + 1);
   g.visible = min(kWindow, g.right);
   if (requested > 0) g.visible = min(g.visible, requested);
@@ -218,55 +220,48 @@ __device__ __forceinline__ TokenGeometry token_geometry_warp(const Params& p, in
 // position right - visible + s of the raw cache; compressed rank r is kept when r < min(TOPK,
 // C, cutoff), no entry before it is negative and its index is below the cutoff; a kept entry
 // goes through the request's block table. Lane l returns slots 32 i + l in resolved[i] (the
-// physical cache row, or -1). This one routine serves the attention kernel (its resolver warp)
-// and the index-set export (`resolve_rows_kernel`), so that the exported set is the gathered set.
-__device__ __forceinline__ void resolve_token_warp(const Params& p, int token, int lane,
-                                                   int (&resolved)[kSlots / 32]) {
+// physical cache row, or -1): neighbouring slots of a sorted list have neighbouring pages, so that a
+// load of the table touches few sectors. This one routine serves the attention kernel (its resolver
+// warp) and the index-set export (`resolve_rows_kernel`), so that the exported set is the gathered set.
+__device__ __forceinline__ void resolve_token_warp(const Params& p, int token, int lane, int (&resolved)[kSlots / 32]) {
+  constexpr int kWindowSteps = kWindow / 32, kListSteps = kTopK / 32;
   // The index list does not depend on the geometry: its loads go out first.
-  const int32_t* list = p.indices + (size_t)token * kTopK;
-  int index[kTopK / 32];
+  const int32_t* list = p.indices + (size_t)token * kTopK + lane;
+  int index[kListSteps];
 #pragma unroll
-  for (int i = 0; i < kTopK / 32; ++i) index[i] = __ldg(list + i * 32 + lane);
+  for (int i = 0; i < kListSteps; ++i) index[i] = __ldg(list + i * 32);
   const TokenGeometry g = token_geometry_warp(p, token, lane);
   int first = kTopK;
 #pragma unroll
-  for (int i = 0; i < kTopK / 32; ++i)
-    if (index[i] < 0 && first == kTopK) first = i * 32 + lane;
+  for (int i = kListSteps - 1; i >= 0; --i)
+    if (index[i] < 0) first = i * 32 + lane;
   const int first_negative = __reduce_min_sync(0xffffffffu, first);
-  const int cmp_shift = p.cmp_page == 64 ? 6 : 7;
-  // Three passes so that all block-table loads are in flight together (a branch or vote between
-  // them would serialise twenty dependent round trips to memory): columns, loads, rows.
-  int column[kSlots / 32], within[kSlots / 32];
-#pragma unroll
-  for (int i = 0; i < kWindow / 32; ++i) {
-    const int slot = i * 32 + lane;
-    const int position = g.right - g.visible + slot;
-    const bool live = slot < g.visible;
-    column[i] = live ? position / kPage : -1;
-    within[i] = position % kPage;
-  }
-#pragma unroll
-  for (int i = 0; i < kTopK / 32; ++i) {
-    const int rank = i * 32 + lane;
-    const bool live = rank < g.bound && rank < first_negative && index[i] < g.cutoff;
-    // cmp_page is 64 or 128: shift and mask instead of a run-time division
-    column[kWindow / 32 + i] = live ? index[i] >> cmp_shift : -1;
-    within[kWindow / 32 + i] = index[i] & (p.cmp_page - 1);
-  }
+  const int cmp_shift = p.cmp_page == 64 ? 6 : 7;  // cmp_page is 64 or 128: shift and mask instead of a run-time division
+  // Two passes so that all block-table loads are in flight together (a branch or vote between
+  // them would serialise twenty dependent round trips to memory): columns and loads, rows.
+  const int first_position = g.right - g.visible + lane;
+  const int rank_end = min(g.bound, first_negative);
+  const int32_t* ori_table = p.ori_table + (size_t)g.batch * p.pages;
+  const int32_t* cmp_table = p.cmp_table + (size_t)g.batch * p.pages;
+  int column[kSlots / 32];  // -1: not live
 #pragma unroll
   for (int i = 0; i < kSlots / 32; ++i) {
-    const int32_t* table = (i < kWindow / 32 ? p.ori_table : p.cmp_table) + (size_t)g.batch * p.pages;
-    resolved[i] = __ldg(table + min(max(column[i], 0), p.pages - 1));  // the page, for now
+    const bool window = i < kWindowSteps;
+    const int slot = i * 32 + lane, rank = slot - kWindow, entry = index[window ? 0 : i - kWindowSteps];
+    const bool live = window ? slot < g.visible : rank < rank_end && entry < g.cutoff;
+    column[i] = !live ? -1 : window ? (first_position + i * 32) / kPage : entry >> cmp_shift;
+    resolved[i] = __ldg((window ? ori_table : cmp_table) + min(unsigned(column[i]), unsigned(p.pages - 1)));  // the page, for now
   }
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < kSlots / 32; ++i) {
-    const bool window = i < kWindow / 32;
+    const bool window = i < kWindowSteps;
     const int blocks = window ? p.ori_blocks : p.cmp_blocks, page_rows = window ? kPage : p.cmp_page;
+    const int within = window ? (first_position + i * 32) % kPage : index[window ? 0 : i - kWindowSteps] & (p.cmp_page - 1);
     const bool live = column[i] >= 0;
     const bool legal = column[i] < p.pages && (unsigned)resolved[i] < (unsigned)blocks;
     bad |= live && !legal;
-    resolved[i] = live && legal ? resolved[i] * page_rows + within[i] : -1;
+    resolved[i] = live && legal ? resolved[i] * page_rows + within : -1;
   }
   if (bad) report(p, kStatusBadPage, token, lane);
 }
@@ -307,20 +302,24 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
          !warp_wait(sm.bar(kInfoRead0 + buffer), ((token_count >> 1) & 1) ^ 1, abort_flag))) return;
     int resolved[kSlots / 32];
     resolve_token_warp(p, token, lane, resolved);
-    int live_chunks = 0;  // bit c set: chunk c holds a live slot (same in all lanes)
+    unsigned live_chunks = 0;  // bit c set: chunk c holds a live slot (same in all lanes)
+    unsigned mine = 0;         // lane l: live bits of slots 32 l ..
 #pragma unroll
     for (int i = 0; i < kSlots / 32; ++i) {
       rows[i * 32 + lane] = resolved[i];
       const unsigned live = __ballot_sync(0xffffffffu, resolved[i] >= 0);
-      if (live != 0) live_chunks |= 1 << (i * 32 / kChunkRows);
-      if (lane == 0) info->live[i] = live;
+      if (live != 0) live_chunks |= 1u << (i * 32 / kChunkRows);
+      if (lane == i) mine = live;
+    }
+    const int chunk = lane >> 1;     // two lanes per chunk (no bit beyond kMaxChunks - 1 is set)
+    if (live_chunks >> chunk & 1) {
+      const int item = __popc(live_chunks & ((1u << chunk) - 1));
+      reinterpret_cast<unsigned*>(&info->live[item])[lane & 1] = mine;
+      info->chunk[item] = (unsigned char)chunk;
     }
     if (lane == 0) {
-      int count = 0;
-      for (int chunk = 0; chunk < kMaxChunks; ++chunk)
-        if (live_chunks >> chunk & 1) info->chunk[count++] = (unsigned char)chunk;
       info->token = token;
-      info->chunks = count;
+      info->chunks = __popc(live_chunks);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(sm.bar(kTokenReady0 + buffer));
@@ -711,8 +710,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
     // sink's own weight exp2(sink - run_max) = 1.
     float run_max = sink, run_sum = half ? 0.f : 1.f;
     for (int i = 0; i < chunks; ++i, ++chunk_count) {
-      const int chunk = info->chunk[i];
-      const unsigned live_lo = info->live[2 * chunk], live_hi = info->live[2 * chunk + 1];
+      const unsigned live_lo = info->live[i].x, live_hi = info->live[i].y;
 
       if (!warp_wait(sm.bar(kSFull), chunk_count & 1, abort_flag)) return;
       tc_fence_after_sync();
@@ -845,6 +843,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  // Up to here nothing has touched global memory: a block's start, and the launch itself, overlap
+  // the end of the kernel before.
+  wait_for_predecessor();
+  let_successor_start();
 
   if (warp < kSoftmaxWarps) {
     softmax_role<kFormat>(p, sm, tmem);
@@ -883,8 +885,7 @@ inline int launch(const Params& p, cudaStream_t stream, int multiprocessors) {
   Params launch_params = p;
   const int per_block = p.tokens / (grid * 4);
   launch_params.token_group = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
-  attention_kernel<kFormat><<<grid, kThreads, kSmemBytes, stream>>>(launch_params);
-  return int(cudaGetLastError());
+  return int(launch_overlapped(attention_kernel<kFormat>, grid, kThreads, kSmemBytes, stream, launch_params));
 }
 
 }  // namespace umma

@@ -12,6 +12,32 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ---- programmatic dependent launch -------------------------------------------------------------
+
+// A kernel launched with programmatic stream serialisation may start while the kernel before it in
+// the stream is still running. Nothing that kernel writes (or reads, if this one overwrites it) is
+// touched before `wait_for_predecessor`: it returns when that kernel has completed and its memory
+// is visible.
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// The kernel behind this one may be started (it waits by itself for this one's completion).
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+// Launch `kernel` with one argument so that its start overlaps its predecessor's end.
+template <typename Kernel, typename Argument>
+inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_t shared_bytes, cudaStream_t stream, const Argument& argument) {
+  cudaLaunchAttribute overlap = {};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(grid));
+  config.blockDim = dim3(unsigned(threads));
+  config.dynamicSmemBytes = shared_bytes;
+  config.stream = stream;
+  config.attrs = &overlap;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, argument);
+}
+
 // ---- mbarrier -----------------------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

@@ -35,7 +35,7 @@ def set_fallback(function):
     """The front end's call for what the registered op refuses."""
     global _fallback
     _fallback = function
-    calls.configure(0, 0, 0, 0, function)
+    calls.configure(0, 0, 0, function)
 
 
 def connect():
@@ -48,7 +48,6 @@ def connect():
 
     library = _library(library_path())
     addresses = (ct.cast(getattr(library, name), ct.c_void_p).value for name in (
-        "launch_sparse_mla", "launch_sparse_mla_f16", "launch_sparse_mla_topk_indices",
-        "launch_sparse_mla_cache_append_flagged"))
+        "launch_sparse_mla_kept_status", "launch_sparse_mla_topk_indices", "launch_sparse_mla_cache_append_flagged"))
     calls.configure(*addresses, _fallback)
     _connected = True

@@ -114,6 +114,14 @@ int launch_sparse_mla_f16(void* stream, void* arg_q, void* arg_ori_kv, void* arg
                           void* arg_attention_out, void* npu_workspace, int64_t B, int64_t T,
                           int64_t PAGES, int64_t ORI_BLOCKS, int64_t CMP_BLOCKS, int64_t CMP_PAGE);
 
+/* ---- The same two launches for a caller that keeps its workspace: `npu_workspace` is zero before its
+ * first use and is not cleared in front of the launch (a memset costs a small call a fifth of its
+ * time), so that its status block holds the first report of all calls made with it. `f16`: 0 for
+ * bfloat16, 1 for IEEE half; `tensors` (host): the 13 device pointers in signature order. */
+int launch_sparse_mla_kept_status(void* stream, int64_t f16, void* const* tensors, void* npu_workspace,
+                                  int64_t B, int64_t T, int64_t PAGES, int64_t ORI_BLOCKS,
+                                  int64_t CMP_BLOCKS, int64_t CMP_PAGE);
+
 /* ---- BF16 cross-check kernel: the same operator on the warp-level tensor instructions
  * (ldmatrix + mma.sync) instead of tcgen05. Same arguments and contract as launch_sparse_mla.
  * It has no counterpart in the reference; tests compare the two implementations on full-size
