@@ -795,15 +795,18 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         partial_max[k] = fmaxf(partial_max[k], raw[4 * k + 3].y);
       }
       const float own_max = fmaxf(fmaxf(partial_max[0], partial_max[1]), fmaxf(partial_max[2], partial_max[3])) * p.scale_log2;  // scale > 0
-      // The running maximum only moves when it is exceeded by more than 8 (a factor 256), so the
-      // accumulator is rescaled rarely; probabilities stay below 2^8 and all terms of one head
-      // share the same reference, which cancels in the final division. So the two lanes of a head
+      // The running maximum is that of the sink and the first chunk (moving it costs nothing while
+      // O is empty; with the sink alone a tenth of all chunks moved some head's) and from then on
+      // only moves when it is exceeded by more than 8 (a factor 256), so the accumulator is rescaled
+      // rarely (1500 cycles, for which everybody waits); probabilities stay below 2^8 and all terms
+      // of one head share the same reference, which cancels in the final division. So the two lanes of a head
       // exchange their maxima only in the rare case: a shuffle waits in the same queue as the
       // producers' copies, a vote does not.
       float alpha = 1.f;
-      if (__any_sync(0xffffffffu, own_max > run_max + 8.f)) {
+      const float slack = i == 0 ? 0.f : 8.f;
+      if (__any_sync(0xffffffffu, own_max > run_max + slack)) {
         const float chunk_max = fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16));
-        if (chunk_max > run_max + 8.f) {
+        if (chunk_max > run_max + slack) {
           alpha = exp2f(run_max - chunk_max);
           run_max = chunk_max;
         }
