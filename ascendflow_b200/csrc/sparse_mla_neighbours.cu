@@ -69,15 +69,15 @@ __device__ __forceinline__ void load_keys(const float* row, int i, int candidate
 }
 
 constexpr int kSelectBins = 256;
-constexpr int kSelectWindow = 65536;  // row positions covered by the bitmap of winners at a time
 
 // Shared memory of one selecting block.
 template <int kThreads, int kCapacity>
 struct SelectShared {
+  static constexpr int kWindow = kThreads >= 256 ? 65536 : 256 * kThreads;  // row positions covered by the bitmap of winners at a time
   uint2 list[kCapacity];               // candidates: row position, score
-  __align__(16) unsigned bitmap[kSelectWindow / 32];
-  unsigned short place[kSelectWindow / 32];  // winners before each word of the bitmap
-  unsigned histogram[kSelectBins];
+  __align__(16) unsigned bitmap[kWindow / 32];
+  unsigned short place[kWindow / 32];  // winners before each word of the bitmap
+  __align__(16) unsigned histogram[kSelectBins];
   unsigned warp_sum[kThreads / 32];
   unsigned count, low, high;           // candidates listed; extremes of what is being binned
   unsigned bin, before, in_bin;        // result of find_bin
@@ -102,22 +102,26 @@ __device__ __forceinline__ unsigned warp_scan(unsigned value, int lane) {
 
 // The bin in which the running count over the histogram reaches `wanted`, what lies before it and
 // what it holds (s.bin stays as it was if the whole histogram holds fewer). Clears the histogram.
-// Called by the whole block after a barrier; ends with one.
+// One warp does it, eight bins per lane. Called by the whole block after a barrier; ends with one.
 template <typename Shared>
 __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned mine = 0, scan = 0;
-  if (threadIdx.x < kSelectBins) {
-    mine = s.histogram[threadIdx.x];
-    s.histogram[threadIdx.x] = 0;
-    scan = warp_scan(mine, lane);
-    if (lane == 31) s.warp_sum[warp] = scan;
-  }
-  __syncthreads();
-  if (threadIdx.x < kSelectBins) {
-    unsigned before = scan - mine;
-    for (int w = 0; w < warp; ++w) before += s.warp_sum[w];
-    if (before < wanted && wanted <= before + mine) { s.bin = threadIdx.x; s.before = before; s.in_bin = mine; }
+  if (threadIdx.x < 32) {
+    static_assert(kSelectBins == 8 * 32, "eight bins per lane");
+    uint4* bins = reinterpret_cast<uint4*>(&s.histogram[threadIdx.x * 8]);
+    const uint4 a = bins[0], b = bins[1];
+    bins[0] = bins[1] = make_uint4(0, 0, 0, 0);
+    const unsigned count[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    unsigned mine = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine += count[i];
+    unsigned before = warp_scan(mine, threadIdx.x) - mine;
+    if (before < wanted && wanted <= before + mine) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (before < wanted && wanted <= before + count[i]) { s.bin = threadIdx.x * 8 + i; s.before = before; s.in_bin = count[i]; }
+        before += count[i];
+      }
+    }
   }
   __syncthreads();
 }
@@ -160,10 +164,10 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
       }
     }
     __syncthreads();
-    if (threadIdx.x < 256) {
+    for (int bin = threadIdx.x; bin < 256; bin += kThreads) {
       unsigned sum = 0;
-      for (int w = 0; w < kWarps; ++w) sum += histogram[w][threadIdx.x];
-      totals[threadIdx.x] = sum;
+      for (int w = 0; w < kWarps; ++w) sum += histogram[w][bin];
+      totals[bin] = sum;
     }
     __syncthreads();
     if (threadIdx.x == 0) {  // walk down from the highest bin until `wanted` entries are covered
@@ -228,17 +232,20 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
 // ties going to the lower index; winners are written in ascending index order, the rest of the 512
 // entries is -1.
 //
-// Bound by memory: the row is streamed once. A strided sample (one or two thousand scores, eight
-// to a sector) gives a floor that about twice TopK scores lie above; the stream lists what reaches
+// Bound by memory for long rows (768 x 65536 scores: 51 us, 60 % of the copy bandwidth; the radix
+// select that read the row five times took 335 us) and by issue slots for many short ones (8192 x
+// 12-16 K: 127 us, 3.8 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
+// two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the stream lists what reaches
 // the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256
 // bins, normally once; the few entries of the threshold's bin are ranked by comparison; a bitmap
 // of winning positions gives the output order. The list holds every score that reaches the
 // floor, so the result is exact whenever the list has at least TopK entries and did not
 // overflow; otherwise (hardly ever, unless most of the row is equal) `select_row_by_digits`.
-template <int kThreads, int kCapacity, int kBlocks>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
   using Shared = SelectShared<kThreads, kCapacity>;
+  constexpr int kWindow = Shared::kWindow;
   extern __shared__ __align__(16) unsigned char select_smem[];
   Shared& s = *reinterpret_cast<Shared*>(select_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -252,47 +259,49 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     for (int i = threadIdx.x; i < kTopK; i += kThreads) list[i] = i < candidates ? i : -1;
     return;
   }
-  for (int i = threadIdx.x * 4; i < min(candidates + 31, kSelectWindow) / 32; i += kThreads * 4)
+  for (int i = threadIdx.x * 4; i < min(candidates + 31, kWindow) / 32; i += kThreads * 4)
     *reinterpret_cast<uint4*>(&s.bitmap[i]) = make_uint4(0, 0, 0, 0);
-  if (threadIdx.x < kSelectBins) s.histogram[threadIdx.x] = 0;
+  for (int i = threadIdx.x; i < kSelectBins; i += kThreads) s.histogram[i] = 0;
   if (threadIdx.x == 0) { s.count = s.few_count = 0; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
   __syncthreads();
 
   // ---- floor ----------------------------------------------------------------------------------
   unsigned floor_key = 0;  // short rows: everything is listed
   if (candidates > kCapacity) {
-    constexpr int kMostQuads = 2;  // sampled 16-byte quads per thread, at most; two neighbouring threads share a sector
-    const int quads = candidates >= 160 * kThreads ? 2 : 1, sampled = quads * kThreads;
-    const unsigned row_pairs = unsigned(candidates) >> 3;
+    // An eighth of the row, or kMostQuads 16-byte quads per thread: eight threads share a 128-byte
+    // segment, and the segments lie at equal distances.
+    constexpr int kSegments = kThreads / 8;
+    const int quads = max(1, min(kMostQuads, candidates / (32 * kThreads))), sampled = quads * kThreads;
+    const unsigned step = (unsigned(candidates) >> 2) / unsigned(quads * kSegments);  // at least eight quads
+    float4 v[kMostQuads];
+#pragma unroll
+    for (int q = 0; q < kMostQuads; ++q)
+      if (q < quads) v[q] = __ldg(reinterpret_cast<const float4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
+    // The row's head on its way to L2 behind the sample, while the floor is found.
+    if (threadIdx.x == 0) prefetch_l2(row, min(unsigned(candidates) * 4u & ~15u, 65536u));
     uint32_t key[4 * kMostQuads];
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q) {
-      if (q < quads) {
-        const unsigned pair = (q * kThreads + threadIdx.x) >> 1;
-        const unsigned at = unsigned((unsigned long long)pair * row_pairs / unsigned(sampled / 2)) * 2 + (threadIdx.x & 1);
-        const float4 v = __ldg(reinterpret_cast<const float4*>(row) + at);
-        key[4 * q + 0] = score_key(v.x); key[4 * q + 1] = score_key(v.y);
-        key[4 * q + 2] = score_key(v.z); key[4 * q + 3] = score_key(v.w);
-      } else {
-        key[4 * q + 0] = key[4 * q + 1] = key[4 * q + 2] = key[4 * q + 3] = 0;
-      }
+      key[4 * q + 0] = q < quads ? score_key(v[q].x) : 0; key[4 * q + 1] = q < quads ? score_key(v[q].y) : 0;
+      key[4 * q + 2] = q < quads ? score_key(v[q].z) : 0; key[4 * q + 3] = q < quads ? score_key(v[q].w) : 0;
     }
-    // The row's head on its way to L2 (behind the sample) while the floor is found.
-    if (threadIdx.x == 0) prefetch_l2(row, min(unsigned(candidates) * 4u & ~15u, 65536u));
-    // Only the sample's upper end matters: its maximum, and the lowest of the maxima of four
-    // threads each, above which lie at least kThreads / 4 samples (about four times as many).
+    // Samples expected among the TopK best, and five standard deviations of that count on top:
+    // the floor lies below the TopK-th best score in all but a few rows in a million.
+    const float expected = float(kTopK) * float(4 * sampled) / float(candidates);
+    unsigned wanted = unsigned(expected + 5.f * sqrtf(expected) + 2.f);
+    // Only the sample's upper end matters: its maximum, and the lowest of the maxima of G groups, above
+    // which lie about four G samples: G = all threads, or a quarter of them where that is enough.
     unsigned best = 0;
 #pragma unroll
     for (int e = 0; e < 4 * kMostQuads; ++e) best = max(best, key[e]);
-    best = max(best, __shfl_xor_sync(0xffffffffu, best, 1));
-    best = max(best, __shfl_xor_sync(0xffffffffu, best, 2));
+    if (wanted <= unsigned(kThreads / 4)) {
+      best = max(best, __shfl_xor_sync(0xffffffffu, best, 1));
+      best = max(best, __shfl_xor_sync(0xffffffffu, best, 2));
+    }
     const unsigned warp_low = __reduce_min_sync(0xffffffffu, best), warp_high = __reduce_max_sync(0xffffffffu, best);
     if (lane == 0) { atomicMin(&s.low, warp_low); atomicMax(&s.high, warp_high); }
     __syncthreads();
-    // Samples expected among the TopK best, and five standard deviations of that count on top:
-    // the floor lies below the TopK-th best score in all but a few rows in a hundred thousand.
-    const float expected = float(kTopK) * float(4 * sampled) / float(candidates);
-    unsigned wanted = unsigned(expected + 5.f * sqrtf(expected) + 2.f), lower = s.low, upper = s.high;
+    unsigned lower = s.low, upper = s.high;
     while (true) {  // normally once; again inside a bin that holds too many (a sample of both signs, say)
       const int shift = max(0, 24 - __clz(int(upper - lower)));  // 256 bins over [lower, upper]
 #pragma unroll
@@ -400,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     __syncthreads();
     find_bin(s, wanted);
     prefix = prefix << (above - shift) | s.bin;
-    if (prefix == 0 && !exact) {
+    if (prefix == 0 && !exact && ties == 0xffffffffu) {
       find_extremes();
       above = 32 - __clz(int(top - bottom));
       shift = max(0, above - 8);
@@ -424,10 +433,11 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~key << 32 | entry.x;
   }
   __syncthreads();
-  if (threadIdx.x < s.few_count) {
-    unsigned before = 0;
-    for (unsigned i = 0; i < s.few_count; ++i) before += s.few[i] < s.few[threadIdx.x];
-    if (before + 1 == wanted) s.limit = s.few[threadIdx.x];
+  const int few = int(s.few_count);  // 32 at most
+  for (int i = warp; i < few; i += kThreads / 32) {
+    const unsigned long long candidate = s.few[i];
+    const unsigned before = __popc(__ballot_sync(0xffffffffu, lane < few && s.few[lane] < candidate));
+    if (before + 1 == wanted && lane == 0) s.limit = candidate;
   }
   __syncthreads();
   const unsigned long long limit = s.limit;
@@ -436,9 +446,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   // A bitmap of winning positions and the number of winners before each of its words: every winner
   // finds its place in the output by itself.
   unsigned written = 0;
-  for (int window = 0; window < candidates; window += kSelectWindow) {
+  for (int window = 0; window < candidates; window += kWindow) {
     if (window > 0) {
-      for (int i = threadIdx.x; i < kSelectWindow / 32; i += kThreads) s.bitmap[i] = 0;
+      for (int i = threadIdx.x; i < kWindow / 32; i += kThreads) s.bitmap[i] = 0;
       __syncthreads();
     }
     unsigned winners = 0;  // of this thread's entries (ten at most)
@@ -446,15 +456,15 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     for (int i = threadIdx.x, bit = 0; i < listed; i += kThreads, ++bit) {
       const uint2 entry = s.list[i];
       const unsigned index = entry.x - window;
-      if (index < kSelectWindow && ((unsigned long long)~score_key(__uint_as_float(entry.y)) << 32 | entry.x) <= limit) {
+      if (index < kWindow && ((unsigned long long)~score_key(__uint_as_float(entry.y)) << 32 | entry.x) <= limit) {
         atomicOr(&s.bitmap[index >> 5], 1u << (index & 31));
         winners |= 1u << bit;
       }
     }
     __syncthreads();
-    const int words = (min(candidates - window, kSelectWindow) + 31) / 32;
+    const int words = (min(candidates - window, kWindow) + 31) / 32;
     // Eight words (32 bytes) per thread: threads beyond the words have none.
-    static_assert(kSelectWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
+    static_assert(kWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
     const int first = threadIdx.x * 8;
     uint4 a = make_uint4(0, 0, 0, 0), b = a;
     if (first < words) a = *reinterpret_cast<const uint4*>(&s.bitmap[first]);
@@ -523,9 +533,9 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
-template <int kThreads, int kCapacity, int kBlocks>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks>;
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads>;
   constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity>));
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
@@ -562,10 +572,14 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   int device = 0, multiprocessors = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Few tokens, or rows whose list of candidates would not fit the small blocks: one large block per
-  // SM and token. Otherwise small blocks, eight to an SM, whose phases overlap.
-  if (T < 2 * multiprocessors || SPAN > 131072) return launch_select<1024, 8192, 1>(p, s);
-  return launch_select<256, 2560, 6>(p, s);
+  // Few tokens, or rows so long that a small block's sample says too little: one large block per SM
+  // and token (16 tokens of 65536 scores: 11 us). Otherwise small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
+  // more than a wave of them (8192 rows of 12-16 K scores: 127 us against 144 with eight warps, which
+  // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
+  // 38) or where the row needs the larger sample.
+  if (T < 2 * multiprocessors || SPAN > 131072) return launch_select<1024, 8192, 1, 2>(p, s);
+  if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768) return launch_select<128, 2048, 9, 4>(p, s);
+  return launch_select<256, 2560, 6, 2>(p, s);
 }
 
 int launch_sparse_mla_cache_append_flagged(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,

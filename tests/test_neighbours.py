@@ -137,10 +137,12 @@ def test_gpu_selection_over_long_rows(max_seq, ratio):
     (320, (1, 4, 511, 512, 513, 2559, 2560, 2561, 4095, 4097, 16383, 32769, 65535, 65536, 65537, 70001)),
     # 1024-thread blocks: the list (8192) and one step (16384)
     (19, (512, 513, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
+    # 128-thread blocks: the list (2048), one step (2048), the window of winners (32768), the longest
+    (1800, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 8191, 16385, 32767, 32768)),
 ])
 def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
-    """One token per request, every row length in turn; continuous, 8-bit-mantissa, offset and
-    clustered scores in turn (what a sample of the row says about it differs)."""
+    """One token per request, every row length in turn; continuous, 8-bit-mantissa, offset,
+    clustered and few-valued scores in turn (what a sample of the row says about it differs)."""
     import torch
 
     from ascendflow_b200 import neighbours
@@ -156,7 +158,7 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     span = -(-max(visible) // 4) * 4
     scores = rng.normal(size=(tokens, span)).astype(np.float32)
     for token in range(tokens):
-        kind = (token // len(visible) + token) % 4
+        kind = (token // len(visible) + token) % 5
         if kind == 1:
             scores[token] = (scores[token].view(np.uint32) & 0xFFFF0000).view(np.float32)
         elif kind == 2:
@@ -164,6 +166,8 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
         elif kind == 3:  # the winners side by side, between the places a sample looks at
             first = int(rng.integers(0, max(1, lengths[token] - 600)))
             scores[token, first:first + 600] += 50.0
+        elif kind == 4:  # hundreds of equal scores at the threshold: the position decides
+            scores[token] = np.round(scores[token] * 8) / 8
     expected = O.select_topk_indices(scores, data, policy)
     device = {k: torch.from_numpy(v).cuda() for k, v in data.items()}
     actual = neighbours.topk_indices(torch.from_numpy(scores).cuda(), device["cu_seqlens_q"], device["seqused_cmp_kv"],
