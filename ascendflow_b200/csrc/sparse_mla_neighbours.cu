@@ -267,7 +267,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
 
   // ---- floor ----------------------------------------------------------------------------------
   unsigned floor_key = 0;  // short rows: everything is listed
-  if (candidates > kCapacity) {
+  constexpr int kListed = 4 * kThreads > 1024 ? 4 * kThreads : 1024;  // (listing 8 K scores costs more than sampling them)
+  static_assert(kListed <= kCapacity, "the whole row fits the list");
+  if (candidates > kListed) {
     // An eighth of the row, or kMostQuads 16-byte quads per thread: eight threads share a 128-byte
     // segment, and the segments lie at equal distances.
     constexpr int kSegments = kThreads / 8;
@@ -572,12 +574,15 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   int device = 0, multiprocessors = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Few tokens, or rows so long that a small block's sample says too little: one large block per SM
-  // and token (16 tokens of 65536 scores: 11 us). Otherwise small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
+  // Rows so long that a small block's sample says too little: large blocks. No more tokens than SMs: a
+  // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
+  // with thirty-two; of 65536: 11 us against 15). Otherwise
+  // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
   // more than a wave of them (8192 rows of 12-16 K scores: 127 us against 144 with eight warps, which
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
   // 38) or where the row needs the larger sample.
-  if (T < 2 * multiprocessors || SPAN > 131072) return launch_select<1024, 8192, 1, 2>(p, s);
+  if (SPAN > 131072) return launch_select<1024, 8192, 1, 2>(p, s);
+  if (T <= multiprocessors) return launch_select<512, 4096, 2, 2>(p, s);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768) return launch_select<128, 2048, 9, 4>(p, s);
   return launch_select<256, 2560, 6, 2>(p, s);
 }

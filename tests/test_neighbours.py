@@ -132,11 +132,13 @@ def test_gpu_selection_over_long_rows(max_seq, ratio):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("tokens,visible", [
-    # 256-thread blocks: TopK, the candidate list (2560), one step of the stream (4096), the sample's
+    # 256-thread blocks: TopK, listed whole (1024), the list (2560), one step of the stream (4096), the sample's
     # sizes, the window of winners (65536), each with its neighbours
-    (320, (1, 4, 511, 512, 513, 2559, 2560, 2561, 4095, 4097, 16383, 32769, 65535, 65536, 65537, 70001)),
-    # 1024-thread blocks: the list (8192) and one step (16384)
-    (19, (512, 513, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
+    (320, (1, 4, 511, 512, 513, 1024, 1025, 2559, 2560, 2561, 4095, 4097, 16383, 32769, 65535, 65536, 65537, 70001)),
+    # 512-thread blocks: listed whole (2048), the list (4096), one step (8192), the longest
+    (19, (512, 513, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
+    # 1024-thread blocks: listed whole (4096), the list (8192), one step (16384), more than a window of winners
+    (7, (4096, 4097, 8193, 16385, 131073, 200001, 150000)),
     # 128-thread blocks: the list (2048), one step (2048), the window of winners (32768), the longest
     (1800, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 8191, 16385, 32767, 32768)),
 ])
@@ -148,7 +150,7 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     from ascendflow_b200 import neighbours
 
     rng = np.random.default_rng(tokens)
-    policy = O.make_policy(tokens, tokens, ratio=1, max_seq=131072, blocks=8)
+    policy = O.make_policy(tokens, tokens, ratio=1, max_seq=-(-max(max(visible), 131072) // 128) * 128, blocks=8)
     lengths = np.array([visible[i % len(visible)] for i in range(tokens)], dtype=np.int32)
     data = {
         "cu_seqlens_q": np.arange(tokens + 1, dtype=np.int32),
@@ -167,7 +169,8 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
             first = int(rng.integers(0, max(1, lengths[token] - 600)))
             scores[token, first:first + 600] += 50.0
         elif kind == 4:  # hundreds of equal scores at the threshold: the position decides
-            scores[token] = np.round(scores[token] * 8) / 8
+            # (+ 0.0: no negative zeros, which the kernel's keys have always put below zero and the oracle ties with it)
+            scores[token] = np.round(scores[token] * 8) / 8 + np.float32(0.0)
     expected = O.select_topk_indices(scores, data, policy)
     device = {k: torch.from_numpy(v).cuda() for k, v in data.items()}
     actual = neighbours.topk_indices(torch.from_numpy(scores).cuda(), device["cu_seqlens_q"], device["seqused_cmp_kv"],
