@@ -111,7 +111,7 @@ def is_current():
     return LIBRARY.exists() and STAMP.exists() and STAMP.read_text() == _identity()
 
 
-ATTENTION_KERNEL_SOURCES = ("sparse_mla_common.cuh", "tcgen05_ptx.cuh", "sparse_mla_tcgen05.cuh")
+ATTENTION_KERNEL_SOURCES = ("sparse_mla_common.cuh", "tcgen05_ptx.cuh", "sparse_mla_tcgen05.cuh", "sparse_mla_team.cuh")
 
 
 def attention_kernel_identity():

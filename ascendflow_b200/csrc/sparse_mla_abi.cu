@@ -13,6 +13,7 @@
 #include "sparse_mla_common.cuh"
 #include "sparse_mla_mma_sync.cuh"
 #include "sparse_mla_tcgen05.cuh"
+#include "sparse_mla_team.cuh"
 
 namespace sparse_mla {
 namespace {
@@ -213,7 +214,7 @@ int launch_sparse_mla(void* stream, void* arg_q, void* arg_ori_kv, void* arg_cmp
     return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (int status = clear_workspace(s, npu_workspace)) return status;
-  return umma::launch<1>(p, s, multiprocessors());
+  return team::launch<1>(p, s, multiprocessors());
 }
 
 int launch_sparse_mla_f16(void* stream, void* arg_q, void* arg_ori_kv, void* arg_cmp_kv,
@@ -231,7 +232,7 @@ int launch_sparse_mla_f16(void* stream, void* arg_q, void* arg_ori_kv, void* arg
     return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (int status = clear_workspace(s, npu_workspace)) return status;
-  return umma::launch<0>(p, s, multiprocessors());
+  return team::launch<0>(p, s, multiprocessors());
 }
 
 int launch_sparse_mla_kept_status(void* stream, int64_t f16, void* const* tensors, void* npu_workspace, int64_t B,
@@ -241,7 +242,7 @@ int launch_sparse_mla_kept_status(void* stream, int64_t f16, void* const* tensor
             tensors[9], tensors[10], tensors[11], tensors[12], npu_workspace, B, T, PAGES, ORI_BLOCKS, CMP_BLOCKS, CMP_PAGE))
     return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return f16 != 0 ? umma::launch<0>(p, s, multiprocessors()) : umma::launch<1>(p, s, multiprocessors());
+  return f16 != 0 ? team::launch<0>(p, s, multiprocessors()) : team::launch<1>(p, s, multiprocessors());
 }
 
 // The portable-instruction BF16 kernel under its own name: the cross-check of the tcgen05 kernel.
@@ -312,7 +313,7 @@ int launch_sparse_mla_static_workspace(void* stream, void* arg_q, void* arg_ori_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // The array keeps whatever the previous call left: the status block must start at zero.
   if (int status = int(cudaMemsetAsync(workspace, 0, kStaticWorkspaceBytes, s))) return status;
-  return umma::launch<1>(p, s, multiprocessors());
+  return team::launch<1>(p, s, multiprocessors());
 }
 
 int launch_sparse_mla_wait_expiry_selftest(void* stream, void* npu_workspace, int64_t limit_cycles) {

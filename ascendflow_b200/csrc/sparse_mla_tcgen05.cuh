@@ -139,6 +139,12 @@ struct Shared {
   __device__ __forceinline__ volatile int* abort_flag() const {
     return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 4);
   }
+  __device__ __forceinline__ volatile uint32_t* rescale_mask() const {  // (team kernel)
+    return reinterpret_cast<volatile uint32_t*>(ptr + kSmemMisc + 8);
+  }
+  __device__ __forceinline__ const volatile float* maxima(int offset) const {  // (team kernel)
+    return reinterpret_cast<const volatile float*>(ptr + offset);
+  }
 };
 
 // The tokens of one persistent block, in order. Blocks take `group` consecutive tokens per round
@@ -279,6 +285,55 @@ __global__ void resolve_rows_kernel(const Params p, int32_t* out) {
   }
 }
 
+// Resolve the 640 slots of a token into row buffer `buffer` and list its live chunks (one warp).
+__device__ __forceinline__ void publish_token(const Params& p, const Shared& sm, int token, int buffer, int lane) {
+  int* rows = sm.rows(buffer);
+  TokenInfo* info = sm.info(buffer);
+  int resolved[kSlots / 32];
+  resolve_token_warp(p, token, lane, resolved);
+  unsigned live_chunks = 0;  // bit c set: chunk c holds a live slot (same in all lanes)
+  unsigned mine = 0;         // lane l: live bits of slots 32 l ..
+#pragma unroll
+  for (int i = 0; i < kSlots / 32; ++i) {
+    rows[i * 32 + lane] = resolved[i];
+    const unsigned live = __ballot_sync(0xffffffffu, resolved[i] >= 0);
+    if (live != 0) live_chunks |= 1u << (i * 32 / kChunkRows);
+    if (lane == i) mine = live;
+  }
+  const int chunk = lane >> 1;     // two lanes per chunk (no bit beyond kMaxChunks - 1 is set)
+  if (live_chunks >> chunk & 1) {
+    const int item = __popc(live_chunks & ((1u << chunk) - 1));
+    reinterpret_cast<unsigned*>(&info->live[item])[lane & 1] = mine;
+    info->chunk[item] = (unsigned char)chunk;
+  }
+  if (lane == 0) {
+    info->token = token;
+    info->chunks = __popc(live_chunks);
+  }
+}
+
+// What a block reads first, for its first token, asked for on the way to L2 (and its pages'
+// translations with it) while the kernel before is still running: L2 sees what that kernel writes,
+// so nothing stale is read later.
+__device__ __forceinline__ void prefetch_first(const Params& p, int token) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp == kResolverWarp) {
+    if (lane < 16) prefetch_l2(p.indices + (size_t)token * kTopK + lane * 32);
+    else if (lane == 16) prefetch_l2(p.topk_len + token);
+    else if (lane == 17) prefetch_l2(p.cu);
+    else if (lane == 18) prefetch_l2(p.seq_ori);
+    else if (lane == 19) prefetch_l2(p.seq_cmp);
+    else if (lane == 20) prefetch_l2(p.residual);
+    else if (lane == 21) prefetch_l2(p.ori_table);
+    else if (lane == 22) prefetch_l2(p.cmp_table);
+    else if (lane == 23) prefetch_l2(p.sinks);
+  } else if (warp >= kFirstProducerWarp && warp < kPvWarp) {
+    const char* q = static_cast<const char*>(p.q) + (size_t)token * kHeads * kRowBytes + (threadIdx.x - kFirstProducerWarp * 32) * 256;
+    prefetch_l2(q);
+    prefetch_l2(q + 128);
+  }
+}
+
 // ---- resolver warp ----------------------------------------------------------------------------
 // Runs ahead of everybody else: for each token of this block it resolves the 640 slots into row
 // buffer `token_count & 1`, lists the live chunks and publishes both.
@@ -289,8 +344,6 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
   TokenWalk walk(p);
   for (int token = walk.next(); token >= 0; token = walk.next(), ++token_count) {
     const int buffer = token_count & 1;
-    int* rows = sm.rows(buffer);
-    TokenInfo* info = sm.info(buffer);
     // The buffer is free once the softmax warps have finished the token that used it two tokens
     // ago. (Barriers that one role may pass without the others keeping up exist once per buffer:
     // a phase parity can only tell two consecutive phases apart.)
@@ -300,27 +353,7 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
     if (token_count >= 2 &&
         (!warp_wait(sm.bar(kTokenDone0 + buffer), ((token_count >> 1) & 1) ^ 1, abort_flag) ||
          !warp_wait(sm.bar(kInfoRead0 + buffer), ((token_count >> 1) & 1) ^ 1, abort_flag))) return;
-    int resolved[kSlots / 32];
-    resolve_token_warp(p, token, lane, resolved);
-    unsigned live_chunks = 0;  // bit c set: chunk c holds a live slot (same in all lanes)
-    unsigned mine = 0;         // lane l: live bits of slots 32 l ..
-#pragma unroll
-    for (int i = 0; i < kSlots / 32; ++i) {
-      rows[i * 32 + lane] = resolved[i];
-      const unsigned live = __ballot_sync(0xffffffffu, resolved[i] >= 0);
-      if (live != 0) live_chunks |= 1u << (i * 32 / kChunkRows);
-      if (lane == i) mine = live;
-    }
-    const int chunk = lane >> 1;     // two lanes per chunk (no bit beyond kMaxChunks - 1 is set)
-    if (live_chunks >> chunk & 1) {
-      const int item = __popc(live_chunks & ((1u << chunk) - 1));
-      reinterpret_cast<unsigned*>(&info->live[item])[lane & 1] = mine;
-      info->chunk[item] = (unsigned char)chunk;
-    }
-    if (lane == 0) {
-      info->token = token;
-      info->chunks = __popc(live_chunks);
-    }
+    publish_token(p, sm, token, buffer, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(sm.bar(kTokenReady0 + buffer));
   }
@@ -348,12 +381,34 @@ __device__ __forceinline__ void transpose_octet(uint32_t* words, int lane) {
   }
 }
 
+// Copies of the 64 rows of a chunk into a tile, by the 256 producer threads.
+__device__ __forceinline__ void gather_chunk(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
+  // Sixteen threads per row and quarter: eight 16-byte units of block q, eight of block q + 4.
+  const int sub = tid & 15;
+  const char* source[kChunkRows / (kProducerThreads / 16)];
+  bool live[kChunkRows / (kProducerThreads / 16)];
+#pragma unroll
+  for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
+    const int slot = chunk * kChunkRows + (tid >> 4) + k * (kProducerThreads / 16);
+    const int row = rows[slot];
+    live[k] = row >= 0;
+    source[k] = static_cast<const char*>(slot < kWindow ? p.ori_kv : p.cmp_kv) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int unit = (q + 4 * (sub >> 3)) * 8 + (sub & 7);
+#pragma unroll
+    for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
+      const int r = (tid >> 4) + k * (kProducerThreads / 16);
+      cp_async16(tile + swizzled(r, unit), source[k] + unit * 16, live[k]);
+    }
+  }
+}
+
 __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32;
   const int lane = tid & 31;
   volatile int* abort_flag = sm.abort_flag();
-  const char* window_base = static_cast<const char*>(p.ori_kv);
-  const char* compressed_base = static_cast<const char*>(p.cmp_kv);
   // Q goes from global memory to tensor memory through registers, never through the ring. A warp
   // reaches the 32 tensor-memory lanes of subpartition (warp index % 4): two producer warps
   // share each subpartition and take 64 columns (256 bytes of every half row) each. Lane l of a
@@ -417,27 +472,7 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
       const uint32_t stage = ring % kStages, use = ring / kStages;
       if (use > 0 && !warp_wait(sm.bar(kKvFree0 + stage), (use - 1) & 1, abort_flag)) return;
       const uint32_t tile = sm.base + kSmemKv + stage * kTileBytes;
-      const int chunk = info->chunk[item];
-      // Sixteen threads per row and quarter: eight 16-byte units of block q, eight of block q + 4.
-      const int sub = tid & 15;
-      const char* source[kChunkRows / (kProducerThreads / 16)];
-      bool live[kChunkRows / (kProducerThreads / 16)];
-#pragma unroll
-      for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
-        const int slot = chunk * kChunkRows + (tid >> 4) + k * (kProducerThreads / 16);
-        const int row = rows[slot];
-        live[k] = row >= 0;
-        source[k] = (slot < kWindow ? window_base : compressed_base) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int unit = (q + 4 * (sub >> 3)) * 8 + (sub & 7);
-#pragma unroll
-        for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
-          const int r = (tid >> 4) + k * (kProducerThreads / 16);
-          cp_async16(tile + swizzled(r, unit), source[k] + unit * 16, live[k]);
-        }
-      }
+      gather_chunk(p, rows, info->chunk[item], tile, tid);
       cp_async_arrive(sm.bar(kKvFull0 + stage));
       if (item == 0 && lane == 0) mbar_arrive(sm.bar(kInfoRead0 + (token_count & 1)));
       if (item == 0) {
@@ -489,9 +524,9 @@ __device__ __forceinline__ void issue_qk_steps(uint32_t s_tmem, uint32_t q_tmem,
 // thrown away, but M = 128 runs at the full rate of the pipe and N = 128 is above its
 // per-instruction floor: 16 instructions of 64 cycles replace 32 of about 56.
 template <int kFormat, int kBegin = 0, int kEnd = kQkSteps>
-__device__ __forceinline__ void issue_qk(const Shared& sm, uint32_t tmem, int stage) {
+__device__ __forceinline__ void issue_qk(const Shared& sm, uint32_t tmem, int stage, uint32_t scores = kTmemS) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, 16, 1024);
-  issue_qk_steps<kFormat, kBegin, kEnd>(tmem + kTmemS, tmem + kTmemQ, x_desc);
+  issue_qk_steps<kFormat, kBegin, kEnd>(tmem + scores, tmem + kTmemQ, x_desc);
 }
 
 constexpr int kPvSteps = 2 * (kChunkRows / 16);
@@ -888,6 +923,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
   const uint32_t tmem = *tmem_slot;
   // Up to here nothing has touched global memory: a block's start, and the launch itself, overlap
   // the end of the kernel before.
+  if (const int first = TokenWalk(p).next(); first >= 0) prefetch_first(p, first);
   wait_for_predecessor();
   let_successor_start();
 

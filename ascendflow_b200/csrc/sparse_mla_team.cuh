@@ -1,0 +1,522 @@
+// Sparse MLA attention for calls of few tokens: a cluster of four blocks works on one token. The
+// arithmetic is that of `attention_kernel`, operation for operation (a token's result does not
+// depend on how many others are in the call); what is spread over the blocks is what does not
+// depend on the order of the chunks.
+//
+//   1. Every block resolves the token and gathers up to three of its ten chunks (items r, r + 4 and
+//      r + 8 for block r).
+//   2. Q X^T of its own chunks, and their maxima per head, which go to all four blocks.
+//   3. With all maxima known every block can follow the running reference through the chunks
+//      (examples/sparse_attention/attention.py:398-490): it takes its own chunks' exponentials and sends
+//      P and the partial sums to the other three (bulk copies), while it gathers, of all chunks, the
+//      128 features it will produce.
+//   4. O += P X over all chunks in order for its 128 features (M = 64, N = 128), normalise, store.
+//
+// Bound by latency. One token on one block takes 30 k cycles: 9 k until its first scores, 1.9 k per
+// chunk, 3 k for the output pass. Here the chunks' first product and softmax run side by side, and
+// the output pass is a quarter; what stays serial is the second product, whose instructions wait for
+// one another (about 700 cycles per chunk). 17.3 -> 14.7 us for one token, 17.4 -> 15.1 for 16, 17.6 ->
+// 16.1 for 24. (Eight blocks: 14.1 us for one token, 15.2 for eight; P written to the other blocks by
+// the softmax threads instead of bulk copies: 19.9.) Copies between blocks are of local shared
+// memory; nothing multicasts.
+//
+// Tensor memory: columns 0-127, 128-255 and 384-511 the scores of the own chunks, 256-383 Q as in
+// `attention_kernel` and, once all scores are computed, 256-319 O (128 features).
+#pragma once
+
+#include "sparse_mla_tcgen05.cuh"
+
+namespace sparse_mla {
+namespace team {
+
+using namespace sm100;
+using namespace umma;
+
+constexpr int kBlocks = 4;                       // of a cluster
+constexpr int kOwnItems = 3;                     // chunks of a block, at most
+constexpr int kSliceBytes = 2 * kBlockBytes;     // 64 rows x 128 features
+static_assert(kOwnItems * kBlocks >= kMaxChunks && kFeatures == kBlocks * 128, "four blocks cover a token");
+
+// Shared memory (bytes from the 1024-aligned base; the row list, token info and misc words lie where
+// `attention_kernel` has them). The own chunks' tiles fill the ring's place. Once all blocks have
+// computed their scores it holds eight slices (the last two chunks' come when the first two have been
+// used) and, behind them, all P tiles and partial sums.
+constexpr int kPBytes = kHeads * 128;
+constexpr int kSumBytes = 2 * kHeads * 4;        // float[2 row halves][64 heads]
+constexpr int kSliceSlots = 8;
+constexpr int kTeamSlices = 0;
+constexpr int kTeamP = kSliceSlots * kSliceBytes;
+constexpr int kTeamSums = kTeamP + kMaxChunks * kPBytes;
+constexpr int kTeamMaxima = kTeamSums + kMaxChunks * kSumBytes;  // float[10][64]
+static_assert(kTeamMaxima + kMaxChunks * kHeads * 4 <= kSmemRows && kTeamMaxima >= kOwnItems * kTileBytes,
+              "areas do not meet; maxima arrive while tiles are in use");
+static_assert(kMaxChunks - kSliceSlots == 2, "two late slices");
+__host__ __device__ constexpr uint32_t score_columns(int own) { return own == 0 ? 0 : own == 1 ? 128 : 384; }
+constexpr uint32_t kTeamO = kTmemQ;
+
+enum TeamBar {
+  kReady = 0, kQReady, kTile0, kTile1, kTile2, kScores0, kScores1, kScores2, kMaskReady, kPvDone, kRescaled, kOutput,
+  kSlices0,                                   // of two chunks each
+  kP0 = kSlices0 + kMaxChunks / 2,
+  kSliceFree0 = kP0 + kMaxChunks, kSliceFree1,
+  kTeamBarCount
+};
+static_assert(kTeamBarCount <= 32, "the barrier area holds 32 mbarriers");
+
+template <int kFormat> constexpr uint32_t kIdescTeamPv = idesc_f16(64, 128, kFormat, 0, 1);  // issued as .ws
+
+// The lazy running reference of one head through the chunks, from their maxima: `visit(item, reference,
+// alpha)` for every chunk. The same comparisons as in `attention_kernel`. (All maxima are loaded
+// first: a chain of shared loads behind the slices' copies takes a thousand cycles.)
+template <typename Visit>
+__device__ __forceinline__ void follow_reference(const volatile float* maxima, float sink, int chunks, Visit visit) {
+  float chunk_max[kMaxChunks];
+#pragma unroll
+  for (int i = 0; i < kMaxChunks; ++i) chunk_max[i] = maxima[i * kHeads];
+  float reference = sink;
+#pragma unroll
+  for (int i = 0; i < kMaxChunks; ++i) {
+    float alpha = 1.f;
+    if (i < chunks && chunk_max[i] > reference + (i == 0 ? 0.f : 8.f)) {
+      alpha = exp2f(reference - chunk_max[i]);
+      reference = chunk_max[i];
+    }
+    visit(i, reference, alpha);
+  }
+}
+
+// Phase A, producer warps: Q to tensor memory, the own chunks' tiles.
+__device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, int token, int rank) {
+  const int tid = threadIdx.x - kFirstProducerWarp * 32, lane = tid & 31, warp = threadIdx.x >> 5;
+  const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
+  volatile int* abort_flag = sm.abort_flag();
+  const char* q = static_cast<const char*>(p.q) + (size_t)token * kHeads * kRowBytes +
+                  (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + (lane >> 4) * 512 + part * 256 + (lane & 7) * 16;
+  uint32_t words[64];  // see producer_role
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(q + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128));
+    words[4 * j + 0] = v.x; words[4 * j + 1] = v.y; words[4 * j + 2] = v.z; words[4 * j + 3] = v.w;
+  }
+  transpose_octet(words, lane);
+  transpose_octet(words + 32, lane);
+  if (!warp_wait(sm.bar(kReady), 0, abort_flag)) return;
+  const int* rows = sm.rows(0);
+  const TokenInfo* info = sm.info(0);
+  const int chunks = info->chunks;
+  for (int j = 0; j < kOwnItems; ++j) {
+    const int item = rank + j * kBlocks;
+    if (item >= chunks) break;
+    gather_chunk(p, rows, info->chunk[item], sm.base + kSmemKv + j * kTileBytes, tid);
+    cp_async_arrive(sm.bar(kTile0 + j));
+    if (j > 0) continue;
+    const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tmem_st16(q_tmem + k * 16, *reinterpret_cast<uint32_t(*)[16]>(&words[16 * k]));
+    tmem_wait_st();
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sm.bar(kQReady));
+  }
+}
+
+// Copies of a chunk's slice, this block's 128 features of its 64 rows, by `threads` threads: sixteen per row.
+__device__ __forceinline__ void gather_slice(const Params& p, const Shared& sm, int rank, int item, int thread, int threads) {
+  const int chunk = sm.info(0)->chunk[item], unit = thread & 15;
+  const int* rows = sm.rows(0);
+#pragma unroll 4
+  for (int r = thread >> 4; r < kChunkRows; r += threads >> 4) {
+    const int slot = chunk * kChunkRows + r, row = rows[slot];
+    const char* source = static_cast<const char*>(slot < kWindow ? p.ori_kv : p.cmp_kv) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
+    cp_async16(sm.base + kTeamSlices + item % kSliceSlots * kSliceBytes + (unit >> 3) * kBlockBytes + r * 128 + (((unit & 7) ^ (r & 7)) << 4),
+               source + rank * 256 + unit * 16, row >= 0);
+  }
+}
+
+// Phase B, producer warps: the first eight chunks' slices; then four of the warps rescale O where a
+// reference moves, the other four gather the last two slices.
+__device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, int rank) {
+  const int tid = threadIdx.x - kFirstProducerWarp * 32, lane = tid & 31, warp = threadIdx.x >> 5;
+  volatile int* abort_flag = sm.abort_flag();
+  const int chunks = sm.info(0)->chunks, early = min(chunks, kSliceSlots);
+  for (int item = 0; item < early; ++item) {
+    gather_slice(p, sm, rank, item, tid, kProducerThreads);
+    if ((item & 1) || item == early - 1) cp_async_arrive(sm.bar(kSlices0 + item / 2));
+  }
+  if (chunks == 0) return;
+  if (warp >= kFirstProducerWarp + 4) {
+    if (chunks <= kSliceSlots) return;
+    for (int item = kSliceSlots; item < chunks; ++item) {
+      if (!warp_wait(sm.bar(kSliceFree0 + item - kSliceSlots), 0, abort_flag)) return;
+      gather_slice(p, sm, rank, item, tid - 128, 128);
+    }
+    cp_async_arrive(sm.bar(kSlices0 + kSliceSlots / 2));
+  } else {
+    if (!warp_wait(sm.bar(kMaskReady), 0, abort_flag)) return;
+    const int o_head = (warp & 1) * 32 + lane;  // lane l of tensor memory: head l % 64 (see softmax_role)
+    const uint32_t o_addr = tmem + kTeamO + (uint32_t((warp & 3) * 32) << 16);
+    const float sink = __ldg(p.sinks + o_head) * 1.4426950408889634f;
+    uint32_t phase = 0;
+    for (uint32_t left = *sm.rescale_mask(); left != 0; left &= left - 1) {
+      const int item = __ffs(left) - 1;
+      float factor = 1.f;
+      follow_reference(sm.maxima(kTeamMaxima) + o_head, sink, chunks, [&](int i, float, float alpha) { if (i == item) factor = alpha; });
+      if (!warp_wait(sm.bar(kPvDone), phase++ & 1, abort_flag)) return;
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 16) {
+        uint32_t o[16];
+        tmem_ld16(o_addr + c, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * factor);
+        tmem_st16(o_addr + c, o);
+      }
+      tmem_wait_st();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sm.bar(kRescaled));
+    }
+  }
+}
+
+// Phase B, one warp: the chunks after the first that move some head's reference.
+__device__ void team_mask(const Shared& sm, float sink, float other_sink) {  // of heads lane, 32 + lane
+  const int lane = threadIdx.x & 31, chunks = sm.info(0)->chunks;
+  uint32_t moved = 0;
+  auto note = [&](int i, float, float alpha) { moved |= uint32_t(i > 0 && alpha != 1.f) << i; };
+  follow_reference(sm.maxima(kTeamMaxima) + lane, sink, chunks, note);
+  follow_reference(sm.maxima(kTeamMaxima) + 32 + lane, other_sink, chunks, note);
+  moved = __reduce_or_sync(0xffffffffu, moved);
+  if (lane == 0) {
+    *sm.rescale_mask() = moved;
+    mbar_arrive(sm.bar(kMaskReady));
+  }
+}
+
+// Phase A, one thread: the own chunks' scores.
+template <int kFormat>
+__device__ void team_qk(const Shared& sm, uint32_t tmem, int rank) {
+  volatile int* abort_flag = sm.abort_flag();
+  if (!mbar_wait(sm.bar(kReady), 0, abort_flag)) return;
+  const int chunks = sm.info(0)->chunks;
+  if (rank >= chunks || !mbar_wait(sm.bar(kQReady), 0, abort_flag)) return;
+#pragma unroll
+  for (int j = 0; j < kOwnItems; ++j) {
+    if (rank + j * kBlocks >= chunks || !mbar_wait(sm.bar(kTile0 + j), 0, abort_flag)) return;
+    tc_fence_after_sync();
+    issue_qk<kFormat>(sm, tmem, j, score_columns(j));
+    mma_commit(sm.bar(kScores0 + j));
+  }
+}
+
+// Phase B, one warp: O = P X over all chunks, this block's 128 features. The whole warp runs the loop and
+// one thread of it issues (by a predicate on the instruction), so that descriptors stay in uniform
+// registers: with a loop of one thread every instruction took 83 cycles to issue.
+template <int kFormat>
+__device__ void team_pv(const Shared& sm, uint32_t tmem) {
+  volatile int* abort_flag = sm.abort_flag();
+  const int chunks = sm.info(0)->chunks;
+  if (chunks == 0 || !warp_wait(sm.bar(kMaskReady), 0, abort_flag)) return;
+  const uint32_t issuer = (threadIdx.x & 31) == 0;
+  const uint32_t rescale_mask = __shfl_sync(0xffffffffu, *sm.rescale_mask(), 0);
+  uint32_t rescales = 0;
+  for (int i = 0; i < chunks; ++i) {
+    if ((i & 1) == 0 && !warp_wait(sm.bar(kSlices0 + i / 2), 0, abort_flag)) return;
+    if (!warp_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
+    if (rescale_mask >> i & 1) {  // some head's reference moves here: O is rescaled first
+      if (issuer) mma_commit(sm.bar(kPvDone));
+      __syncwarp();
+      if (!warp_wait(sm.bar(kRescaled), rescales++ & 1, abort_flag)) return;
+    }
+    tc_fence_after_sync();
+    const uint64_t p_desc = smem_desc_sw128(sm.base + kTeamP + i * kPBytes, 16, 1024);
+    const uint64_t x_desc = smem_desc_sw128(sm.base + kTeamSlices + i % kSliceSlots * kSliceBytes, kBlockBytes, 1024);
+#pragma unroll
+    for (int k = 0; k < kChunkRows / 16; ++k)
+      mma_ws_ss_if(issuer, tmem + kTeamO, p_desc + ((k * 32) >> 4), x_desc + ((k * 2048) >> 4), kIdescTeamPv<kFormat>, k > 0 || i > 0);
+    if (issuer && i + kSliceSlots < chunks) mma_commit(sm.bar(kSliceFree0 + i));
+    __syncwarp();
+  }
+  if (issuer) mma_commit(sm.bar(kOutput));
+}
+
+// Phase B, one thread: every own chunk's P and partial sums to the other blocks.
+__device__ void team_send(const Shared& sm, int rank) {
+  volatile int* abort_flag = sm.abort_flag();
+  const int chunks = sm.info(0)->chunks;
+  for (int item = rank; item < chunks; item += kBlocks) {
+    if (!mbar_wait(sm.bar(kP0 + item), 0, abort_flag)) return;
+    const uint32_t tile = sm.base + kTeamP + item * kPBytes, sums = sm.base + kTeamSums + item * kSumBytes;
+    for (int other = 1; other < kBlocks; ++other) {
+      const uint32_t to = uint32_t(rank + other) % kBlocks, bar = cluster_address(sm.bar(kP0 + item), to);
+      bulk_copy_to_block(cluster_address(tile, to), tile, kPBytes, bar);
+      bulk_copy_to_block(cluster_address(sums, to), sums, kSumBytes, bar);
+    }
+  }
+}
+
+// A thread's scores of own chunk `own` (as in softmax_role): 32 rows of its head.
+__device__ __forceinline__ void team_scores(uint32_t tmem, int own, unsigned live, float2 (&raw)[16]) {
+  const uint32_t s_addr = tmem + score_columns(own) + (uint32_t((threadIdx.x >> 5) * 32) << 16);
+  uint32_t low_a[16], low_b[16], high_a[16], high_b[16];
+  tmem_ld16_halves<32>(s_addr, low_a);
+  tmem_ld16_halves<32>(s_addr + 16, low_b);
+  tmem_ld16_halves<32>(s_addr + kHalfLanes + 64, high_a);
+  tmem_ld16_halves<32>(s_addr + kHalfLanes + 80, high_b);
+  tmem_wait_ld();
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    raw[e] = add_pair(make_float2(__uint_as_float(low_a[2 * e]), __uint_as_float(low_a[2 * e + 1])),
+                      make_float2(__uint_as_float(high_a[2 * e]), __uint_as_float(high_a[2 * e + 1])));
+    raw[8 + e] = add_pair(make_float2(__uint_as_float(low_b[2 * e]), __uint_as_float(low_b[2 * e + 1])),
+                          make_float2(__uint_as_float(high_b[2 * e]), __uint_as_float(high_b[2 * e + 1])));
+  }
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    if (!(live >> (2 * e) & 1u)) raw[e].x = -INFINITY;
+    if (!(live >> (2 * e + 1) & 1u)) raw[e].y = -INFINITY;
+  }
+}
+
+// Phase A, softmax warps: the own chunks' maxima to all blocks.
+__device__ __forceinline__ void team_maxima(const Params& p, const Shared& sm, uint32_t tmem, int rank) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4, head = warp * 16 + (lane & 15);
+  volatile int* abort_flag = sm.abort_flag();
+  if (!warp_wait(sm.bar(kReady), 0, abort_flag)) return;
+  const TokenInfo* info = sm.info(0);
+  const int chunks = info->chunks;
+  int own = 0;
+  for (int item = rank; item < chunks; item += kBlocks, ++own) {
+    if (!warp_wait(sm.bar(kScores0 + own), 0, abort_flag)) return;
+    tc_fence_after_sync();
+    float2 raw[16];
+    team_scores(tmem, own, half ? info->live[item].y : info->live[item].x, raw);
+    float own_max = -INFINITY, other_max = -INFINITY;
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+      own_max = max3(own_max, raw[e].x, raw[e].y);
+      other_max = max3(other_max, raw[e + 1].x, raw[e + 1].y);
+    }
+    own_max = fmaxf(own_max, other_max) * p.scale_log2;
+    const float chunk_max = fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16));
+    // Each of a head's two threads tells two blocks.
+    const uint32_t at = sm.base + kTeamMaxima + (item * kHeads + head) * 4;
+#pragma unroll
+    for (int b = 0; b < kBlocks / 2; ++b) cluster_store(cluster_address(at, half * (kBlocks / 2) + b), chunk_max);
+  }
+  tc_fence_before_sync();
+}
+
+// Phase B, softmax warps: P of the own chunks, the denominators, the output.
+template <int kFormat>
+__device__ __forceinline__ void team_softmax(const Params& p, const Shared& sm, uint32_t tmem, int token, int rank, float sink, float o_sink) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4, head = warp * 16 + (lane & 15);
+  const int o_head = (warp & 1) * 32 + lane;  // see softmax_role
+  const uint32_t o_addr = tmem + kTeamO + (uint32_t(warp * 32) << 16);
+  volatile int* abort_flag = sm.abort_flag();
+  const TokenInfo* info = sm.info(0);
+  const int chunks = info->chunks;
+  char* out = static_cast<char*>(p.out) + ((size_t)token * kHeads + o_head) * kRowBytes + rank * 256 + (warp >> 1) * 128;
+  if (chunks == 0) {  // nothing visible: the output row is zero whatever the sink
+    for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(out + u * 16) = make_uint4(0, 0, 0, 0);
+    return;
+  }
+  const volatile float* maxima = sm.maxima(kTeamMaxima);
+  int own = 0;
+  for (int item = rank; item < chunks; item += kBlocks, ++own) {
+    float run_max = sink;
+    follow_reference(maxima + head, sink, chunks, [&](int i, float reference, float) { if (i == item) run_max = reference; });
+    tc_fence_after_sync();
+    float2 prob[16];
+    team_scores(tmem, own, half ? info->live[item].y : info->live[item].x, prob);
+    const float2 scale = make_float2(p.scale_log2, p.scale_log2), reference = make_float2(-run_max, -run_max);
+    float2 sum_a = make_float2(0.f, 0.f), sum_b = sum_a;  // four partial sums
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      prob[e] = fma_pair(prob[e], scale, reference);
+      prob[e].x = exp2f(prob[e].x);
+      prob[e].y = exp2f(prob[e].y);
+      if (e & 1) sum_b = add_pair(sum_b, prob[e]); else sum_a = add_pair(sum_a, prob[e]);
+    }
+    unsigned char* tile = sm.ptr + kTeamP + item * kPBytes;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint4 v;
+      v.x = pack_pair<kFormat>(prob[4 * u + 0].x, prob[4 * u + 0].y); v.y = pack_pair<kFormat>(prob[4 * u + 1].x, prob[4 * u + 1].y);
+      v.z = pack_pair<kFormat>(prob[4 * u + 2].x, prob[4 * u + 2].y); v.w = pack_pair<kFormat>(prob[4 * u + 3].x, prob[4 * u + 3].y);
+      *reinterpret_cast<uint4*>(tile + p_offset(head, half * 4 + u)) = v;
+    }
+    reinterpret_cast<float*>(sm.ptr + kTeamSums)[(item * 2 + half) * kHeads + head] = (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
+    fence_proxy_async();  // the PV and the copies to the other blocks read the tile through the async proxy
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sm.bar(kP0 + item));
+  }
+  // The denominator: the two row halves' sums follow the reference, then add up (see softmax_role).
+  // From here on the head of this thread is that of its accumulator lane.
+  for (int i = 0; i < chunks; ++i)
+    if (!warp_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
+  float low = 1.f, high = 0.f;  // the low half's share includes the sink's own weight
+  follow_reference(maxima + o_head, o_sink, chunks, [&](int i, float, float alpha) {
+    const volatile float* sums = reinterpret_cast<const volatile float*>(sm.ptr + kTeamSums + i * kSumBytes);
+    if (i < chunks) {
+      low = low * alpha + sums[o_head];
+      high = high * alpha + sums[kHeads + o_head];
+    }
+  });
+  const float inverse = 1.f / (low + high);
+  if (!warp_wait(sm.bar(kOutput), 0, abort_flag)) return;
+  tc_fence_after_sync();
+  uint32_t o[64];
+#pragma unroll
+  for (int q = 0; q < 64; q += 16) tmem_ld16(o_addr + q, *reinterpret_cast<uint32_t(*)[16]>(&o[q]));
+  tmem_wait_ld();
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    uint4 v;
+    v.x = pack_pair<kFormat>(__uint_as_float(o[8 * u + 0]) * inverse, __uint_as_float(o[8 * u + 1]) * inverse);
+    v.y = pack_pair<kFormat>(__uint_as_float(o[8 * u + 2]) * inverse, __uint_as_float(o[8 * u + 3]) * inverse);
+    v.z = pack_pair<kFormat>(__uint_as_float(o[8 * u + 4]) * inverse, __uint_as_float(o[8 * u + 5]) * inverse);
+    v.w = pack_pair<kFormat>(__uint_as_float(o[8 * u + 6]) * inverse, __uint_as_float(o[8 * u + 7]) * inverse);
+    __stcs(reinterpret_cast<uint4*>(out + u * 16), v);
+  }
+}
+
+// Every thread passes the cluster's barrier three times: all blocks have started (their shared memory
+// may be written); all maxima are in place and all scores read (P may take the tiles' place); all
+// copies have arrived (shared memory may be given up). No role leaves before it has.
+template <int kFormat>
+__global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
+  extern __shared__ unsigned char smem_raw[];
+  Shared sm;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
+  sm.base = raw + pad;
+  sm.ptr = smem_raw + pad;
+  const int warp = threadIdx.x >> 5, rank = int(cluster_rank()), token = int(blockIdx.x) / kBlocks;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm.ptr + kSmemMisc);
+
+  if (threadIdx.x < kTeamBarCount) {
+    const int i = threadIdx.x;
+    const bool a_chunk = i >= kP0 && i < kSliceFree0, mine = a_chunk && (i - kP0) % kBlocks == rank;
+    const int count = i == kQReady ? kProducerWarps
+                    : i == kSlices0 + kSliceSlots / 2 ? kProducerThreads / 2
+                    : (i >= kTile0 && i <= kTile2) || (i >= kSlices0 && i < kP0) ? kProducerThreads
+                    : mine || i == kRescaled ? kSoftmaxWarps : 1;
+    mbar_init(sm.bar(i), count);
+    mbar_fence_init();
+    if (a_chunk && !mine) mbar_arrive_expect(sm.bar(i), kPBytes + kSumBytes);  // comes from the block that owns it
+  }
+  if (threadIdx.x == 0) { *sm.abort_flag() = 0; *sm.rescale_mask() = 0; }
+  if (warp == kMmaWarp) { tmem_alloc(smem_u32(tmem_slot), kTmemColumns); tmem_relinquish(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  prefetch_first(p, token);
+  wait_for_predecessor();
+  let_successor_start();
+  cluster_wait();
+
+  // Sinks (log2 domain), loaded early: of the thread's score head in the softmax warps, of heads lane and
+  // 32 + lane in the others.
+  const int lane = threadIdx.x & 31;
+  const float sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? warp * 16 + (lane & 15) : lane)) * 1.4426950408889634f;
+  const float other_sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? (warp & 1) * 32 : 32) + lane) * 1.4426950408889634f;
+  if (warp < kSoftmaxWarps) {
+    team_maxima(p, sm, tmem, rank);
+  } else if (warp == kMmaWarp) {
+    if ((threadIdx.x & 31) == 0) team_qk<kFormat>(sm, tmem, rank);
+  } else if (warp == kResolverWarp) {
+    publish_token(p, sm, token, 0, threadIdx.x & 31);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(sm.bar(kReady));
+  } else if (warp != kPvWarp) {
+    team_gather(p, sm, tmem, token, rank);
+  }
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (*sm.abort_flag() == 0) {
+    tc_fence_after_sync();
+    if (warp < kSoftmaxWarps) {
+      team_softmax<kFormat>(p, sm, tmem, token, rank, sink, other_sink);
+    } else if (warp == kPvWarp) {
+      team_pv<kFormat>(sm, tmem);
+    } else if (warp == kResolverWarp) {
+      if ((threadIdx.x & 31) == 0) team_send(sm, rank);
+    } else if (warp == kMmaWarp) {
+      if (sm.info(0)->chunks > 0) team_mask(sm, sink, other_sink);
+    } else {
+      team_slices(p, sm, tmem, rank);
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+    }
+  }
+  __syncwarp();
+  // (A wait has given up: what is still on its way to or from this block gets time to arrive.)
+  if (*sm.abort_flag() != 0)
+    for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  tc_fence_before_sync();
+  cluster_arrive();
+  cluster_wait();
+  if (threadIdx.x == 0 && *sm.abort_flag() != 0) report(p, kStatusWaitExpired, blockIdx.x, 0);
+  __syncthreads();
+  if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemColumns);
+}
+
+inline cudaLaunchConfig_t team_config(cudaLaunchAttribute (&attributes)[2], int tokens, cudaStream_t stream) {
+  attributes[0] = {};
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = kBlocks;
+  attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+  attributes[1] = {};
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(tokens * kBlocks));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmemBytes;
+  config.stream = stream;
+  config.attrs = attributes;
+  config.numAttrs = 2;
+  return config;
+}
+
+// How many tokens (clusters) the current device works on at a time; 0 if it cannot. Asked once per device
+// (a word that everybody sets to the same value).
+template <int kFormat>
+inline int team_capacity(int device) {
+  static int known[64] = {0};  // capacity + 1
+  if (known[device] == 0) {
+    cudaLaunchAttribute attributes[2];
+    cudaLaunchConfig_t config = team_config(attributes, 1, nullptr);
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(team_kernel<kFormat>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, team_kernel<kFormat>, &config) != cudaSuccess) {
+      cudaGetLastError();  // not on this device, then; nothing has failed
+      clusters = 0;
+    }
+    known[device] = clusters + 1;
+  }
+  return known[device] - 1;
+}
+
+// One cluster per token while all of them fit the device at once (33 on a B200); the persistent blocks
+// beyond: a second round of clusters would take longer than they do.
+template <int kFormat>
+inline int launch(const Params& p, cudaStream_t stream, int multiprocessors) {
+  int device = 0;
+  const cudaError_t error = cudaGetDevice(&device);
+  if (error != cudaSuccess) return int(error);
+  if (device < 0 || device >= 64) return -1;
+  if (p.tokens > team_capacity<kFormat>(device)) return umma::launch<kFormat>(p, stream, multiprocessors);
+  cudaLaunchAttribute attributes[2];
+  const cudaLaunchConfig_t config = team_config(attributes, p.tokens, stream);
+  return int(cudaLaunchKernelEx(&config, team_kernel<kFormat>, p));
+}
+
+}  // namespace team
+}  // namespace sparse_mla

@@ -22,6 +22,8 @@ __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepco
 // The kernel behind this one may be started (it waits by itself for this one's completion).
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+__device__ __forceinline__ void prefetch_l2(const void* at) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(at)); }
+
 // Launch `kernel` with one argument so that its start overlaps its predecessor's end.
 template <typename Kernel, typename Argument>
 inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_t shared_bytes, cudaStream_t stream, const Argument& argument) {
@@ -48,6 +50,10 @@ __device__ __forceinline__ void mbar_fence_init() {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// Arrive, and expect `bytes` of bulk copies in the current phase besides.
+__device__ __forceinline__ void mbar_arrive_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
@@ -103,6 +109,32 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 }
 __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+}
+
+// ---- clusters and distributed shared memory ------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  return rank;
+}
+// The cluster's barrier, executed by every thread of every block: first arrive, then wait.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+// Address of this block's shared-memory word `address` in the block of rank `rank`.
+__device__ __forceinline__ uint32_t cluster_address(uint32_t address, uint32_t rank) {
+  uint32_t mapped;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(mapped) : "r"(address), "r"(rank));
+  return mapped;
+}
+__device__ __forceinline__ void cluster_store(uint32_t address, float value) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(address), "f"(value) : "memory");
+}
+// Copy shared memory of this block to another block of the cluster (16-byte aligned addresses, a
+// multiple of 16 bytes); counts as `bytes` on that block's barrier.
+__device__ __forceinline__ void bulk_copy_to_block(uint32_t target, uint32_t source, uint32_t bytes, uint32_t target_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+               ::"r"(target), "r"(source), "r"(bytes), "r"(target_bar) : "memory");
 }
 
 // ---- tensor memory ---------------------------------------------------------------------------
@@ -202,6 +234,16 @@ __device__ __forceinline__ void mma_ws_ss_c(uint32_t d_tmem, uint64_t a_desc, ui
         "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
         "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc) : "memory");
   }
+}
+// The weight-stationary form for a whole warp: the lane with `issuer` set issues.
+__device__ __forceinline__ void mma_ws_ss_if(uint32_t issuer, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.b32 q, %0, 0;\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "@q tcgen05.mma.ws.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n"
+      "}\n" ::"r"(issuer), "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // Arrive on `bar` once all tcgen05.mma issued so far by this thread have completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
