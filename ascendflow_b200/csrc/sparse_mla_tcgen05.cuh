@@ -634,6 +634,26 @@ __device__ __forceinline__ float max3(float a, float b, float c) {  // one instr
   return d;
 }
 
+// The running reference of a head (log2 domain; it starts at the sink) moves to a chunk's maximum when
+// that exceeds it by more than 8 (a factor 256): the accumulator is rescaled rarely (1500 cycles, for
+// which everybody waits), probabilities stay below 2^8 and all terms of one head share the same
+// reference, which cancels in the final division. With the token's first chunk O is still empty and
+// moving is free: it then moves whenever it can, by whole powers of two, which changes no rounding.
+// (Without that a tenth of all chunks rescaled some head with a low sink.) Returns the factor of
+// what has been accumulated.
+__device__ __forceinline__ float move_reference(float& reference, float chunk_max, bool first) {
+  float alpha = 1.f;
+  if (chunk_max > reference + 8.f) {
+    alpha = exp2f(reference - chunk_max);
+    reference = chunk_max;
+  } else if (first && chunk_max > reference + 1.f) {
+    const float steps = floorf(chunk_max - reference);
+    alpha = exp2f(-steps);
+    reference += steps;
+  }
+  return alpha;
+}
+
 // Two FP32 additions / multiply-adds in one instruction.
 __device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
   float2 d;
@@ -830,22 +850,12 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         partial_max[k] = fmaxf(partial_max[k], raw[4 * k + 3].y);
       }
       const float own_max = fmaxf(fmaxf(partial_max[0], partial_max[1]), fmaxf(partial_max[2], partial_max[3])) * p.scale_log2;  // scale > 0
-      // The running maximum is that of the sink and the first chunk (moving it costs nothing while
-      // O is empty; with the sink alone a tenth of all chunks moved some head's) and from then on
-      // only moves when it is exceeded by more than 8 (a factor 256), so the accumulator is rescaled
-      // rarely (1500 cycles, for which everybody waits); probabilities stay below 2^8 and all terms
-      // of one head share the same reference, which cancels in the final division. So the two lanes of a head
-      // exchange their maxima only in the rare case: a shuffle waits in the same queue as the
-      // producers' copies, a vote does not.
+      // `move_reference` says when the running reference moves. Usually it does not, so the two lanes
+      // of a head exchange their maxima only in the rare case: a shuffle waits in the same queue as
+      // the producers' copies, a vote does not.
       float alpha = 1.f;
-      const float slack = i == 0 ? 0.f : 8.f;
-      if (__any_sync(0xffffffffu, own_max > run_max + slack)) {
-        const float chunk_max = fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16));
-        if (chunk_max > run_max + slack) {
-          alpha = exp2f(run_max - chunk_max);
-          run_max = chunk_max;
-        }
-      }
+      if (__any_sync(0xffffffffu, own_max > run_max + (i == 0 ? 1.f : 8.f)))
+        alpha = move_reference(run_max, fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16)), i == 0);
       if (i > 0) {
         // O holds earlier chunks. The factor of a head is known to the thread that has its scores;
         // the head's accumulator rows are in other threads' lanes: hand the factors over.

@@ -76,11 +76,7 @@ __device__ __forceinline__ void follow_reference(const volatile float* maxima, f
   float reference = sink;
 #pragma unroll
   for (int i = 0; i < kMaxChunks; ++i) {
-    float alpha = 1.f;
-    if (i < chunks && chunk_max[i] > reference + (i == 0 ? 0.f : 8.f)) {
-      alpha = exp2f(reference - chunk_max[i]);
-      reference = chunk_max[i];
-    }
+    const float alpha = i < chunks ? move_reference(reference, chunk_max[i], i == 0) : 1.f;
     visit(i, reference, alpha);
   }
 }
