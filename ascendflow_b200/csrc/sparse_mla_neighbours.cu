@@ -232,9 +232,9 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
 // ties going to the lower index; winners are written in ascending index order, the rest of the 512
 // entries is -1.
 //
-// Bound by memory for long rows (768 x 65536 scores: 51 us, 60 % of the copy bandwidth; the radix
+// Bound by memory for long rows (768 x 65536 scores: 45 us, 68 % of the copy bandwidth; the radix
 // select that read the row five times took 335 us) and by issue slots for many short ones (8192 x
-// 12-16 K: 127 us, 3.8 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
+// 12-16 K: 122 us, 3.8 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
 // two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the stream lists what reaches
 // the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256
@@ -265,6 +265,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   if (threadIdx.x == 0) { s.count = s.few_count = 0; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
   __syncthreads();
 
+  constexpr int kInFlight = 4;  // 16-byte loads in flight per thread of the pass over the row
+  constexpr unsigned kStep = kInFlight * 4 * kThreads, kAhead = kStep > 4096 ? kStep : 4096;
+  const unsigned end = unsigned(candidates);  // unsigned: a step may reach past INT32_MAX
+
   // ---- floor ----------------------------------------------------------------------------------
   unsigned floor_key = 0;  // short rows: everything is listed
   constexpr int kListed = 4 * kThreads > 1024 ? 4 * kThreads : 1024;  // (listing 8 K scores costs more than sampling them)
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     for (int q = 0; q < kMostQuads; ++q)
       if (q < quads) v[q] = __ldg(reinterpret_cast<const float4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
     // The row's head on its way to L2 behind the sample, while the floor is found.
-    if (threadIdx.x == 0) prefetch_l2(row, min(unsigned(candidates) * 4u & ~15u, 65536u));
+    if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kAhead));
     uint32_t key[4 * kMostQuads];
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q) {
@@ -329,9 +333,11 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
     return;
   }
-  constexpr int kInFlight = 4;  // 16-byte loads in flight per thread
-  const unsigned end = unsigned(candidates);  // unsigned: a step may reach past INT32_MAX
-  for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kInFlight * 4 * kThreads) {
+  // What lies kAhead scores (16 KiB) further on is on its way to L2 meanwhile: a block's own loads are
+  // not in flight while it looks at what they brought (768 x 65536 scores: 51.1 -> 45.0 us, 1800 x 65536:
+  // 105 -> 89; 12 and 32 KiB: 46.1, and 64 KiB at the row's head alone, 51.1).
+  for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
+    if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
     float4 v[kInFlight];
 #pragma unroll
     for (int h = 0; h < kInFlight; ++h) {
