@@ -234,7 +234,7 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
 //
 // Bound by memory for long rows (768 x 65536 scores: 45 us, 68 % of the copy bandwidth; the radix
 // select that read the row five times took 335 us) and by issue slots for many short ones (8192 x
-// 12-16 K: 122 us, 3.8 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
+// 12-16 K: 120 us, 3.9 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
 // two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the stream lists what reaches
 // the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256
@@ -242,7 +242,7 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
 // of winning positions gives the output order. The list holds every score that reaches the
 // floor, so the result is exact whenever the list has at least TopK entries and did not
 // overflow; otherwise (hardly ever, unless most of the row is equal) `select_row_by_digits`.
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
   using Shared = SelectShared<kThreads, kCapacity>;
   constexpr int kWindow = Shared::kWindow;
@@ -251,7 +251,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int token = blockIdx.x;
   sm100::wait_for_predecessor();
-  sm100::let_successor_start();
+  // Many rows: blocks of the next launch come when these end. Waiting beside them they take the slots
+  // of SMs that got fewer rows, and so spread their own unevenly (600 x 16 K: 19.3 against 16.4 us).
+  if constexpr (kThreads >= 512) sm100::let_successor_start();
   const int candidates = int(min((int64_t)visible_compressed_rows(p, token, lane), p.span));
   int32_t* list = p.out + (size_t)token * kTopK;
   const float* row = p.scores + (size_t)token * p.span;
@@ -265,7 +267,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   if (threadIdx.x == 0) { s.count = s.few_count = 0; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
   __syncthreads();
 
-  constexpr int kInFlight = 4;  // 16-byte loads in flight per thread of the pass over the row
+  // kInFlight: 16-byte loads in flight per thread of the pass over the row
+  static_assert(kInFlight <= 8, "a word of signs");
   constexpr unsigned kStep = kInFlight * 4 * kThreads, kAhead = kStep > 4096 ? kStep : 4096;
   const unsigned end = unsigned(candidates);  // unsigned: a step may reach past INT32_MAX
 
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       const unsigned i = first + h * kThreads * 4;
       v[h] = i < end ? __ldcs(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    // The sign of score - floor, shifted in: bit 15 - (4 h + e) is clear where the score reaches it.
+    // The sign of score - floor, shifted in: bit 4 (kInFlight - 1 - h) + 3 - e is clear where the score reaches it.
     unsigned below = 0;
 #pragma unroll
     for (int h = 0; h < kInFlight; ++h) {
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       below = __funnelshift_l(__float_as_uint(v[h].z - floor_value), below, 1);
       below = __funnelshift_l(__float_as_uint(v[h].w - floor_value), below, 1);
     }
-    unsigned hits = ~below & 0xffffu;
+    unsigned hits = ~below & (0xffffffffu >> (32 - 4 * kInFlight));
     if (first + (kInFlight - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
 #pragma unroll
       for (int h = 0; h < kInFlight; ++h) {
@@ -541,9 +544,9 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads>;
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight>;
   constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity>));
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
@@ -584,12 +587,14 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
   // with thirty-two; of 65536: 11 us against 15). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
-  // more than a wave of them (8192 rows of 12-16 K scores: 127 us against 144 with eight warps, which
+  // more than a wave of them (8192 rows of 12-16 K scores: 120 us against 144 with eight warps, which
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
-  // 38) or where the row needs the larger sample.
+  // 38) or where the row needs the larger sample. Eight loads in flight per thread need one block fewer per
+  // SM: better where a row has several steps (1800 x 32 K: 59.5 -> 54.0 us; 4000 x 4 K: 42.7 -> 43.4).
   if (SPAN > 131072) return launch_select<1024, 8192, 1, 2>(p, s);
   if (T <= multiprocessors) return launch_select<512, 4096, 2, 2>(p, s);
-  if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768) return launch_select<128, 2048, 9, 4>(p, s);
+  if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
+    return SPAN <= 8192 ? launch_select<128, 2048, 9, 4>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
   return launch_select<256, 2560, 6, 2>(p, s);
 }
 

@@ -139,7 +139,9 @@ def test_gpu_selection_over_long_rows(max_seq, ratio):
     (19, (512, 513, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
     # 1024-thread blocks: listed whole (4096), the list (8192), one step (16384), more than a window of winners
     (7, (4096, 4097, 8193, 16385, 131073, 200001, 150000)),
-    # 128-thread blocks: the list (2048), one step (2048), the window of winners (32768), the longest
+    # 128-thread blocks, rows of at most 8192 scores: the list and one step (2048)
+    (1900, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 6143, 8191, 8192)),
+    # 128-thread blocks, longer rows: the list (2048), one step (4096), the window of winners (32768), the longest
     (1800, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 8191, 16385, 32767, 32768)),
 ])
 def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
