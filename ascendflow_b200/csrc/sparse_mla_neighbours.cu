@@ -519,6 +519,8 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
                                     int page_rows, int32_t* status, volatile int32_t* flag) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
+  sm100::wait_for_predecessor();
+  sm100::let_successor_start();
   for (int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; token < tokens; token += warps) {
     int lo = 0, hi = batches;  // invariant: cu[lo] <= token < cu[hi]
     while (hi - lo > 1) {
@@ -605,11 +607,10 @@ int launch_sparse_mla_cache_append_flagged(void* stream, void* arg_new_rows, voi
   if (PAGE_ROWS != 64 && PAGE_ROWS != 128) return -1;
   if (B > INT32_MAX || T > INT32_MAX || PAGES > INT32_MAX || BLOCKS > INT32_MAX / kPage) return -1;
   const int64_t blocks = (T + 7) / 8;  // eight warps = eight rows per block
-  cache_append_kernel<<<int(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const char*>(arg_new_rows), static_cast<char*>(arg_cache), static_cast<const int32_t*>(arg_block_table),
-      static_cast<const int32_t*>(arg_cu_seqlens_q), static_cast<const int32_t*>(arg_seqused_kv), int(B), int(T), int(PAGES),
-      int(BLOCKS), int(PAGE_ROWS), static_cast<int32_t*>(status_words), static_cast<volatile int32_t*>(flag));
-  return int(cudaGetLastError());
+  return int(sm100::launch_overlapped(cache_append_kernel, int(blocks), 256, 0, static_cast<cudaStream_t>(stream),
+                                      static_cast<const char*>(arg_new_rows), static_cast<char*>(arg_cache), static_cast<const int32_t*>(arg_block_table),
+                                      static_cast<const int32_t*>(arg_cu_seqlens_q), static_cast<const int32_t*>(arg_seqused_kv), int(B), int(T), int(PAGES),
+                                      int(BLOCKS), int(PAGE_ROWS), static_cast<int32_t*>(status_words), static_cast<volatile int32_t*>(flag)));
 }
 
 int launch_sparse_mla_cache_append(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,

@@ -24,9 +24,9 @@ __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcon
 
 __device__ __forceinline__ void prefetch_l2(const void* at) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(at)); }
 
-// Launch `kernel` with one argument so that its start overlaps its predecessor's end.
-template <typename Kernel, typename Argument>
-inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_t shared_bytes, cudaStream_t stream, const Argument& argument) {
+// Launch `kernel` so that its start overlaps its predecessor's end.
+template <typename Kernel, typename... Arguments>
+inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_t shared_bytes, cudaStream_t stream, const Arguments&... arguments) {
   cudaLaunchAttribute overlap = {};
   overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -37,7 +37,7 @@ inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_
   config.stream = stream;
   config.attrs = &overlap;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, argument);
+  return cudaLaunchKernelEx(&config, kernel, arguments...);
 }
 
 // ---- mbarrier -----------------------------------------------------------------------------
