@@ -38,3 +38,32 @@ def test_search_finds_the_request_of_every_token(requests):
     resolved = ops.resolve_rows(*(torch.from_numpy(np.ascontiguousarray(data[n])).cuda() for n in names),
                                 ori_blocks=requests * pages, cmp_blocks=requests * pages, cmp_page=64)
     assert np.array_equal(resolved.cpu().numpy(), O.resolve_rows(data, policy))
+
+
+@pytest.mark.parametrize("requests", [1, 2, 31, 32, 33, 64, 1025])
+def test_append_and_selection_find_the_request_of_every_token(requests):
+    """The cache append, and the selection of few rows, whose lanes load a request's scalars with the probe."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    rng = np.random.default_rng(requests)
+    counts = np.zeros(requests, dtype=np.int64)
+    counts[rng.choice(requests, min(requests, 40), replace=False)] = rng.integers(1, 3, min(requests, 40))
+    tokens, pages = int(counts.sum()), 8
+    cu = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    lengths = np.maximum(counts, rng.integers(1, pages * 128 + 1, requests)).astype(np.int32)
+    table = rng.permutation(requests * pages).reshape(requests, pages).astype(np.int32)
+    used = int(table.max()) + 1
+    cache, rows = np.zeros((used, 128, 1, 512), dtype=np.int16), rng.integers(-32768, 32768, (tokens, 512)).astype(np.int16)
+    on_gpu = lambda array: torch.from_numpy(np.ascontiguousarray(array)).cuda()
+    device_cache = on_gpu(cache).view(torch.bfloat16)
+    status = neighbours.cache_append(on_gpu(rows).view(torch.bfloat16), device_cache, on_gpu(table), on_gpu(cu), on_gpu(lengths))
+    assert tuple(status) == (0,) * 8
+    assert np.array_equal(device_cache.view(torch.int16).cpu().numpy(), O.append_rows(cache, rows, table, cu, lengths))
+
+    data = {"cu_seqlens_q": cu, "seqused_ori_kv": lengths, "seqused_cmp_kv": lengths, "cmp_residual_kv": np.zeros(requests, dtype=np.int32)}
+    policy = O.make_policy(requests, tokens, ratio=1, max_seq=pages * 128, blocks=8)
+    scores = rng.normal(size=(tokens, pages * 128)).astype(np.float32)
+    selected = neighbours.topk_indices(on_gpu(scores), on_gpu(cu), on_gpu(lengths), on_gpu(data["cmp_residual_kv"]), ratio=1)
+    assert np.array_equal(selected.cpu().numpy(), O.select_topk_indices(scores, data, policy))
