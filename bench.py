@@ -48,11 +48,11 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # count, since traffic is Q + O + gathered rows per token. The figures belong to the kernel
 # sources whose hash is recorded with them: a line measured with other sources says so.
 MEASURED_TRAFFIC = {
-    "prefill": {"bytes_per_token": 1078.24e6 / 8192, "profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md"},
+    "prefill": {"bytes_per_token": 1075.76e6 / 8192, "profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md"},
     # decode: one-pass captures of the full-size calls (768 / 384 / 96 query tokens per launch)
-    "decode": {"bytes_per_token": 503.43e6 / 768, "profile": "profiles/attention_kernel_decode_dram_traffic.md",
-               "per_launch": {768: 503.43e6, 384: 245.31e6, 96: 58.76e6}},
-    "attention_kernel_sha256": "cf219b2916c73021fcc7b13f2ccb3d2f10457042d5341a70c42cd3ad2728e22b",
+    "decode": {"bytes_per_token": 500.34e6 / 768, "profile": "profiles/attention_kernel_decode_dram_traffic.md",
+               "per_launch": {768: 500.34e6, 384: 242.30e6, 96: 58.77e6}},
+    "attention_kernel_sha256": "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3",
 }
 EXTRA_WORKLOADS = ("prefill_q32k_ctx32k", "decode_b64_q6_ctx128k", "decode_b128_q6_ctx128k")
 CONFIG_KEYS = {"heads": 64, "features": 512, "topk": 512, "window": 128, "ratio": 2, "values": "N(0,1)",
