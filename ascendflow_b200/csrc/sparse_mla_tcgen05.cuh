@@ -501,6 +501,16 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   }
 }
 
+// Wait for copies announced by `cp_async_arrive`, then make them visible to the async proxy. cp.async writes
+// through the generic proxy and the barrier orders it for generic readers only; the tensor core reads
+// operands through the async proxy. The copying threads cannot fence (they do not wait for their
+// copies), so the thread that issues the product does: one instruction per tile.
+__device__ __forceinline__ bool wait_for_copies(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (!mbar_wait(bar, parity, abort_flag)) return false;
+  fence_proxy_async();
+  return true;
+}
+
 // ---- MMA warp (one thread) --------------------------------------------------------------------
 
 // Compile-time unrolled issue loops: every operand offset and accumulate flag is an immediate,
@@ -580,7 +590,7 @@ __device__ void qk_role(const Params& p, const Shared& sm, uint32_t tmem) {
       const uint32_t stage = chunk_count % kStages;
       // One barrier says both that the tile has landed and that the single score buffer is free
       // (the softmax warps have read the previous chunk out of it).
-      if (!mbar_wait(sm.bar(kKvFull0 + stage), (chunk_count / kStages) & 1, abort_flag)) return;
+      if (!wait_for_copies(sm.bar(kKvFull0 + stage), (chunk_count / kStages) & 1, abort_flag)) return;
       tc_fence_after_sync();
       issue_qk<kFormat>(sm, tmem, stage);
       mma_commit(sm.bar(kSFull));

@@ -199,7 +199,7 @@ __device__ void team_qk(const Shared& sm, uint32_t tmem, int rank) {
   if (rank >= chunks || !mbar_wait(sm.bar(kQReady), 0, abort_flag)) return;
 #pragma unroll
   for (int j = 0; j < kOwnItems; ++j) {
-    if (rank + j * kBlocks >= chunks || !mbar_wait(sm.bar(kTile0 + j), 0, abort_flag)) return;
+    if (rank + j * kBlocks >= chunks || !wait_for_copies(sm.bar(kTile0 + j), 0, abort_flag)) return;
     tc_fence_after_sync();
     issue_qk<kFormat>(sm, tmem, j, score_columns(j));
     mma_commit(sm.bar(kScores0 + j));
@@ -218,7 +218,7 @@ __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   const uint32_t rescale_mask = __shfl_sync(0xffffffffu, *sm.rescale_mask(), 0);
   uint32_t rescales = 0;
   for (int i = 0; i < chunks; ++i) {
-    if ((i & 1) == 0 && !warp_wait(sm.bar(kSlices0 + i / 2), 0, abort_flag)) return;
+    if ((i & 1) == 0 && !__all_sync(0xffffffffu, wait_for_copies(sm.bar(kSlices0 + i / 2), 0, abort_flag))) return;
     if (!warp_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
     if (rescale_mask >> i & 1) {  // some head's reference moves here: O is rescaled first
       if (issuer) mma_commit(sm.bar(kPvDone));

@@ -99,8 +99,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // ---- proxies and tcgen05 ordering ------------------------------------------------------------
 
-// Make this thread's earlier generic-proxy shared memory writes visible to the async proxy
-// (tcgen05.mma operand reads, TMA).
+// Make generic-proxy shared memory writes that happened before (this thread's own, and those that a
+// barrier has ordered before it) visible to the async proxy (tcgen05.mma operand reads, TMA).
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 }
