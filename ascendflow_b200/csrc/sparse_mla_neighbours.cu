@@ -54,7 +54,7 @@ __device__ __forceinline__ Request request_of(const int32_t* cu, int batches, in
       begin = __ldg(cu + probe);
       if (ahead) { end = __ldg(cu + probe + 1); a = __ldg(first + probe); b = __ldg(second + probe); }
     }
-    const int winner = 31 - __clz(__ballot_sync(0xffffffffu, begin <= token));  // lane 0 probes cu[lo]: always set
+    const int winner = 31 - __clz(__ballot_sync(0xffffffffu, begin <= token) | 1u);  // a token before cu[0] counts to the first request
     lo += winner * step;
     if (ahead) {
       begin = __shfl_sync(0xffffffffu, begin, winner);

@@ -198,14 +198,14 @@ __device__ __forceinline__ TokenGeometry token_geometry_warp(const Params& p, in
     const int step = (hi - lo + 31) >> 5;
     const int probe = lo + lane * step;
     const bool below = probe < hi && __ldg(p.cu + probe) <= token;
-    const unsigned mask = __ballot_sync(0xffffffffu, below);  // lane 0 probes cu[lo]: always set
+    const unsigned mask = __ballot_sync(0xffffffffu, below) | 1u;  // a token before cu[0] counts to the first request
     lo += (31 - __clz(mask)) * step;
     hi = min(hi, lo + step);
   }
   const int mine = min(lo + lane, hi - 1);
   const int my_begin = __ldg(p.cu + mine), my_end = __ldg(p.cu + mine + 1);
   const int my_length = __ldg(p.seq_ori + mine), my_available = __ldg(p.seq_cmp + mine), my_residual = __ldg(p.residual + mine);
-  const int found = 31 - __clz(__ballot_sync(0xffffffffu, lo + lane < hi && my_begin <= token));
+  const int found = 31 - __clz(__ballot_sync(0xffffffffu, lo + lane < hi && my_begin <= token) | 1u);
   const int begin = __shfl_sync(0xffffffffu, my_begin, found), end = __shfl_sync(0xffffffffu, my_end, found);
   const int length = __shfl_sync(0xffffffffu, my_length, found), available = __shfl_sync(0xffffffffu, my_available, found);
   const int residual = __shfl_sync(0xffffffffu, my_residual, found);

@@ -67,3 +67,38 @@ def test_append_and_selection_find_the_request_of_every_token(requests):
     scores = rng.normal(size=(tokens, pages * 128)).astype(np.float32)
     selected = neighbours.topk_indices(on_gpu(scores), on_gpu(cu), on_gpu(lengths), on_gpu(data["cmp_residual_kv"]), ratio=1)
     assert np.array_equal(selected.cpu().numpy(), O.select_topk_indices(scores, data, policy))
+
+
+@pytest.mark.parametrize("requests", [1, 2, 33, 1100])
+def test_tokens_in_front_of_the_first_request_count_to_it(requests):
+    """`cu_seqlens_q` need not start at 0: the binary search of the search's contract ends at request 0."""
+    import torch
+
+    from ascendflow_b200 import neighbours, ops
+
+    front, length, pages = 5, 300, 4
+    tokens = front + requests
+    cu = front + np.arange(requests + 1, dtype=np.int32)
+    table = np.random.default_rng(1).permutation(requests * pages).reshape(requests, pages).astype(np.int32)
+    of = np.maximum(0, np.arange(tokens) - front)                       # request of every token
+    position = length - 1 + np.minimum(0, np.arange(tokens) - front)    # last row it sees, its own
+    on_gpu = lambda array: torch.from_numpy(np.ascontiguousarray(array)).cuda()  # noqa: E731
+    lengths, zeros = np.full(requests, length, dtype=np.int32), np.zeros(requests, dtype=np.int32)
+
+    none = np.full((tokens, 1, 512), -1, dtype=np.int32)
+    resolved = ops.resolve_rows(*map(on_gpu, (none, table, table, cu, lengths, lengths, zeros, np.zeros((tokens, 1), dtype=np.int32))),
+                                ori_blocks=requests * pages, cmp_blocks=requests * pages, cmp_page=128).cpu().numpy()
+    window = position[:, None] - 127 + np.arange(128)
+    assert np.array_equal(resolved[:, :128], table[of[:, None], window // 128] * 128 + window % 128)
+
+    rows = np.random.default_rng(2).integers(-32768, 32768, (tokens, 512)).astype(np.int16)
+    cache = torch.zeros((requests * pages, 128, 1, 512), dtype=torch.bfloat16, device="cuda")
+    status = neighbours.cache_append(on_gpu(rows).view(torch.bfloat16), cache, on_gpu(table), on_gpu(cu), on_gpu(lengths))
+    assert tuple(status) == (0,) * 8
+    written = cache.view(-1, 512).view(torch.int16).cpu().numpy()
+    assert np.array_equal(written[table[of, position // 128] * 128 + position % 128], rows)
+
+    scores = np.random.default_rng(3).normal(size=(tokens, 512)).astype(np.float32)
+    selected = neighbours.topk_indices(on_gpu(scores), on_gpu(cu), on_gpu(lengths), on_gpu(zeros), ratio=1).cpu().numpy()
+    for token in range(tokens):
+        assert np.array_equal(selected[token, 0], np.where(np.arange(512) <= position[token], np.arange(512), -1))
