@@ -88,6 +88,9 @@ __device__ __forceinline__ void load_keys(const float* row, int i, int candidate
 }
 
 constexpr int kSelectBins = 256;
+// The longest row. Loops over a row reach up to one of their steps past its end: signed ones step by 4 K scores,
+// all others count unsigned (the windows of winners step by 64 K).
+constexpr int kMostSpan = INT32_MAX - 8192;
 
 // Shared memory of one selecting block.
 template <int kThreads, int kCapacity>
@@ -159,6 +162,7 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
   constexpr int kWarps = kThreads / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kStep = kThreads * 4;
+  static_assert(kMostSpan <= INT32_MAX - 2 * kStep, "signed positions");
   if (threadIdx.x == 0) { prefix_key = 0; wanted = kTopK; }
   for (int digit = 3; digit >= 0; --digit) {
     const int shift = digit * 8;
@@ -476,7 +480,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   // A bitmap of winning positions and the number of winners before each of its words: every winner
   // finds its place in the output by itself.
   unsigned written = 0;
-  for (int window = 0; window < candidates; window += kWindow) {
+  static_assert(uint64_t(kMostSpan) + kWindow <= UINT32_MAX, "unsigned positions");
+  for (unsigned window = 0; window < end; window += kWindow) {
     if (window > 0) {
       for (int i = threadIdx.x; i < kWindow / 32; i += kThreads) s.bitmap[i] = 0;
       __syncthreads();
@@ -492,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       }
     }
     __syncthreads();
-    const int words = (min(candidates - window, kWindow) + 31) / 32;
+    const int words = int(min(end - window, unsigned(kWindow)) + 31) / 32;
     // Eight words (32 bytes) per thread: threads beyond the words have none.
     static_assert(kWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
     const int first = threadIdx.x * 8;
@@ -588,7 +593,7 @@ extern "C" {
 int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_seqlens_q, void* arg_seqused_cmp_kv,
                                    void* arg_cmp_residual_kv, void* arg_cmp_sparse_indices, int64_t B, int64_t T,
                                    int64_t SPAN, int64_t CMP_PAGE) {
-  if (B <= 0 || T <= 0 || SPAN <= 0 || B > INT32_MAX || T > INT32_MAX || SPAN > INT32_MAX - 8192 || SPAN % 4 != 0) return -1;
+  if (B <= 0 || T <= 0 || SPAN <= 0 || B > INT32_MAX || T > INT32_MAX || SPAN > kMostSpan || SPAN % 4 != 0) return -1;
   if (CMP_PAGE != 64 && CMP_PAGE != 128) return -1;
   SelectParams p = {};
   p.scores = static_cast<const float*>(arg_scores);

@@ -228,3 +228,44 @@ def test_gpu_append_matches_the_oracle_byte_for_byte():
     status = neighbours.cache_append(as_bf16(new), device_cache, torch.from_numpy(table).cuda(),
                                      torch.from_numpy(cu).cuda(), torch.from_numpy(bad).cuda())
     assert status[0] == 1 and status[1] == sum(lens) - 1
+
+
+def selection_steps(source):
+    """The type and the step of the loop over the windows of winners, from the kernel's source."""
+    import re
+
+    kind, step = re.search(r"for \((\w+) window = 0; window < \w+; window \+= (\w+)\)", source).groups()
+    return kind, {"kWindow": 65536}[step]
+
+
+def test_windows_of_winners_end_on_the_longest_row():
+    """The last window of the longest accepted row starts below 2^31 and ends above: the position behind it must
+    not come out negative (the loop would not end)."""
+    from pathlib import Path
+
+    kind, step = selection_steps((Path(__file__).resolve().parents[1] / "ascendflow_b200/csrc/sparse_mla_neighbours.cu").read_text())
+    longest = 2**31 - 1 - 8192
+    behind = (longest - 1) // step * step + step
+    wrapped = behind - 2**32 if kind == "int" and behind >= 2**31 else behind % 2**32
+    assert wrapped >= longest
+
+
+@pytest.mark.gpu
+def test_gpu_selection_over_the_longest_row():
+    """2^31 - 8196 scores (8.6 GB). The sampled head of the row holds high scores, so that the list is short and
+    its winners are put in order window by window, up to the row's end."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    span = 2**31 - 1 - 8192 - 3
+    scores = torch.empty((1, span), dtype=torch.float32, device="cuda").normal_()
+    generator = torch.Generator(device="cuda")
+    generator.manual_seed(3)
+    for first, count in ((0, 900), (span // 2 + 5000, 300), (span - 70000, 300), (span - 300, 300)):
+        scores[0, first:first + count] = 100 + torch.rand(count, device="cuda", generator=generator)
+    i32 = lambda *values: torch.tensor(values, dtype=torch.int32, device="cuda")  # noqa: E731
+    actual = neighbours.topk_indices(scores, i32(0, 1), i32(span), i32(0), ratio=1)[0, 0].long()
+    places = torch.cat([torch.arange(first, first + count) for first, count in ((0, 900), (span // 2 + 5000, 300), (span - 70000, 300), (span - 300, 300))]).cuda()
+    order = torch.argsort(scores[0, places], descending=True, stable=True)   # ties: the lower index
+    assert torch.equal(actual, places[order[:512]].sort().values)
