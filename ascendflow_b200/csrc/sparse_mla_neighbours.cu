@@ -17,7 +17,8 @@
 namespace sparse_mla {
 namespace {
 
-// Monotone map of a finite FP32 value to an unsigned key: larger value, larger key.
+// Monotone map of an FP32 value to an unsigned key: larger value, larger key. NaNs lie beyond the infinities,
+// on the side that their sign says.
 __device__ __forceinline__ uint32_t score_key(float value) {
   const uint32_t bits = __float_as_uint(value);
   return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
@@ -123,7 +124,7 @@ __device__ __forceinline__ unsigned warp_scan(unsigned value, int lane) {
 }
 
 // The bin in which the running count over the histogram reaches `wanted`, what lies before it and
-// what it holds (s.bin stays as it was if the whole histogram holds fewer). Clears the histogram.
+// what it holds (s.bin is kSelectBins if the whole histogram holds fewer). Clears the histogram.
 // One warp does it, eight bins per lane. Called by the whole block after a barrier; ends with one.
 template <typename Shared>
 __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
@@ -137,7 +138,9 @@ __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) mine += count[i];
     unsigned before = warp_scan(mine, threadIdx.x) - mine;
-    if (before < wanted && wanted <= before + mine) {
+    const bool here = before < wanted && wanted <= before + mine;
+    if (!__any_sync(0xffffffffu, here)) s.bin = kSelectBins;
+    if (here) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         if (before < wanted && wanted <= before + count[i]) { s.bin = threadIdx.x * 8 + i; s.before = before; s.in_bin = count[i]; }
@@ -352,8 +355,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   }
 
   // ---- one pass over the row --------------------------------------------------------------------
-  // Scores that reach the floor are listed in any order. (Subnormals are flushed in what follows:
-  // a floor among them would not tell them and the zeros apart.)
+  // Scores that reach the floor are listed in any order, and NaNs, whatever their sign: those with a
+  // sign have the lowest keys of all and do not count below. (Subnormals are flushed in what follows: a
+  // floor among them would not tell them and the zeros apart.)
   const float floor_value = floor_key == 0 ? -INFINITY : __uint_as_float(floor_key & 0x80000000u ? floor_key ^ 0x80000000u : ~floor_key);
   if ((__float_as_uint(floor_value) & 0x7f800000u) == 0) {
     select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
@@ -437,11 +441,15 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       const uint2 entry = s.list[i];
       const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
       const unsigned value = ties == 0xffffffffu ? distance : entry.x;
-      if ((unsigned long long)value >> above == prefix && (ties == 0xffffffffu || distance == ties))
+      if ((unsigned long long)value >> above == prefix && (ties == 0xffffffffu || distance == ties) && key >= floor_key)
         atomicAdd(&s.histogram[value >> shift & (kSelectBins - 1)], 1u);
     }
     __syncthreads();
     find_bin(s, wanted);
+    if (s.bin == kSelectBins) {  // fewer than TopK of the list are as high as the floor: the rest are NaNs with a sign
+      select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
+      return;
+    }
     prefix = prefix << (above - shift) | s.bin;
     if (prefix == 0 && !exact && ties == 0xffffffffu) {
       find_extremes();
@@ -463,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   for (int i = threadIdx.x; i < listed; i += kThreads) {
     const uint2 entry = s.list[i];
     const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
-    if (ties == 0xffffffffu ? distance >> shift == prefix : distance == ties && entry.x >> shift == prefix)
+    if (key >= floor_key && (ties == 0xffffffffu ? distance >> shift == prefix : distance == ties && entry.x >> shift == prefix))
       s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~key << 32 | entry.x;
   }
   __syncthreads();

@@ -269,3 +269,56 @@ def test_gpu_selection_over_the_longest_row():
     places = torch.cat([torch.arange(first, first + count) for first, count in ((0, 900), (span // 2 + 5000, 300), (span - 70000, 300), (span - 300, 300))]).cuda()
     order = torch.argsort(scores[0, places], descending=True, stable=True)   # ties: the lower index
     assert torch.equal(actual, places[order[:512]].sort().values)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,span", [(1800, 14336), (320, 65536), (19, 16384), (7, 150000)])  # 128, 256, 512 and 1024 threads
+def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
+    """NaNs above and below the infinities by their sign, masks of -inf and of the lowest finite value, more and
+    fewer of them than are selected."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    rng = np.random.default_rng(span)
+    scores = rng.normal(size=(tokens, span)).astype(np.float32)
+    bits = scores.view(np.uint32)
+    for token in range(tokens):
+        few, many = rng.choice(span, 300, replace=False), rng.choice(span, 2000, replace=False)
+        kind = token % 10
+        if kind == 9:                                 # NaNs with a sign next to the floor, in order of their keys
+            scores[token] = np.finfo(np.float32).min
+            bits[token, many] = 0xFF800001
+            scores[token, few] = rng.normal(size=300) * 1e37
+        elif kind == 0:
+            bits[token, many] = 0xFFC00000            # more NaNs with a sign than the list has room for beside the winners
+        elif kind == 1:                               # few winners above the sample's floor, NaNs with a sign beside them
+            first = int(rng.integers(0, span - 700))
+            scores[token, first:first + 400] += 50.0
+            bits[token, many[:700]] = 0xFFFFFFFF
+        elif kind == 2:
+            bits[token, few] = 0x7FC00000
+            bits[token, many] = 0xFFC00001
+        elif kind == 3:
+            bits[token, many] = 0x7F800001 + np.arange(2000, dtype=np.uint32) % 7
+        elif kind == 4:                               # nearly everything is masked: the threshold is a mask
+            scores[token, np.setdiff1d(np.arange(span), few)] = -np.inf
+        elif kind == 5:
+            scores[token, np.setdiff1d(np.arange(span), many)] = np.finfo(np.float32).min
+        elif kind == 6:
+            scores[token] = -np.inf
+            bits[token, few] = 0xFFC00000
+        elif kind == 7:
+            bits[token] = 0xFFC00000
+            scores[token, many[:600]] = 1.0
+        else:
+            scores[token, many] = np.inf
+    device = lambda array: torch.from_numpy(np.ascontiguousarray(array)).cuda()  # noqa: E731
+    lengths = np.full(tokens, span, dtype=np.int32)
+    actual = neighbours.topk_indices(device(scores), device(np.arange(tokens + 1, dtype=np.int32)), device(lengths),
+                                     device(np.zeros(tokens, dtype=np.int32)), ratio=1).cpu().numpy()[:, 0]
+    for token in range(tokens):
+        key = np.where(bits[token] >> 31, ~bits[token], bits[token] | 0x80000000)
+        threshold = np.sort(key)[-512]
+        above, equal = np.flatnonzero(key > threshold), np.flatnonzero(key == threshold)
+        assert np.array_equal(actual[token], np.sort(np.concatenate([above, equal[:512 - len(above)]])))
