@@ -10,7 +10,9 @@
 
 #include <Python.h>
 
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/core/Tensor.h>
+#include <ATen/core/grad_mode.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -167,13 +169,18 @@ void sparse_mla_op(const at::Tensor& q, const at::Tensor& ori_kv, const at::Tens
   Py_DECREF(result);
 }
 
-// The output is written in place: its version counts up, as for any in-place operation.
+// The output is written in place: its version counts up, as for any in-place operation. The op has no gradient. Plain autograd leaves the output without one, but
+// functorch's transforms would take what they track for a constant and return zeros: refused.
 void sparse_mla_mutates(const at::Tensor& q, const at::Tensor& ori_kv, const at::Tensor& cmp_kv, const at::Tensor& indices,
                         const at::Tensor& ori_table, const at::Tensor& cmp_table, const at::Tensor& cu, const at::Tensor& seq_ori,
                         const at::Tensor& seq_cmp, const at::Tensor& residual, const at::Tensor& topk_length,
                         const at::Tensor& sinks, at::Tensor& out) {
   static const auto op =
       c10::Dispatcher::singleton().findSchemaOrThrow("ascendflow_b200::sparse_mla", "").typed<decltype(sparse_mla_op)>();
+  if (const auto& functorch = at::functorch::functorchTLSAccessor(); functorch != nullptr && at::GradMode::is_enabled())
+    for (const at::Tensor* tensor : std::initializer_list<const at::Tensor*>{&q, &ori_kv, &cmp_kv, &indices, &ori_table, &cmp_table, &cu,
+                                                                             &seq_ori, &seq_cmp, &residual, &topk_length, &sinks, &out})
+      if (tensor->defined() && tensor->requires_grad()) functorch->checkSupportsCppAutogradFunction();  // throws inside a transform
   {
     at::AutoDispatchBelowADInplaceOrView below;
     op.call(q, ori_kv, cmp_kv, indices, ori_table, cmp_table, cu, seq_ori, seq_cmp, residual, topk_length, sinks, out);

@@ -1,0 +1,40 @@
+"""The native host side where there is no device: what the registered op does with tensors of other backends and
+under torch's transforms, and whose errors the functions raise."""
+
+import pytest
+import torch
+
+from ascendflow_b200 import ops  # noqa: F401  (registers the op)
+
+
+def arguments(device):
+    shapes = [(4, 64, 512), (8, 128, 1, 512), (8, 64, 1, 512), (4, 1, 512), (2, 3), (2, 3), (3,), (2,), (2,), (2,), (4, 1), (64,), (4, 64, 512)]
+    types = [torch.bfloat16] * 3 + [torch.int32] * 8 + [torch.float32, torch.bfloat16]
+    return [torch.empty(shape, dtype=dtype, device=device) for shape, dtype in zip(shapes, types)]
+
+
+op = torch.ops.ascendflow_b200.sparse_mla
+
+
+@pytest.mark.parametrize("tracked", [0, 12])  # q; the output
+def test_op_cannot_be_differentiated_by_functorch(tracked):
+    def loss(factor):
+        call = arguments("meta")
+        call[tracked] = call[tracked] * factor
+        op(*call)
+        return call[12].sum()
+
+    with pytest.raises(RuntimeError):
+        torch.func.grad(loss)(torch.ones((), dtype=torch.bfloat16, device="meta"))
+
+
+def test_op_is_a_constant_to_functorch_where_nothing_of_it_is_tracked():
+    def loss(factor):
+        op(*arguments("meta"))
+        with torch.no_grad():
+            call = arguments("meta")
+            call[0] = call[0] * factor
+            op(*call)
+        return factor * 2
+
+    assert torch.func.grad(loss)(torch.ones((), device="meta")).shape == ()
