@@ -169,7 +169,8 @@ void sparse_mla_op(const at::Tensor& q, const at::Tensor& ori_kv, const at::Tens
   Py_DECREF(result);
 }
 
-// The output is written in place: its version counts up, as for any in-place operation. The op has no gradient. Plain autograd leaves the output without one, but
+// The output is written in place: its version counts up, as for any in-place operation (a tensor made in
+// inference mode has none). The op has no gradient. Plain autograd leaves the output without one, but
 // functorch's transforms would take what they track for a constant and return zeros: refused.
 void sparse_mla_mutates(const at::Tensor& q, const at::Tensor& ori_kv, const at::Tensor& cmp_kv, const at::Tensor& indices,
                         const at::Tensor& ori_table, const at::Tensor& cmp_table, const at::Tensor& cu, const at::Tensor& seq_ori,
@@ -185,7 +186,7 @@ void sparse_mla_mutates(const at::Tensor& q, const at::Tensor& ori_kv, const at:
     at::AutoDispatchBelowADInplaceOrView below;
     op.call(q, ori_kv, cmp_kv, indices, ori_table, cmp_table, cu, seq_ori, seq_cmp, residual, topk_length, sinks, out);
   }
-  torch::autograd::increment_version(out);
+  if (out.defined() && !out.is_inference()) torch::autograd::increment_version(out);
 }
 
 TORCH_LIBRARY(ascendflow_b200, m) {

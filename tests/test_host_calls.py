@@ -38,3 +38,15 @@ def test_op_is_a_constant_to_functorch_where_nothing_of_it_is_tracked():
         return factor * 2
 
     assert torch.func.grad(loss)(torch.ones((), device="meta")).shape == ()
+
+
+def test_op_writes_outputs_made_in_inference_mode():
+    call = arguments("meta")
+    with torch.inference_mode():
+        call[12] = torch.empty_like(call[0])
+    op(*call)                                    # outside of inference mode
+    with torch.inference_mode():
+        op(*call)
+    normal = arguments("meta")
+    op(*normal)
+    assert normal[12]._version == 1
