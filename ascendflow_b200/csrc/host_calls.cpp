@@ -126,7 +126,8 @@ at::Tensor workspace_for(const c10::cuda::CUDAStream& stream) {
 // Launches an accepted call on the current stream. -1000: not accepted, nothing enqueued.
 constexpr int kRefused = -1000;
 int attention(const Tensors& t) {
-  if (launch_attention == nullptr) return kRefused;
+  // (Nothing is asked of the CUDA runtime for tensors that are elsewhere: there may be no device.)
+  if (launch_attention == nullptr || !t[kQ]->defined() || !t[kQ]->is_cuda()) return kRefused;
   const c10::DeviceIndex device = c10::cuda::current_device();
   Sizes s;
   if (!accepted(t, device, &s)) return kRefused;
@@ -233,8 +234,9 @@ PyObject* call_select(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
   HANDLE_TH_ERRORS
   std::array<const at::Tensor*, 4> t;
   if (count != 6 || launch_select == nullptr || !tensors_of(arguments, &t) || !PyLong_CheckExact(arguments[4])) Py_RETURN_NONE;
-  const long ratio = PyLong_AsLong(arguments[4]);
-  if (ratio == -1 && PyErr_Occurred()) return nullptr;
+  int overflow = 0;
+  const long ratio = PyLong_AsLongAndOverflow(arguments[4], &overflow);
+  if (overflow != 0 || !t[0]->is_cuda()) Py_RETURN_NONE;
   const c10::DeviceIndex device = c10::cuda::current_device();
   if ((ratio != 1 && ratio != 2) || !plain(*t[0], at::kFloat, device) || t[0]->dim() != 2) Py_RETURN_NONE;
   for (int i = 1; i < 4; ++i)
@@ -325,7 +327,7 @@ int append_and_wait(int device, cudaStream_t stream, void* const (&p)[5], int64_
 PyObject* call_append(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
   HANDLE_TH_ERRORS
   std::array<const at::Tensor*, 5> t;
-  if (count != 5 || launch_append == nullptr || !tensors_of(arguments, &t)) Py_RETURN_NONE;
+  if (count != 5 || launch_append == nullptr || !tensors_of(arguments, &t) || !t[0]->is_cuda()) Py_RETURN_NONE;
   const c10::DeviceIndex device = c10::cuda::current_device();
   const at::ScalarType type = t[0]->scalar_type();
   if ((type != at::kBFloat16 && type != at::kHalf) || !plain(*t[0], type, device) || !plain(*t[1], type, device)) Py_RETURN_NONE;

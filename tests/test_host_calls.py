@@ -4,7 +4,8 @@ under torch's transforms, and whose errors the functions raise."""
 import pytest
 import torch
 
-from ascendflow_b200 import ops  # noqa: F401  (registers the op)
+from ascendflow_b200 import host, neighbours, ops
+from ascendflow_b200.diagnostics import CompileError
 
 
 def arguments(device):
@@ -50,3 +51,18 @@ def test_op_writes_outputs_made_in_inference_mode():
     normal = arguments("meta")
     op(*normal)
     assert normal[12]._version == 1
+
+
+@pytest.mark.parametrize("device", ["cpu", "meta"])
+def test_tensors_elsewhere_get_the_front_ends_error(device):
+    """Also once the native side is connected, and on a machine without a device."""
+    host.connect()
+    with pytest.raises(CompileError, match="CUDA tensor"):
+        ops.sparse_mla(*arguments(device))
+    i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=device)  # noqa: E731
+    for ratio in (1, 2, 1 << 70):
+        with pytest.raises(CompileError, match="CUDA tensor"):
+            neighbours.topk_indices(torch.empty((2, 8), device=device), i32(2), i32(1), i32(1), ratio=ratio)
+    rows, cache = (torch.empty(shape, dtype=torch.bfloat16, device=device) for shape in ((2, 512), (2, 128, 1, 512)))
+    with pytest.raises(CompileError, match="CUDA tensors"):
+        neighbours.cache_append(rows, cache, i32(1, 2), i32(2), i32(1))
