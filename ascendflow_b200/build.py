@@ -68,41 +68,55 @@ HOST_LIBRARY = PACKAGE / "lib" / "_host_calls.so"
 HOST_STAMP = HOST_LIBRARY.with_suffix(".stamp")
 
 
-def _host_command():
+HOST_FLAGS = ("-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden")
+HOST_LINKED = ("-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lcudart")
+
+
+def _host_command(output):
     """How the native host side is compiled: a CPython module against this interpreter's torch."""
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension
 
-    flags = ["-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden",
-             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    abi = f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"
     includes = [f"-I{path}" for path in (*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"])]
     libraries = [f"-L{path}" for path in cpp_extension.library_paths("cuda")]
-    return [os.environ.get("CXX", "g++"), *flags, *includes, "-o", str(HOST_LIBRARY), str(HOST_SOURCE), *libraries,
-            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lcudart"]
+    return [os.environ.get("CXX", "g++"), *HOST_FLAGS, abi, *includes, "-o", str(output), str(HOST_SOURCE), *libraries, *HOST_LINKED]
 
 
 def _host_identity():
+    """What the command is made of. (Not the compiler's path: a built file is carried to machines that have another.)"""
     import sys
 
     import torch
 
-    digest = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    parts = (torch.__version__, torch.__file__, sys.version, *HOST_FLAGS, *HOST_LINKED)
+    digest = hashlib.sha256("\n".join(parts).encode())
     for path in (HOST_SOURCE, ROOT / "include" / "sparse_mla.h"):
         digest.update(path.read_bytes())
     return digest.hexdigest()
 
 
 def build_host_library(force=False):
-    """Compile the native host side when its source, the header or torch changed; return its path."""
+    """Compile the native host side when its source, the header, the command or torch changed; return its path.
+
+    Built on import, so possibly by several ranks at a time: each compiles to a name of its own and
+    moves the file into place, where another may be loading the one before."""
     identity = _host_identity()
     if not force and HOST_LIBRARY.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text() == identity:
         return HOST_LIBRARY
     HOST_LIBRARY.parent.mkdir(parents=True, exist_ok=True)
-    result = subprocess.run(_host_command(), capture_output=True, text=True)
-    require(result.returncode == 0, "building the native host side failed:\n" + result.stderr[-4000:], kind=ErrorKind.RESOURCE)
-    HOST_STAMP.write_text(identity)
+    built = HOST_LIBRARY.with_name(f"{HOST_LIBRARY.stem}.{os.getpid()}.tmp.so")
+    try:
+        result = subprocess.run(_host_command(built), capture_output=True, text=True)
+        require(result.returncode == 0, "building the native host side failed:\n" + result.stderr[-4000:], kind=ErrorKind.RESOURCE)
+        os.replace(built, HOST_LIBRARY)
+    finally:
+        built.unlink(missing_ok=True)
+    stamp = HOST_STAMP.with_name(f"{HOST_STAMP.name}.{os.getpid()}")
+    stamp.write_text(identity)
+    os.replace(stamp, HOST_STAMP)
     return HOST_LIBRARY
 
 

@@ -66,3 +66,26 @@ def test_tensors_elsewhere_get_the_front_ends_error(device):
     rows, cache = (torch.empty(shape, dtype=torch.bfloat16, device=device) for shape in ((2, 512), (2, 128, 1, 512)))
     with pytest.raises(CompileError, match="CUDA tensors"):
         neighbours.cache_append(rows, cache, i32(1, 2), i32(2), i32(1))
+
+
+def test_host_library_is_identified_by_its_command_and_replaced_as_a_whole(tmp_path, monkeypatch):
+    from ascendflow_b200 import build
+
+    identity = build._host_identity()
+    monkeypatch.setattr(build, "HOST_FLAGS", ("-O0", *build.HOST_FLAGS[1:]))
+    assert build._host_identity() != identity
+
+    library = tmp_path / "_host_calls.so"
+    library.write_bytes(b"in use by another rank")
+    inode = library.stat().st_ino
+    monkeypatch.setattr(build, "HOST_LIBRARY", library)
+    monkeypatch.setattr(build, "HOST_STAMP", library.with_suffix(".stamp"))
+    monkeypatch.setenv("CXX", str(tmp_path / "compiler"))
+    (tmp_path / "compiler").write_text("#!/bin/sh\nwhile [ \"$1\" != -o ]; do shift; done\necho built > \"$2\"\n")
+    (tmp_path / "compiler").chmod(0o755)
+    with open(library, "rb") as loaded:
+        assert build.build_host_library() == library
+        assert loaded.read() == b"in use by another rank"   # the file that was there is untouched
+    assert library.read_bytes() == b"built\n" and library.stat().st_ino != inode
+    assert build.HOST_STAMP.read_text() == build._host_identity()
+    assert sorted(path.name for path in tmp_path.iterdir()) == ["_host_calls.so", "_host_calls.stamp", "compiler"]
