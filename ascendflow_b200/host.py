@@ -5,6 +5,9 @@ registered torch op.
 been enqueued, and the Python front end (`runtime/`) finds out why. Until `connect()` has given
 it the kernel library's entry points it refuses everything, so that the first call of a process goes
 through the front end, which builds or verifies that library.
+
+Where the module cannot be had (a torch without CUDA, no compiler) the package still imports and traces:
+a stand-in refuses everything, and `connect()`, on the way of every call with CUDA tensors, says why.
 """
 
 from __future__ import annotations
@@ -16,6 +19,7 @@ import importlib.util
 import torch  # noqa: F401  (its libraries are what the module links against)
 
 from .build import build_host_library
+from .diagnostics import CompileError
 
 
 def _load():
@@ -26,7 +30,39 @@ def _load():
     return module
 
 
-calls = _load()
+class _Unavailable:
+    """Refuses every call; registers the op for tracing, with calls that go through the front end."""
+
+    def __init__(self, error):
+        self.error = error
+
+    def configure(self, attention, select, append, fallback):
+        if not hasattr(self, "registration"):
+            self.registration = torch.library.Library("ascendflow_b200", "DEF")
+            self.registration.define(SCHEMA, tags=(torch.Tag.pt2_compliant_tag,))
+            self.registration.impl("sparse_mla", fallback, "CUDA")
+
+    def sparse_mla(self, *tensors):
+        return False
+
+    def topk_indices(self, *arguments):
+        return None
+
+    def cache_append(self, *arguments):
+        return None
+
+    def release_workspaces(self):
+        pass
+
+
+SCHEMA = ("sparse_mla(Tensor q, Tensor ori_kv, Tensor cmp_kv, Tensor cmp_sparse_indices, Tensor ori_block_table, "
+          "Tensor cmp_block_table, Tensor cu_seqlens_q, Tensor seqused_ori_kv, Tensor seqused_cmp_kv, "
+          "Tensor cmp_residual_kv, Tensor ori_topk_length, Tensor sinks, Tensor(a12!) attention_out) -> ()")
+
+try:
+    calls = _load()
+except (CompileError, ImportError, OSError) as error:
+    calls = _Unavailable(error)
 _fallback = None
 _connected = False
 
@@ -43,6 +79,8 @@ def connect():
     global _connected
     if _connected:
         return
+    if isinstance(calls, _Unavailable):
+        raise RuntimeError("the native host side is not available") from calls.error
     from .build import library_path
     from .runtime.torch import _library
 

@@ -47,7 +47,8 @@ def kernel(name="sparse_mla"):
 
 def _checked(*tensors):
     """The call through the Python front end."""
-    host.connect()
+    if tensors[0].is_cuda:
+        host.connect()
     kernel("sparse_mla_f16" if tensors[0].dtype == torch.float16 else "sparse_mla")(*tensors)
 
 

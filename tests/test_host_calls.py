@@ -68,6 +68,45 @@ def test_tensors_elsewhere_get_the_front_ends_error(device):
         neighbours.cache_append(rows, cache, i32(1, 2), i32(2), i32(1))
 
 
+def test_package_imports_and_traces_where_the_native_module_cannot_be_built(tmp_path):
+    """A copy of the package on a machine with no compiler and nothing built: as with a torch without CUDA."""
+    import os
+    import shutil
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parents[1]
+    shutil.copytree(root / "ascendflow_b200", tmp_path / "ascendflow_b200", ignore=shutil.ignore_patterns("lib", "__pycache__"))
+    shutil.copytree(root / "include", tmp_path / "include")
+    program = """
+import torch
+from ascendflow_b200 import host, neighbours, ops
+from ascendflow_b200.diagnostics import CompileError
+shapes = [(4, 64, 512), (8, 128, 1, 512), (8, 64, 1, 512), (4, 1, 512), (2, 3), (2, 3), (3,), (2,), (2,), (2,), (4, 1), (64,), (4, 64, 512)]
+types = [torch.bfloat16] * 3 + [torch.int32] * 8 + [torch.float32, torch.bfloat16]
+make = lambda device: [torch.empty(s, dtype=t, device=device) for s, t in zip(shapes, types)]
+call = make("meta")
+torch.ops.ascendflow_b200.sparse_mla(*call)
+for function, arguments in ((neighbours.topk_indices, (call[11],) * 4), (neighbours.cache_append, call[:5])):
+    try:
+        function(*arguments)
+    except CompileError:
+        continue
+    raise SystemExit("not refused")
+try:
+    host.connect()
+except RuntimeError as error:
+    assert "not available" in str(error) and error.__cause__ is not None
+else:
+    raise SystemExit("connected")
+print("imported")
+"""
+    result = subprocess.run([sys.executable, "-c", program], cwd=tmp_path, capture_output=True, text=True,
+                            env=dict(os.environ, CXX="/bin/false", PYTHONPATH=str(tmp_path)))
+    assert result.stdout.strip().endswith("imported"), result.stderr[-2000:]
+
+
 def test_host_library_is_identified_by_its_command_and_replaced_as_a_whole(tmp_path, monkeypatch):
     from ascendflow_b200 import build
 
