@@ -266,9 +266,18 @@ PyObject* call_select(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
   END_HANDLE_TH_ERRORS
 }
 
+// Allocations in a call that may run while another thread (or this one) captures a stream.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // What one running append needs: the kernel's status block (device, all zero between calls) and a
 // word of host memory that the kernel sets when it has written one. A call holds a pair until its
-// stream has been waited for, so the pool grows to the number of calls that run at the same time.
+// stream has been waited for, so there are as many as calls run at the same time, at most kMostWorkspaces of
+// them kept. Blocks are cleared on the stream of the call that has them, and that stream is waited for before
+// another call gets them: a plain cudaMemset runs on the default stream, for which others do not wait.
 struct AppendStatus {
   int device;
   int32_t* words;        // device
@@ -278,7 +287,7 @@ struct AppendStatus {
 std::mutex append_mutex;
 std::vector<AppendStatus>* append_pool = new std::vector<AppendStatus>;
 
-cudaError_t take_append_status(int device, AppendStatus* s) {
+cudaError_t take_append_status(int device, cudaStream_t stream, AppendStatus* s) {
   {
     std::lock_guard<std::mutex> lock(append_mutex);
     for (size_t i = 0; i < append_pool->size(); ++i)
@@ -288,9 +297,10 @@ cudaError_t take_append_status(int device, AppendStatus* s) {
         return cudaSuccess;
       }
   }
+  const RelaxedCapture relaxed;
   void *words = nullptr, *flag = nullptr, *flag_on_device = nullptr;
   cudaError_t error = cudaMalloc(&words, kWorkspaceBytes);
-  if (error == cudaSuccess) error = cudaMemset(words, 0, kWorkspaceBytes);
+  if (error == cudaSuccess) error = cudaMemsetAsync(words, 0, kWorkspaceBytes, stream);
   if (error == cudaSuccess) error = cudaHostAlloc(&flag, 64, cudaHostAllocMapped | cudaHostAllocPortable);
   if (error == cudaSuccess) error = cudaHostGetDevicePointer(&flag_on_device, flag, 0);
   if (error != cudaSuccess) {
@@ -303,22 +313,32 @@ cudaError_t take_append_status(int device, AppendStatus* s) {
   return cudaSuccess;
 }
 
+void free_append_status(const AppendStatus& s) {
+  const RelaxedCapture relaxed;
+  cudaFree(s.words);
+  cudaFreeHost(const_cast<int32_t*>(s.flag));
+}
+
 // Launch, wait for the stream, read the status: the status block only travels when there is one.
 int append_and_wait(int device, cudaStream_t stream, void* const (&p)[5], int64_t batches, int64_t tokens, int64_t pages,
                     int64_t blocks, int64_t page_rows, int32_t (&words)[SPARSE_MLA_STATUS_WORDS]) {
   AppendStatus s;
-  if (cudaError_t error = take_append_status(device, &s)) return int(error);
+  if (cudaError_t error = take_append_status(device, stream, &s)) return int(error);
   std::fill(std::begin(words), std::end(words), 0);
   const int status = launch_append(stream, p[0], p[1], p[2], p[3], p[4], s.words, s.flag_on_device, batches, tokens, pages, blocks, page_rows);
   cudaError_t error = cudaStreamSynchronize(stream);
   if (error == cudaSuccess && *s.flag != 0) {
-    error = cudaMemcpy(words, s.words, sizeof(words), cudaMemcpyDeviceToHost);
-    if (error == cudaSuccess) error = cudaMemset(s.words, 0, kWorkspaceBytes);
+    error = cudaMemcpyAsync(words, s.words, sizeof(words), cudaMemcpyDeviceToHost, stream);
+    if (error == cudaSuccess) error = cudaMemsetAsync(s.words, 0, kWorkspaceBytes, stream);
+    if (error == cudaSuccess) error = cudaStreamSynchronize(stream);
     *s.flag = 0;
   }
   if (error == cudaSuccess) {  // (after an error the pair is left alone)
-    std::lock_guard<std::mutex> lock(append_mutex);
-    append_pool->push_back(s);
+    std::unique_lock<std::mutex> lock(append_mutex);
+    const bool kept = append_pool->size() < kMostWorkspaces;
+    if (kept) append_pool->push_back(s);
+    lock.unlock();
+    if (!kept) free_append_status(s);
   }
   return status != 0 ? status : int(error);
 }
@@ -364,8 +384,16 @@ PyObject* configure(PyObject*, PyObject* arguments) {
 }
 
 PyObject* release_workspaces(PyObject*, PyObject*) {
-  std::lock_guard<std::mutex> lock(workspace_mutex);
-  workspaces->clear();
+  {
+    std::lock_guard<std::mutex> lock(workspace_mutex);
+    workspaces->clear();
+  }
+  std::vector<AppendStatus> unused;
+  {
+    std::lock_guard<std::mutex> lock(append_mutex);
+    unused.swap(*append_pool);
+  }
+  for (const AppendStatus& s : unused) free_append_status(s);
   Py_RETURN_NONE;
 }
 

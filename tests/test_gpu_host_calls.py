@@ -98,3 +98,30 @@ def test_append_reports_a_bad_page_once_and_is_clean_afterwards():
         if code:
             assert status[1:3] in ((1, 512), (2, 513))
     assert np.array_equal(cache.view(512, 512)[:, 0].float().cpu().numpy().nonzero()[0], [0, 1, 2, 509, 510, 511])
+
+
+def test_append_reports_on_side_streams_neither_stay_nor_vanish():
+    """Bad and good appends in turn on streams that do not wait for the default stream, while that one is
+    busy: each call's report is its own. Blocks are new on every other round."""
+    import torch
+
+    from ascendflow_b200 import host, neighbours
+
+    cache = torch.zeros((4, 128, 1, 512), dtype=torch.bfloat16, device="cuda")
+    rows = torch.ones((3, 512), dtype=torch.bfloat16, device="cuda")
+    cu = torch.tensor([0, 3], dtype=torch.int32, device="cuda")
+    table = torch.tensor([[0, 1, 2, 3]], dtype=torch.int32, device="cuda")
+    lengths = {code: torch.tensor([length], dtype=torch.int32, device="cuda") for code, length in ((0, 100), (1, 515))}
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    work = torch.zeros(1 << 24, device="cuda")
+    torch.cuda.synchronize()
+    for turn in range(30):
+        if turn % 2 == 0:
+            host.calls.release_workspaces()
+        for _ in range(4):
+            work.add_(1)
+        with torch.cuda.stream(streams[turn % 3]):
+            code = (turn % 5) % 2
+            status = neighbours.cache_append(rows, cache, table, cu, lengths[code])
+            assert status[0] == code
+            assert status[1:3] in ((0, 512), (1, 513), (2, 514)) if code else status == (0,) * 8
