@@ -99,9 +99,9 @@ bool accepted(const Tensors& t, int device, Sizes* s) {
   return true;
 }
 
-// One status block per device and stream, kept (and zero: no call clears it). At most kMostWorkspaces of them: a program that makes
-// streams without end gets the oldest one's memory back for the newest (the allocator holds freed
-// memory until its stream is done with it).
+// One status block per device and stream, kept (and zero: no call clears it, `read_status` does). At most
+// kMostWorkspaces of them: a program that makes streams without end gets the oldest one's memory back for the
+// newest (the allocator holds freed memory until its stream is done with it).
 constexpr size_t kWorkspaceBytes = 1024, kMostWorkspaces = 64;
 struct Workspace {
   int device;
@@ -383,6 +383,43 @@ PyObject* configure(PyObject*, PyObject* arguments) {
   Py_RETURN_NONE;
 }
 
+// The first report of the calls on the current stream since it was last read: waits for the stream, and leaves what it
+// has read zero.
+int take_report(cudaStream_t stream, void* block, int32_t (&words)[SPARSE_MLA_STATUS_WORDS]) {
+  cudaError_t error = cudaMemcpyAsync(words, block, sizeof(words), cudaMemcpyDeviceToHost, stream);
+  if (error == cudaSuccess) error = cudaStreamSynchronize(stream);
+  if (error == cudaSuccess && words[0] != 0) {
+    error = cudaMemsetAsync(block, 0, kWorkspaceBytes, stream);
+    if (error == cudaSuccess) error = cudaStreamSynchronize(stream);
+  }
+  return int(error);
+}
+
+PyObject* read_status(PyObject*, PyObject*) {
+  HANDLE_TH_ERRORS
+  int32_t words[SPARSE_MLA_STATUS_WORDS] = {};
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+  at::Tensor own;
+  {
+    std::lock_guard<std::mutex> lock(workspace_mutex);
+    for (const Workspace& w : *workspaces)
+      if (w.device == stream.device_index() && w.stream == stream.stream()) own = w.memory;
+  }
+  int status = 0;
+  {
+    pybind11::gil_scoped_release no_gil;
+    if (own.defined()) status = take_report(stream.stream(), own.mutable_data_ptr(), words);
+  }
+  if (status != 0) {
+    PyErr_Format(PyExc_RuntimeError, "status read failed with CUDA error %d; device retries are disabled", status);
+    return nullptr;
+  }
+  PyObject* result = PyTuple_New(SPARSE_MLA_STATUS_WORDS);
+  for (int i = 0; i < SPARSE_MLA_STATUS_WORDS; ++i) PyTuple_SET_ITEM(result, i, PyLong_FromLong(words[i]));
+  return result;
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* release_workspaces(PyObject*, PyObject*) {
   {
     std::lock_guard<std::mutex> lock(workspace_mutex);
@@ -402,6 +439,7 @@ PyMethodDef methods[] = {
     {"sparse_mla", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_attention)), METH_FASTCALL, nullptr},
     {"topk_indices", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_select)), METH_FASTCALL, nullptr},
     {"cache_append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_append)), METH_FASTCALL, nullptr},
+    {"read_status", read_status, METH_NOARGS, nullptr},
     {"release_workspaces", release_workspaces, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

@@ -51,6 +51,9 @@ class _Unavailable:
     def cache_append(self, *arguments):
         return None
 
+    def read_status(self):
+        raise RuntimeError("the native host side is not available") from self.error
+
     def release_workspaces(self):
         pass
 
@@ -75,10 +78,10 @@ def set_fallback(function):
 
 
 def connect():
-    """Hand the verified kernel library's entry points over, once."""
+    """Hand the verified kernel library's entry points over, once; true when they were not there before."""
     global _connected
     if _connected:
-        return
+        return False
     if isinstance(calls, _Unavailable):
         raise RuntimeError("the native host side is not available") from calls.error
     from .build import library_path
@@ -89,3 +92,4 @@ def connect():
         "launch_sparse_mla_kept_status", "launch_sparse_mla_topk_indices", "launch_sparse_mla_cache_append_flagged"))
     calls.configure(*addresses, _fallback)
     _connected = True
+    return True

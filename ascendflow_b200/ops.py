@@ -47,8 +47,8 @@ def kernel(name="sparse_mla"):
 
 def _checked(*tensors):
     """The call through the Python front end."""
-    if tensors[0].is_cuda:
-        host.connect()
+    if tensors[0].is_cuda and host.connect() and _launch(*tensors):
+        return  # the first call of the process
     kernel("sparse_mla_f16" if tensors[0].dtype == torch.float16 else "sparse_mla")(*tensors)
 
 
@@ -63,6 +63,13 @@ def sparse_mla(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block
                  cu_seqlens_q, seqused_ori_kv, seqused_cmp_kv, cmp_residual_kv, ori_topk_length,
                  sinks, attention_out)
     return attention_out
+
+
+def status():
+    """Wait for the current stream and return the first report of the calls made on it since the last
+    reading, as eight ints (word 0: 0 ok, 1 bad block-table entry, 2 an on-chip wait expired; 1 and 2: token
+    and slot)."""
+    return host.calls.read_status()
 
 
 # `torch.ops.ascendflow_b200.sparse_mla` is registered by the native module when it is loaded: no

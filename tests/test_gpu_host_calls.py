@@ -125,3 +125,35 @@ def test_append_reports_on_side_streams_neither_stay_nor_vanish():
             status = neighbours.cache_append(rows, cache, table, cu, lengths[code])
             assert status[0] == code
             assert status[1:3] in ((0, 512), (1, 513), (2, 514)) if code else status == (0,) * 8
+
+
+def with_a_bad_page(call):
+    """The call with page numbers in the first request's table that no cache has, and as it was."""
+    table = call["ori_block_table"].clone()
+    table[0, :] = 1 << 20
+    return arguments(call, ori_block_table=table), arguments(call)
+
+
+@pytest.mark.parametrize("entry", ["function", "op"])
+def test_status_reports_a_bad_page_once(call, entry):
+    import torch
+
+    from ascendflow_b200 import ops
+
+    launch = ops.sparse_mla if entry == "function" else torch.ops.ascendflow_b200.sparse_mla
+    bad, good = with_a_bad_page(call)
+    ops.status()                            # what other tests' calls on this stream have left
+    side = torch.cuda.Stream()
+    for stream in (torch.cuda.current_stream(), side):
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for arguments_, code in ((good, 0), (bad, 1), (good, 0), (bad, 1), (bad, 1)):
+                launch(*arguments_)
+                status = ops.status()
+                assert status[0] == code and len(status) == 8
+                assert ops.status() == (0,) * 8
+                assert code or status == (0,) * 8
+            launch(*bad)
+            launch(*good)
+            assert ops.status()[0] == 1     # a good call does not take a report away
+    torch.cuda.synchronize()
