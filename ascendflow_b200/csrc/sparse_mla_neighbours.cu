@@ -17,10 +17,10 @@
 namespace sparse_mla {
 namespace {
 
-// Monotone map of an FP32 value to an unsigned key: larger value, larger key. NaNs lie beyond the infinities,
-// on the side that their sign says.
-__device__ __forceinline__ uint32_t score_key(float value) {
-  const uint32_t bits = __float_as_uint(value);
+// Monotone map of an FP32 value, given by its bits, to an unsigned key: larger value, larger key. NaNs lie beyond the infinities,
+// on the side that their sign says. (Scores are loaded as words where their keys are wanted: comparing the key of
+// a float, the compiler may compare the floats, and NaNs come out wrong.)
+__device__ __forceinline__ uint32_t score_key(uint32_t bits) {
   return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
 }
 
@@ -78,19 +78,19 @@ __device__ __forceinline__ int visible_compressed_rows(const SelectParams& p, in
   return min(available, max(0, completed - request.count + (token - request.begin) + 1) / p.ratio);
 }
 
-// Four consecutive scores as keys (one 16-byte load); `span` is a multiple of four, so every row
-// starts on a 16-byte boundary and a load may run past `candidates` but never past the row.
-__device__ __forceinline__ void load_keys(const float* row, int i, int candidates, uint32_t (&key)[4], bool (&valid)[4]) {
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (i < candidates) v = __ldg(reinterpret_cast<const float4*>(row + i));
+// Four consecutive scores and their keys (one 16-byte load); `span` is a multiple of four, so every row
+// starts on a 16-byte boundary and a load may run past `end` but never past the row.
+__device__ __forceinline__ uint4 load_keys(const float* row, unsigned i, unsigned end, uint32_t (&key)[4], bool (&valid)[4]) {
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (i < end) v = __ldg(reinterpret_cast<const uint4*>(row + i));
   key[0] = score_key(v.x); key[1] = score_key(v.y); key[2] = score_key(v.z); key[3] = score_key(v.w);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) valid[e] = i + e < candidates;
+  for (int e = 0; e < 4; ++e) valid[e] = i + e < end;
+  return v;
 }
 
 constexpr int kSelectBins = 256;
-// The longest row. Loops over a row reach up to one of their steps past its end: signed ones step by 4 K scores,
-// all others count unsigned (the windows of winners step by 64 K).
+// The longest row. Loops over a row reach up to one of their steps past its end and count unsigned.
 constexpr int kMostSpan = INT32_MAX - 8192;
 
 // Shared memory of one selecting block.
@@ -101,10 +101,11 @@ struct SelectShared {
   __align__(16) unsigned bitmap[kWindow / 32];
   unsigned short place[kWindow / 32];  // winners before each word of the bitmap
   __align__(16) unsigned histogram[kSelectBins];
-  unsigned warp_sum[kThreads / 32];
+  unsigned warp_sum[2][kThreads / 32];
   unsigned count, low, high;           // candidates listed; extremes of what is being binned
   unsigned bin, before, in_bin;        // result of find_bin
   unsigned few_count;                  // entries in `few`
+  bool mass;                           // many scores of the sample equal the key below the floor
   unsigned long long few[32], limit;   // the threshold bin's entries; the last winner
 };
 
@@ -124,7 +125,8 @@ __device__ __forceinline__ unsigned warp_scan(unsigned value, int lane) {
 }
 
 // The bin in which the running count over the histogram reaches `wanted`, what lies before it and
-// what it holds (s.bin is kSelectBins if the whole histogram holds fewer). Clears the histogram.
+// what it holds. If the whole histogram holds fewer, s.bin is kSelectBins and s.before what it holds. Clears
+// the histogram.
 // One warp does it, eight bins per lane. Called by the whole block after a barrier; ends with one.
 template <typename Shared>
 __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
@@ -139,7 +141,7 @@ __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
     for (int i = 0; i < 8; ++i) mine += count[i];
     unsigned before = warp_scan(mine, threadIdx.x) - mine;
     const bool here = before < wanted && wanted <= before + mine;
-    if (!__any_sync(0xffffffffu, here)) s.bin = kSelectBins;
+    if (!__any_sync(0xffffffffu, here) && threadIdx.x == 31) { s.bin = kSelectBins; s.before = before + mine; }
     if (here) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -151,104 +153,310 @@ __device__ __forceinline__ void find_bin(Shared& s, unsigned wanted) {
   __syncthreads();
 }
 
-// The selection for any row, whatever its scores: an MSB-first radix select over the keys (four
-// 8-bit digits, one histogram per warp, one addition per warp and bin) finds the key of the
-// TopK-th highest score and how many entries equal to it are taken; one more pass in index order
-// writes the winners through a block-wide prefix count. Reads the row five times. Used where the
-// listed candidates of `topk_select_kernel` turn out to be too few or too many (masses of equal
-// scores, or scores whose sample says little about the row). Called by the whole block.
-template <int kThreads>
-__device__ __noinline__ void select_row_by_digits(const float* row, int candidates, int32_t* list, unsigned (*histogram)[256],
-                                                  unsigned* totals) {
-  __shared__ unsigned long long warp_count[kThreads / 32], base_count;
-  __shared__ unsigned prefix_key, wanted;
-  constexpr int kWarps = kThreads / 32;
+// Every candidate above `threshold`, and the first `equal_taken` of those equal to it, in index order; TopK of
+// them at most. Returns how many equal ones there were up to the last winner. Sixteen scores side by
+// side per thread and step, one barrier per step. Called by the whole block after a barrier.
+template <int kThreads, typename Shared>
+__device__ __noinline__ unsigned write_winners(Shared& s, const float* row, unsigned end, int32_t* list, unsigned threshold, unsigned equal_taken) {
+  constexpr int kPerThread = 16;
+  static_assert(kPerThread * kThreads < 65536, "two counts to a word");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kStep = kThreads * 4;
-  static_assert(kMostSpan <= INT32_MAX - 2 * kStep, "signed positions");
-  if (threadIdx.x == 0) { prefix_key = 0; wanted = kTopK; }
-  for (int digit = 3; digit >= 0; --digit) {
-    const int shift = digit * 8;
-    for (int i = threadIdx.x; i < kWarps * 256; i += kThreads) (&histogram[0][0])[i] = 0;
-    __syncthreads();
-    const unsigned prefix = prefix_key;
-    const unsigned mask = digit == 3 ? 0u : (0xffffffffu << (shift + 8));
-    for (int first = 0; first < candidates; first += kStep) {
+  unsigned greater = 0, equal = 0;  // before this step
+  for (unsigned first = 0, buffer = 0; first < end && greater + min(equal, equal_taken) < kTopK; first += kPerThread * kThreads, buffer ^= 1) {
+    const unsigned mine = first + threadIdx.x * kPerThread;
+    unsigned is_greater = 0, is_equal = 0;
+#pragma unroll
+    for (int h = 0; h < kPerThread; h += 4) {
       uint32_t key[4];
       bool valid[4];
-      load_keys(row, first + threadIdx.x * 4, candidates, key, valid);
+      load_keys(row, mine + h, end, key, valid);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const bool counted = valid[e] && (key[e] & mask) == prefix;
-        // from the second digit on, most warps hold no entry with the prefix: nothing to vote on
-        if (__ballot_sync(0xffffffffu, counted) == 0u) continue;
-        // Lanes that fall into the same bin (most of them, for the exponent digit) add once,
-        // through their lowest lane.
-        const unsigned bin = counted ? (key[e] >> shift) & 255u : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        if (counted && lane == __ffs(peers) - 1) atomicAdd(&histogram[warp][bin], unsigned(__popc(peers)));
+        is_greater |= unsigned(valid[e] && key[e] > threshold) << (h + e);
+        is_equal |= unsigned(valid[e] && key[e] == threshold) << (h + e);
       }
     }
-    __syncthreads();
-    for (int bin = threadIdx.x; bin < 256; bin += kThreads) {
-      unsigned sum = 0;
-      for (int w = 0; w < kWarps; ++w) sum += histogram[w][bin];
-      totals[bin] = sum;
+    const unsigned counts = unsigned(__popc(is_greater)) | unsigned(__popc(is_equal)) << 16;
+    const unsigned scan = warp_scan(counts, lane);
+    if (lane == 31) s.warp_sum[buffer][warp] = scan;
+    __syncthreads();  // (the other buffer is read until everybody has come here)
+    unsigned before = scan - counts, total = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      const unsigned sum = s.warp_sum[buffer][w];
+      if (w < warp) before += sum;
+      total += sum;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // walk down from the highest bin until `wanted` entries are covered
-      unsigned above = 0;
-      int bin = 255;
-      while (bin > 0 && above + totals[bin] < wanted) above += totals[bin--];
-      prefix_key = prefix | (unsigned(bin) << shift);
-      wanted -= above;  // entries still to take among those that share the longer prefix
+    unsigned greater_before = greater + (before & 0xffffu), equal_before = equal + (before >> 16);
+    for (unsigned left = is_greater | is_equal; left != 0; left &= left - 1) {
+      const int bit = __ffs(left) - 1;
+      const unsigned at = greater_before + min(equal_before, equal_taken);
+      const bool above = is_greater >> bit & 1;
+      if ((above || equal_before < equal_taken) && at < kTopK) list[at] = int32_t(mine + bit);
+      if (above) ++greater_before; else ++equal_before;
     }
-    __syncthreads();
+    greater += total & 0xffffu;
+    equal += total >> 16;
   }
-  const unsigned threshold = prefix_key, equal_taken = wanted;  // wanted >= 1
-  // Counts are packed: entries above the threshold in the low half, entries equal to it in the
-  // high half of a 64-bit word.
-  if (threadIdx.x == 0) base_count = 0;
-  __syncthreads();
-  for (int first = 0; first < candidates; first += kStep) {
-    const int i = first + threadIdx.x * 4;
-    uint32_t key[4];
-    bool valid[4];
-    load_keys(row, i, candidates, key, valid);
-    unsigned long long mine = 0;
+  return equal;
+}
+
+// For rows that the sample said too little about: a key that at least TopK candidates reach and at most
+// `most`. Or, where so many are equal that there is none, the threshold itself (`equal` of the candidates
+// equal to it are winners).
+//
+// Histograms over the whole row, 256 bins between `lower` and `upper`, then inside the bin that the
+// `wanted`-th highest key up to `upper` lies in. Keys above `upper` are TopK - wanted winners; or, if
+// `open`, any number of candidates (a sample's maximum is no maximum). One pass is the rule: scores that
+// fool the sample are few in the bins. Called by the whole block after a barrier.
+struct Floor {
+  unsigned key, equal;
+};
+template <int kThreads, typename Shared>
+__device__ __noinline__ Floor find_floor(Shared& s, const float* row, unsigned end, unsigned most, unsigned lower, unsigned upper, unsigned wanted, bool open) {
+  const int lane = threadIdx.x & 31;
+  // Six passes at most: the open range, four digits of one that holds the threshold, one that turns out not to.
+  // (Scores that change meanwhile have no TopK best, but must not keep the block.)
+  for (int pass = 0; pass < 8; ++pass) {
+    const int shift = max(0, 24 - __clz(int(upper - lower)));
+    for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += 16 * kThreads) {
+      uint32_t key[4][4];
+      bool valid[4][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (valid[e]) mine += key[e] > threshold ? 1ull : (key[e] == threshold ? (1ull << 32) : 0ull);
-    unsigned long long scan = mine;  // inclusive scan over the warp
+      for (int h = 0; h < 4; ++h) load_keys(row, first + h * 4 * kThreads, end, key[h], valid[h]);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long up = __shfl_up_sync(0xffffffffu, scan, d);
-      if (lane >= d) scan += up;
+      for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool counted = valid[h][e] && key[h][e] >= lower && (open || key[h][e] <= upper);
+          if (!__any_sync(0xffffffffu, counted)) continue;
+          // Lanes that fall into the same bin (most of them, among equal scores) add once.
+          const unsigned bin = counted ? (upper - min(key[h][e], upper)) >> shift : kSelectBins;
+          const unsigned peers = __match_any_sync(0xffffffffu, bin);
+          if (counted && lane == __ffs(peers) - 1) atomicAdd(&s.histogram[bin], unsigned(__popc(peers)));
+        }
     }
-    if (lane == 31) warp_count[warp] = scan;
     __syncthreads();
-    unsigned long long before = base_count + scan - mine;
-    for (int w = 0; w < warp; ++w) before += warp_count[w];
-    unsigned greater_before = unsigned(before), equal_before = unsigned(before >> 32);
-    // An entry equal to the threshold is a winner while fewer than `equal_taken` such entries
-    // precede it; every winner's position is the number of winners before it.
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (!valid[e]) continue;
-      if (key[e] > threshold) {
-        list[greater_before + min(equal_before, equal_taken)] = i + e;
-        ++greater_before;
-      } else if (key[e] == threshold) {
-        if (equal_before < equal_taken) list[greater_before + equal_before] = i + e;
-        ++equal_before;
+    find_bin(s, wanted);
+    if (s.bin == kSelectBins) {  // everything here is a winner, and more below
+      wanted -= s.before;
+      upper = lower - 1;
+      lower = 0;
+      open = false;
+      continue;
+    }
+    const unsigned depth = ((s.bin + 1) << shift) - 1;
+    const unsigned bottom = depth >= upper - lower ? lower : upper - depth;
+    const bool beyond = open && s.bin == 0;  // the bin goes on above `upper`
+    if (kTopK - wanted + s.before + s.in_bin <= most) return {bottom, 0};
+    if (shift == 0 && !beyond) return {bottom, wanted - s.before};
+    upper = beyond ? 0xffffffffu : upper - (s.bin << shift);
+    lower = bottom;
+    wanted -= s.before;
+    open = false;
+  }
+  return {lower, wanted};
+}
+
+// The TopK best of the `listed` entries (not more than there is room for), written in index order. False, and nothing
+// written, if fewer than TopK of them reach the floor. Called by the whole block after a barrier.
+template <int kThreads, int kCapacity, typename Shared>
+__device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int listed, unsigned floor_key, int32_t* list) {
+  constexpr int kWindow = Shared::kWindow;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // ---- the TopK best of the list ----------------------------------------------------------------
+  // Ordered by (distance of the key from the highest, row position): smaller is better, all
+  // distinct. First the distance, then (more than 32 equal scores at the threshold) the position.
+  // "The highest" is the sample's, and what lies above it counts as distance 0, until the
+  // threshold turns out to lie there.
+  unsigned top = s.high, bottom = floor_key;
+  bool exact = false;
+  auto find_extremes = [&]() {
+    unsigned low = 0xffffffffu, high = 0;
+    for (int i = threadIdx.x; i < listed; i += kThreads) {
+      const unsigned key = score_key(s.list[i].y);
+      low = min(low, key);
+      high = max(high, key);
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    if (lane == 0) { atomicMin(&s.low, low); atomicMax(&s.high, high); }
+    __syncthreads();
+    top = s.high;
+    bottom = s.low;
+    exact = true;
+  };
+  if (floor_key == 0) find_extremes();  // nothing was sampled
+  unsigned wanted = kTopK;
+  int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
+  unsigned prefix = 0;  // leading bits found so far
+  unsigned ties = 0xffffffffu;  // distance of the threshold, once the position decides
+  while (true) {
+    for (int i = threadIdx.x; i < listed; i += kThreads) {
+      const uint2 entry = s.list[i];
+      const unsigned key = score_key(entry.y), distance = top - min(key, top);
+      const unsigned value = ties == 0xffffffffu ? distance : entry.x;
+      if ((unsigned long long)value >> above == prefix && (ties == 0xffffffffu || distance == ties) && key >= floor_key)
+        atomicAdd(&s.histogram[value >> shift & (kSelectBins - 1)], 1u);
+    }
+    __syncthreads();
+    find_bin(s, wanted);
+    if (s.bin == kSelectBins) return false;  // the rest are NaNs with a sign
+    prefix = prefix << (above - shift) | s.bin;
+    if (prefix == 0 && !exact && ties == 0xffffffffu) {
+      find_extremes();
+      above = 32 - __clz(int(top - bottom));
+      shift = max(0, above - 8);
+      continue;
+    }
+    wanted -= s.before;
+    if (s.in_bin <= 32) break;
+    above = shift;
+    if (shift == 0) {  // (positions are distinct: only for the distance)
+      ties = prefix;
+      prefix = 0;
+      above = 32 - __clz(int(end - 1));
+    }
+    shift = max(0, above - 8);
+  }
+  // The threshold bin's entries side by side: the wanted-th smallest of them is the last winner.
+  for (int i = threadIdx.x; i < listed; i += kThreads) {
+    const uint2 entry = s.list[i];
+    const unsigned key = score_key(entry.y), distance = top - min(key, top);
+    if (key >= floor_key && (ties == 0xffffffffu ? distance >> shift == prefix : distance == ties && entry.x >> shift == prefix))
+      s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~key << 32 | entry.x;
+  }
+  __syncthreads();
+  const int few = int(s.few_count);  // 32 at most
+  for (int i = warp; i < few; i += kThreads / 32) {
+    const unsigned long long candidate = s.few[i];
+    const unsigned before = __popc(__ballot_sync(0xffffffffu, lane < few && s.few[lane] < candidate));
+    if (before + 1 == wanted && lane == 0) s.limit = candidate;
+  }
+  __syncthreads();
+  const unsigned long long limit = s.limit;
+
+  // ---- winners in index order ---------------------------------------------------------------------
+  // A bitmap of winning positions and the number of winners before each of its words: every winner
+  // finds its place in the output by itself.
+  unsigned written = 0;
+  static_assert(uint64_t(kMostSpan) + kWindow <= UINT32_MAX, "unsigned positions");
+  for (unsigned window = 0; window < end; window += kWindow) {
+    if (window > 0) {
+      for (int i = threadIdx.x; i < kWindow / 32; i += kThreads) s.bitmap[i] = 0;
+      __syncthreads();
+    }
+    unsigned winners = 0;  // of this thread's entries (16 at most)
+    static_assert(kCapacity <= 32 * kThreads, "a bit per entry of a thread");
+    for (int i = threadIdx.x, bit = 0; i < listed; i += kThreads, ++bit) {
+      const uint2 entry = s.list[i];
+      const unsigned index = entry.x - window;
+      if (index < kWindow && ((unsigned long long)~score_key(entry.y) << 32 | entry.x) <= limit) {
+        atomicOr(&s.bitmap[index >> 5], 1u << (index & 31));
+        winners |= 1u << bit;
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long add = 0;
-      for (int w = 0; w < kWarps; ++w) add += warp_count[w];
-      base_count += add;
+    const int words = int(min(end - window, unsigned(kWindow)) + 31) / 32;
+    // Eight words (32 bytes) per thread: threads beyond the words have none.
+    static_assert(kWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
+    const int first = threadIdx.x * 8;
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    if (first < words) a = *reinterpret_cast<const uint4*>(&s.bitmap[first]);
+    if (first + 4 < words) b = *reinterpret_cast<const uint4*>(&s.bitmap[first + 4]);
+    const unsigned counts[8] = {unsigned(__popc(a.x)), unsigned(__popc(a.y)), unsigned(__popc(a.z)), unsigned(__popc(a.w)),
+                                unsigned(__popc(b.x)), unsigned(__popc(b.y)), unsigned(__popc(b.z)), unsigned(__popc(b.w))};
+    unsigned mine = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine += counts[i];
+    const unsigned scan = warp_scan(mine, lane);
+    if (lane == 31) s.warp_sum[0][warp] = scan;
+    __syncthreads();
+    unsigned at = written + scan - mine;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) at += s.warp_sum[0][w];
+      written += s.warp_sum[0][w];
     }
+    if (first < words) {
+      unsigned packed[4];  // a count is at most 512: two to a word
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        packed[i] = at | (at + counts[2 * i]) << 16;
+        at += counts[2 * i] + counts[2 * i + 1];
+      }
+      *reinterpret_cast<uint4*>(&s.place[first]) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+    __syncthreads();
+    for (; winners != 0; winners &= winners - 1) {
+      const unsigned position = s.list[(__ffs(winners) - 1) * kThreads + threadIdx.x].x, index = position - window;
+      list[s.place[index >> 5] + __popc(s.bitmap[index >> 5] & ((1u << (index & 31)) - 1))] = position;
+    }
+    __syncthreads();  // the bitmap and the sums are free again
+  }
+  return true;
+}
+
+// What is left of `topk_select_kernel` where the list of what reaches the floor is too short or too long, or has not
+// been made (`listed`), since the floor is zero, subnormal, infinite or a NaN. All by keys, and not inline: the
+// usual row's instructions stay together.
+template <int kThreads, int kCapacity, typename Shared>
+__device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigned end, int32_t* list, unsigned floor_key, bool listed) {
+  bool fits = false;  // the floor has been found to
+  while (true) {
+    if (!listed) {
+      for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += 16 * kThreads) {
+        uint32_t key[4][4];
+        bool valid[4][4];
+        uint4 v[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) v[h] = load_keys(row, first + h * 4 * kThreads, end, key[h], valid[h]);
+        unsigned hits = 0;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) hits |= unsigned(valid[e >> 2][e & 3] && key[e >> 2][e & 3] >= floor_key) << e;
+        if (hits == 0) continue;
+        unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+        if (at + unsigned(__popc(hits)) > kCapacity) continue;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (hits >> (4 * h + e) & 1) s.list[at++] = make_uint2(first + h * 4 * kThreads + e, values[e]);
+        }
+      }
+      __syncthreads();
+      const unsigned count = s.count;
+      if (count >= kTopK && count <= kCapacity && select_from_list<kThreads, kCapacity>(s, end, int(count), floor_key, list)) return;
+      if (fits) return;  // the scores have changed since they were counted
+    }
+    Floor found;
+    const unsigned count = s.count;
+    if (count > kCapacity) {
+      found = find_floor<kThreads>(s, row, end, kCapacity, floor_key, max(s.high, floor_key), kTopK, true);
+    } else {
+      unsigned reached = 0;  // of the list, without NaNs
+      for (unsigned i = threadIdx.x; i < count; i += kThreads) reached += score_key(s.list[i].y) >= floor_key;
+      reached = __reduce_add_sync(0xffffffffu, reached);
+      if ((threadIdx.x & 31) == 0) atomicAdd(&s.few_count, reached);
+      __syncthreads();
+      unsigned missing = kTopK - s.few_count, upper = floor_key - 1, lower = min(s.low, upper);
+      if (s.mass) {
+        const unsigned equal = write_winners<kThreads>(s, row, end, list, upper, missing);
+        if (equal >= missing) return;
+        missing -= equal;
+        --upper;
+        lower = 0;
+      }
+      found = find_floor<kThreads>(s, row, end, kCapacity, lower, upper, missing, false);
+    }
+    if (found.equal != 0) {
+      write_winners<kThreads>(s, row, end, list, found.key, found.equal);
+      return;
+    }
+    floor_key = found.key;
+    fits = true;
+    listed = false;
+    __syncthreads();
+    if (threadIdx.x == 0) s.count = s.few_count = 0;
     __syncthreads();
   }
 }
@@ -267,14 +475,22 @@ __device__ __noinline__ void select_row_by_digits(const float* row, int candidat
 // bins, normally once; the few entries of the threshold's bin are ranked by comparison; a bitmap
 // of winning positions gives the output order. The list holds every score that reaches the
 // floor, so the result is exact whenever the list has at least TopK entries and did not
-// overflow; otherwise (hardly ever, unless most of the row is equal) `select_row_by_digits`.
+// overflow. Otherwise the row is gone through again, by keys (`select_by_keys`):
+//   many equal scores  (zeros behind a ReLU, masks) show in the sample as a floor that many samples are
+//                      equal to. What lies above it is listed; if that is too little, one more pass in index
+//                      order takes the first of the equal ones (`write_winners`).
+//   a sample that      (scores that change slowly along the row) is set right by `find_floor`, and the
+//   says too little    row streamed once more with a floor that is known to fit.
+// 768 x 65536 scores, against the radix select that read every row five times: constant 373 -> 55 us, zeros 383
+// -> 80, all but 300 masked 360 -> 142, correlated over 64 positions 326 -> 192 (a fifth of the rows);
+// 100 rows of the latter 114 -> 80. With that select as the way out they took 461, 433, 457, 283 and 127.
 template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
   using Shared = SelectShared<kThreads, kCapacity>;
   constexpr int kWindow = Shared::kWindow;
   extern __shared__ __align__(16) unsigned char select_smem[];
   Shared& s = *reinterpret_cast<Shared*>(select_smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const int token = blockIdx.x;
   sm100::wait_for_predecessor();
   // Many rows: blocks of the next launch come when these end. Waiting beside them they take the slots
@@ -290,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   for (int i = threadIdx.x * 4; i < min(candidates + 31, kWindow) / 32; i += kThreads * 4)
     *reinterpret_cast<uint4*>(&s.bitmap[i]) = make_uint4(0, 0, 0, 0);
   for (int i = threadIdx.x; i < kSelectBins; i += kThreads) s.histogram[i] = 0;
-  if (threadIdx.x == 0) { s.count = s.few_count = 0; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
+  if (threadIdx.x == 0) { s.count = s.few_count = 0; s.mass = false; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
   __syncthreads();
 
   // kInFlight: 16-byte loads in flight per thread of the pass over the row
@@ -308,10 +524,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     constexpr int kSegments = kThreads / 8;
     const int quads = max(1, min(kMostQuads, candidates / (32 * kThreads))), sampled = quads * kThreads;
     const unsigned step = (unsigned(candidates) >> 2) / unsigned(quads * kSegments);  // at least eight quads
-    float4 v[kMostQuads];
+    uint4 v[kMostQuads];
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q)
-      if (q < quads) v[q] = __ldg(reinterpret_cast<const float4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
+      if (q < quads) v[q] = __ldg(reinterpret_cast<const uint4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
     // The row's head on its way to L2 behind the sample, while the floor is found.
     if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kAhead));
     uint32_t key[4 * kMostQuads];
@@ -336,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     const unsigned warp_low = __reduce_min_sync(0xffffffffu, best), warp_high = __reduce_max_sync(0xffffffffu, best);
     if (lane == 0) { atomicMin(&s.low, warp_low); atomicMax(&s.high, warp_high); }
     __syncthreads();
-    unsigned lower = s.low, upper = s.high;
+    unsigned lower = s.low, upper = s.high, above = 0;  // (samples above `upper`)
     while (true) {  // normally once; again inside a bin that holds too many (a sample of both signs, say)
       const int shift = max(0, 24 - __clz(int(upper - lower)));  // 256 bins over [lower, upper]
 #pragma unroll
@@ -347,200 +563,75 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       if (s.bin == kSelectBins) break;  // fewer samples than wanted: all of them
       const unsigned depth = ((s.bin + 1) << shift) - 1;
       lower = depth >= upper - lower ? lower : upper - depth;
-      if (s.in_bin <= 32 || shift == 0) break;
+      if (s.in_bin <= 32) break;
+      if (shift == 0) {  // many are equal to the floor: what lies above it, unless all of them are likely to fit
+        above += s.before + s.in_bin;
+        if (float(above) * float(candidates) > 0.8f * kCapacity * float(4 * sampled) && lower != 0xffffffffu) {
+          ++lower;
+          if (threadIdx.x == 0) s.mass = true;
+        }
+        break;
+      }
       upper -= s.bin << shift;
       wanted -= s.before;
+      above += s.before;
     }
     floor_key = lower;
   }
 
   // ---- one pass over the row --------------------------------------------------------------------
-  // Scores that reach the floor are listed in any order, and NaNs, whatever their sign: those with a
-  // sign have the lowest keys of all and do not count below. (Subnormals are flushed in what follows: a
-  // floor among them would not tell them and the zeros apart.)
-  const float floor_value = floor_key == 0 ? -INFINITY : __uint_as_float(floor_key & 0x80000000u ? floor_key ^ 0x80000000u : ~floor_key);
-  if ((__float_as_uint(floor_value) & 0x7f800000u) == 0) {
-    select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
-    return;
-  }
-  // What lies kAhead scores (16 KiB) further on is on its way to L2 meanwhile: a block's own loads are
-  // not in flight while it looks at what they brought (768 x 65536 scores: 51.1 -> 45.0 us, 1800 x 65536:
-  // 105 -> 89; 12 and 32 KiB: 46.1, and 64 KiB at the row's head alone, 51.1).
-  for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
-    if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
-    float4 v[kInFlight];
-#pragma unroll
-    for (int h = 0; h < kInFlight; ++h) {
-      const unsigned i = first + h * kThreads * 4;
-      v[h] = i < end ? __ldcs(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    // The sign of score - floor, shifted in: bit 4 (kInFlight - 1 - h) + 3 - e is clear where the score reaches it.
-    unsigned below = 0;
-#pragma unroll
-    for (int h = 0; h < kInFlight; ++h) {
-      below = __funnelshift_l(__float_as_uint(v[h].x - floor_value), below, 1);
-      below = __funnelshift_l(__float_as_uint(v[h].y - floor_value), below, 1);
-      below = __funnelshift_l(__float_as_uint(v[h].z - floor_value), below, 1);
-      below = __funnelshift_l(__float_as_uint(v[h].w - floor_value), below, 1);
-    }
-    unsigned hits = ~below & (0xffffffffu >> (32 - 4 * kInFlight));
-    if (first + (kInFlight - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
+  // Scores that reach the floor are listed in any order, by the sign of score - floor: two instructions per
+  // score. That is no less exact than the keys but for NaNs, which are listed whatever their sign (those with one
+  // have the lowest keys of all and do not count), and for subnormals, which are flushed.
+  const unsigned floor_bits = floor_key == 0 ? 0xff800000u : floor_key & 0x80000000u ? floor_key ^ 0x80000000u : ~floor_key;
+  const unsigned exponent = floor_bits & 0x7f800000u;
+  const bool normal = floor_key == 0 || (exponent != 0 && exponent != 0x7f800000u);
+  const float floor_value = __uint_as_float(floor_bits);
+  if (normal) {
+    // What lies kAhead scores (16 KiB) further on is on its way to L2 meanwhile: a block's own loads are
+    // not in flight while it looks at what they brought (768 x 65536 scores: 51.1 -> 45.0 us, 1800 x 65536:
+    // 105 -> 89; 12 and 32 KiB: 46.1, and 64 KiB at the row's head alone, 51.1).
+    for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
+      if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
+      uint4 v[kInFlight];
 #pragma unroll
       for (int h = 0; h < kInFlight; ++h) {
-        const unsigned i = first + h * kThreads * 4, left = i < end ? min(end - i, 4u) : 0u;
-        hits &= ~((15u >> left) << (4 * (kInFlight - 1 - h)));
+        const unsigned i = first + h * kThreads * 4;
+        v[h] = i < end ? __ldcs(reinterpret_cast<const uint4*>(row + i)) : make_uint4(0, 0, 0, 0);
       }
-    }
-    if (hits == 0) continue;
-    unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
-    if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
+      // The sign of score - floor, shifted in: bit 4 (kInFlight - 1 - h) + 3 - e is clear where the score reaches it.
+      unsigned below = 0;
 #pragma unroll
-    for (int h = 0; h < kInFlight; ++h) {
-      const float values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+      for (int h = 0; h < kInFlight; ++h) {
+        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].x) - floor_value), below, 1);
+        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].y) - floor_value), below, 1);
+        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].z) - floor_value), below, 1);
+        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].w) - floor_value), below, 1);
+      }
+      unsigned hits = ~below & (0xffffffffu >> (32 - 4 * kInFlight));
+      if (first + (kInFlight - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (hits >> (4 * (kInFlight - 1 - h) + 3 - e) & 1) s.list[at++] = make_uint2(first + h * kThreads * 4 + e, __float_as_uint(values[e]));
-    }
-  }
-  __syncthreads();
-  const int listed = int(s.count);
-  if (listed < kTopK || listed > kCapacity) {
-    select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
-    return;
-  }
-
-  // ---- the TopK best of the list ----------------------------------------------------------------
-  // Ordered by (distance of the key from the highest, row position): smaller is better, all
-  // distinct. First the distance, then (more than 32 equal scores at the threshold) the position.
-  // "The highest" is the sample's, and what lies above it counts as distance 0, until the
-  // threshold turns out to lie there.
-  unsigned top = s.high, bottom = floor_key;
-  bool exact = false;
-  auto find_extremes = [&]() {
-    unsigned low = 0xffffffffu, high = 0;
-    for (int i = threadIdx.x; i < listed; i += kThreads) {
-      const unsigned key = score_key(__uint_as_float(s.list[i].y));
-      low = min(low, key);
-      high = max(high, key);
-    }
-    low = __reduce_min_sync(0xffffffffu, low);
-    high = __reduce_max_sync(0xffffffffu, high);
-    if (lane == 0) { atomicMin(&s.low, low); atomicMax(&s.high, high); }
-    __syncthreads();
-    top = s.high;
-    bottom = s.low;
-    exact = true;
-  };
-  if (floor_key == 0) find_extremes();  // nothing was sampled
-  unsigned wanted = kTopK;
-  int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
-  unsigned prefix = 0;  // leading bits found so far
-  unsigned ties = 0xffffffffu;  // distance of the threshold, once the position decides
-  while (true) {
-    for (int i = threadIdx.x; i < listed; i += kThreads) {
-      const uint2 entry = s.list[i];
-      const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
-      const unsigned value = ties == 0xffffffffu ? distance : entry.x;
-      if ((unsigned long long)value >> above == prefix && (ties == 0xffffffffu || distance == ties) && key >= floor_key)
-        atomicAdd(&s.histogram[value >> shift & (kSelectBins - 1)], 1u);
-    }
-    __syncthreads();
-    find_bin(s, wanted);
-    if (s.bin == kSelectBins) {  // fewer than TopK of the list are as high as the floor: the rest are NaNs with a sign
-      select_row_by_digits<kThreads>(row, candidates, list, reinterpret_cast<unsigned (*)[256]>(s.list), s.histogram);
-      return;
-    }
-    prefix = prefix << (above - shift) | s.bin;
-    if (prefix == 0 && !exact && ties == 0xffffffffu) {
-      find_extremes();
-      above = 32 - __clz(int(top - bottom));
-      shift = max(0, above - 8);
-      continue;
-    }
-    wanted -= s.before;
-    if (s.in_bin <= 32) break;
-    above = shift;
-    if (shift == 0) {  // (positions are distinct: only for the distance)
-      ties = prefix;
-      prefix = 0;
-      above = 32 - __clz(candidates - 1);
-    }
-    shift = max(0, above - 8);
-  }
-  // The threshold bin's entries side by side: the wanted-th smallest of them is the last winner.
-  for (int i = threadIdx.x; i < listed; i += kThreads) {
-    const uint2 entry = s.list[i];
-    const unsigned key = score_key(__uint_as_float(entry.y)), distance = top - min(key, top);
-    if (key >= floor_key && (ties == 0xffffffffu ? distance >> shift == prefix : distance == ties && entry.x >> shift == prefix))
-      s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~key << 32 | entry.x;
-  }
-  __syncthreads();
-  const int few = int(s.few_count);  // 32 at most
-  for (int i = warp; i < few; i += kThreads / 32) {
-    const unsigned long long candidate = s.few[i];
-    const unsigned before = __popc(__ballot_sync(0xffffffffu, lane < few && s.few[lane] < candidate));
-    if (before + 1 == wanted && lane == 0) s.limit = candidate;
-  }
-  __syncthreads();
-  const unsigned long long limit = s.limit;
-
-  // ---- winners in index order ---------------------------------------------------------------------
-  // A bitmap of winning positions and the number of winners before each of its words: every winner
-  // finds its place in the output by itself.
-  unsigned written = 0;
-  static_assert(uint64_t(kMostSpan) + kWindow <= UINT32_MAX, "unsigned positions");
-  for (unsigned window = 0; window < end; window += kWindow) {
-    if (window > 0) {
-      for (int i = threadIdx.x; i < kWindow / 32; i += kThreads) s.bitmap[i] = 0;
-      __syncthreads();
-    }
-    unsigned winners = 0;  // of this thread's entries (ten at most)
-    static_assert(kCapacity <= 32 * kThreads, "a bit per entry of a thread");
-    for (int i = threadIdx.x, bit = 0; i < listed; i += kThreads, ++bit) {
-      const uint2 entry = s.list[i];
-      const unsigned index = entry.x - window;
-      if (index < kWindow && ((unsigned long long)~score_key(__uint_as_float(entry.y)) << 32 | entry.x) <= limit) {
-        atomicOr(&s.bitmap[index >> 5], 1u << (index & 31));
-        winners |= 1u << bit;
+        for (int h = 0; h < kInFlight; ++h) {
+          const unsigned i = first + h * kThreads * 4, left = i < end ? min(end - i, 4u) : 0u;
+          hits &= ~((15u >> left) << (4 * (kInFlight - 1 - h)));
+        }
+      }
+      if (hits == 0) continue;
+      unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+      if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
+#pragma unroll
+      for (int h = 0; h < kInFlight; ++h) {
+        const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (hits >> (4 * (kInFlight - 1 - h) + 3 - e) & 1) s.list[at++] = make_uint2(first + h * kThreads * 4 + e, values[e]);
       }
     }
     __syncthreads();
-    const int words = int(min(end - window, unsigned(kWindow)) + 31) / 32;
-    // Eight words (32 bytes) per thread: threads beyond the words have none.
-    static_assert(kWindow / 32 <= 8 * kThreads, "eight words per thread cover the window");
-    const int first = threadIdx.x * 8;
-    uint4 a = make_uint4(0, 0, 0, 0), b = a;
-    if (first < words) a = *reinterpret_cast<const uint4*>(&s.bitmap[first]);
-    if (first + 4 < words) b = *reinterpret_cast<const uint4*>(&s.bitmap[first + 4]);
-    const unsigned counts[8] = {unsigned(__popc(a.x)), unsigned(__popc(a.y)), unsigned(__popc(a.z)), unsigned(__popc(a.w)),
-                                unsigned(__popc(b.x)), unsigned(__popc(b.y)), unsigned(__popc(b.z)), unsigned(__popc(b.w))};
-    unsigned mine = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) mine += counts[i];
-    const unsigned scan = warp_scan(mine, lane);
-    if (lane == 31) s.warp_sum[warp] = scan;
-    __syncthreads();
-    unsigned at = written + scan - mine;
-    for (int w = 0; w < kThreads / 32; ++w) {
-      if (w < warp) at += s.warp_sum[w];
-      written += s.warp_sum[w];
-    }
-    if (first < words) {
-      unsigned packed[4];  // a count is at most 512: two to a word
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        packed[i] = at | (at + counts[2 * i]) << 16;
-        at += counts[2 * i] + counts[2 * i + 1];
-      }
-      *reinterpret_cast<uint4*>(&s.place[first]) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    }
-    __syncthreads();
-    for (; winners != 0; winners &= winners - 1) {
-      const unsigned position = s.list[(__ffs(winners) - 1) * kThreads + threadIdx.x].x, index = position - window;
-      list[s.place[index >> 5] + __popc(s.bitmap[index >> 5] & ((1u << (index & 31)) - 1))] = position;
-    }
-    __syncthreads();  // the bitmap and the sums are free again
+    const int listed = int(s.count);
+    if (listed >= kTopK && listed <= kCapacity && select_from_list<kThreads, kCapacity>(s, end, listed, floor_key, list)) return;
   }
+  select_by_keys<kThreads, kCapacity>(s, row, end, list, floor_key, normal);
 }
 
 // One warp per new row: token j of n of request b goes to logical position L_b - n + j of the raw

@@ -322,3 +322,58 @@ def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
         threshold = np.sort(key)[-512]
         above, equal = np.flatnonzero(key > threshold), np.flatnonzero(key == threshold)
         assert np.array_equal(actual[token], np.sort(np.concatenate([above, equal[:512 - len(above)]])))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (19, 16384), (7, 150000)])  # 128, 128, 256, 512, 1024 threads
+def test_gpu_selection_of_rows_that_a_sample_says_little_about(tokens, span):
+    """Many equal scores at, above and below the threshold, at zero, among subnormals and at a mask; scores that
+    change slowly along the row, in both directions of a missed floor; winners the sample has not seen."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    rng = np.random.default_rng(span + tokens)
+    scores = rng.normal(size=(tokens, span)).astype(np.float32)
+    slow = np.convolve(rng.normal(size=tokens + span), np.exp(-np.arange(400) / 64), mode="same").astype(np.float32)
+    place = np.arange(span)
+    for token in range(tokens):
+        few, kind = rng.choice(span, 400, replace=False), token % 14
+        if kind == 0:
+            scores[token] = np.maximum(scores[token] - 2.9, 0)              # fewer winners than TopK above zero
+        elif kind == 1:
+            scores[token] = np.maximum(scores[token] - 0.5, 0)
+        elif kind == 2:
+            scores[token] = 0.25
+        elif kind == 3:
+            scores[token] = np.where(np.isin(place, few), scores[token], -np.inf)
+        elif kind == 4:
+            scores[token] = np.round(scores[token] * 2) + np.float32(0.0)
+        elif kind in (5, 6, 7):
+            scores[token] = slow[token:token + span] + (0.01 * scores[token] if kind == 6 else 0)
+        elif kind == 8:                                                      # the highest all in one place, away from a sample's start
+            scores[token, 40:40 + 300] = 30 + rng.random(300)
+        elif kind == 9:                                                      # far more high ones in the sampled head than elsewhere
+            scores[token, :64] = 30
+        elif kind == 10:                                                     # zeros of both signs and subnormals
+            scores[token] = np.where(np.isin(place, few), np.float32(1e-41) * (place % 5), np.float32(-0.0))
+        elif kind == 11:
+            scores[token] = np.where(place % 3 == 0, np.float32(-1e-40), np.where(place % 3 == 1, np.float32(0.0), np.float32(-1.0)))
+        elif kind == 12:                                                     # 400 above a plateau that is rare in the sample
+            scores[token] = -np.abs(scores[token])
+            scores[token, few] = 5
+            scores[token, rng.choice(span, 120, replace=False)] = 4
+        else:                                                                # ascending
+            scores[token] = np.sort(scores[token])
+    device = lambda array: torch.from_numpy(np.ascontiguousarray(array)).cuda()  # noqa: E731
+    lengths = np.full(tokens, span, dtype=np.int32)
+    lengths[::3] -= 5
+    actual = neighbours.topk_indices(device(scores), device(np.arange(tokens + 1, dtype=np.int32)), device(lengths),
+                                     device(np.zeros(tokens, dtype=np.int32)), ratio=1).cpu().numpy()[:, 0]
+    bits = scores.view(np.uint32)
+    for token in range(tokens):
+        row = bits[token, :lengths[token]]
+        key = np.where(row >> 31, ~row, row | 0x80000000)
+        threshold = np.sort(key)[-512]
+        above, equal = np.flatnonzero(key > threshold), np.flatnonzero(key == threshold)
+        assert np.array_equal(actual[token], np.sort(np.concatenate([above, equal[:512 - len(above)]]))), (token, token % 14)
