@@ -705,7 +705,10 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   int device = 0, multiprocessors = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Rows so long that a small block's sample says too little: large blocks. No more tokens than SMs: a
+  // Rows so long that a small block's sample says too little: large blocks (16 x 1 M scores: 98 us against 398
+  // with 512 threads, 300 x 1 M: 357 against 695, 16 x 200 K: 32.8 against 35.8), for many rows only beyond 256 K.
+  // Two blocks of 512 threads to an SM are better before that, and where the buffer is wide but the rows are
+  // not (600 x 200 K: 131 us against 154, 2000 rows of 2 K in a buffer of 140000: 68 against 120). No more tokens than SMs: a
   // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
   // with thirty-two; of 65536: 11 us against 15). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
@@ -713,8 +716,8 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
   // 38) or where the row needs the larger sample. Eight loads in flight per thread need one block fewer per
   // SM: better where a row has several steps (1800 x 32 K: 59.5 -> 54.0 us; 4000 x 4 K: 42.7 -> 43.4).
-  if (SPAN > 131072) return launch_select<1024, 8192, 1, 2>(p, s);
-  if (T <= multiprocessors) return launch_select<512, 4096, 2, 2>(p, s);
+  if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
+  if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
     return SPAN <= 8192 ? launch_select<128, 2048, 9, 4>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
   return launch_select<256, 2560, 6, 2>(p, s);
