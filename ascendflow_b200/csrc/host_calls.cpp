@@ -99,6 +99,13 @@ bool accepted(const Tensors& t, int device, Sizes* s) {
   return true;
 }
 
+// Allocations in a call that may run while another thread (or this one) captures a stream.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // One status block per device and stream, kept (and zero: no call clears it, `read_status` does). At most
 // kMostWorkspaces of them: a program that makes streams without end gets the oldest one's memory back for the
 // newest (the allocator holds freed memory until its stream is done with it).
@@ -123,6 +130,39 @@ at::Tensor workspace_for(const c10::cuda::CUDAStream& stream) {
   return memory;
 }
 
+// A captured launch runs whenever its graph is replayed, on any stream, for as long as the graph lives. All
+// captured launches of a device share one block (its first report counts, as everywhere), which is
+// allocated and cleared outside of the capture and never given back.
+constexpr int kMostDevices = 64;
+std::array<void*, kMostDevices> captured_blocks = {};
+
+cudaError_t captured_block(int device, void** block) {
+  if (device < 0 || device >= kMostDevices) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(workspace_mutex);
+  cudaError_t error = cudaSuccess;
+  if (captured_blocks[device] == nullptr) {
+    const RelaxedCapture relaxed;
+    cudaStream_t aside = nullptr;  // not the capturing one, and none that waits for it
+    void* memory = nullptr;
+    error = cudaStreamCreateWithFlags(&aside, cudaStreamNonBlocking);
+    if (error == cudaSuccess) error = cudaMalloc(&memory, kWorkspaceBytes);
+    if (error == cudaSuccess) error = cudaMemsetAsync(memory, 0, kWorkspaceBytes, aside);
+    if (error == cudaSuccess) error = cudaStreamSynchronize(aside);
+    if (aside != nullptr) cudaStreamDestroy(aside);
+    if (error == cudaSuccess) captured_blocks[device] = memory;
+    else if (memory != nullptr) cudaFree(memory);
+  }
+  *block = captured_blocks[device];
+  return error;
+}
+
+cudaError_t is_capturing(cudaStream_t stream, bool* capturing) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaError_t error = cudaStreamIsCapturing(stream, &status);
+  *capturing = status != cudaStreamCaptureStatusNone;
+  return error;
+}
+
 // Launches an accepted call on the current stream. -1000: not accepted, nothing enqueued.
 constexpr int kRefused = -1000;
 int attention(const Tensors& t) {
@@ -137,9 +177,14 @@ int attention(const Tensors& t) {
   for (const at::Tensor* tensor : t) c10::cuda::CUDACachingAllocator::recordStream(tensor->storage().data_ptr(), stream);
   void* p[kTensors];
   for (int i = 0; i < kTensors; ++i) p[i] = const_cast<void*>(t[i]->const_data_ptr());
-  const at::Tensor workspace = workspace_for(stream);
-  return launch_attention(stream.stream(), t[kQ]->scalar_type() == at::kHalf, p, workspace.mutable_data_ptr(), s.batches, s.tokens,
-                          s.pages, s.ori_blocks, s.cmp_blocks, s.cmp_page);
+  bool capturing = false;
+  if (const cudaError_t error = is_capturing(stream.stream(), &capturing)) return int(error);
+  at::Tensor kept;
+  void* workspace = nullptr;
+  if (!capturing) workspace = (kept = workspace_for(stream)).mutable_data_ptr();
+  else if (const cudaError_t error = captured_block(device, &workspace)) return int(error);
+  return launch_attention(stream.stream(), t[kQ]->scalar_type() == at::kHalf, p, workspace, s.batches, s.tokens, s.pages, s.ori_blocks,
+                          s.cmp_blocks, s.cmp_page);
 }
 
 // ---- the registered op -----------------------------------------------------------------------------
@@ -266,13 +311,6 @@ PyObject* call_select(PyObject*, PyObject* const* arguments, Py_ssize_t count) {
   END_HANDLE_TH_ERRORS
 }
 
-// Allocations in a call that may run while another thread (or this one) captures a stream.
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 // What one running append needs: the kernel's status block (device, all zero between calls) and a
 // word of host memory that the kernel sets when it has written one. A call holds a pair until its
 // stream has been waited for, so there are as many as calls run at the same time, at most kMostWorkspaces of
@@ -383,8 +421,8 @@ PyObject* configure(PyObject*, PyObject* arguments) {
   Py_RETURN_NONE;
 }
 
-// The first report of the calls on the current stream since it was last read: waits for the stream, and leaves what it
-// has read zero.
+// The first report of the calls on the current stream since it was last read, or else of the device's captured launches:
+// waits for the stream, and leaves what it has read zero.
 int take_report(cudaStream_t stream, void* block, int32_t (&words)[SPARSE_MLA_STATUS_WORDS]) {
   cudaError_t error = cudaMemcpyAsync(words, block, sizeof(words), cudaMemcpyDeviceToHost, stream);
   if (error == cudaSuccess) error = cudaStreamSynchronize(stream);
@@ -400,15 +438,18 @@ PyObject* read_status(PyObject*, PyObject*) {
   int32_t words[SPARSE_MLA_STATUS_WORDS] = {};
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
   at::Tensor own;
+  void* captured = nullptr;
   {
     std::lock_guard<std::mutex> lock(workspace_mutex);
     for (const Workspace& w : *workspaces)
       if (w.device == stream.device_index() && w.stream == stream.stream()) own = w.memory;
+    if (stream.device_index() < kMostDevices) captured = captured_blocks[stream.device_index()];
   }
   int status = 0;
   {
     pybind11::gil_scoped_release no_gil;
     if (own.defined()) status = take_report(stream.stream(), own.mutable_data_ptr(), words);
+    if (status == 0 && words[0] == 0 && captured != nullptr) status = take_report(stream.stream(), captured, words);
   }
   if (status != 0) {
     PyErr_Format(PyExc_RuntimeError, "status read failed with CUDA error %d; device retries are disabled", status);

@@ -68,7 +68,7 @@ def sparse_mla(q, ori_kv, cmp_kv, cmp_sparse_indices, ori_block_table, cmp_block
 def status():
     """Wait for the current stream and return the first report of the calls made on it since the last
     reading, as eight ints (word 0: 0 ok, 1 bad block-table entry, 2 an on-chip wait expired; 1 and 2: token
-    and slot)."""
+    and slot). Calls captured in CUDA graphs report per device: theirs follow when the stream has none."""
     return host.calls.read_status()
 
 

@@ -157,3 +157,31 @@ def test_status_reports_a_bad_page_once(call, entry):
             launch(*good)
             assert ops.status()[0] == 1     # a good call does not take a report away
     torch.cuda.synchronize()
+
+
+def test_captured_calls_report_and_outlive_kept_blocks(call):
+    """A first call on a capturing stream, replayed after every kept block has been given back and its memory reused."""
+    import torch
+
+    from ascendflow_b200 import host, ops
+
+    bad, good = with_a_bad_page(call)
+    ops.sparse_mla(*good)
+    expected = call["attention_out"].clone()
+    ops.status()
+    graphs = []
+    for arguments_ in (good, bad):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.sparse_mla(*arguments_)
+        graphs.append(graph)
+    host.calls.release_workspaces()
+    filled = [torch.full((1024,), 0x5A, dtype=torch.uint8, device="cuda") for _ in range(64)]
+    for graph, code in zip((graphs[0], graphs[1], graphs[0], graphs[1]), (0, 1, 0, 1)):
+        call["attention_out"].zero_()
+        graph.replay()
+        status = ops.status()
+        assert status[0] == code and (code or torch.equal(call["attention_out"], expected))
+    ops.sparse_mla(*good)
+    assert ops.status() == (0,) * 8
+    assert all(bool((block == 0x5A).all()) for block in filled)
