@@ -516,12 +516,12 @@ __device__ __forceinline__ bool wait_for_copies(uint32_t bar, uint32_t parity, v
 // Compile-time unrolled issue loops: every operand offset and accumulate flag is an immediate,
 // so the issuing thread spends a couple of instructions per MMA and stays ahead of the pipe.
 constexpr int kQkSteps = kFeatures / 32;  // K = 16 steps over one half of the features
-template <int kFormat, int K, int kEnd = kQkSteps>
+template <int kFormat, int K = 0>
 __device__ __forceinline__ void issue_qk_steps(uint32_t s_tmem, uint32_t q_tmem, uint64_t x_desc) {
-  if constexpr (K < kEnd) {
+  if constexpr (K < kQkSteps) {
     constexpr uint32_t offset = block_position(K >> 2) * kBlockBytes + (K & 3) * 32;
     mma_ts_c<K != 0>(s_tmem, q_tmem + K * 8, x_desc + (offset >> 4), kIdescQK<kFormat>);
-    issue_qk_steps<kFormat, K + 1, kEnd>(s_tmem, q_tmem, x_desc);
+    issue_qk_steps<kFormat, K + 1>(s_tmem, q_tmem, x_desc);
   }
 }
 
@@ -533,20 +533,20 @@ __device__ __forceinline__ void issue_qk_steps(uint32_t s_tmem, uint32_t q_tmem,
 // (Q_hi . X_hi); the other two quadrants mix the halves and are ignored. Half the products are
 // thrown away, but M = 128 runs at the full rate of the pipe and N = 128 is above its
 // per-instruction floor: 16 instructions of 64 cycles replace 32 of about 56.
-template <int kFormat, int kBegin = 0, int kEnd = kQkSteps>
+template <int kFormat>
 __device__ __forceinline__ void issue_qk(const Shared& sm, uint32_t tmem, int stage, uint32_t scores = kTmemS) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, 16, 1024);
-  issue_qk_steps<kFormat, kBegin, kEnd>(tmem + scores, tmem + kTmemQ, x_desc);
+  issue_qk_steps<kFormat>(tmem + scores, tmem + kTmemQ, x_desc);
 }
 
 constexpr int kPvSteps = 2 * (kChunkRows / 16);
-template <int kFormat, int I, bool kFirst, int kEnd = kPvSteps>
+template <int kFormat, int I, bool kFirst>
 __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc, uint64_t x_desc) {
-  if constexpr (I < kEnd) {
+  if constexpr (I < kPvSteps) {
     constexpr int h = I / (kChunkRows / 16), k = I % (kChunkRows / 16);
     constexpr uint32_t offset = h * kBlockBytes + k * 2048;
     mma_ws_ss_c<!(kFirst && k == 0)>(o_tmem + h * kTmemOHalf, p_desc + ((k * 32) >> 4), x_desc + (offset >> 4), kIdescPV<kFormat>);
-    issue_pv_steps<kFormat, I + 1, kFirst, kEnd>(o_tmem, p_desc, x_desc);
+    issue_pv_steps<kFormat, I + 1, kFirst>(o_tmem, p_desc, x_desc);
   }
 }
 
@@ -555,12 +555,12 @@ __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc,
 // A = P from shared memory (one 128-byte row per head, 32 bytes per K = 16 step); B = X with
 // features contiguous: the four 64-feature blocks of a half are two block positions apart,
 // 8-row groups 1024 bytes apart.
-template <int kFormat, int kBegin = 0, int kEnd = kPvSteps>
+template <int kFormat>
 __device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, bool accumulate) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, 2 * kBlockBytes, 1024);
   const uint64_t p_desc = smem_desc_sw128(sm.base + kSmemP, 16, 1024);
-  if (accumulate) issue_pv_steps<kFormat, kBegin, false, kEnd>(tmem + kTmemO, p_desc, x_desc);
-  else issue_pv_steps<kFormat, kBegin, true, kEnd>(tmem + kTmemO, p_desc, x_desc);
+  if (accumulate) issue_pv_steps<kFormat, 0, false>(tmem + kTmemO, p_desc, x_desc);
+  else issue_pv_steps<kFormat, 0, true>(tmem + kTmemO, p_desc, x_desc);
 }
 
 // Two issuing threads in two warps, one per product. Each follows its own data: the QK thread

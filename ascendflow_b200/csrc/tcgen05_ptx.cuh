@@ -67,19 +67,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return done != 0;
 }
 
-// Non-blocking test (try_wait may suspend the thread for a while before answering).
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
-}
-
 // Wait for the phase with the given parity, giving up after `limit` SM clock cycles or as soon
 // as `*abort_flag` (shared memory) is non-zero. Returns false when it gave up; the caller must
 // then leave its loop and go to the kernel's common exit.
@@ -195,24 +182,6 @@ __device__ __forceinline__ void mma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint6
         "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
   }
 }
-template <bool kAccumulate>
-__device__ __forceinline__ void mma_ss_c(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-  if constexpr (kAccumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.eq.b32 p, 0, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc) : "memory");
-  } else {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, 0, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc) : "memory");
-  }
-}
 // Weight-stationary form (tcgen05.mma.ws): with M = 64 the accumulator spreads over all 128
 // tensor-memory lanes (lanes 0-63 hold rows 0-63 x columns [0, N/2), lanes 64-127 hold the same
 // rows x columns [N/2, N); N/2 tensor-memory columns), and the instruction runs at 80 % of the
@@ -273,12 +242,6 @@ __device__ __forceinline__ void tmem_ld16_halves(uint32_t taddr, uint32_t (&r)[1
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr), "n"(kSplit) : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
