@@ -469,8 +469,8 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
 // Bound by memory for long rows (768 x 65536 scores: 45 us, 68 % of the copy bandwidth; the radix
 // select that read the row five times took 335 us) and by issue slots for many short ones (8192 x
 // 12-16 K: 120 us, 3.9 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
-// two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the stream lists what reaches
-// the floor (two instructions per score, next to nothing listed), and the exact selection runs on
+// two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the
+// stream lists what reaches the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256
 // bins, normally once; the few entries of the threshold's bin are ranked by comparison; a bitmap
 // of winning positions gives the output order. The list holds every score that reaches the
@@ -536,8 +536,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       key[4 * q + 0] = q < quads ? score_key(v[q].x) : 0; key[4 * q + 1] = q < quads ? score_key(v[q].y) : 0;
       key[4 * q + 2] = q < quads ? score_key(v[q].z) : 0; key[4 * q + 3] = q < quads ? score_key(v[q].w) : 0;
     }
-    // Samples expected among the TopK best, and five standard deviations of that count on top:
-    // the floor lies below the TopK-th best score in all but a few rows in a million.
+    // Samples expected among the TopK best, and five standard deviations of that count on top: of
+    // independent scores, the floor lies below the TopK-th best in all but a few rows in a million. (A piece of
+    // neighbours that are alike is one draw and not 32: such rows miss more often, see `select_by_keys`.)
     const float expected = float(kTopK) * float(4 * sampled) / float(candidates);
     unsigned wanted = unsigned(expected + 5.f * sqrtf(expected) + 2.f);
     // Only the sample's upper end matters: its maximum, and the lowest of the maxima of G groups, above

@@ -677,7 +677,7 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // are busy back to back. Their time is latency (tensor-memory loads, votes, shared loads that queue
 // behind the producers' copies, the special-function unit: 32 exponentials of a warp take 256
 // cycles), so nothing that is known a chunk earlier is fetched late, and additions go two to an
-// instruction. Prefill of 8192 tokens at 32K: 1000 -> 935 us; decode 128x6 at 128K: 127 -> 122 us.
+// instruction. Prefill of 8192 tokens at 32K: 1038 -> 978 us; decode 128x6 at 128K: 135 -> 132 us.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -15,10 +15,10 @@
 // Bound by latency. One token on one block takes 30 k cycles: 9 k until its first scores, 1.9 k per
 // chunk, 3 k for the output pass. Here the chunks' first product and softmax run side by side, and
 // the output pass is a quarter; what stays serial is the second product, whose instructions wait for
-// one another (about 700 cycles per chunk). 17.3 -> 14.7 us for one token, 17.4 -> 15.1 for 16, 17.6 ->
-// 16.1 for 24. (Eight blocks: 14.1 us for one token, 15.2 for eight; P written to the other blocks by
-// the softmax threads instead of bulk copies: 19.9.) Copies between blocks are of local shared
-// memory; nothing multicasts.
+// one another (about 700 cycles per chunk), and rescaling where a reference moves. 16.9 -> 15.4 us for one
+// token, 18.0 -> 16.7 for 16, 18.5 -> 18.1 for 33. (Eight blocks: half a microsecond less for one token, none for
+// eight; P written to the other blocks by the softmax threads instead of bulk copies: 19.9.) Copies between
+// blocks are of local shared memory; nothing multicasts.
 //
 // Tensor memory: columns 0-127, 128-255 and 384-511 the scores of the own chunks, 256-383 Q as in
 // `attention_kernel` and, once all scores are computed, 256-319 O (128 features).

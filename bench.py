@@ -48,11 +48,12 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # count, since traffic is Q + O + gathered rows per token. The figures belong to the kernel
 # sources whose hash is recorded with them: a line measured with other sources says so.
 MEASURED_TRAFFIC = {
-    "prefill": {"bytes_per_token": 1075.76e6 / 8192, "profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md"},
+    "prefill": {"bytes_per_token": 1077.56e6 / 8192, "profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md",
+                "attention_kernel_sha256": "f5dd2139a677fe6cfe153ae3fa822e4fb305045993558e579c836f3f99ec42b7"},
     # decode: one-pass captures of the full-size calls (768 / 384 / 96 query tokens per launch)
     "decode": {"bytes_per_token": 500.34e6 / 768, "profile": "profiles/attention_kernel_decode_dram_traffic.md",
-               "per_launch": {768: 500.34e6, 384: 242.30e6, 96: 58.77e6}},
-    "attention_kernel_sha256": "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3",
+               "per_launch": {768: 500.34e6, 384: 242.30e6, 96: 58.79e6},
+               "attention_kernel_sha256": "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3"},
 }
 EXTRA_WORKLOADS = ("prefill_q32k_ctx32k", "decode_b64_q6_ctx128k", "decode_b128_q6_ctx128k")
 CONFIG_KEYS = {"heads": 64, "features": 512, "topk": 512, "window": 128, "ratio": 2, "values": "N(0,1)",
@@ -251,8 +252,8 @@ def roofline_of(config, work, ms, world, source_sha):
     record["traffic"] = measured if measured else traffic["bytes_per_token"] * work["tokens"] / world
     record["traffic_source"] = (f"ncu capture summarised in {traffic['profile']}, "
                                 f"{'of this very call' if measured else 'scaled by tokens'}; captured with "
-                                f"kernel sources {MEASURED_TRAFFIC['attention_kernel_sha256'][:12]}"
-                                + ("" if MEASURED_TRAFFIC["attention_kernel_sha256"] == source_sha else
+                                f"kernel sources {traffic['attention_kernel_sha256'][:12]}"
+                                + ("" if traffic["attention_kernel_sha256"] == source_sha else
                                    f" (this run: {source_sha[:12]}, so the figure may be stale)"))
     record["peak_source"] = f"{source} (burst figure: each launch is timed alone between L2 evictions)"
     record["per_gpu"] = "achieved is per GPU: the whole call's work / GPUs / slowest rank's time"

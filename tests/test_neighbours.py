@@ -100,9 +100,8 @@ def test_gpu_selection_matches_the_oracle_bit_for_bit(ratio, seed):
 @pytest.mark.gpu
 @pytest.mark.parametrize("max_seq,ratio", [(131072, 2), (32768, 2), (131072, 1), (262144, 2)])
 def test_gpu_selection_over_long_rows(max_seq, ratio):
-    """Decode-sized rows: up to 65536 scores are selected from one read (upper key halves kept in
-    shared memory), longer rows by the streaming kernel. Continuous scores, heavy ties, one row of
-    nothing but ties (more of them than the kernel's tie list holds), one of negative values."""
+    """Decode-sized rows, selected from one read, and one longer than a window of winners. Continuous scores,
+    heavy ties, one row of nothing but ties (more of them than the list holds), one of negative values."""
     import torch
 
     from ascendflow_b200 import neighbours
