@@ -21,14 +21,15 @@
 //                    rescaled only when the running maximum moved by more than 2^8, final
 //                    normalisation and store (after the next token's first chunk).
 //
-// Tensor memory (512 columns x 128 lanes), all of it in use:
+// Tensor memory (512 columns x 128 lanes):
 //   columns   0-255  O: two weight-stationary M = 64, N = 256 accumulators (columns 0-127: features
 //                    0-255, columns 128-255: features 256-511). Lane l holds head l % 64 and,
 //                    of each accumulator, features 128 (l / 64) .. + 127.
-//   columns 256-383  Q as 16-bit pairs, same split: lanes 0-15 hold Q[:, 0:256] of 16 heads, lanes
-//                    16-31 hold Q[:, 256:512] of the same heads.
-//   columns 384-511  the score buffer of the stacked QK product (see `issue_qk`): a low-half lane
-//                    finds its partial scores in columns 0-63, a high-half lane in columns 64-127.
+//   columns 256-383  Q as 16-bit pairs: lanes 0-15 of every warp's 32 hold the even pairs of 16 heads
+//                    (features 4 c and 4 c + 1 in column c), lanes 16-31 the odd pairs of the same heads.
+//   columns 384-447  the score buffer of the QK product (see `issue_qk`): the partial scores of a
+//                    lane's pairs.
+//   columns 448-463  which pairs a lane holds, as the sparse product's metadata (written once).
 // Thread (lane & 15) + 16 * half of softmax warp w owns head 16 w + (lane & 15) of that half; the
 // two lanes of a head add their partial scores with one shuffle per score and split the 64 rows
 // of the chunk between them.
@@ -85,7 +86,8 @@ constexpr int kSmemBytes = kSmemEnd + 1024;  // + slack for the 1024-byte alignm
 constexpr uint32_t kTmemColumns = 512;
 constexpr uint32_t kTmemO = 0;
 constexpr uint32_t kTmemQ = 256;
-constexpr uint32_t kTmemS = 384;                             // one 128-column score buffer
+constexpr uint32_t kTmemS = 384;                             // one 64-column score buffer
+constexpr uint32_t kTmemPlaces = 448;                        // which features a lane of Q holds (see `issue_qk`)
 constexpr uint32_t kTmemOHalf = 128;                         // columns of one 256-feature accumulator
 constexpr uint32_t kHalfLanes = 16u << 16;                   // lane offset of the high-half lanes in a tensor-memory address
 
@@ -106,18 +108,13 @@ enum Bar {
 static_assert(kBarCount <= 32, "the barrier area holds 32 mbarriers");
 
 // Storage formats of kind::f16 instructions: 0 = IEEE half, 1 = BF16.
-template <int kFormat> constexpr uint32_t kIdescQK = idesc_f16(128, 128, kFormat, 0, 0);
+template <int kFormat> constexpr uint32_t kIdescQK = idesc_f16(128, kChunkRows, kFormat, 0, 0) | kSparseA;
 template <int kFormat> constexpr uint32_t kIdescPV = idesc_f16(64, 256, kFormat, 0, 1);  // issued as .ws
-
-// Position of 64-feature block b in a tile: blocks b and b + 4 (the same features of the low
-// and the high half of a row) are neighbours, so that a K-major operand of 128 "rows" with
-// 8-row groups 1024 bytes apart reads rows 0-63 from block b and rows 64-127 from block b + 4.
-__host__ __device__ constexpr int block_position(int b) { return (b & 3) * 2 + (b >> 2); }
 
 // Byte offset of 16-byte unit `unit` (0..63) of row `row` in a K-major 128-byte-swizzled tile
 // of 64 rows: eight 64-feature blocks of [64 rows x 128 bytes].
 __device__ __forceinline__ uint32_t swizzled(int row, int unit) {
-  return block_position(unit >> 3) * kBlockBytes + row * 128 + (((unit & 7) ^ (row & 7)) << 4);
+  return (unit >> 3) * kBlockBytes + row * 128 + (((unit & 7) ^ (row & 7)) << 4);
 }
 
 // The P tile (64 heads x 64 rows of 16-bit probabilities, K-major, 128-byte swizzle: one
@@ -359,10 +356,22 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
   }
 }
 
+// Q on its way through the registers of a producer thread: 64 words, the even ones of every 16 bytes
+// in words[0..31] and the odd ones in words[32..63], so that 16 columns of tensor memory are 16
+// registers in a row when they are stored. Place of word i of the thread's 256 bytes:
+__host__ __device__ constexpr int q_place(int i) { return (i & 1) * 32 + (i >> 1); }
+
+__device__ __forceinline__ void load_q_unit(uint32_t (&words)[64], int unit, const void* source) {
+  const uint4 v = __ldg(static_cast<const uint4*>(source));
+  words[q_place(4 * unit)] = v.x; words[q_place(4 * unit + 1)] = v.y;
+  words[q_place(4 * unit + 2)] = v.z; words[q_place(4 * unit + 3)] = v.w;
+}
+
 // 8 x 8 transpose of 16-byte elements across the eight lanes of an octet: on entry lane a holds
-// element (a, b) ... of row b in words[4 b .. 4 b + 3]; on return it holds element (b, a) there,
+// element (a, b) ... of row b as unit kFirst + b; on return it holds element (b, a) there,
 // i.e. what lane b held at index a. Three butterfly stages, register indices all static.
-__device__ __forceinline__ void transpose_octet(uint32_t* words, int lane) {
+template <int kFirst>
+__device__ __forceinline__ void transpose_octet(uint32_t (&words)[64], int lane) {
 #pragma unroll
   for (int m = 1; m < 8; m <<= 1) {
     const bool upper = (lane & m) != 0;
@@ -371,8 +380,8 @@ __device__ __forceinline__ void transpose_octet(uint32_t* words, int lane) {
       if (b & m) continue;
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        uint32_t& low = words[4 * b + w];
-        uint32_t& high = words[4 * (b | m) + w];
+        uint32_t& low = words[q_place(4 * (kFirst + b) + w)];
+        uint32_t& high = words[q_place(4 * (kFirst + (b | m)) + w)];
         const uint32_t send = upper ? low : high;
         const uint32_t got = __shfl_xor_sync(0xffffffffu, send, m);
         if (upper) low = got; else high = got;
@@ -381,10 +390,39 @@ __device__ __forceinline__ void transpose_octet(uint32_t* words, int lane) {
   }
 }
 
+// The two lanes of a head (lane and lane + 16) hold 256 contiguous bytes of its row each, the low lane the
+// first; on return the low lane has the even words of the 512 bytes and the high lane the odd ones, in order.
+__device__ __forceinline__ void split_pairs(uint32_t (&words)[64], int lane) {
+  const bool high = (lane & 16) != 0;
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    const uint32_t even = words[c], odd = words[32 + c];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? even : odd, 16);
+    words[c] = high ? got : even;
+    words[32 + c] = high ? odd : got;
+  }
+}
+
+// 64 columns of Q to tensor memory.
+__device__ __forceinline__ void store_q(uint32_t q_tmem, const uint32_t (&words)[64]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) tmem_st16(q_tmem + j * 16, *reinterpret_cast<const uint32_t(*)[16]>(&words[16 * j]));
+}
+
+// The metadata of the sparse QK product: of every four features a lane of Q holds numbers 0 and 1 (low
+// lanes) or 2 and 3 (high lanes), two bits per number. The two entries of a word belong to two heads
+// eight apart, whose lanes hold the same numbers: a lane's words are all alike. (Four columns are
+// read at most; a store is sixteen wide.)
+__device__ __forceinline__ void store_places(uint32_t places_tmem, int lane) {
+  uint32_t columns[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) columns[e] = lane & 16 ? 0xeeeeeeeeu : 0x44444444u;
+  tmem_st16(places_tmem, columns);
+}
+
 // Copies of the 64 rows of a chunk into a tile, by the 256 producer threads.
 __device__ __forceinline__ void gather_chunk(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
-  // Sixteen threads per row and quarter: eight 16-byte units of block q, eight of block q + 4.
-  const int sub = tid & 15;
+  const int sub = tid & 15;  // sixteen threads per row: 256 bytes at a time
   const char* source[kChunkRows / (kProducerThreads / 16)];
   bool live[kChunkRows / (kProducerThreads / 16)];
 #pragma unroll
@@ -396,7 +434,7 @@ __device__ __forceinline__ void gather_chunk(const Params& p, const int* rows, i
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int unit = (q + 4 * (sub >> 3)) * 8 + (sub & 7);
+    const int unit = q * 16 + sub;
 #pragma unroll
     for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
       const int r = (tid >> 4) + k * (kProducerThreads / 16);
@@ -411,14 +449,15 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   volatile int* abort_flag = sm.abort_flag();
   // Q goes from global memory to tensor memory through registers, never through the ring. A warp
   // reaches the 32 tensor-memory lanes of subpartition (warp index % 4): two producer warps
-  // share each subpartition and take 64 columns (256 bytes of every half row) each. Lane l of a
-  // subpartition holds head 16 * subpartition + (l & 15), feature half l >> 4.
+  // share each subpartition and take 64 columns (512 bytes of every row) each. Lane l of a
+  // subpartition holds head 16 * subpartition + (l & 15), its even 32-bit words (l < 16) or its odd ones.
   const int warp = threadIdx.x >> 5;
   const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
   // Loads are coalesced: in load j the eight lanes of an octet read 128 contiguous bytes of the
-  // half row that belongs to the octet's lane (j & 7); an 8 x 8 transpose by shuffles within
-  // the octet then gives every lane its own half row (see `transpose_octet`).
-  const size_t q_octet_offset = (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + (lane >> 4) * 512 + part * 256 + (lane & 7) * 16;
+  // 256 bytes that belong to the octet's lane (j & 7); an 8 x 8 transpose by shuffles within
+  // the octet then gives every lane its own 256 bytes (see `transpose_octet`), and the two lanes of a
+  // head exchange words (`split_pairs`).
+  const size_t q_octet_offset = (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + part * 512 + (lane >> 4) * 256 + (lane & 7) * 16;
   const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
   // Ring bookkeeping: stage s is free again once the PV of the tile it held has completed
   // (kKvFree0 + s, committed by the MMA thread). A tile is announced without anybody waiting
@@ -428,8 +467,8 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   uint32_t ring = 0;  // tiles placed so far (all tokens)
   uint32_t token_count = 0, q_loads = 0;
   // Q staging registers: `words` holds (part of) the Q slice of `staged_token`; step s < 4 loads
-  // a quarter of it, steps 4 and 5 transpose the two halves.
-  constexpr int kQSteps = 6;
+  // a quarter of it, steps 4 and 5 transpose the two halves, step 6 splits even and odd words.
+  constexpr int kQSteps = 7;
   constexpr int kQFirstItem = 2;  // the first two tiles of a token are issued without delay
   uint32_t words[64];
   int staged_token = -1, q_step = kQSteps;
@@ -438,18 +477,17 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
     auto load4 = [&](auto first) {
       constexpr int kFirst = decltype(first)::value;
 #pragma unroll
-      for (int j = kFirst; j < kFirst + 4; ++j) {  // row (j & 7) of the octet, units 8 (j >> 3) .. + 7
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(source + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128));
-        words[4 * j + 0] = v.x; words[4 * j + 1] = v.y; words[4 * j + 2] = v.z; words[4 * j + 3] = v.w;
-      }
+      for (int j = kFirst; j < kFirst + 4; ++j)  // row (j & 7) of the octet, units 8 (j >> 3) .. + 7
+        load_q_unit(words, j, source + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128);
     };
     switch (q_step) {
       case 0: load4(std::integral_constant<int, 0>{}); break;
       case 1: load4(std::integral_constant<int, 4>{}); break;
       case 2: load4(std::integral_constant<int, 8>{}); break;
       case 3: load4(std::integral_constant<int, 12>{}); break;
-      case 4: transpose_octet(words, lane); break;
-      default: transpose_octet(words + 32, lane); break;
+      case 4: transpose_octet<0>(words, lane); break;
+      case 5: transpose_octet<8>(words, lane); break;
+      default: split_pairs(words, lane); break;
     }
     ++q_step;
   };
@@ -484,9 +522,7 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
         while (q_step < kQSteps) q_advance();
         if (q_loads > 0 && !warp_wait(sm.bar(kQFree), (q_loads - 1) & 1, abort_flag)) return;
         tc_fence_after_sync();
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          tmem_st16(q_tmem + j * 16, *reinterpret_cast<uint32_t(*)[16]>(&words[16 * j]));
+        store_q(q_tmem, words);
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
@@ -515,28 +551,31 @@ __device__ __forceinline__ bool wait_for_copies(uint32_t bar, uint32_t parity, v
 
 // Compile-time unrolled issue loops: every operand offset and accumulate flag is an immediate,
 // so the issuing thread spends a couple of instructions per MMA and stays ahead of the pipe.
-constexpr int kQkSteps = kFeatures / 32;  // K = 16 steps over one half of the features
+constexpr int kQkSteps = kFeatures / 32;
 template <int kFormat, int K = 0>
-__device__ __forceinline__ void issue_qk_steps(uint32_t s_tmem, uint32_t q_tmem, uint64_t x_desc) {
+__device__ __forceinline__ void issue_qk_steps(uint32_t s_tmem, uint32_t q_tmem, uint64_t x_desc, uint32_t places_tmem) {
   if constexpr (K < kQkSteps) {
-    constexpr uint32_t offset = block_position(K >> 2) * kBlockBytes + (K & 3) * 32;
-    mma_ts_c<K != 0>(s_tmem, q_tmem + K * 8, x_desc + (offset >> 4), kIdescQK<kFormat>);
-    issue_qk_steps<kFormat, K + 1>(s_tmem, q_tmem, x_desc);
+    constexpr uint32_t offset = (K >> 1) * kBlockBytes + (K & 1) * 64;
+    mma_sparse_ts_c<K != 0>(s_tmem, q_tmem + K * 8, x_desc + (offset >> 4), places_tmem, kIdescQK<kFormat>);
+    issue_qk_steps<kFormat, K + 1>(s_tmem, q_tmem, x_desc, places_tmem);
   }
 }
 
-// S = Q X^T for one 64-row tile as ONE M = 128, N = 128 product per K step. Operand rows
-// (tensor-memory lanes) 16-31 of every subpartition hold the high feature half of the heads
-// whose low half is in lanes 0-15; operand "rows" 64-127 of B are the tile's rows again, high
-// feature half (block b + 4 next to block b). Of the 128 x 128 result a thread's useful scores
-// are columns 0-63 in a low-half lane (Q_lo . X_lo) and 64-127 in a high-half lane
-// (Q_hi . X_hi); the other two quadrants mix the halves and are ignored. Half the products are
-// thrown away, but M = 128 runs at the full rate of the pipe and N = 128 is above its
-// per-instruction floor: 16 instructions of 64 cycles replace 32 of about 56.
+// S = Q X^T for one 64-row tile. 64 heads fill half of the M = 128 operand rows (tensor-memory lanes)
+// that the pipe's full rate wants, so the features of a head are split between two lanes: lanes 0-15 of
+// every subpartition hold the even pairs of features of 16 heads, lanes 16-31 the odd pairs. Either
+// is a 2:4 sparse row, two of every four neighbours, and the sparse product multiplies just those: 16
+// instructions M = 128, N = 64, K = 32 give every lane the partial scores of its pairs, no product is
+// wasted, and the tile is read once.
+//
+// Bound by the 44 cycles that an instruction takes at least: 704 cycles per tile. Dense, with the low
+// and the high half of the features stacked along M and along N (M = 128, N = 128, K = 16; two of
+// the four quadrants thrown away) it was 1030 cycles and twice the multiplications, which the board's power
+// limit turned into a lower clock; M = 64 without stacking takes 1420.
 template <int kFormat>
 __device__ __forceinline__ void issue_qk(const Shared& sm, uint32_t tmem, int stage, uint32_t scores = kTmemS) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, 16, 1024);
-  issue_qk_steps<kFormat>(tmem + scores, tmem + kTmemQ, x_desc);
+  issue_qk_steps<kFormat>(tmem + scores, tmem + kTmemQ, x_desc, tmem + kTmemPlaces);
 }
 
 constexpr int kPvSteps = 2 * (kChunkRows / 16);
@@ -544,7 +583,7 @@ template <int kFormat, int I, bool kFirst>
 __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc, uint64_t x_desc) {
   if constexpr (I < kPvSteps) {
     constexpr int h = I / (kChunkRows / 16), k = I % (kChunkRows / 16);
-    constexpr uint32_t offset = h * kBlockBytes + k * 2048;
+    constexpr uint32_t offset = h * 4 * kBlockBytes + k * 2048;
     mma_ws_ss_c<!(kFirst && k == 0)>(o_tmem + h * kTmemOHalf, p_desc + ((k * 32) >> 4), x_desc + (offset >> 4), kIdescPV<kFormat>);
     issue_pv_steps<kFormat, I + 1, kFirst>(o_tmem, p_desc, x_desc);
   }
@@ -553,11 +592,10 @@ __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc,
 // O += P X for one 64-row tile as two weight-stationary M = 64, N = 256 products (features 0-255
 // and 256-511): with 64 heads a plain M = 64 instruction would leave half of the pipe idle.
 // A = P from shared memory (one 128-byte row per head, 32 bytes per K = 16 step); B = X with
-// features contiguous: the four 64-feature blocks of a half are two block positions apart,
-// 8-row groups 1024 bytes apart.
+// features contiguous: 64-feature blocks kBlockBytes apart, 8-row groups 1024 bytes apart.
 template <int kFormat>
 __device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, bool accumulate) {
-  const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, 2 * kBlockBytes, 1024);
+  const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, kBlockBytes, 1024);
   const uint64_t p_desc = smem_desc_sw128(sm.base + kSmemP, 16, 1024);
   if (accumulate) issue_pv_steps<kFormat, 0, false>(tmem + kTmemO, p_desc, x_desc);
   else issue_pv_steps<kFormat, 0, true>(tmem + kTmemO, p_desc, x_desc);
@@ -696,7 +734,12 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   __nv_bfloat16* out_base = static_cast<__nv_bfloat16*>(p.out);
   const uint32_t s_addr = tmem + kTmemS + lane_base;
 
-  if (lane == 0) mbar_arrive(sm.bar(kKvFull0));  // the score buffer starts out free (first chunk, stage 0)
+  store_places(tmem + kTmemPlaces + lane_base, lane);
+  tmem_wait_st();
+  tc_fence_before_sync();
+  __syncwarp();
+  // The score buffer starts out free (first chunk, stage 0), and the metadata is in place.
+  if (lane == 0) mbar_arrive(sm.bar(kKvFull0));
   // Step c (c >= 1) of this block's chunk stream is one phase of one barrier: it completes once
   // all four softmax warps have published what they hand each other for chunk c (rescale factors,
   // or the finished token's reciprocal denominators) AND the PV of chunk c - 1 has completed
@@ -795,12 +838,12 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
 
       if (!warp_wait(sm.bar(kSFull), chunk_count & 1, abort_flag)) return;
       tc_fence_after_sync();
-      // Lane (head, low half) holds Q_lo . X_lo in columns 0-63, lane (head, high half) holds
-      // Q_hi . X_hi in columns 64-127. The two threads of a head share the softmax work: the low
+      // Lane (head, low half) holds the scores' sums over the even pairs of features, lane (head, high
+      // half) those over the odd pairs. The two threads of a head share the softmax work: the low
       // thread owns tile rows 0-31, the high thread rows 32-63. Both partial scores of a row come
       // straight to the thread that owns it: a load over the 16 low lanes gives threads 0-15
-      // columns j and threads 16-31 columns 32 + j of the low partials; a load over the 16 high
-      // lanes gives them columns 64 + j and 96 + j of the high partials. No exchange between lanes.
+      // columns j and threads 16-31 columns 32 + j of the low lanes' partials; a load over the 16 high
+      // lanes gives them the same columns of the high lanes' partials. No exchange between lanes.
       const unsigned live = half ? live_hi : live_lo;
       const bool all_live = (live_lo & live_hi) == 0xffffffffu;  // the usual case: nothing to mask
       float2 raw[16];  // unscaled scores: the scale goes into the exponent's FMA
@@ -808,8 +851,8 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         uint32_t low_a[16], low_b[16], high_a[16], high_b[16];
         tmem_ld16_halves<32>(s_addr, low_a);                       // rows 0-15 | 32-47, low partial
         tmem_ld16_halves<32>(s_addr + 16, low_b);                  // rows 16-31 | 48-63
-        tmem_ld16_halves<32>(s_addr + kHalfLanes + 64, high_a);    // the same rows, high partial
-        tmem_ld16_halves<32>(s_addr + kHalfLanes + 80, high_b);
+        tmem_ld16_halves<32>(s_addr + kHalfLanes, high_a);         // the same rows, high partial
+        tmem_ld16_halves<32>(s_addr + kHalfLanes + 16, high_b);
         tmem_wait_ld();
         // The scores are in registers: the next QK may overwrite the buffer. Its tile's full
         // barrier counts this as well as the copies.

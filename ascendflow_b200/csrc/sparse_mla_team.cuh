@@ -20,8 +20,8 @@
 // eight; P written to the other blocks by the softmax threads instead of bulk copies: 19.9.) Copies between
 // blocks are of local shared memory; nothing multicasts.
 //
-// Tensor memory: columns 0-127, 128-255 and 384-511 the scores of the own chunks, 256-383 Q as in
-// `attention_kernel` and, once all scores are computed, 256-319 O (128 features).
+// Tensor memory: columns 0-63, 128-191 and 384-447 the scores of the own chunks, 256-383 Q and 448-463 its
+// metadata as in `attention_kernel`; once all scores are computed, 256-319 O (128 features).
 #pragma once
 
 #include "sparse_mla_tcgen05.cuh"
@@ -87,15 +87,13 @@ __device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, in
   const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
   volatile int* abort_flag = sm.abort_flag();
   const char* q = static_cast<const char*>(p.q) + (size_t)token * kHeads * kRowBytes +
-                  (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + (lane >> 4) * 512 + part * 256 + (lane & 7) * 16;
+                  (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + part * 512 + (lane >> 4) * 256 + (lane & 7) * 16;
   uint32_t words[64];  // see producer_role
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(q + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128));
-    words[4 * j + 0] = v.x; words[4 * j + 1] = v.y; words[4 * j + 2] = v.z; words[4 * j + 3] = v.w;
-  }
-  transpose_octet(words, lane);
-  transpose_octet(words + 32, lane);
+  for (int j = 0; j < 16; ++j) load_q_unit(words, j, q + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128);
+  transpose_octet<0>(words, lane);
+  transpose_octet<8>(words, lane);
+  split_pairs(words, lane);
   if (!warp_wait(sm.bar(kReady), 0, abort_flag)) return;
   const int* rows = sm.rows(0);
   const TokenInfo* info = sm.info(0);
@@ -107,8 +105,8 @@ __device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, in
     cp_async_arrive(sm.bar(kTile0 + j));
     if (j > 0) continue;
     const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) tmem_st16(q_tmem + k * 16, *reinterpret_cast<uint32_t(*)[16]>(&words[16 * k]));
+    store_q(q_tmem, words);
+    if (part == 0) store_places(tmem + kTmemPlaces + (uint32_t(subpartition * 32) << 16), lane);
     tmem_wait_st();
     tc_fence_before_sync();
     __syncwarp();
@@ -258,8 +256,8 @@ __device__ __forceinline__ void team_scores(uint32_t tmem, int own, unsigned liv
   uint32_t low_a[16], low_b[16], high_a[16], high_b[16];
   tmem_ld16_halves<32>(s_addr, low_a);
   tmem_ld16_halves<32>(s_addr + 16, low_b);
-  tmem_ld16_halves<32>(s_addr + kHalfLanes + 64, high_a);
-  tmem_ld16_halves<32>(s_addr + kHalfLanes + 80, high_b);
+  tmem_ld16_halves<32>(s_addr + kHalfLanes, high_a);
+  tmem_ld16_halves<32>(s_addr + kHalfLanes + 16, high_b);
   tmem_wait_ld();
 #pragma unroll
   for (int e = 0; e < 8; ++e) {

@@ -154,7 +154,8 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo,
 }
 
 // Instruction descriptor for kind::f16 with FP32 accumulation. format: 0 = f16, 1 = bf16.
-// a_mn / b_mn: 1 when that operand is MN-major in shared memory.
+// a_mn / b_mn: 1 when that operand is MN-major in shared memory. kSparseA: A is 2:4 sparse.
+constexpr uint32_t kSparseA = 1u << 2;
 __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, int format, int a_mn, int b_mn) {
   return (1u << 4) | (uint32_t(format) << 7) | (uint32_t(format) << 10) | (uint32_t(a_mn) << 15) |
          (uint32_t(b_mn) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
@@ -164,22 +165,25 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, int format, int a
 
 // The accumulate flag is a template argument: no predicate set-up per instruction, and the issuing
 // thread's unrolled sequences carry nothing but immediates.
+//
+// The form with a 2:4 sparse A: of every four neighbours along K a row of A holds two, and the metadata (two
+// bits for each of these: its place among the four) lies in tensor memory at `meta_tmem`. K = 32 per instruction.
 template <bool kAccumulate>
-__device__ __forceinline__ void mma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
+__device__ __forceinline__ void mma_sparse_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t meta_tmem, uint32_t idesc) {
   if constexpr (kAccumulate) {
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
         "setp.eq.b32 p, 0, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
+        "tcgen05.mma.sp.cta_group::1.kind::f16 [%0], [%1], %2, [%3], %4, p;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(meta_tmem), "r"(idesc) : "memory");
   } else {
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
         "setp.ne.b32 p, 0, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
+        "tcgen05.mma.sp.cta_group::1.kind::f16 [%0], [%1], %2, [%3], %4, p;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(meta_tmem), "r"(idesc) : "memory");
   }
 }
 // Weight-stationary form (tcgen05.mma.ws): with M = 64 the accumulator spreads over all 128
