@@ -683,8 +683,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {  // one instr
 }
 
 // The running reference of a head (log2 domain; it starts at the sink) moves to a chunk's maximum when
-// that exceeds it by more than 8 (a factor 256): the accumulator is rescaled rarely (1500 cycles, for
-// which everybody waits), probabilities stay below 2^8 and all terms of one head share the same
+// that exceeds it by more than 8 (a factor 256): the accumulator is rescaled rarely (everybody waits for it), probabilities stay below 2^8 and all terms of one head share the same
 // reference, which cancels in the final division. A smaller step is not free even while O is empty: in
 // IEEE half small probabilities would then lose up to eight of their bits to the subnormal range (1.7 %
 // off for rows 2^-20 below the best; it would spare rescaling for heads with a low sink, 1 to 3 % of a
@@ -926,14 +925,18 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       }
       if (__any_sync(0xffffffffu, o_alpha != 1.f)) {  // the previous PV has landed (wait above)
         tc_fence_after_sync();
+        // 32 columns at a time: a round trip to tensor memory each (in 16s the pass took 1500 cycles, and a
+        // quarter of the chunks has one in some warp; prefill of 8K tokens, one call at a time, 896 -> 859 us).
 #pragma unroll 1
-        for (int c = 0; c < 256; c += 16) {
-          uint32_t o[16];
-          tmem_ld16(tmem + kTmemO + c + lane_base, o);
+        for (int c = 0; c < 256; c += 32) {
+          uint32_t o[32];
+          tmem_ld16(tmem + kTmemO + c + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[0]));
+          tmem_ld16(tmem + kTmemO + c + 16 + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[16]));
           tmem_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * o_alpha);
-          tmem_st16(tmem + kTmemO + c + lane_base, o);
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * o_alpha);
+          tmem_st16(tmem + kTmemO + c + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[0]));
+          tmem_st16(tmem + kTmemO + c + 16 + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[16]));
         }
         tmem_wait_st();
       }
