@@ -139,6 +139,9 @@ struct Shared {
   __device__ __forceinline__ volatile uint32_t* rescale_mask() const {  // (team kernel)
     return reinterpret_cast<volatile uint32_t*>(ptr + kSmemMisc + 8);
   }
+  __device__ __forceinline__ volatile int* first_negative() const {  // one per softmax warp
+    return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 16);
+  }
   __device__ __forceinline__ const volatile float* maxima(int offset) const {  // (team kernel)
     return reinterpret_cast<const volatile float*>(ptr + offset);
   }
@@ -309,6 +312,81 @@ __device__ __forceinline__ void publish_token(const Params& p, const Shared& sm,
   }
 }
 
+// The first token of a block, resolved by five warps together: the softmax warps, which have nothing else to
+// do yet, take a quarter of the list each and the resolver warp the window, four slots per lane instead of
+// twenty. One warp's straight line of code over twenty slots is fetched cold, once, and took 6.7 k
+// cycles of the 26 k of a one-token call; nothing of the token can start before. The rows and chunks are those
+// of `publish_token`.
+constexpr int kFirstThreads = (kSoftmaxWarps + 1) * 32;
+constexpr int kFirstSlots = kWindow / 32;  // per lane
+static_assert(kTopK == kSoftmaxWarps * kWindow, "five parts of 128 slots");
+__device__ __forceinline__ void publish_first_token(const Params& p, const Shared& sm, int token, int warp, int lane, uint32_t ready_bar) {
+  const bool window = warp == kResolverWarp;
+  const int first_rank = warp * kWindow + lane;  // (list warps)
+  TokenInfo* info = sm.info(0);
+  int index[kFirstSlots];
+  if (!window) {
+#pragma unroll
+    for (int i = 0; i < kFirstSlots; ++i) index[i] = __ldg(p.indices + (size_t)token * kTopK + first_rank + i * 32);
+  }
+  const TokenGeometry g = token_geometry_warp(p, token, lane);
+  const int first_position = g.right - g.visible + lane;
+  const int shift = window || p.cmp_page != 64 ? 7 : 6;
+  const int32_t* table = (window ? p.ori_table : p.cmp_table) + (size_t)g.batch * p.pages;
+  const int blocks = window ? p.ori_blocks : p.cmp_blocks;
+  int column[kFirstSlots], page[kFirstSlots];  // column: -1 where not live
+  int negative = kTopK;                        // rank of the list's first negative entry
+#pragma unroll
+  for (int i = kFirstSlots - 1; i >= 0; --i) {
+    if (window) index[i] = first_position + i * 32;
+    else if (index[i] < 0) negative = first_rank + i * 32;
+    const bool live = window ? lane + i * 32 < g.visible : index[i] >= 0 && index[i] < g.cutoff && first_rank + i * 32 < g.bound;
+    column[i] = live ? index[i] >> shift : -1;
+    page[i] = __ldg(table + min(unsigned(column[i]), unsigned(p.pages - 1)));
+  }
+  negative = __reduce_min_sync(0xffffffffu, negative);
+  if (!window && lane == 0) sm.first_negative()[warp] = negative;
+  named_barrier_sync(1, kFirstThreads);
+  if (!window) {
+#pragma unroll
+    for (int w = 0; w < kSoftmaxWarps; ++w) negative = min(negative, sm.first_negative()[w]);
+  }
+  const int part = window ? 0 : warp + 1;
+  int* rows = sm.rows(0) + part * kWindow + lane;
+  bool bad = false;
+  unsigned mask[kFirstSlots];
+#pragma unroll
+  for (int i = 0; i < kFirstSlots; ++i) {
+    const bool live = column[i] >= 0 && (window || first_rank + i * 32 < negative);
+    const bool legal = column[i] < p.pages && (unsigned)page[i] < (unsigned)blocks;
+    bad |= live && !legal;
+    const int row = live && legal ? (page[i] << shift) + (index[i] & ((1 << shift) - 1)) : -1;
+    rows[i * 32] = row;
+    mask[i] = __ballot_sync(0xffffffffu, row >= 0);
+  }
+  if (lane < 2) info->live[part * 2 + lane] = lane == 0 ? make_uint2(mask[0], mask[1]) : make_uint2(mask[2], mask[3]);
+  if (bad) report(p, kStatusBadPage, token, lane);
+  if (!window) {
+    named_barrier_arrive(2, kFirstThreads);
+    return;
+  }
+  named_barrier_sync(2, kFirstThreads);
+  // The live chunks, in order.
+  const uint2 live = lane < kMaxChunks ? info->live[lane] : make_uint2(0, 0);
+  const unsigned live_chunks = __ballot_sync(0xffffffffu, (live.x | live.y) != 0);
+  if (live_chunks >> lane & 1) {
+    const int item = __popc(live_chunks & ((1u << lane) - 1));
+    info->live[item] = live;
+    info->chunk[item] = (unsigned char)lane;
+  }
+  if (lane == 0) {
+    info->token = token;
+    info->chunks = __popc(live_chunks);
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive(ready_bar);
+}
+
 // What a block reads first, for its first token, asked for on the way to L2 (and its pages'
 // translations with it) while the kernel before is still running: L2 sees what that kernel writes,
 // so nothing stale is read later.
@@ -332,13 +410,15 @@ __device__ __forceinline__ void prefetch_first(const Params& p, int token) {
 }
 
 // ---- resolver warp ----------------------------------------------------------------------------
-// Runs ahead of everybody else: for each token of this block it resolves the 640 slots into row
+// Runs ahead of everybody else: for each token of this block after the first it resolves the 640 slots into row
 // buffer `token_count & 1`, lists the live chunks and publishes both.
 __device__ void resolver_role(const Params& p, const Shared& sm) {
   const int lane = threadIdx.x & 31;
   volatile int* abort_flag = sm.abort_flag();
   uint32_t token_count = 0;
   TokenWalk walk(p);
+  walk.next();  // the first token: `publish_first_token`
+  ++token_count;
   for (int token = walk.next(); token >= 0; token = walk.next(), ++token_count) {
     const int buffer = token_count & 1;
     // The buffer is free once the softmax warps have finished the token that used it two tokens
@@ -983,9 +1063,13 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
   const uint32_t tmem = *tmem_slot;
   // Up to here nothing has touched global memory: a block's start, and the launch itself, overlap
   // the end of the kernel before.
-  if (const int first = TokenWalk(p).next(); first >= 0) prefetch_first(p, first);
+  const int first = TokenWalk(p).next();  // (there is one: no more blocks than tokens)
+  prefetch_first(p, first);
   wait_for_predecessor();
   let_successor_start();
+
+  if (warp < kSoftmaxWarps || warp == kResolverWarp)
+    publish_first_token(p, sm, first, warp, threadIdx.x & 31, sm.bar(kTokenReady0));
 
   if (warp < kSoftmaxWarps) {
     softmax_role<kFormat>(p, sm, tmem);

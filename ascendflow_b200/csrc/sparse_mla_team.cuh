@@ -114,35 +114,62 @@ __device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, in
   }
 }
 
-// Copies of a chunk's slice, this block's 128 features of its 64 rows, by `threads` threads: sixteen per row.
-__device__ __forceinline__ void gather_slice(const Params& p, const Shared& sm, int rank, int item, int thread, int threads) {
-  const int chunk = sm.info(0)->chunk[item], unit = thread & 15;
-  const int* rows = sm.rows(0);
-#pragma unroll 4
-  for (int r = thread >> 4; r < kChunkRows; r += threads >> 4) {
-    const int slot = chunk * kChunkRows + r, row = rows[slot];
-    const char* source = static_cast<const char*>(slot < kWindow ? p.ori_kv : p.cmp_kv) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
-    cp_async16(sm.base + kTeamSlices + item % kSliceSlots * kSliceBytes + (unit >> 3) * kBlockBytes + r * 128 + (((unit & 7) ^ (r & 7)) << 4),
-               source + rank * 256 + unit * 16, row >= 0);
+// Copies of `kItems` chunks' slices (as many of them as there are), this block's 128 features of their 64 rows, by
+// `kThreadCount` threads: sixteen per row. All row numbers first: a round trip to shared memory per row would
+// take as long as the copies.
+template <int kItems, int kThreadCount>
+__device__ __forceinline__ void gather_slices(const Params& p, const Shared& sm, int rank, int item, int chunks, int thread) {
+  constexpr int kRows = kChunkRows / (kThreadCount / 16);
+  const int unit = thread & 15;
+  int chunk[kItems], row[kItems][kRows];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) chunk[i] = sm.info(0)->chunk[min(item + i, chunks - 1)];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i)
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) row[i][k] = sm.rows(0)[chunk[i] * kChunkRows + (thread >> 4) + k * (kThreadCount / 16)];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    if (item + i >= chunks) break;
+    const char* cache = static_cast<const char*>(chunk[i] * kChunkRows < kWindow ? p.ori_kv : p.cmp_kv) + rank * 256 + unit * 16;
+    const uint32_t slice = sm.base + kTeamSlices + (item + i) % kSliceSlots * kSliceBytes + (unit >> 3) * kBlockBytes;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const int r = (thread >> 4) + k * (kThreadCount / 16);
+      cp_async16(slice + r * 128 + (((unit & 7) ^ (r & 7)) << 4), cache + (size_t)max(row[i][k], 0) * kRowBytes, row[i][k] >= 0);
+    }
   }
 }
 
-// Phase B, producer warps: the first eight chunks' slices; then four of the warps rescale O where a
-// reference moves, the other four gather the last two slices.
+// Phase A, producer warps, behind their part in the cluster's barrier: the first eight chunks' slices. They fill
+// the places of the own chunks' first two tiles, four each, which are free when these have been multiplied.
+__device__ void team_early_slices(const Params& p, const Shared& sm, int rank) {
+  const int tid = threadIdx.x - kFirstProducerWarp * 32;
+  volatile int* abort_flag = sm.abort_flag();
+  if (*abort_flag != 0) return;  // (the token may not be there)
+  const int chunks = sm.info(0)->chunks;
+  static_assert(kTileBytes == 4 * kSliceBytes && kSliceSlots == 8, "four slices to a tile");
+#pragma unroll 1
+  for (int item = 0; item < min(chunks, kSliceSlots); item += 2) {
+    const int own = item / 4;
+    if (item % 4 == 0 && rank + own * kBlocks < chunks && !warp_wait(sm.bar(kScores0 + own), 0, abort_flag)) return;
+    gather_slices<2, kProducerThreads>(p, sm, rank, item, chunks, tid);
+    cp_async_arrive(sm.bar(kSlices0 + item / 2));
+  }
+}
+
+// Phase B, producer warps: four of them rescale O where a reference moves, the other four gather the last two
+// slices.
 __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, int rank) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32, lane = tid & 31, warp = threadIdx.x >> 5;
   volatile int* abort_flag = sm.abort_flag();
-  const int chunks = sm.info(0)->chunks, early = min(chunks, kSliceSlots);
-  for (int item = 0; item < early; ++item) {
-    gather_slice(p, sm, rank, item, tid, kProducerThreads);
-    if ((item & 1) || item == early - 1) cp_async_arrive(sm.bar(kSlices0 + item / 2));
-  }
+  const int chunks = sm.info(0)->chunks;
   if (chunks == 0) return;
   if (warp >= kFirstProducerWarp + 4) {
     if (chunks <= kSliceSlots) return;
     for (int item = kSliceSlots; item < chunks; ++item) {
       if (!warp_wait(sm.bar(kSliceFree0 + item - kSliceSlots), 0, abort_flag)) return;
-      gather_slice(p, sm, rank, item, tid - 128, 128);
+      gather_slices<1, 128>(p, sm, rank, item, chunks, tid - 128);
     }
     cp_async_arrive(sm.bar(kSlices0 + kSliceSlots / 2));
   } else {
@@ -419,19 +446,18 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   const int lane = threadIdx.x & 31;
   const float sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? warp * 16 + (lane & 15) : lane)) * 1.4426950408889634f;
   const float other_sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? (warp & 1) * 32 : 32) + lane) * 1.4426950408889634f;
+  if (warp < kSoftmaxWarps || warp == kResolverWarp) publish_first_token(p, sm, token, warp, lane, sm.bar(kReady));
   if (warp < kSoftmaxWarps) {
     team_maxima(p, sm, tmem, rank);
   } else if (warp == kMmaWarp) {
     if ((threadIdx.x & 31) == 0) team_qk<kFormat>(sm, tmem, rank);
-  } else if (warp == kResolverWarp) {
-    publish_token(p, sm, token, 0, threadIdx.x & 31);
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(sm.bar(kReady));
-  } else if (warp != kPvWarp) {
+  } else if (warp >= kFirstProducerWarp && warp != kPvWarp) {
     team_gather(p, sm, tmem, token, rank);
   }
   __syncwarp();
   cluster_arrive();
+  if (warp >= kFirstProducerWarp && warp != kPvWarp) team_early_slices(p, sm, rank);
+  __syncwarp();
   cluster_wait();
   if (*sm.abort_flag() == 0) {
     tc_fence_after_sync();
@@ -452,8 +478,11 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   // (A wait has given up: what is still on its way to or from this block gets time to arrive.)
   if (*sm.abort_flag() != 0)
     for (int i = 0; i < 100; ++i) __nanosleep(1000);
+  // What the last barrier is for is that the other blocks' copies to this one have arrived, which its waits have
+  // seen, and that they have finished reading: nothing written here is read behind it, so nobody waits
+  // for the output's way to memory (2.2 k cycles).
   tc_fence_before_sync();
-  cluster_arrive();
+  cluster_arrive_relaxed();
   cluster_wait();
   if (threadIdx.x == 0 && *sm.abort_flag() != 0) report(p, kStatusWaitExpired, blockIdx.x, 0);
   __syncthreads();

@@ -40,6 +40,11 @@ inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_
   return cudaLaunchKernelEx(&config, kernel, arguments...);
 }
 
+// ---- barriers of some of a block's warps --------------------------------------------------------
+
+__device__ __forceinline__ void named_barrier_sync(int id, int threads) { asm volatile("barrier.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_barrier_arrive(int id, int threads) { asm volatile("barrier.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+
 // ---- mbarrier -----------------------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -107,6 +112,8 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 }
 // The cluster's barrier, executed by every thread of every block: first arrive, then wait.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+// The same for threads whose writes nobody in the cluster reads behind the barrier.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 // Address of this block's shared-memory word `address` in the block of rank `rank`.
 __device__ __forceinline__ uint32_t cluster_address(uint32_t address, uint32_t rank) {
