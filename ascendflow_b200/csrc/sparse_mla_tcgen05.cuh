@@ -320,8 +320,9 @@ __device__ __forceinline__ void publish_token(const Params& p, const Shared& sm,
 constexpr int kFirstThreads = (kSoftmaxWarps + 1) * 32;
 constexpr int kFirstSlots = kWindow / 32;  // per lane
 static_assert(kTopK == kSoftmaxWarps * kWindow, "five parts of 128 slots");
-__device__ __forceinline__ void publish_first_token(const Params& p, const Shared& sm, int token, int warp, int lane, uint32_t ready_bar) {
-  const bool window = warp == kResolverWarp;
+template <bool window>
+__device__ __forceinline__ void publish_first_token(const Params& p, const Shared& sm, int token, uint32_t ready_bar) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first_rank = warp * kWindow + lane;  // (list warps)
   TokenInfo* info = sm.info(0);
   int index[kFirstSlots];
@@ -436,57 +437,35 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
   }
 }
 
-// Q on its way through the registers of a producer thread: 64 words, the even ones of every 16 bytes
-// in words[0..31] and the odd ones in words[32..63], so that 16 columns of tensor memory are 16
-// registers in a row when they are stored. Place of word i of the thread's 256 bytes:
-__host__ __device__ constexpr int q_place(int i) { return (i & 1) * 32 + (i >> 1); }
-
-__device__ __forceinline__ void load_q_unit(uint32_t (&words)[64], int unit, const void* source) {
-  const uint4 v = __ldg(static_cast<const uint4*>(source));
-  words[q_place(4 * unit)] = v.x; words[q_place(4 * unit + 1)] = v.y;
-  words[q_place(4 * unit + 2)] = v.z; words[q_place(4 * unit + 3)] = v.w;
+// Q on its way to tensor memory: every thread of a producer warp loads 16 bytes of rows t / 4 and t / 4 + 8 of
+// the warp's 16 heads in each of eight 64-byte segments. The 16-lane stores put the even words (two heads' each)
+// to the low lanes and the odd words to the high lanes as they are: no exchange between lanes. (Loads of
+// whole lines with 96 shuffles for a transpose and 32 for the split took 450 instructions more per thread and
+// token, and their queue is the one that everybody's shared memory accesses stand in.)
+constexpr int kQLoads = 16;
+__device__ __forceinline__ const char* q_rows(const Params& p, int token, int subpartition, int part, int lane) {
+  return static_cast<const char*>(p.q) + ((size_t)token * kHeads + subpartition * 16 + (lane >> 2)) * kRowBytes + part * 512 + (lane & 3) * 16;
 }
-
-// 8 x 8 transpose of 16-byte elements across the eight lanes of an octet: on entry lane a holds
-// element (a, b) ... of row b as unit kFirst + b; on return it holds element (b, a) there,
-// i.e. what lane b held at index a. Three butterfly stages, register indices all static.
-template <int kFirst>
-__device__ __forceinline__ void transpose_octet(uint32_t (&words)[64], int lane) {
+template <int kFirst, int kCount>
+__device__ __forceinline__ void load_q(const char* rows, uint32_t (&words)[64]) {
 #pragma unroll
-  for (int m = 1; m < 8; m <<= 1) {
-    const bool upper = (lane & m) != 0;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      if (b & m) continue;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        uint32_t& low = words[q_place(4 * (kFirst + b) + w)];
-        uint32_t& high = words[q_place(4 * (kFirst + (b | m)) + w)];
-        const uint32_t send = upper ? low : high;
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, send, m);
-        if (upper) low = got; else high = got;
-      }
-    }
-  }
-}
-
-// The two lanes of a head (lane and lane + 16) hold 256 contiguous bytes of its row each, the low lane the
-// first; on return the low lane has the even words of the 512 bytes and the high lane the odd ones, in order.
-__device__ __forceinline__ void split_pairs(uint32_t (&words)[64], int lane) {
-  const bool high = (lane & 16) != 0;
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    const uint32_t even = words[c], odd = words[32 + c];
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? even : odd, 16);
-    words[c] = high ? got : even;
-    words[32 + c] = high ? odd : got;
+  for (int k = kFirst; k < kFirst + kCount; ++k) {  // segment k / 2, row (k & 1) * 8
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(rows + (k >> 1) * 64 + (k & 1) * 8 * kRowBytes));
+    words[4 * k + 0] = v.x; words[4 * k + 1] = v.y; words[4 * k + 2] = v.z; words[4 * k + 3] = v.w;
   }
 }
 
 // 64 columns of Q to tensor memory.
 __device__ __forceinline__ void store_q(uint32_t q_tmem, const uint32_t (&words)[64]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) tmem_st16(q_tmem + j * 16, *reinterpret_cast<const uint32_t(*)[16]>(&words[16 * j]));
+  for (int half = 0; half < 2; ++half)
+#pragma unroll
+    for (int quad = 0; quad < 2; ++quad) {  // four segments: 32 columns
+      uint32_t columns[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) columns[c] = words[32 * quad + 2 * c + half];
+      tmem_st_16x256b(q_tmem + half * kHalfLanes + quad * 32, columns);
+    }
 }
 
 // The metadata of the sparse QK product: of every four features a lane of Q holds numbers 0 and 1 (low
@@ -533,11 +512,6 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   // subpartition holds head 16 * subpartition + (l & 15), its even 32-bit words (l < 16) or its odd ones.
   const int warp = threadIdx.x >> 5;
   const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
-  // Loads are coalesced: in load j the eight lanes of an octet read 128 contiguous bytes of the
-  // 256 bytes that belong to the octet's lane (j & 7); an 8 x 8 transpose by shuffles within
-  // the octet then gives every lane its own 256 bytes (see `transpose_octet`), and the two lanes of a
-  // head exchange words (`split_pairs`).
-  const size_t q_octet_offset = (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + part * 512 + (lane >> 4) * 256 + (lane & 7) * 16;
   const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
   // Ring bookkeeping: stage s is free again once the PV of the tile it held has completed
   // (kKvFree0 + s, committed by the MMA thread). A tile is announced without anybody waiting
@@ -546,39 +520,26 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   // the warps need not stay in step with each other.
   uint32_t ring = 0;  // tiles placed so far (all tokens)
   uint32_t token_count = 0, q_loads = 0;
-  // Q staging registers: `words` holds (part of) the Q slice of `staged_token`; step s < 4 loads
-  // a quarter of it, steps 4 and 5 transpose the two halves, step 6 splits even and odd words.
-  constexpr int kQSteps = 7;
+  // Q staging registers: `words` holds (part of) the Q slice of `staged_token`, a quarter more with every step.
+  constexpr int kQSteps = 4;
   constexpr int kQFirstItem = 2;  // the first two tiles of a token are issued without delay
   uint32_t words[64];
-  int staged_token = -1, q_step = kQSteps;
+  int q_step = kQSteps;
+  const char* q = nullptr;
   auto q_advance = [&]() {
-    const char* source = static_cast<const char*>(p.q) + (size_t)staged_token * kHeads * kRowBytes + q_octet_offset;
-    auto load4 = [&](auto first) {
-      constexpr int kFirst = decltype(first)::value;
-#pragma unroll
-      for (int j = kFirst; j < kFirst + 4; ++j)  // row (j & 7) of the octet, units 8 (j >> 3) .. + 7
-        load_q_unit(words, j, source + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128);
-    };
     switch (q_step) {
-      case 0: load4(std::integral_constant<int, 0>{}); break;
-      case 1: load4(std::integral_constant<int, 4>{}); break;
-      case 2: load4(std::integral_constant<int, 8>{}); break;
-      case 3: load4(std::integral_constant<int, 12>{}); break;
-      case 4: transpose_octet<0>(words, lane); break;
-      case 5: transpose_octet<8>(words, lane); break;
-      default: split_pairs(words, lane); break;
+      case 0: load_q<0, 4>(q, words); break;
+      case 1: load_q<4, 4>(q, words); break;
+      case 2: load_q<8, 4>(q, words); break;
+      default: load_q<12, 4>(q, words); break;
     }
     ++q_step;
   };
   TokenWalk walk(p);
   // The first token's Q does not depend on the resolver: its loads go out while the token is
   // being resolved (a block that only gets a few tokens spends a good part of its time here).
-  staged_token = walk.peek();
-  if (staged_token >= 0) {
-    q_step = 0;
-    while (q_step < kQSteps) q_advance();
-  }
+  int staged_token = walk.peek();
+  if (staged_token >= 0) load_q<0, kQLoads>(q_rows(p, staged_token, subpartition, part, lane), words);
   for (int token = walk.next(); token >= 0; token = walk.next(), ++token_count) {
     if (!warp_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) return;
     const int* rows = sm.rows(token_count & 1);
@@ -598,7 +559,7 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
         // previous token's tiles were being issued, unless this is the block's first working
         // token or the walk skipped an empty one. The wait (the previous working token's last
         // QK has read the old Q) cannot depend on this thread: all its tiles have been issued.
-        if (staged_token != token) { staged_token = token; q_step = 0; }
+        if (staged_token != token) { q = q_rows(p, token, subpartition, part, lane); q_step = 0; }
         while (q_step < kQSteps) q_advance();
         if (q_loads > 0 && !warp_wait(sm.bar(kQFree), (q_loads - 1) & 1, abort_flag)) return;
         tc_fence_after_sync();
@@ -609,6 +570,7 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
         if (lane == 0) mbar_arrive(sm.bar(kQFull));
         ++q_loads;
         staged_token = walk.peek();  // start on the next token's Q
+        q = q_rows(p, max(staged_token, 0), subpartition, part, lane);
         q_step = staged_token >= 0 ? 0 : kQSteps;
       } else if (item >= kQFirstItem && q_step < kQSteps) {
         q_advance();  // one slice of the next token's Q per tile, so that it never comes as a burst
@@ -1068,10 +1030,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
   wait_for_predecessor();
   let_successor_start();
 
-  if (warp < kSoftmaxWarps || warp == kResolverWarp)
-    publish_first_token(p, sm, first, warp, threadIdx.x & 31, sm.bar(kTokenReady0));
-
   if (warp < kSoftmaxWarps) {
+    publish_first_token<false>(p, sm, first, sm.bar(kTokenReady0));
     softmax_role<kFormat>(p, sm, tmem);
   } else if (warp == kMmaWarp) {
     if ((threadIdx.x & 31) == 0) qk_role<kFormat>(p, sm, tmem);
@@ -1080,6 +1040,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
     if ((threadIdx.x & 31) == 0) pv_role<kFormat>(p, sm, tmem);
     __syncwarp();
   } else if (warp == kResolverWarp) {
+    publish_first_token<true>(p, sm, first, sm.bar(kTokenReady0));
     resolver_role(p, sm);
   } else {
     producer_role(p, sm, tmem);

@@ -86,14 +86,8 @@ __device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, in
   const int tid = threadIdx.x - kFirstProducerWarp * 32, lane = tid & 31, warp = threadIdx.x >> 5;
   const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
   volatile int* abort_flag = sm.abort_flag();
-  const char* q = static_cast<const char*>(p.q) + (size_t)token * kHeads * kRowBytes +
-                  (size_t)(subpartition * 16 + (lane & 8)) * kRowBytes + part * 512 + (lane >> 4) * 256 + (lane & 7) * 16;
   uint32_t words[64];  // see producer_role
-#pragma unroll
-  for (int j = 0; j < 16; ++j) load_q_unit(words, j, q + (size_t)(j & 7) * kRowBytes + (j >> 3) * 128);
-  transpose_octet<0>(words, lane);
-  transpose_octet<8>(words, lane);
-  split_pairs(words, lane);
+  load_q<0, kQLoads>(q_rows(p, token, subpartition, part, lane), words);
   if (!warp_wait(sm.bar(kReady), 0, abort_flag)) return;
   const int* rows = sm.rows(0);
   const TokenInfo* info = sm.info(0);
@@ -446,8 +440,10 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   const int lane = threadIdx.x & 31;
   const float sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? warp * 16 + (lane & 15) : lane)) * 1.4426950408889634f;
   const float other_sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? (warp & 1) * 32 : 32) + lane) * 1.4426950408889634f;
-  if (warp < kSoftmaxWarps || warp == kResolverWarp) publish_first_token(p, sm, token, warp, lane, sm.bar(kReady));
-  if (warp < kSoftmaxWarps) {
+  if (warp == kResolverWarp) {
+    publish_first_token<true>(p, sm, token, sm.bar(kReady));
+  } else if (warp < kSoftmaxWarps) {
+    publish_first_token<false>(p, sm, token, sm.bar(kReady));
     team_maxima(p, sm, tmem, rank);
   } else if (warp == kMmaWarp) {
     if ((threadIdx.x & 31) == 0) team_qk<kFormat>(sm, tmem, rank);
