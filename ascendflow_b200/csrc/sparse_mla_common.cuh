@@ -55,6 +55,8 @@ struct Params {
   int32_t cmp_blocks;
   float scale_log2;          // 512^-0.5 * log2(e)
   int32_t token_group;       // consecutive tokens a persistent block takes per round (>= 1)
+  int32_t whole_rounds;      // tokens in rounds that are full
+  int32_t last_group;        // tokens that a block takes, at most, of those behind them
 };
 
 struct TokenGeometry {

@@ -147,25 +147,34 @@ struct Shared {
   }
 };
 
-// The tokens of one persistent block, in order. Blocks take `group` consecutive tokens per round
-// (round r, block b: tokens (r * grid + b) * group ...), so that a block's successive tokens
-// share most of their window rows in L2 while different blocks read different windows at any one
-// time. Every role of a block walks the same sequence.
+// The tokens of one persistent block, in order. Blocks take `token_group` consecutive tokens per round, so
+// that a block's successive tokens share most of their window rows in L2 while different blocks read
+// different windows at any one time. The last round, which is not full, is dealt in groups as small as it
+// takes: 1493 tokens on 148 blocks in twos would be 12 for some, dealt singly in the end they are 11 at most.
+// Every role of a block walks the same sequence.
 struct TokenWalk {
-  unsigned start, within, group, stride, tokens;  // start < tokens + stride < 2^32
-  __device__ __forceinline__ explicit TokenWalk(const Params& p)
-      : start(blockIdx.x * p.token_group), within(0), group(p.token_group), stride(gridDim.x * p.token_group), tokens(p.tokens) {}
+  const Params& p;
+  unsigned round, at, end;  // first token of the round; of it, the block's next token and the end of its group
+  __device__ __forceinline__ explicit TokenWalk(const Params& params) : p(params), round(0) { enter(); }
+  __device__ __forceinline__ unsigned stride() const { return gridDim.x * unsigned(p.token_group); }
+  __device__ __forceinline__ void enter() {
+    const unsigned group = round < unsigned(p.whole_rounds) ? p.token_group : p.last_group;
+    at = round + blockIdx.x * group;  // (below 2^31 + 2^31)
+    end = min(at + group, unsigned(p.tokens));
+  }
   __device__ __forceinline__ int next() {  // next token of this block, or -1 when done
-    if (within == group) { start += stride; within = 0; }
-    const unsigned token = start + within;
-    if (token >= tokens) return -1;  // (and so is every later one)
-    ++within;
-    return int(token);
+    if (at >= end) {
+      if (round >= unsigned(p.whole_rounds)) return -1;
+      round += stride();
+      enter();
+      if (at >= end) return -1;
+    }
+    return int(at++);
   }
   __device__ __forceinline__ int peek() const { TokenWalk copy = *this; return copy.next(); }
-  __device__ __forceinline__ int count() const {  // how many tokens next() hands out in all
-    const unsigned rounds = tokens / stride, rest = tokens - rounds * stride, mine = blockIdx.x * group;
-    return int(rounds * group + (rest <= mine ? 0 : min(rest - mine, group)));
+  static __device__ __forceinline__ int count(const Params& p) {  // how many tokens next() hands out in all
+    const unsigned whole = unsigned(p.whole_rounds), rest = unsigned(p.tokens) - whole, mine = blockIdx.x * unsigned(p.last_group);
+    return int(whole / gridDim.x + (rest <= mine ? 0 : min(rest - mine, unsigned(p.last_group))));
   }
 };
 
@@ -656,7 +665,7 @@ template <int kFormat>
 __device__ void qk_role(const Params& p, const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
   uint32_t chunk_count = 0, working_tokens = 0;
-  const uint32_t my_tokens = uint32_t(TokenWalk(p).count());  // closed form: no walk on this thread
+  const uint32_t my_tokens = uint32_t(TokenWalk::count(p));  // closed form: no walk on this thread
   for (uint32_t token_count = 0; token_count < my_tokens; ++token_count) {
     if (!mbar_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) return;
     const int chunks = sm.info(token_count & 1)->chunks;
@@ -686,7 +695,7 @@ template <int kFormat>
 __device__ void pv_role(const Params& p, const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
   uint32_t chunk_count = 0, working_tokens = 0;
-  const uint32_t my_tokens = uint32_t(TokenWalk(p).count());
+  const uint32_t my_tokens = uint32_t(TokenWalk::count(p));
   for (uint32_t token_count = 0; token_count < my_tokens; ++token_count) {
     if (!mbar_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) return;
     const int chunks = sm.info(token_count & 1)->chunks;
@@ -1069,6 +1078,9 @@ inline int launch(const Params& p, cudaStream_t stream, int multiprocessors) {
   Params launch_params = p;
   const int per_block = p.tokens / (grid * 4);
   launch_params.token_group = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
+  const int rest = p.tokens % (grid * launch_params.token_group);
+  launch_params.whole_rounds = p.tokens - rest;
+  launch_params.last_group = (rest + grid - 1) / grid;
   return int(launch_overlapped(attention_kernel<kFormat>, grid, kThreads, kSmemBytes, stream, launch_params));
 }
 
