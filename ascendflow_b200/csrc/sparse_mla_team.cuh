@@ -5,11 +5,11 @@
 //
 //   1. Every block resolves the token and gathers up to three of its ten chunks (items r, r + 4 and
 //      r + 8 for block r).
-//   2. Q X^T of its own chunks, and their maxima per head, which go to all four blocks.
+//   2. Q X^T of its own chunks, and their maxima per head, which go to all four blocks. Meanwhile it gathers, of
+//      all chunks, the 128 features it will produce.
 //   3. With all maxima known every block can follow the running reference through the chunks
 //      (examples/sparse_attention/attention.py:398-490): it takes its own chunks' exponentials and sends
-//      P and the partial sums to the other three (bulk copies), while it gathers, of all chunks, the
-//      128 features it will produce.
+//      P and the partial sums to the other three (bulk copies).
 //   4. O += P X over all chunks in order for its 128 features (M = 64, N = 128), normalise, store.
 //
 // Bound by latency. One token on one block takes 30 k cycles: 9 k until its first scores, 1.9 k per
@@ -55,7 +55,7 @@ __host__ __device__ constexpr uint32_t score_columns(int own) { return own == 0 
 constexpr uint32_t kTeamO = kTmemQ;
 
 enum TeamBar {
-  kReady = 0, kQReady, kTile0, kTile1, kTile2, kScores0, kScores1, kScores2, kMaskReady, kPvDone, kRescaled, kOutput,
+  kReady = 0, kQReady, kTile0, kTile1, kTile2, kScores0, kScores1, kScores2, kMaxima, kMaskReady, kPvDone, kRescaled, kOutput,
   kSlices0,                                   // of two chunks each
   kP0 = kSlices0 + kMaxChunks / 2,
   kSliceFree0 = kP0 + kMaxChunks, kSliceFree1,
@@ -135,7 +135,7 @@ __device__ __forceinline__ void gather_slices(const Params& p, const Shared& sm,
   }
 }
 
-// Phase A, producer warps, behind their part in the cluster's barrier: the first eight chunks' slices. They fill
+// Phase A, producer warps: the first eight chunks' slices. They fill
 // the places of the own chunks' first two tiles, four each, which are free when these have been multiplied.
 __device__ void team_early_slices(const Params& p, const Shared& sm, int rank) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32;
@@ -157,6 +157,7 @@ __device__ void team_early_slices(const Params& p, const Shared& sm, int rank) {
 __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, int rank) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32, lane = tid & 31, warp = threadIdx.x >> 5;
   volatile int* abort_flag = sm.abort_flag();
+  if (*abort_flag != 0) return;
   const int chunks = sm.info(0)->chunks;
   if (chunks == 0) return;
   if (warp >= kFirstProducerWarp + 4) {
@@ -167,7 +168,7 @@ __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, in
     }
     cp_async_arrive(sm.bar(kSlices0 + kSliceSlots / 2));
   } else {
-    if (!warp_wait(sm.bar(kMaskReady), 0, abort_flag)) return;
+    if (!warp_wait(sm.bar(kMaskReady), 0, abort_flag) || !warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;
     const int o_head = (warp & 1) * 32 + lane;  // lane l of tensor memory: head l % 64 (see softmax_role)
     const uint32_t o_addr = tmem + kTeamO + (uint32_t((warp & 3) * 32) << 16);
     const float sink = __ldg(p.sinks + o_head) * 1.4426950408889634f;
@@ -197,6 +198,8 @@ __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, in
 
 // Phase B, one warp: the chunks after the first that move some head's reference.
 __device__ void team_mask(const Shared& sm, float sink, float other_sink) {  // of heads lane, 32 + lane
+  volatile int* abort_flag = sm.abort_flag();
+  if (!warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;
   const int lane = threadIdx.x & 31, chunks = sm.info(0)->chunks;
   uint32_t moved = 0;
   auto note = [&](int i, float, float alpha) { moved |= uint32_t(i > 0 && alpha != 1.f) << i; };
@@ -225,40 +228,45 @@ __device__ void team_qk(const Shared& sm, uint32_t tmem, int rank) {
   }
 }
 
-// Phase B, one warp: O = P X over all chunks, this block's 128 features. The whole warp runs the loop and
-// one thread of it issues (by a predicate on the instruction), so that descriptors stay in uniform
-// registers: with a loop of one thread every instruction took 83 cycles to issue.
+template <int kFormat, int K, bool kFirst>
+__device__ __forceinline__ void issue_team_pv(uint32_t tmem, uint64_t p_desc, uint64_t x_desc) {
+  if constexpr (K < kChunkRows / 16) {
+    mma_ws_ss_c<!(kFirst && K == 0)>(tmem + kTeamO, p_desc + ((K * 32) >> 4), x_desc + ((K * 2048) >> 4), kIdescTeamPv<kFormat>);
+    issue_team_pv<kFormat, K + 1, kFirst>(tmem, p_desc, x_desc);
+  }
+}
+
+// Phase B, one thread: O = P X over all chunks, this block's 128 features.
 template <int kFormat>
 __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
+  if (!mbar_wait(sm.bar(kMaskReady), 0, abort_flag)) return;
   const int chunks = sm.info(0)->chunks;
-  if (chunks == 0 || !warp_wait(sm.bar(kMaskReady), 0, abort_flag)) return;
-  const uint32_t issuer = (threadIdx.x & 31) == 0;
-  const uint32_t rescale_mask = __shfl_sync(0xffffffffu, *sm.rescale_mask(), 0);
+  if (chunks == 0) return;
+  const uint32_t rescale_mask = *sm.rescale_mask();
   uint32_t rescales = 0;
+#pragma unroll 1
   for (int i = 0; i < chunks; ++i) {
-    if ((i & 1) == 0 && !__all_sync(0xffffffffu, wait_for_copies(sm.bar(kSlices0 + i / 2), 0, abort_flag))) return;
-    if (!warp_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
+    if ((i & 1) == 0 && !wait_for_copies(sm.bar(kSlices0 + i / 2), 0, abort_flag)) return;
+    if (!mbar_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
     if (rescale_mask >> i & 1) {  // some head's reference moves here: O is rescaled first
-      if (issuer) mma_commit(sm.bar(kPvDone));
-      __syncwarp();
-      if (!warp_wait(sm.bar(kRescaled), rescales++ & 1, abort_flag)) return;
+      mma_commit(sm.bar(kPvDone));
+      if (!mbar_wait(sm.bar(kRescaled), rescales++ & 1, abort_flag)) return;
     }
     tc_fence_after_sync();
     const uint64_t p_desc = smem_desc_sw128(sm.base + kTeamP + i * kPBytes, 16, 1024);
     const uint64_t x_desc = smem_desc_sw128(sm.base + kTeamSlices + i % kSliceSlots * kSliceBytes, kBlockBytes, 1024);
-#pragma unroll
-    for (int k = 0; k < kChunkRows / 16; ++k)
-      mma_ws_ss_if(issuer, tmem + kTeamO, p_desc + ((k * 32) >> 4), x_desc + ((k * 2048) >> 4), kIdescTeamPv<kFormat>, k > 0 || i > 0);
-    if (issuer && i + kSliceSlots < chunks) mma_commit(sm.bar(kSliceFree0 + i));
-    __syncwarp();
+    if (i == 0) issue_team_pv<kFormat, 0, true>(tmem, p_desc, x_desc);
+    else issue_team_pv<kFormat, 0, false>(tmem, p_desc, x_desc);
+    if (i + kSliceSlots < chunks) mma_commit(sm.bar(kSliceFree0 + i));
   }
-  if (issuer) mma_commit(sm.bar(kOutput));
+  mma_commit(sm.bar(kOutput));
 }
 
 // Phase B, one thread: every own chunk's P and partial sums to the other blocks.
 __device__ void team_send(const Shared& sm, int rank) {
   volatile int* abort_flag = sm.abort_flag();
+  if (!mbar_wait(sm.bar(kReady), 0, abort_flag)) return;
   const int chunks = sm.info(0)->chunks;
   for (int item = rank; item < chunks; item += kBlocks) {
     if (!mbar_wait(sm.bar(kP0 + item), 0, abort_flag)) return;
@@ -318,7 +326,10 @@ __device__ __forceinline__ void team_maxima(const Params& p, const Shared& sm, u
     // Each of a head's two threads tells two blocks.
     const uint32_t at = sm.base + kTeamMaxima + (item * kHeads + head) * 4;
 #pragma unroll
-    for (int b = 0; b < kBlocks / 2; ++b) cluster_store(cluster_address(at, half * (kBlocks / 2) + b), chunk_max);
+    for (int b = 0; b < kBlocks / 2; ++b) {
+      const uint32_t to = half * (kBlocks / 2) + b;
+      cluster_store_async(cluster_address(at, to), chunk_max, cluster_address(sm.bar(kMaxima), to));
+    }
   }
   tc_fence_before_sync();
 }
@@ -338,6 +349,7 @@ __device__ __forceinline__ void team_softmax(const Params& p, const Shared& sm, 
     return;
   }
   const volatile float* maxima = sm.maxima(kTeamMaxima);
+  if (!warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;  // all blocks' (and so all own scores have been read)
   int own = 0;
   for (int item = rank; item < chunks; item += kBlocks, ++own) {
     float run_max = sink;
@@ -398,9 +410,10 @@ __device__ __forceinline__ void team_softmax(const Params& p, const Shared& sm, 
   }
 }
 
-// Every thread passes the cluster's barrier three times: all blocks have started (their shared memory
-// may be written); all maxima are in place and all scores read (P may take the tiles' place); all
-// copies have arrived (shared memory may be given up). No role leaves before it has.
+// Every thread passes the cluster's barrier twice: all blocks have started (their shared memory may be
+// written); all copies have arrived (it may be given up). No role leaves before it has. In between a block waits
+// for what the others send: all maxima, with which all of them say too that their scores have been read (so that
+// P may take the tiles' place; a barrier of the cluster there took 1.7 k cycles), and every chunk's P.
 template <int kFormat>
 __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   extern __shared__ unsigned char smem_raw[];
@@ -442,33 +455,25 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   const float other_sink = __ldg(p.sinks + (warp < kSoftmaxWarps ? (warp & 1) * 32 : 32) + lane) * 1.4426950408889634f;
   if (warp == kResolverWarp) {
     publish_first_token<true>(p, sm, token, sm.bar(kReady));
+    if (lane == 0) {
+      mbar_arrive_expect(sm.bar(kMaxima), uint32_t(sm.info(0)->chunks * kHeads) * 4);
+      team_send(sm, rank);
+    }
   } else if (warp < kSoftmaxWarps) {
     publish_first_token<false>(p, sm, token, sm.bar(kReady));
     team_maxima(p, sm, tmem, rank);
+    team_softmax<kFormat>(p, sm, tmem, token, rank, sink, other_sink);
   } else if (warp == kMmaWarp) {
-    if ((threadIdx.x & 31) == 0) team_qk<kFormat>(sm, tmem, rank);
-  } else if (warp >= kFirstProducerWarp && warp != kPvWarp) {
+    if (lane == 0) team_qk<kFormat>(sm, tmem, rank);
+    __syncwarp();
+    team_mask(sm, sink, other_sink);
+  } else if (warp == kPvWarp) {
+    if (lane == 0) team_pv<kFormat>(sm, tmem);
+  } else {
     team_gather(p, sm, tmem, token, rank);
-  }
-  __syncwarp();
-  cluster_arrive();
-  if (warp >= kFirstProducerWarp && warp != kPvWarp) team_early_slices(p, sm, rank);
-  __syncwarp();
-  cluster_wait();
-  if (*sm.abort_flag() == 0) {
-    tc_fence_after_sync();
-    if (warp < kSoftmaxWarps) {
-      team_softmax<kFormat>(p, sm, tmem, token, rank, sink, other_sink);
-    } else if (warp == kPvWarp) {
-      team_pv<kFormat>(sm, tmem);
-    } else if (warp == kResolverWarp) {
-      if ((threadIdx.x & 31) == 0) team_send(sm, rank);
-    } else if (warp == kMmaWarp) {
-      if (sm.info(0)->chunks > 0) team_mask(sm, sink, other_sink);
-    } else {
-      team_slices(p, sm, tmem, rank);
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-    }
+    team_early_slices(p, sm, rank);
+    team_slices(p, sm, tmem, rank);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
   }
   __syncwarp();
   // (A wait has given up: what is still on its way to or from this block gets time to arrive.)

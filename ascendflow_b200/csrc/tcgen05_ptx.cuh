@@ -121,8 +121,10 @@ __device__ __forceinline__ uint32_t cluster_address(uint32_t address, uint32_t r
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(mapped) : "r"(address), "r"(rank));
   return mapped;
 }
-__device__ __forceinline__ void cluster_store(uint32_t address, float value) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(address), "f"(value) : "memory");
+// Store to another block; counts as four bytes on that block's barrier `bar`.
+__device__ __forceinline__ void cluster_store_async(uint32_t address, float value, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n"
+               ::"r"(address), "r"(__float_as_uint(value)), "r"(bar) : "memory");
 }
 // Copy shared memory of this block to another block of the cluster (16-byte aligned addresses, a
 // multiple of 16 bytes); counts as `bytes` on that block's barrier.
