@@ -323,9 +323,11 @@ __device__ __forceinline__ void publish_token(const Params& p, const Shared& sm,
 
 // The first token of a block, resolved by five warps together: the softmax warps, which have nothing else to
 // do yet, take a quarter of the list each and the resolver warp the window, four slots per lane instead of
-// twenty. One warp's straight line of code over twenty slots is fetched cold, once, and took 6.7 k
-// cycles of the 26 k of a one-token call; nothing of the token can start before. The rows and chunks are those
-// of `publish_token`.
+// twenty. Nothing of the token can start before, and one warp took 6.7 k of the 26 k cycles of a one-token
+// call for it, now 3.5 k (the queue for loads and shared memory, which Q's loads stand in too, is most of
+// it: with its instructions fetched beforehand it was hardly faster). 64 x 6 tokens at 128K 64.5 -> 62.0 us, 256
+// tokens at 4K 31.1 -> 30.4. The rows and chunks are those of `publish_token`. One instantiation per kind of
+// warp, each inside its role: a common one in front of the roles cost the loops behind it 3 %.
 constexpr int kFirstThreads = (kSoftmaxWarps + 1) * 32;
 constexpr int kFirstSlots = kWindow / 32;  // per lane
 static_assert(kTopK == kSoftmaxWarps * kWindow, "five parts of 128 slots");
@@ -450,7 +452,9 @@ __device__ void resolver_role(const Params& p, const Shared& sm) {
 // the warp's 16 heads in each of eight 64-byte segments. The 16-lane stores put the even words (two heads' each)
 // to the low lanes and the odd words to the high lanes as they are: no exchange between lanes. (Loads of
 // whole lines with 96 shuffles for a transpose and 32 for the split took 450 instructions more per thread and
-// token, and their queue is the one that everybody's shared memory accesses stand in.)
+// token, and their queue is the one that everybody's shared memory accesses stand in: prefill of 8K tokens
+// 920 -> 900 us, 256 tokens at 4K 32.7 -> 31.0. 32-byte loads, which need no shuffles either if both lanes of a head
+// load the same or the tile's units are permuted, were slower: 918, and 1600 as copies then split sectors.)
 constexpr int kQLoads = 16;
 __device__ __forceinline__ const char* q_rows(const Params& p, int token, int subpartition, int part, int lane) {
   return static_cast<const char*>(p.q) + ((size_t)token * kHeads + subpartition * 16 + (lane >> 2)) * kRowBytes + part * 512 + (lane & 3) * 16;
@@ -765,7 +769,8 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // are busy back to back. Their time is latency (tensor-memory loads, votes, shared loads that queue
 // behind the producers' copies, the special-function unit: 32 exponentials of a warp take 256
 // cycles), so nothing that is known a chunk earlier is fetched late, and additions go two to an
-// instruction. Prefill of 8192 tokens at 32K: 1038 -> 978 us; decode 128x6 at 128K: 135 -> 132 us.
+// instruction. Prefill of 8192 tokens at 32K: 1038 -> 978 us; decode 128x6 at 128K: 135 -> 132 us. In a
+// steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides and not cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

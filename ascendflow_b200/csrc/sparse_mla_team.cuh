@@ -12,13 +12,15 @@
 //      P and the partial sums to the other three (bulk copies).
 //   4. O += P X over all chunks in order for its 128 features (M = 64, N = 128), normalise, store.
 //
-// Bound by latency. One token on one block takes 30 k cycles: 9 k until its first scores, 1.9 k per
-// chunk, 3 k for the output pass. Here the chunks' first product and softmax run side by side, and
-// the output pass is a quarter; what stays serial is the second product, whose instructions wait for
-// one another (about 700 cycles per chunk), and rescaling where a reference moves. 16.9 -> 15.4 us for one
-// token, 18.0 -> 16.7 for 16, 18.5 -> 18.1 for 33. (Eight blocks: half a microsecond less for one token, none for
-// eight; P written to the other blocks by the softmax threads instead of bulk copies: 19.9.) Copies between
-// blocks are of local shared memory; nothing multicasts.
+// Bound by latency. One token on one block takes 30 k cycles: 6 k until its first scores, 2 k per chunk, 3 k for
+// the output pass. Here the chunks' first product and softmax run side by side, and the output pass is a
+// quarter. Of the 20 k cycles that are left the token's resolution takes 3.5 k, gather, scores and maxima of up to
+// three chunks 5.5 k, the first P 1.3 k, the second product, in the order of the chunks, 8 k (700 per chunk, and
+// rescaling where a reference moves), output 1.5 k. A call of one token 15.6 -> 11.8 us, of 16 tokens 16.8 -> 12.5
+// (one warp resolving the token, all slices gathered behind a barrier of the cluster, products issued by a whole
+// warp before). Eight blocks had less for one token, nothing for eight; P written to the other blocks by
+// the softmax threads instead of bulk copies was slower by a fifth. Copies between blocks are of local shared
+// memory; nothing multicasts.
 //
 // Tensor memory: columns 0-63, 128-191 and 384-447 the scores of the own chunks, 256-383 Q and 448-463 its
 // metadata as in `attention_kernel`; once all scores are computed, 256-319 O (128 features).
