@@ -14,9 +14,9 @@
 //
 // Bound by latency. One token on one block takes 30 k cycles: 6 k until its first scores, 2 k per chunk, 3 k for
 // the output pass. Here the chunks' first product and softmax run side by side, and the output pass is a
-// quarter. Of the 20 k cycles that are left the token's resolution takes 3.5 k, gather, scores and maxima of up to
-// three chunks 5.5 k, the first P 1.3 k, the second product, in the order of the chunks, 8 k (700 per chunk, and
-// rescaling where a reference moves), output 1.5 k. A call of one token 15.6 -> 11.8 us, of 16 tokens 16.8 -> 12.5
+// quarter. Of the 19 k cycles that are left the token's resolution takes 3.5 k, gather, scores and maxima of up to
+// three chunks 5.5 k, the first P 1.3 k, the second product, in the order of the chunks, 6.5 k (and rescaling
+// where a reference moves), output 1.5 k. A call of one token 15.3 -> 10.9 us, of 16 tokens 16.3 -> 11.4
 // (one warp resolving the token, all slices gathered behind a barrier of the cluster, products issued by a whole
 // warp before). Eight blocks had less for one token, nothing for eight; P written to the other blocks by
 // the softmax threads instead of bulk copies was slower by a fifth. Copies between blocks are of local shared
@@ -238,7 +238,9 @@ __device__ __forceinline__ void issue_team_pv(uint32_t tmem, uint64_t p_desc, ui
   }
 }
 
-// Phase B, one thread: O = P X over all chunks, this block's 128 features.
+// Phase B, one thread: O = P X over all chunks, this block's 128 features. Unrolled over the chunks: in a loop the
+// descriptors of every instruction are moved to uniform registers first, and a chunk's four instructions take
+// twice as long (one token 11.7 -> 11.0 us, 16 tokens 12.5 -> 11.7).
 template <int kFormat>
 __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
@@ -247,8 +249,10 @@ __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   if (chunks == 0) return;
   const uint32_t rescale_mask = *sm.rescale_mask();
   uint32_t rescales = 0;
-#pragma unroll 1
-  for (int i = 0; i < chunks; ++i) {
+  const uint64_t p_first = smem_desc_sw128(sm.base + kTeamP, 16, 1024), x_first = smem_desc_sw128(sm.base + kTeamSlices, kBlockBytes, 1024);
+#pragma unroll
+  for (int i = 0; i < kMaxChunks; ++i) {
+    if (i >= chunks) break;
     if ((i & 1) == 0 && !wait_for_copies(sm.bar(kSlices0 + i / 2), 0, abort_flag)) return;
     if (!mbar_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
     if (rescale_mask >> i & 1) {  // some head's reference moves here: O is rescaled first
@@ -256,8 +260,8 @@ __device__ void team_pv(const Shared& sm, uint32_t tmem) {
       if (!mbar_wait(sm.bar(kRescaled), rescales++ & 1, abort_flag)) return;
     }
     tc_fence_after_sync();
-    const uint64_t p_desc = smem_desc_sw128(sm.base + kTeamP + i * kPBytes, 16, 1024);
-    const uint64_t x_desc = smem_desc_sw128(sm.base + kTeamSlices + i % kSliceSlots * kSliceBytes, kBlockBytes, 1024);
+    const uint64_t p_desc = p_first + uint32_t(i * (kPBytes >> 4));
+    const uint64_t x_desc = x_first + uint32_t((i & (kSliceSlots - 1)) * (kSliceBytes >> 4));
     if (i == 0) issue_team_pv<kFormat, 0, true>(tmem, p_desc, x_desc);
     else issue_team_pv<kFormat, 0, false>(tmem, p_desc, x_desc);
     if (i + kSliceSlots < chunks) mma_commit(sm.bar(kSliceFree0 + i));
