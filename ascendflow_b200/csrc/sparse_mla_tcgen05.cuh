@@ -179,8 +179,9 @@ struct TokenWalk {
 };
 
 // A wait whose outcome is uniform across the calling warp (all 32 lanes must call it).
+template <bool kCluster = false>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+  return __all_sync(0xffffffffu, mbar_wait<kCluster>(bar, parity, abort_flag));
 }
 
 // ---- producer warps ---------------------------------------------------------------------------

@@ -170,7 +170,7 @@ __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, in
     }
     cp_async_arrive(sm.bar(kSlices0 + kSliceSlots / 2));
   } else {
-    if (!warp_wait(sm.bar(kMaskReady), 0, abort_flag) || !warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;
+    if (!warp_wait(sm.bar(kMaskReady), 0, abort_flag) || !warp_wait<true>(sm.bar(kMaxima), 0, abort_flag)) return;
     const int o_head = (warp & 1) * 32 + lane;  // lane l of tensor memory: head l % 64 (see softmax_role)
     const uint32_t o_addr = tmem + kTeamO + (uint32_t((warp & 3) * 32) << 16);
     const float sink = __ldg(p.sinks + o_head) * 1.4426950408889634f;
@@ -201,7 +201,7 @@ __device__ void team_slices(const Params& p, const Shared& sm, uint32_t tmem, in
 // Phase B, one warp: the chunks after the first that move some head's reference.
 __device__ void team_mask(const Shared& sm, float sink, float other_sink) {  // of heads lane, 32 + lane
   volatile int* abort_flag = sm.abort_flag();
-  if (!warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;
+  if (!warp_wait<true>(sm.bar(kMaxima), 0, abort_flag)) return;
   const int lane = threadIdx.x & 31, chunks = sm.info(0)->chunks;
   uint32_t moved = 0;
   auto note = [&](int i, float, float alpha) { moved |= uint32_t(i > 0 && alpha != 1.f) << i; };
@@ -254,7 +254,7 @@ __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   for (int i = 0; i < kMaxChunks; ++i) {
     if (i >= chunks) break;
     if ((i & 1) == 0 && !wait_for_copies(sm.bar(kSlices0 + i / 2), 0, abort_flag)) return;
-    if (!mbar_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
+    if (!mbar_wait<true>(sm.bar(kP0 + i), 0, abort_flag)) return;
     if (rescale_mask >> i & 1) {  // some head's reference moves here: O is rescaled first
       mma_commit(sm.bar(kPvDone));
       if (!mbar_wait(sm.bar(kRescaled), rescales++ & 1, abort_flag)) return;
@@ -355,7 +355,7 @@ __device__ __forceinline__ void team_softmax(const Params& p, const Shared& sm, 
     return;
   }
   const volatile float* maxima = sm.maxima(kTeamMaxima);
-  if (!warp_wait(sm.bar(kMaxima), 0, abort_flag)) return;  // all blocks' (and so all own scores have been read)
+  if (!warp_wait<true>(sm.bar(kMaxima), 0, abort_flag)) return;  // all blocks' (and so all own scores have been read)
   int own = 0;
   for (int item = rank; item < chunks; item += kBlocks, ++own) {
     float run_max = sink;
@@ -389,7 +389,7 @@ __device__ __forceinline__ void team_softmax(const Params& p, const Shared& sm, 
   // The denominator: the two row halves' sums follow the reference, then add up (see softmax_role).
   // From here on the head of this thread is that of its accumulator lane.
   for (int i = 0; i < chunks; ++i)
-    if (!warp_wait(sm.bar(kP0 + i), 0, abort_flag)) return;
+    if (!warp_wait<true>(sm.bar(kP0 + i), 0, abort_flag)) return;
   float low = 1.f, high = 0.f;  // the low half's share includes the sink's own weight
   follow_reference(maxima + o_head, o_sink, chunks, [&](int i, float, float alpha) {
     const volatile float* sums = reinterpret_cast<const volatile float*>(sm.ptr + kTeamSums + i * kSumBytes);

@@ -60,27 +60,41 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
+// kCluster: what completes the phase are stores and copies of other blocks of the cluster. They release at cluster
+// scope, and a wait synchronises with them only if it acquires at that scope (the default is the block's own).
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if constexpr (kCluster) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  } else {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  }
   return done != 0;
 }
 
 // Wait for the phase with the given parity, giving up after `limit` SM clock cycles or as soon
 // as `*abort_flag` (shared memory) is non-zero. Returns false when it gave up; the caller must
 // then leave its loop and go to the kernel's common exit.
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           long long limit = (1ll << 31)) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<kCluster>(bar, parity)) return true;
   const long long start = clock64();
   int spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
+  while (!mbar_try_wait<kCluster>(bar, parity)) {
     if ((++spins & 63) == 0) {
       if (*abort_flag != 0) return false;
       if (clock64() - start > limit) { *abort_flag = 1; return false; }

@@ -20,3 +20,19 @@ def test_operands_copied_by_cp_async_are_fenced_before_the_tensor_core_reads_the
     common = (CSRC / "sparse_mla_tcgen05.cuh").read_text()
     body = common[common.index("bool wait_for_copies("):]
     assert "fence_proxy_async();" in body[: body.index("\n}\n")]
+
+
+def test_waits_for_other_blocks_acquire_at_cluster_scope():
+    """What other blocks complete (by remote stores and copies) is waited for at their scope; the sender of P waits for its
+    own block's warps only."""
+    source = (CSRC / "sparse_mla_team.cuh").read_text()
+    remote = set(re.findall(r"cluster_address\(sm\.bar\((\w+)", source))
+    assert remote == {"kMaxima", "kP0"}
+    for barrier in remote:
+        waits = re.findall(rf"(\w+_wait(?:<true>)?)\(sm\.bar\({barrier}([^)]*)\)", source)
+        assert waits
+        for wait, item in waits:
+            assert wait.endswith("<true>") or item == " + item", (barrier, wait, item)
+    wrappers = (CSRC / "tcgen05_ptx.cuh").read_text()
+    body = wrappers[wrappers.index("bool mbar_try_wait("):]
+    assert "mbarrier.try_wait.parity.acquire.cluster." in body[: body.index("\n}\n")]
