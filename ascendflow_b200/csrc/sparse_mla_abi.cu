@@ -287,8 +287,10 @@ int launch_sparse_mla_resolve_rows(void* stream, void* arg_cmp_sparse_indices,
     return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (int status = clear_workspace(s, npu_workspace)) return status;
-  const int64_t blocks = (T + 3) / 4, cap = int64_t(multiprocessors()) * 8;  // four warps = four tokens per block
-  umma::resolve_rows_kernel<<<int(blocks < cap ? blocks : cap), 128, 0, s>>>(p, static_cast<int32_t*>(arg_resolved_rows));
+  const int firsts = umma::persistent_blocks(p, multiprocessors());
+  umma::deal_tokens(p, firsts);
+  const int64_t others = (T - firsts + umma::kExportWarps - 1) / umma::kExportWarps, cap = int64_t(multiprocessors()) * 6;
+  umma::resolve_rows_kernel<<<firsts + int(others < cap ? others : cap), umma::kExportWarps * 32, 0, s>>>(p, firsts, static_cast<int32_t*>(arg_resolved_rows));
   return int(cudaGetLastError());
 }
 

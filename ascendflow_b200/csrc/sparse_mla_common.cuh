@@ -20,6 +20,7 @@ constexpr int kWindow = 128;
 constexpr int kTopK = 512;
 constexpr int kSlots = kWindow + kTopK;  // 640
 constexpr int kPage = 128;
+constexpr int kPageShift = 7;
 constexpr int kRowBytes = kFeatures * 2;  // one latent row, 16-bit elements
 
 constexpr int kStatusWords = 8;

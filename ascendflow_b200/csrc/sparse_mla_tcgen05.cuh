@@ -230,66 +230,110 @@ __device__ __forceinline__ TokenGeometry token_geometry_warp(const Params& p, in
   return g;
 }
 
-// ---- slot -> physical row, one warp per token -------------------------------------------------
+// ---- slot -> physical row -----------------------------------------------------------------------
 // The selection of the reference's oracle (benchmarks/attention/sparse_reference.py:107-124) and
 // of its device routines (examples/sparse_attention/gather.py:39-60, 87-131): window slot s is
 // position right - visible + s of the raw cache; compressed rank r is kept when r < min(TOPK,
 // C, cutoff), no entry before it is negative and its index is below the cutoff; a kept entry
-// goes through the request's block table. Lane l returns slots 32 i + l in resolved[i] (the
-// physical cache row, or -1): neighbouring slots of a sorted list have neighbouring pages, so that a
-// load of the table touches few sectors. This one routine serves the attention kernel (its resolver
-// warp) and the index-set export (`resolve_rows_kernel`), so that the exported set is the gathered set.
-__device__ __forceinline__ void resolve_token_warp(const Params& p, int token, int lane, int (&resolved)[kSlots / 32]) {
-  constexpr int kWindowSteps = kWindow / 32, kListSteps = kTopK / 32;
+// goes through the request's block table. A warp resolves kWindowSteps x 32 slots of the window (all of it or
+// none) and kListSteps x 32 ranks of the list from `first_rank` on; lane l returns the l-th of every 32 in
+// `resolved` (the physical cache row, or -1): neighbouring slots of a sorted list have neighbouring pages, so that
+// a load of the table touches few sectors. `others_end` tells, given the rank of the first negative entry among the
+// warp's own (kTopK when it has none), that among the other warps' ranks of the list.
+//
+// Everybody resolves through this one routine: one warp for all of a token (`resolve_token_warp`), five warps for
+// the first token of a block (`resolve_first_part`), and the index-set export (`resolve_rows_kernel`) in the form
+// that gathers the token, so that the exported set is the gathered set.
+template <int kWindowSteps, int kListSteps, typename OthersEnd>
+__device__ __forceinline__ void resolve_slots(const Params& p, int token, int lane, int first_rank, OthersEnd others_end, int (&resolved)[kWindowSteps + kListSteps]) {
+  constexpr int kSteps = kWindowSteps + kListSteps;
+  static_assert(kWindowSteps == 0 || kWindowSteps * 32 == kWindow, "a window is not split");
   // The index list does not depend on the geometry: its loads go out first.
-  const int32_t* list = p.indices + (size_t)token * kTopK + lane;
-  int index[kListSteps];
+  const int32_t* list = p.indices + (size_t)token * kTopK + first_rank + lane;
+  int place[kSteps];  // position in the raw cache, or entry of the list
 #pragma unroll
-  for (int i = 0; i < kListSteps; ++i) index[i] = __ldg(list + i * 32);
+  for (int i = kWindowSteps; i < kSteps; ++i) place[i] = __ldg(list + (i - kWindowSteps) * 32);
   const TokenGeometry g = token_geometry_warp(p, token, lane);
   int first = kTopK;
 #pragma unroll
-  for (int i = kListSteps - 1; i >= 0; --i)
-    if (index[i] < 0) first = i * 32 + lane;
-  const int first_negative = __reduce_min_sync(0xffffffffu, first);
+  for (int i = kSteps - 1; i >= kWindowSteps; --i)
+    if (place[i] < 0) first = first_rank + (i - kWindowSteps) * 32 + lane;
+  const int own_end = kListSteps == 0 ? kTopK : __reduce_min_sync(0xffffffffu, first);
   const int cmp_shift = p.cmp_page == 64 ? 6 : 7;  // cmp_page is 64 or 128: shift and mask instead of a run-time division
   // Two passes so that all block-table loads are in flight together (a branch or vote between
-  // them would serialise twenty dependent round trips to memory): columns and loads, rows.
+  // them would serialise dependent round trips to memory): columns and loads, rows.
   const int first_position = g.right - g.visible + lane;
-  const int rank_end = min(g.bound, first_negative);
+  const int rank_end = min(g.bound, own_end);
   const int32_t* ori_table = p.ori_table + (size_t)g.batch * p.pages;
   const int32_t* cmp_table = p.cmp_table + (size_t)g.batch * p.pages;
-  int column[kSlots / 32];  // -1: not live
+  int column[kSteps];  // -1: not live
 #pragma unroll
-  for (int i = 0; i < kSlots / 32; ++i) {
+  for (int i = 0; i < kSteps; ++i) {
     const bool window = i < kWindowSteps;
-    const int slot = i * 32 + lane, rank = slot - kWindow, entry = index[window ? 0 : i - kWindowSteps];
-    const bool live = window ? slot < g.visible : rank < rank_end && entry < g.cutoff;
-    column[i] = !live ? -1 : window ? (first_position + i * 32) / kPage : entry >> cmp_shift;
+    const int rank = first_rank + (i - kWindowSteps) * 32 + lane;
+    if (window) place[i] = first_position + i * 32;
+    const bool live = window ? i * 32 + lane < g.visible : rank < rank_end && place[i] < g.cutoff;
+    column[i] = live ? place[i] >> (window ? kPageShift : cmp_shift) : -1;
     resolved[i] = __ldg((window ? ori_table : cmp_table) + min(unsigned(column[i]), unsigned(p.pages - 1)));  // the page, for now
   }
+  const int end = kListSteps == 0 ? kTopK : others_end(own_end);
   bool bad = false;
 #pragma unroll
-  for (int i = 0; i < kSlots / 32; ++i) {
+  for (int i = 0; i < kSteps; ++i) {
     const bool window = i < kWindowSteps;
-    const int blocks = window ? p.ori_blocks : p.cmp_blocks, page_rows = window ? kPage : p.cmp_page;
-    const int within = window ? (first_position + i * 32) % kPage : index[window ? 0 : i - kWindowSteps] & (p.cmp_page - 1);
-    const bool live = column[i] >= 0;
+    const int blocks = window ? p.ori_blocks : p.cmp_blocks, shift = window ? kPageShift : cmp_shift;
+    const bool live = column[i] >= 0 && (window || first_rank + (i - kWindowSteps) * 32 + lane < end);
     const bool legal = column[i] < p.pages && (unsigned)resolved[i] < (unsigned)blocks;
     bad |= live && !legal;
-    resolved[i] = live && legal ? resolved[i] * page_rows + within : -1;
+    resolved[i] = live && legal ? (resolved[i] << shift) + (place[i] & ((1 << shift) - 1)) : -1;
   }
   if (bad) report(p, kStatusBadPage, token, lane);
 }
 
-// The gathered index set of every token, written out: one warp per token runs the routine the
-// attention kernel's resolver warp runs.
-__global__ void resolve_rows_kernel(const Params p, int32_t* out) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int token = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; token < p.tokens; token += warps) {
+// All slots of a token by one warp: slot 32 i + lane in resolved[i].
+__device__ __forceinline__ void resolve_token_warp(const Params& p, int token, int lane, int (&resolved)[kSlots / 32]) {
+  resolve_slots<kWindow / 32, kTopK / 32>(p, token, lane, 0, [](int) { return kTopK; }, resolved);
+}
+
+// A token by five warps: the window by one, a quarter of the list by each of warps 0 to 3, which tell each other through
+// `first_negative` (one word each) and named barrier 1 where the list ends.
+constexpr int kFirstParts = 4;
+constexpr int kFirstSlots = kWindow / 32;  // per lane
+static_assert(kTopK == kFirstParts * kWindow, "five parts of 128 slots");
+template <bool window>
+__device__ __forceinline__ void resolve_first_part(const Params& p, int token, volatile int* first_negative, int (&resolved)[kFirstSlots]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  resolve_slots<window ? kFirstSlots : 0, window ? 0 : kFirstSlots>(p, token, lane, window ? 0 : warp * kWindow, [&](int own) {
+    if (lane == 0) first_negative[warp] = own;
+    named_barrier_sync(1, kFirstParts * 32);
+    int all = first_negative[0];
+#pragma unroll
+    for (int w = 1; w < kFirstParts; ++w) all = min(all, first_negative[w]);
+    return all;
+  }, resolved);
+}
+
+// The gathered index set of every token, written out, every token resolved as in a call of this many: the first token
+// of each of its `firsts` blocks (clusters take a token each, persistent blocks `token_group` in the first round) by
+// the five warps of a block here, the others by a warp each.
+constexpr int kExportWarps = kFirstParts + 1;
+__global__ void resolve_rows_kernel(const Params p, int firsts, int32_t* out) {
+  __shared__ int first_negative[kFirstParts];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (int(blockIdx.x) < firsts) {
+    const int token = int(blockIdx.x) * p.token_group, part = warp == kFirstParts ? 0 : warp + 1;
+    int resolved[kFirstSlots];
+    if (warp == kFirstParts) resolve_first_part<true>(p, token, first_negative, resolved);
+    else resolve_first_part<false>(p, token, first_negative, resolved);
+#pragma unroll
+    for (int i = 0; i < kFirstSlots; ++i) out[(size_t)token * kSlots + part * kWindow + i * 32 + lane] = resolved[i];
+    return;
+  }
+  const unsigned warps = (gridDim.x - firsts) * kExportWarps;
+  for (unsigned token = (blockIdx.x - firsts) * kExportWarps + warp; token < unsigned(p.tokens); token += warps) {
+    if (token % p.token_group == 0 && token / p.token_group < unsigned(firsts)) continue;
     int resolved[kSlots / 32];
-    resolve_token_warp(p, token, lane, resolved);
+    resolve_token_warp(p, int(token), lane, resolved);
 #pragma unroll
     for (int i = 0; i < kSlots / 32; ++i) out[(size_t)token * kSlots + i * 32 + lane] = resolved[i];
   }
@@ -329,56 +373,23 @@ __device__ __forceinline__ void publish_token(const Params& p, const Shared& sm,
 // it: with its instructions fetched beforehand it was hardly faster). 64 x 6 tokens at 128K 64.5 -> 62.0 us, 256
 // tokens at 4K 31.1 -> 30.4. The rows and chunks are those of `publish_token`. One instantiation per kind of
 // warp, each inside its role: a common one in front of the roles cost the loops behind it 3 %.
-constexpr int kFirstThreads = (kSoftmaxWarps + 1) * 32;
-constexpr int kFirstSlots = kWindow / 32;  // per lane
-static_assert(kTopK == kSoftmaxWarps * kWindow, "five parts of 128 slots");
+constexpr int kFirstThreads = (kFirstParts + 1) * 32;
+static_assert(kFirstParts == kSoftmaxWarps, "warps 0 to 3 are the softmax warps");
 template <bool window>
 __device__ __forceinline__ void publish_first_token(const Params& p, const Shared& sm, int token, uint32_t ready_bar) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int first_rank = warp * kWindow + lane;  // (list warps)
   TokenInfo* info = sm.info(0);
-  int index[kFirstSlots];
-  if (!window) {
-#pragma unroll
-    for (int i = 0; i < kFirstSlots; ++i) index[i] = __ldg(p.indices + (size_t)token * kTopK + first_rank + i * 32);
-  }
-  const TokenGeometry g = token_geometry_warp(p, token, lane);
-  const int first_position = g.right - g.visible + lane;
-  const int shift = window || p.cmp_page != 64 ? 7 : 6;
-  const int32_t* table = (window ? p.ori_table : p.cmp_table) + (size_t)g.batch * p.pages;
-  const int blocks = window ? p.ori_blocks : p.cmp_blocks;
-  int column[kFirstSlots], page[kFirstSlots];  // column: -1 where not live
-  int negative = kTopK;                        // rank of the list's first negative entry
-#pragma unroll
-  for (int i = kFirstSlots - 1; i >= 0; --i) {
-    if (window) index[i] = first_position + i * 32;
-    else if (index[i] < 0) negative = first_rank + i * 32;
-    const bool live = window ? lane + i * 32 < g.visible : index[i] >= 0 && index[i] < g.cutoff && first_rank + i * 32 < g.bound;
-    column[i] = live ? index[i] >> shift : -1;
-    page[i] = __ldg(table + min(unsigned(column[i]), unsigned(p.pages - 1)));
-  }
-  negative = __reduce_min_sync(0xffffffffu, negative);
-  if (!window && lane == 0) sm.first_negative()[warp] = negative;
-  named_barrier_sync(1, kFirstThreads);
-  if (!window) {
-#pragma unroll
-    for (int w = 0; w < kSoftmaxWarps; ++w) negative = min(negative, sm.first_negative()[w]);
-  }
   const int part = window ? 0 : warp + 1;
   int* rows = sm.rows(0) + part * kWindow + lane;
-  bool bad = false;
+  int resolved[kFirstSlots];
+  resolve_first_part<window>(p, token, sm.first_negative(), resolved);
   unsigned mask[kFirstSlots];
 #pragma unroll
   for (int i = 0; i < kFirstSlots; ++i) {
-    const bool live = column[i] >= 0 && (window || first_rank + i * 32 < negative);
-    const bool legal = column[i] < p.pages && (unsigned)page[i] < (unsigned)blocks;
-    bad |= live && !legal;
-    const int row = live && legal ? (page[i] << shift) + (index[i] & ((1 << shift) - 1)) : -1;
-    rows[i * 32] = row;
-    mask[i] = __ballot_sync(0xffffffffu, row >= 0);
+    rows[i * 32] = resolved[i];
+    mask[i] = __ballot_sync(0xffffffffu, resolved[i] >= 0);
   }
   if (lane < 2) info->live[part * 2 + lane] = lane == 0 ? make_uint2(mask[0], mask[1]) : make_uint2(mask[2], mask[3]);
-  if (bad) report(p, kStatusBadPage, token, lane);
   if (!window) {
     named_barrier_arrive(2, kFirstThreads);
     return;
@@ -1068,6 +1079,16 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
   if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemColumns);
 }
 
+// How a call's tokens are dealt to the persistent blocks (see `TokenWalk`).
+inline int persistent_blocks(const Params& p, int multiprocessors) { return p.tokens < multiprocessors ? p.tokens : multiprocessors; }
+inline void deal_tokens(Params& p, int grid) {
+  const int per_block = p.tokens / (grid * 4);
+  p.token_group = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
+  const int rest = p.tokens % (grid * p.token_group);
+  p.whole_rounds = p.tokens - rest;
+  p.last_group = (rest + grid - 1) / grid;
+}
+
 template <int kFormat>
 inline int launch(const Params& p, cudaStream_t stream, int multiprocessors) {
   static bool configured[64] = {false};
@@ -1080,13 +1101,9 @@ inline int launch(const Params& p, cudaStream_t stream, int multiprocessors) {
     if (error != cudaSuccess) return int(error);
     configured[device] = true;
   }
-  const int grid = p.tokens < multiprocessors ? p.tokens : multiprocessors;
+  const int grid = persistent_blocks(p, multiprocessors);
   Params launch_params = p;
-  const int per_block = p.tokens / (grid * 4);
-  launch_params.token_group = per_block < 1 ? 1 : (per_block > 8 ? 8 : per_block);
-  const int rest = p.tokens % (grid * launch_params.token_group);
-  launch_params.whole_rounds = p.tokens - rest;
-  launch_params.last_group = (rest + grid - 1) / grid;
+  deal_tokens(launch_params, grid);
   return int(launch_overlapped(attention_kernel<kFormat>, grid, kThreads, kSmemBytes, stream, launch_params));
 }
 

@@ -138,9 +138,10 @@ int launch_sparse_mla_warp_mma(void* stream, void* arg_q, void* arg_ori_kv, void
 /* ---- Gathered index set export -------------------------------------------------------------
  * Writes, for every token and slot 0..639, the physical cache row the attention kernel gathers
  * (a row of ori_kv viewed as [ORI_BLOCKS*128, 512] for slots < 128, a row of cmp_kv viewed as
- * [CMP_BLOCKS*CMP_PAGE, 512] for the rest) or -1 for a masked slot. One warp per token runs
- * `resolve_token_warp`, the device routine that the resolver warp of the tcgen05 attention
- * kernels (launch_sparse_mla, launch_sparse_mla_f16) runs for every token it gathers; the
+ * [CMP_BLOCKS*CMP_PAGE, 512] for the rest) or -1 for a masked slot. The device routine is the one that the
+ * tcgen05 attention kernels (launch_sparse_mla, launch_sparse_mla_f16) gather by, `resolve_slots`,
+ * and every token is resolved in the form in which a call of this many tokens has it: the first token
+ * of each block by five warps, the others by one; the
  * warp-MMA cross-check kernel keeps its own block-wide routine. The reference checks the same fact by
  * reading back its gather workspace (benchmarks/attention/run_sparse.py:111-130, 253-262);
  * this kernel keeps gathered rows on chip, so the set is exported instead.

@@ -36,3 +36,10 @@ def test_waits_for_other_blocks_acquire_at_cluster_scope():
     wrappers = (CSRC / "tcgen05_ptx.cuh").read_text()
     body = wrappers[wrappers.index("bool mbar_try_wait("):]
     assert "mbarrier.try_wait.parity.acquire.cluster." in body[: body.index("\n}\n")]
+
+
+def test_slots_are_resolved_by_one_routine():
+    """The rule from slot to row stands once beside the tcgen05 kernels, and all forms of resolving a token run it."""
+    source = (CSRC / "sparse_mla_tcgen05.cuh").read_text()
+    assert source.count("report(p, kStatusBadPage") == 1
+    assert "kStatusBadPage" not in (CSRC / "sparse_mla_team.cuh").read_text()
