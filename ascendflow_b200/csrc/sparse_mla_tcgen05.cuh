@@ -39,7 +39,6 @@
 #pragma once
 
 #include <cuda_bf16.h>
-#include <type_traits>
 #include <cuda_fp16.h>
 
 #include "sparse_mla_common.cuh"

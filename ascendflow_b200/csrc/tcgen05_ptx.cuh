@@ -231,16 +231,6 @@ __device__ __forceinline__ void mma_ws_ss_c(uint32_t d_tmem, uint64_t a_desc, ui
         "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc) : "memory");
   }
 }
-// The weight-stationary form for a whole warp: the lane with `issuer` set issues.
-__device__ __forceinline__ void mma_ws_ss_if(uint32_t issuer, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.b32 q, %0, 0;\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "@q tcgen05.mma.ws.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n"
-      "}\n" ::"r"(issuer), "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // Arrive on `bar` once all tcgen05.mma issued so far by this thread have completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
