@@ -7,7 +7,7 @@
 // order, as the reference does: examples/sparse_attention/attention.py:42-64, 147-207). The
 // chunks of all the block's tokens form one stream; the issue order is QK(c + 1), PV(c).
 //
-//   resolver warp    resolves slot -> physical row (sparse_mla_common.cuh) up to two tokens ahead.
+//   resolver warp    resolves slot -> physical row (`resolve_slots`) up to two tokens ahead.
 //   producer warps   gather the token's rows with 16-byte cp.async into a three-stage ring of
 //                    128-byte-swizzled shared tiles (a row is fetched once and serves as K and
 //                    V), and move the token's Q from global to tensor memory through registers.
@@ -30,9 +30,8 @@
 //   columns 384-447  the score buffer of the QK product (see `issue_qk`): the partial scores of a
 //                    lane's pairs.
 //   columns 448-463  which pairs a lane holds, as the sparse product's metadata (written once).
-// Thread (lane & 15) + 16 * half of softmax warp w owns head 16 w + (lane & 15) of that half; the
-// two lanes of a head add their partial scores with one shuffle per score and split the 64 rows
-// of the chunk between them.
+// Thread (lane & 15) + 16 * half of softmax warp w works on head 16 w + (lane & 15) and rows 32 half .. + 31 of
+// the chunk; it loads both partial scores of each.
 //
 // Every wait on an mbarrier is bounded (tcgen05_ptx.cuh): on expiry the block records
 // kStatusWaitExpired, all roles leave their loops, tensor memory is released, the kernel returns.
@@ -88,7 +87,7 @@ constexpr uint32_t kTmemQ = 256;
 constexpr uint32_t kTmemS = 384;                             // one 64-column score buffer
 constexpr uint32_t kTmemPlaces = 448;                        // which features a lane of Q holds (see `issue_qk`)
 constexpr uint32_t kTmemOHalf = 128;                         // columns of one 256-feature accumulator
-constexpr uint32_t kHalfLanes = 16u << 16;                   // lane offset of the high-half lanes in a tensor-memory address
+constexpr uint32_t kHalfLanes = 16u << 16;                   // lane offset of lanes 16-31 (the odd pairs) in a tensor-memory address
 
 struct TokenInfo {
   int token;
@@ -780,8 +779,9 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // are busy back to back. Their time is latency (tensor-memory loads, votes, shared loads that queue
 // behind the producers' copies, the special-function unit: 32 exponentials of a warp take 256
 // cycles), so nothing that is known a chunk earlier is fetched late, and additions go two to an
-// instruction. Prefill of 8192 tokens at 32K: 1038 -> 978 us; decode 128x6 at 128K: 135 -> 132 us. In a
-// steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides and not cycles.
+// instruction (with QK still a dense product: prefill of 8192 tokens at 32K 1038 -> 978 us, decode 128x6 at 128K
+// 135 -> 132; they take 850 and 113 now). In a steady loop the large calls are at the board's power limit (1.6 GHz),
+// where energy decides and not cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -904,20 +904,20 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
 
       if (!warp_wait(sm.bar(kSFull), chunk_count & 1, abort_flag)) return;
       tc_fence_after_sync();
-      // Lane (head, low half) holds the scores' sums over the even pairs of features, lane (head, high
-      // half) those over the odd pairs. The two threads of a head share the softmax work: the low
+      // Of a head's two lanes the low one (0-15) holds the scores' sums over the even pairs of features, the
+      // high one (16-31) those over the odd pairs. The two threads of a head share the softmax work: the low
       // thread owns tile rows 0-31, the high thread rows 32-63. Both partial scores of a row come
       // straight to the thread that owns it: a load over the 16 low lanes gives threads 0-15
-      // columns j and threads 16-31 columns 32 + j of the low lanes' partials; a load over the 16 high
-      // lanes gives them the same columns of the high lanes' partials. No exchange between lanes.
+      // columns j and threads 16-31 columns 32 + j of the even pairs' sums; a load over the 16 high
+      // lanes gives them the same columns of the odd pairs' sums. No exchange between lanes.
       const unsigned live = half ? live_hi : live_lo;
       const bool all_live = (live_lo & live_hi) == 0xffffffffu;  // the usual case: nothing to mask
       float2 raw[16];  // unscaled scores: the scale goes into the exponent's FMA
       {
         uint32_t low_a[16], low_b[16], high_a[16], high_b[16];
-        tmem_ld16_halves<32>(s_addr, low_a);                       // rows 0-15 | 32-47, low partial
+        tmem_ld16_halves<32>(s_addr, low_a);                       // rows 0-15 | 32-47, even pairs
         tmem_ld16_halves<32>(s_addr + 16, low_b);                  // rows 16-31 | 48-63
-        tmem_ld16_halves<32>(s_addr + kHalfLanes, high_a);         // the same rows, high partial
+        tmem_ld16_halves<32>(s_addr + kHalfLanes, high_a);         // the same rows, odd pairs
         tmem_ld16_halves<32>(s_addr + kHalfLanes + 16, high_b);
         tmem_wait_ld();
         // The scores are in registers: the next QK may overwrite the buffer. Its tile's full

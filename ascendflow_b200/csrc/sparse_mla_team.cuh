@@ -14,9 +14,9 @@
 //
 // Bound by latency. One token on one block takes 30 k cycles: 6 k until its first scores, 2 k per chunk, 3 k for
 // the output pass. Here the chunks' first product and softmax run side by side, and the output pass is a
-// quarter. Of the 19 k cycles that are left the token's resolution takes 3.5 k, gather, scores and maxima of up to
-// three chunks 5.5 k, the first P 1.3 k, the second product, in the order of the chunks, 6.5 k (and rescaling
-// where a reference moves), output 1.5 k. A call of one token 15.3 -> 10.9 us, of 16 tokens 16.3 -> 11.4
+// quarter. Of the 19 k cycles that are left the token's resolution takes 3.7 k, gather, scores and maxima of up to
+// three chunks 6 k, the first P 1.1 k, the second product, in the order of the chunks, 6.6 k (and a thousand more for
+// every chunk at which a reference moves), output 1.7 k. A call of one token 15.3 -> 11.1 us, of 16 tokens 16.3 -> 11.4
 // (one warp resolving the token, all slices gathered behind a barrier of the cluster, products issued by a whole
 // warp before). Eight blocks had less for one token, nothing for eight; P written to the other blocks by
 // the softmax threads instead of bulk copies was slower by a fifth. Copies between blocks are of local shared
@@ -137,8 +137,8 @@ __device__ __forceinline__ void gather_slices(const Params& p, const Shared& sm,
   }
 }
 
-// Phase A, producer warps: the first eight chunks' slices. They fill
-// the places of the own chunks' first two tiles, four each, which are free when these have been multiplied.
+// Phase A, producer warps: the first eight chunks' slices. They fill the places of the own chunks' first two
+// tiles, four each, which are free when these have been multiplied.
 __device__ void team_early_slices(const Params& p, const Shared& sm, int rank) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32;
   volatile int* abort_flag = sm.abort_flag();
