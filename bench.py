@@ -45,15 +45,16 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # dram__bytes_read.sum + dram__bytes_write.sum of the attention kernel per query token, from the
 # ncu captures summarised under profiles/ (prefill Q8K/ctx32K: whole launch of 8192 tokens; decode
 # B16 x 6 queries at ctx 128K: 96 tokens). Other sizes of the same regime are scaled by token
-# count, since traffic is Q + O + gathered rows per token. The figures belong to the kernel
-# sources whose hash is recorded with them: a line measured with other sources says so.
-MEASURED_TRAFFIC = {
-    "prefill": {"bytes_per_token": 1077.28e6 / 8192, "profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md",
-                "attention_kernel_sha256": "3b33bc9ebe2be71c73fb306a748106a786518f1dc2093ded2bdcf7e584ebfaff"},
-    # decode: one-pass captures of the full-size calls (768 / 384 / 96 query tokens per launch)
-    "decode": {"bytes_per_token": 500.34e6 / 768, "profile": "profiles/attention_kernel_decode_dram_traffic.md",
-               "per_launch": {768: 500.34e6, 384: 242.30e6, 96: 58.79e6},
-               "attention_kernel_sha256": "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3"},
+# count, since traffic is Q + O + gathered rows per token. Every figure belongs to the kernel
+# sources whose hash is recorded with it: a line measured with other sources says so.
+PROFILED_SOURCES = "d47db29731a055163a5544e301b9858134843884ea34ac07a4472763c2749cc4"
+FULL_SIZE_DECODE_SOURCES = "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3"
+MEASURED_TRAFFIC = {  # query tokens of the captured launches: bytes of a launch, sources
+    "prefill": {"profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md",
+                "launches": {8192: (1076.73e6, PROFILED_SOURCES)}, "scaled_from": 8192},
+    "decode": {"profile": "profiles/attention_kernel_decode_dram_traffic.md",
+               "launches": {768: (500.34e6, FULL_SIZE_DECODE_SOURCES), 384: (242.30e6, FULL_SIZE_DECODE_SOURCES),
+                            96: (58.71e6, PROFILED_SOURCES)}, "scaled_from": 768},
 }
 EXTRA_WORKLOADS = ("prefill_q32k_ctx32k", "decode_b64_q6_ctx128k", "decode_b128_q6_ctx128k")
 CONFIG_KEYS = {"heads": 64, "features": 512, "topk": 512, "window": 128, "ratio": 2, "values": "N(0,1)",
@@ -248,12 +249,13 @@ def roofline_of(config, work, ms, world, source_sha):
         record = {"bound": "tensor", "achieved": achieved, "peak": peak["bf16_tflops"], "unit": "TFLOP/s"}
     record["frac"] = record["achieved"] / record["peak"]
     traffic = MEASURED_TRAFFIC[regime]
-    measured = traffic.get("per_launch", {}).get(work["tokens"]) if world == 1 else None
-    record["traffic"] = measured if measured else traffic["bytes_per_token"] * work["tokens"] / world
+    captured = work["tokens"] if world == 1 and work["tokens"] in traffic["launches"] else traffic["scaled_from"]
+    launch_bytes, captured_sha = traffic["launches"][captured]
+    record["traffic"] = launch_bytes * work["tokens"] / captured / world
     record["traffic_source"] = (f"ncu capture summarised in {traffic['profile']}, "
-                                f"{'of this very call' if measured else 'scaled by tokens'}; captured with "
-                                f"kernel sources {traffic['attention_kernel_sha256'][:12]}"
-                                + ("" if traffic["attention_kernel_sha256"] == source_sha else
+                                f"{'of a call of this size' if world == 1 and captured == work['tokens'] else 'scaled by tokens'}; "
+                                f"captured with kernel sources {captured_sha[:12]}"
+                                + ("" if captured_sha == source_sha else
                                    f" (this run: {source_sha[:12]}, so the figure may be stale)"))
     record["peak_source"] = f"{source} (burst figure: each launch is timed alone between L2 evictions)"
     record["per_gpu"] = "achieved is per GPU: the whole call's work / GPUs / slowest rank's time"
