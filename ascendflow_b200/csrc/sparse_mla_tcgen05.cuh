@@ -99,7 +99,7 @@ static_assert(sizeof(TokenInfo) <= 128, "the info area holds two 128-byte entrie
 
 enum Bar {
   kTokenReady0 = 0, kTokenReady1, kTokenDone0, kTokenDone1, kQFull, kQFree,
-  kKvFree0, kKvFree1, kKvFree2,
+  kKvFree0, kKvFree1, kKvFree2, kKvFree3, kKvFree4, kKvFree5,  // halves of the ring stages
   kSFull, kPFull, kOFree,
   kKvFull0, kKvFull1, kKvFull2, kSoftmaxSync, kInfoRead0, kInfoRead1, kBarCount
 };
@@ -502,14 +502,16 @@ __device__ __forceinline__ void store_places(uint32_t places_tmem, int lane) {
   tmem_st16(places_tmem, columns);
 }
 
-// Copies of the 64 rows of a chunk into a tile, by the 256 producer threads.
-__device__ __forceinline__ void gather_chunk(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
+// Copies of a chunk's rows into a tile, all 64 or one half of them, by the 256 producer threads.
+template <int kHalf, int kHalves>
+__device__ __forceinline__ void gather_rows(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
+  constexpr int kRows = kChunkRows / (kProducerThreads / 16) / kHalves;  // of a thread
   const int sub = tid & 15;  // sixteen threads per row: 256 bytes at a time
-  const char* source[kChunkRows / (kProducerThreads / 16)];
-  bool live[kChunkRows / (kProducerThreads / 16)];
+  const char* source[kRows];
+  bool live[kRows];
 #pragma unroll
-  for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
-    const int slot = chunk * kChunkRows + (tid >> 4) + k * (kProducerThreads / 16);
+  for (int k = 0; k < kRows; ++k) {
+    const int slot = chunk * kChunkRows + (tid >> 4) + (kHalf * kRows + k) * (kProducerThreads / 16);
     const int row = rows[slot];
     live[k] = row >= 0;
     source[k] = static_cast<const char*>(slot < kWindow ? p.ori_kv : p.cmp_kv) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
@@ -518,8 +520,8 @@ __device__ __forceinline__ void gather_chunk(const Params& p, const int* rows, i
   for (int q = 0; q < 4; ++q) {
     const int unit = q * 16 + sub;
 #pragma unroll
-    for (int k = 0; k < kChunkRows / (kProducerThreads / 16); ++k) {
-      const int r = (tid >> 4) + k * (kProducerThreads / 16);
+    for (int k = 0; k < kRows; ++k) {
+      const int r = (tid >> 4) + (kHalf * kRows + k) * (kProducerThreads / 16);
       cp_async16(tile + swizzled(r, unit), source[k] + unit * 16, live[k]);
     }
   }
@@ -536,8 +538,8 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
   const int warp = threadIdx.x >> 5;
   const int subpartition = warp & 3, part = (warp - kFirstProducerWarp) >> 2;
   const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
-  // Ring bookkeeping: stage s is free again once the PV of the tile it held has completed
-  // (kKvFree0 + s, committed by the MMA thread). A tile is announced without anybody waiting
+  // Ring bookkeeping: the halves of stage s are free again once the PV of the tile it held has used them
+  // (kKvFree0 + 2 s and + 1, committed by the MMA thread). A tile is announced without anybody waiting
   // for it: every producer thread attaches the completion of its own copies to the stage's
   // full barrier (cp.async.mbarrier.arrive), so the threads never block on data in flight and
   // the warps need not stay in step with each other.
@@ -572,9 +574,12 @@ __device__ void producer_role(const Params& p, const Shared& sm, uint32_t tmem) 
     if (chunks == 0 && lane == 0) mbar_arrive(sm.bar(kInfoRead0 + (token_count & 1)));
     for (int item = 0; item < chunks; ++item, ++ring) {
       const uint32_t stage = ring % kStages, use = ring / kStages;
-      if (use > 0 && !warp_wait(sm.bar(kKvFree0 + stage), (use - 1) & 1, abort_flag)) return;
       const uint32_t tile = sm.base + kSmemKv + stage * kTileBytes;
-      gather_chunk(p, rows, info->chunk[item], tile, tid);
+      const int chunk = info->chunk[item];
+      if (use > 0 && !warp_wait(sm.bar(kKvFree0 + 2 * stage), (use - 1) & 1, abort_flag)) return;
+      gather_rows<0, 2>(p, rows, chunk, tile, tid);
+      if (use > 0 && !warp_wait(sm.bar(kKvFree0 + 2 * stage + 1), (use - 1) & 1, abort_flag)) return;
+      gather_rows<1, 2>(p, rows, chunk, tile, tid);
       cp_async_arrive(sm.bar(kKvFull0 + stage));
       if (item == 0 && lane == 0) mbar_arrive(sm.bar(kInfoRead0 + (token_count & 1)));
       if (item == 0) {
@@ -644,13 +649,13 @@ __device__ __forceinline__ void issue_qk(const Shared& sm, uint32_t tmem, int st
 }
 
 constexpr int kPvSteps = 2 * (kChunkRows / 16);
-template <int kFormat, int I, bool kFirst>
+template <int kFormat, int I, int kEnd, bool kFirst>
 __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc, uint64_t x_desc) {
-  if constexpr (I < kPvSteps) {
-    constexpr int h = I / (kChunkRows / 16), k = I % (kChunkRows / 16);
+  if constexpr (I < kEnd) {
+    constexpr int h = I % 2, k = I / 2;
     constexpr uint32_t offset = h * 4 * kBlockBytes + k * 2048;
     mma_ws_ss_c<!(kFirst && k == 0)>(o_tmem + h * kTmemOHalf, p_desc + ((k * 32) >> 4), x_desc + (offset >> 4), kIdescPV<kFormat>);
-    issue_pv_steps<kFormat, I + 1, kFirst>(o_tmem, p_desc, x_desc);
+    issue_pv_steps<kFormat, I + 1, kEnd, kFirst>(o_tmem, p_desc, x_desc);
   }
 }
 
@@ -658,12 +663,21 @@ __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc,
 // and 256-511): with 64 heads a plain M = 64 instruction would leave half of the pipe idle.
 // A = P from shared memory (one 128-byte row per head, 32 bytes per K = 16 step); B = X with
 // features contiguous: 64-feature blocks kBlockBytes apart, 8-row groups 1024 bytes apart.
+//
+// The tile's rows are used up in order, both products of 16 rows after each other, and its first half is
+// given back when it has been: a tile stays in the ring from its copies' issue to the end of its PV, through QK, softmax and
+// PV, and the next tile of the stage can be 320 cycles on its way by that end. Decode 128 x 6 118.2 -> 115.3 us, 64 x 6 61.1 -> 59.8,
+// prefill of 8K tokens 864 -> 846, 23 mixed requests 170.6 -> 167.1. (Quarters: 115.7, 60.5 and 864: what a wait
+// and its commit cost is what they bring.)
 template <int kFormat>
 __device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, bool accumulate) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, kBlockBytes, 1024);
   const uint64_t p_desc = smem_desc_sw128(sm.base + kSmemP, 16, 1024);
-  if (accumulate) issue_pv_steps<kFormat, 0, false>(tmem + kTmemO, p_desc, x_desc);
-  else issue_pv_steps<kFormat, 0, true>(tmem + kTmemO, p_desc, x_desc);
+  if (accumulate) issue_pv_steps<kFormat, 0, kPvSteps / 2, false>(tmem + kTmemO, p_desc, x_desc);
+  else issue_pv_steps<kFormat, 0, kPvSteps / 2, true>(tmem + kTmemO, p_desc, x_desc);
+  mma_commit(sm.bar(kKvFree0 + 2 * stage));
+  issue_pv_steps<kFormat, kPvSteps / 2, kPvSteps, false>(tmem + kTmemO, p_desc, x_desc);
+  mma_commit(sm.bar(kKvFree0 + 2 * stage + 1));
 }
 
 // Two issuing threads in two warps, one per product. Each follows its own data: the QK thread
@@ -721,8 +735,7 @@ __device__ void pv_role(const Params& p, const Shared& sm, uint32_t tmem) {
       if (i == 0 && !mbar_wait(sm.bar(kOFree), (working_tokens & 1) ^ 1, abort_flag)) return;
       tc_fence_after_sync();
       issue_pv<kFormat>(sm, tmem, stage, i != 0);
-      mma_commit(sm.bar(kKvFree0 + stage));  // frees the ring stage for the producers
-      mma_commit(sm.bar(kSoftmaxSync));      // and counts towards the softmax warps' step c + 1
+      mma_commit(sm.bar(kSoftmaxSync));  // counts towards the softmax warps' step c + 1
     }
     ++working_tokens;
   }
@@ -1041,7 +1054,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
 
   if (threadIdx.x == 0) {
     const int P = kProducerWarps, S = kSoftmaxWarps, T = kProducerThreads;
-    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, S, S, T + S, T + S, T + S, S + 1, P + 2, P + 2};
+    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, 1, 1, 1, S, S, T + S, T + S, T + S, S + 1, P + 2, P + 2};
     for (int i = 0; i < kBarCount; ++i) mbar_init(sm.bar(i), counts[i]);
     mbar_fence_init();
     *sm.abort_flag() = 0;

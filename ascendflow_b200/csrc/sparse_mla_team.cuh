@@ -97,7 +97,7 @@ __device__ void team_gather(const Params& p, const Shared& sm, uint32_t tmem, in
   for (int j = 0; j < kOwnItems; ++j) {
     const int item = rank + j * kBlocks;
     if (item >= chunks) break;
-    gather_chunk(p, rows, info->chunk[item], sm.base + kSmemKv + j * kTileBytes, tid);
+    gather_rows<0, 1>(p, rows, info->chunk[item], sm.base + kSmemKv + j * kTileBytes, tid);
     cp_async_arrive(sm.bar(kTile0 + j));
     if (j > 0) continue;
     const uint32_t q_tmem = tmem + kTmemQ + part * 64 + (uint32_t(subpartition * 32) << 16);
