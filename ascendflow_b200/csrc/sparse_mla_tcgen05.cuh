@@ -65,19 +65,20 @@ constexpr int kTileBytes = 8 * kBlockBytes;                 // 64 rows x 512 fea
 
 // Shared memory map (bytes from a 1024-aligned base).
 constexpr int kSmemKv = 0;
-// The P tile (64 heads x 64 rows, 8 KiB) and, per softmax warp, 4 KiB of epilogue staging
-// (32 x 128-byte rows). Both 1024-byte aligned like the tiles, because the swizzle is a function
-// of the address.
+// Two P tiles (64 heads x 64 rows, 8 KiB) for the chunks in turn and, per softmax warp, 2 KiB of epilogue staging
+// (16 x 128-byte rows; 16 more in the P tile that is not in use then). All 1024-byte aligned like the tiles, because
+// the swizzle is a function of the address.
 constexpr int kSmemP = kSmemKv + kStages * kTileBytes;
-constexpr int kSmemStore = kSmemP + kHeads * 128;
-constexpr int kSmemRows = kSmemStore + kSoftmaxWarps * 4096;   // int[2][640]
+constexpr int kPTileBytes = kHeads * 128;
+constexpr int kSmemStore = kSmemP + 2 * kPTileBytes;
+constexpr int kSmemRows = kSmemStore + kSoftmaxWarps * 2048;   // int[2][640]
 constexpr int kSmemInfo = kSmemRows + 2 * kSlots * 4;       // TokenInfo[2]
 constexpr int kSmemBars = kSmemInfo + 2 * 128;              // mbarriers
 constexpr int kSmemMisc = kSmemBars + 32 * 8;               // tmem slot, abort flag
-// Per-head factors handed between the softmax warps (float[2][64] each, double-buffered): a
+// Per-head factors handed between the softmax warps (float[64] and, double-buffered, float[2][64]): a
 // thread works out the softmax of one head but reads the accumulator of another (see below).
 constexpr int kSmemAlpha = kSmemMisc + 64;
-constexpr int kSmemInverse = kSmemAlpha + 2 * kHeads * 4;
+constexpr int kSmemInverse = kSmemAlpha + kHeads * 4;
 constexpr int kSmemEnd = kSmemInverse + 2 * kHeads * 4;
 constexpr int kSmemBytes = kSmemEnd + 1024;  // + slack for the 1024-byte alignment
 
@@ -100,8 +101,8 @@ static_assert(sizeof(TokenInfo) <= 128, "the info area holds two 128-byte entrie
 enum Bar {
   kTokenReady0 = 0, kTokenReady1, kTokenDone0, kTokenDone1, kQFull, kQFree,
   kKvFree0, kKvFree1, kKvFree2, kKvFree3, kKvFree4, kKvFree5,  // halves of the ring stages
-  kSFull, kPFull, kOFree,
-  kKvFull0, kKvFull1, kKvFull2, kSoftmaxSync, kInfoRead0, kInfoRead1, kBarCount
+  kSFull0, kSFull1, kPFull0, kPFull1, kOFree,
+  kKvFull0, kKvFull1, kKvFull2, kPvDone, kOutReady, kInfoRead0, kInfoRead1, kBarCount
 };
 static_assert(kBarCount <= 32, "the barrier area holds 32 mbarriers");
 
@@ -115,8 +116,8 @@ __device__ __forceinline__ uint32_t swizzled(int row, int unit) {
   return (unit >> 3) * kBlockBytes + row * 128 + (((unit & 7) ^ (row & 7)) << 4);
 }
 
-// The P tile (64 heads x 64 rows of 16-bit probabilities, K-major, 128-byte swizzle: one
-// 128-byte row per head): byte offset of 16-byte unit `unit` (0..7) of head `head` from kSmemP.
+// A P tile (64 heads x 64 rows of 16-bit probabilities, K-major, 128-byte swizzle: one
+// 128-byte row per head): byte offset of 16-byte unit `unit` (0..7) of head `head`.
 __device__ __forceinline__ uint32_t p_offset(int head, int unit) {
   return head * 128 + ((unit ^ (head & 7)) << 4);
 }
@@ -136,6 +137,9 @@ struct Shared {
   }
   __device__ __forceinline__ volatile uint32_t* rescale_mask() const {  // (team kernel)
     return reinterpret_cast<volatile uint32_t*>(ptr + kSmemMisc + 8);
+  }
+  __device__ __forceinline__ volatile int* softmax_failed() const {  // a softmax warp's wait has given up
+    return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 12);
   }
   __device__ __forceinline__ volatile int* first_negative() const {  // one per softmax warp
     return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 16);
@@ -670,9 +674,9 @@ __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc,
 // prefill of 8K tokens 864 -> 846, 23 mixed requests 170.6 -> 167.1. (Quarters: 115.7, 60.5 and 864: what a wait
 // and its commit cost is what they bring.)
 template <int kFormat>
-__device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, bool accumulate) {
+__device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, int p_tile, bool accumulate) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, kBlockBytes, 1024);
-  const uint64_t p_desc = smem_desc_sw128(sm.base + kSmemP, 16, 1024);
+  const uint64_t p_desc = smem_desc_sw128(sm.base + kSmemP + p_tile * kPTileBytes, 16, 1024);
   if (accumulate) issue_pv_steps<kFormat, 0, kPvSteps / 2, false>(tmem + kTmemO, p_desc, x_desc);
   else issue_pv_steps<kFormat, 0, kPvSteps / 2, true>(tmem + kTmemO, p_desc, x_desc);
   mma_commit(sm.bar(kKvFree0 + 2 * stage));
@@ -687,8 +691,8 @@ __device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int st
 // each, far beyond what the pipe's short queue covers) run while the other thread's product
 // executes. Both walk the same token and chunk sequence as everybody else.
 
-// S = Q X^T: chunk c of the block's chunk stream uses ring stage c % kStages and the c-th phase of
-// the score barrier.
+// S = Q X^T: chunk c of the block's chunk stream uses ring stage c % kStages and score barrier c % 2 (the buffer is one;
+// two barriers tell phases two chunks apart from each other).
 template <int kFormat>
 __device__ void qk_role(const Params& p, const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
@@ -710,7 +714,7 @@ __device__ void qk_role(const Params& p, const Shared& sm, uint32_t tmem) {
       if (!wait_for_copies(sm.bar(kKvFull0 + stage), (chunk_count / kStages) & 1, abort_flag)) return;
       tc_fence_after_sync();
       issue_qk<kFormat>(sm, tmem, stage);
-      mma_commit(sm.bar(kSFull));
+      mma_commit(sm.bar(kSFull0 + (chunk_count & 1)));
       if (i + 1 == chunks) mma_commit(sm.bar(kQFree));  // the last QK that reads this token's Q
       if (i == 0) mbar_arrive(sm.bar(kInfoRead0 + (token_count & 1)));  // chunk count read (see resolver)
     }
@@ -731,11 +735,14 @@ __device__ void pv_role(const Params& p, const Shared& sm, uint32_t tmem) {
     if (chunks == 0) continue;
     for (int i = 0; i < chunks; ++i, ++chunk_count) {
       const uint32_t stage = chunk_count % kStages;
-      if (!mbar_wait(sm.bar(kPFull), chunk_count & 1, abort_flag)) return;
+      const int p_tile = chunk_count & 1;
+      if (!mbar_wait(sm.bar(kPFull0 + p_tile), (chunk_count >> 1) & 1, abort_flag)) return;
       if (i == 0 && !mbar_wait(sm.bar(kOFree), (working_tokens & 1) ^ 1, abort_flag)) return;
       tc_fence_after_sync();
-      issue_pv<kFormat>(sm, tmem, stage, i != 0);
-      mma_commit(sm.bar(kSoftmaxSync));  // counts towards the softmax warps' step c + 1
+      issue_pv<kFormat>(sm, tmem, stage, p_tile, i != 0);
+      mma_commit(sm.bar(kSFull0 + p_tile));  // the P tile is free: half of what the softmax warps wait for at chunk c + 2
+      mma_commit(sm.bar(kPvDone));
+      if (i + 1 == chunks) mma_commit(sm.bar(kOutReady));  // O is complete
     }
     ++working_tokens;
   }
@@ -791,13 +798,16 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
   return d;
 }
 
-// What paces the kernel: from scores ready to P handed over, and back to the next scores, these warps
-// are busy back to back. Their time is latency (tensor-memory loads, votes, shared loads that queue
-// behind the producers' copies, the special-function unit: 32 exponentials of a warp take 256
-// cycles), so nothing that is known a chunk earlier is fetched late, and additions go two to an
-// instruction (with QK still a dense product: prefill of 8192 tokens at 32K 1038 -> 978 us, decode 128x6 at 128K
-// 135 -> 132; they take 850 and 113 now). In a steady loop the large calls are at the board's power limit (1.6 GHz),
-// where energy decides and not cycles.
+// What paces the kernel. Inside of a token a chunk takes 1.75 k cycles, and shared memory is what it takes them for: a tile
+// is written once (64 KiB), read by QK and by PV (64 each), and P is written and read (8 and 16): 216 KiB at 128 bytes
+// per cycle are 1.69 k. (The products' instructions, 704 and 640 cycles by themselves, take 920 each beside the copies.)
+// From scores to P handed over these warps need 1.35 k; nothing that is known a chunk earlier is fetched late, and additions
+// go two to an instruction. Between two tokens lie 4 to 5 k cycles more: the output leaves the SM at 32 bytes per cycle (2.05 k for
+// 64 KiB, by stores or bulk copies alike), and the conversion to 16 bits before it takes 1.7 k.
+//
+// A second P tile takes the wait for the previous PV out of the chain, and flags by named barriers a word in shared memory and a
+// wait: 256 tokens at 4K 30.0 -> 28.5 us, 100 tokens 16.9 -> 15.9, 1000 tokens 106.7 -> 104.4, prefill of 8K tokens 840 -> 832.
+// In a steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides and not cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -822,48 +832,45 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   __syncwarp();
   // The score buffer starts out free (first chunk, stage 0), and the metadata is in place.
   if (lane == 0) mbar_arrive(sm.bar(kKvFull0));
-  // Step c (c >= 1) of this block's chunk stream is one phase of one barrier: it completes once
-  // all four softmax warps have published what they hand each other for chunk c (rescale factors,
-  // or the finished token's reciprocal denominators) AND the PV of chunk c - 1 has completed
-  // (the MMA thread commits every PV to it). A warp arrives as early as it can and waits, once,
-  // right before it needs the others' values, O, or the P tile: one wait per chunk for all three.
-  uint32_t steps_arrived = 0, steps_waited = 0;  // steps 1 .. n are done
-  auto step_arrive = [&](uint32_t step) {
-    if (steps_arrived >= step) return;
+  // What the four warps tell each other goes through named barriers: P for chunk c needs no wait but that for the scores (its
+  // barrier counts the end of PV c - 2, which read the same P tile), and a barrier that reduces a flag costs
+  // less than the round trips to shared memory, behind the producers' copies, that an mbarrier and a word would be.
+  // Nobody may be left waiting at one. A warp whose wait gives up says so at the next reduction, and all four leave
+  // behind it.
+  volatile int* failed_word = sm.softmax_failed();
+  bool failed = false;
+  auto give_up = [&]() {
+    failed = true;
+    if (lane == 0) *failed_word = 1;
     __syncwarp();
-    if (lane == 0) mbar_arrive(sm.bar(kSoftmaxSync));
-    steps_arrived = step;
   };
-  auto step_wait = [&](uint32_t step) -> bool {
-    if (steps_waited >= step) return true;
-    if (!warp_wait(sm.bar(kSoftmaxSync), (step - 1) & 1, abort_flag)) return false;
-    steps_waited = step;
-    return true;
-  };
+  auto anybody = [&](bool flag) { return named_barrier_any(3, 32 * kSoftmaxWarps, flag || failed); };
 
   // A finished token waits for its epilogue until the first chunk of the next working token has
   // been through the softmax, so that the MMA thread has a P to go on with while O is written out.
+  uint32_t outputs = 0;         // epilogues so far
   int done_token = -1;          // token whose O is complete (or about to be) and not yet stored
   uint32_t done_count = 0;      // its index in this block's walk
 
   // O / denominator -> 16-bit -> global for `done_token`: 64 columns per pass, tensor memory ->
   // registers -> a swizzled per-warp staging tile -> global, so that every store instruction
   // writes four complete 128-byte lines.
-  auto epilogue = [&]() -> bool {
-    // The token's last PV and everybody's reciprocal denominators: step `chunk_count`. After the
-    // next token's first chunk that step has been waited for already.
-    step_arrive(chunk_count);
-    if (!step_wait(chunk_count)) return false;
+  // `chunks_before`: chunks of the stream whose PV precedes. Everybody's reciprocal denominators are there (a reduction lies between).
+  auto epilogue = [&](uint32_t chunks_before) {
+    if (!warp_wait(sm.bar(kOutReady), outputs & 1, abort_flag)) { give_up(); return; }
+    ++outputs;
     tc_fence_after_sync();
     const float inverse = inverse_exchange[(done_count & 1) * kHeads + o_head];
-    unsigned char* staging = sm.ptr + kSmemStore + warp * 4096;
+    // Rows 0-15 of the staging tile lie in the warp's own 2 KiB, rows 16-31 where its own heads' rows of the unused P tile are.
+    unsigned char* staging_low = sm.ptr + kSmemStore + warp * 2048;
+    unsigned char* staging_high = sm.ptr + kSmemP + ((chunks_before & 1) ^ 1) * kPTileBytes + warp * 2048;
+    unsigned char* staging_row = (half ? staging_high : staging_low) + (lane & 15) * 128;
     __nv_bfloat16* token_out = out_base + (size_t)done_token * kHeads * kFeatures;
+    uint32_t o[64];  // loaded a pass ahead
+#pragma unroll
+    for (int q = 0; q < 64; q += 16) tmem_ld16(tmem + kTmemO + q + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[q]));
 #pragma unroll 1
     for (int c = 0; c < 256; c += 64) {
-      uint32_t o[64];
-#pragma unroll
-      for (int q = 0; q < 64; q += 16)
-        tmem_ld16(tmem + kTmemO + c + q + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[q]));
       tmem_wait_ld();
       if (c == 192) {  // O has been read completely: the next token's first PV may overwrite it
         tc_fence_before_sync();
@@ -877,13 +884,17 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         v.y = pack_pair<kFormat>(__uint_as_float(o[unit * 8 + 2]) * inverse, __uint_as_float(o[unit * 8 + 3]) * inverse);
         v.z = pack_pair<kFormat>(__uint_as_float(o[unit * 8 + 4]) * inverse, __uint_as_float(o[unit * 8 + 5]) * inverse);
         v.w = pack_pair<kFormat>(__uint_as_float(o[unit * 8 + 6]) * inverse, __uint_as_float(o[unit * 8 + 7]) * inverse);
-        *reinterpret_cast<uint4*>(staging + lane * 128 + ((unit ^ (lane & 7)) << 4)) = v;
+        *reinterpret_cast<uint4*>(staging_row + ((unit ^ (lane & 7)) << 4)) = v;
+      }
+      if (c < 192) {
+#pragma unroll
+        for (int q = 0; q < 64; q += 16) tmem_ld16(tmem + kTmemO + c + 64 + q + lane_base, *reinterpret_cast<uint32_t(*)[16]>(&o[q]));
       }
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = i * 4 + (lane >> 3), unit = lane & 7;  // staging row = owning lane
-        const uint4 v = *reinterpret_cast<const uint4*>(staging + row * 128 + ((unit ^ (row & 7)) << 4));
+        const uint4 v = *reinterpret_cast<const uint4*>((i < 4 ? staging_low : staging_high) + (row & 15) * 128 + ((unit ^ (row & 7)) << 4));
         // accumulator columns 0-127: features 0-255 (this warp's 128 of them), 128-255: 256-511
         __nv_bfloat16* dst = token_out + (size_t)((warp & 1) * 32 + row) * kFeatures + (c >> 7) * 256 + o_feature + (c & 127) + unit * 8;
         __stcs(reinterpret_cast<uint4*>(dst), v);  // written once, read by nobody here
@@ -892,18 +903,25 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
     }
     if (lane == 0) mbar_arrive(sm.bar(kTokenDone0 + (done_count & 1)));
     done_token = -1;
-    return true;
   };
 
   TokenWalk walk(p);
-  for (int token = walk.next(); token >= 0; token = walk.next(), ++token_count) {
-    if (!warp_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) return;
+  for (int token = walk.next();; token = walk.next(), ++token_count) {
     const TokenInfo* info = sm.info(token_count & 1);
-    const int chunks = info->chunks;
-    if (chunks == 0) {  // nothing visible: the output row is zero whatever the sink
-      // The resolver needs the finished token's row buffer back before it can publish the token
-      // after this one: no point in holding its epilogue any longer.
-      if (done_token >= 0 && !epilogue()) return;
+    int chunks = 0;
+    if (token >= 0) {
+      if (!warp_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) { give_up(); break; }
+      chunks = info->chunks;
+    }
+    if (chunks == 0) {
+      // No chunk to put the finished token's output behind. (And the resolver needs the finished token's row buffer
+      // back before it can publish the token after this one: no point in holding its epilogue any longer.)
+      if (done_token >= 0) {
+        if (anybody(false)) return;
+        epilogue(chunk_count);
+      }
+      if (token < 0) break;
+      // nothing visible: the output row is zero whatever the sink
       __nv_bfloat16* out = out_base + ((size_t)token * kHeads + head) * kFeatures + half * 256;
       for (int i = 0; i < 256; i += 8) *reinterpret_cast<uint4*>(out + i) = make_uint4(0, 0, 0, 0);
       __syncwarp();
@@ -918,7 +936,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       const unsigned live_lo = next_live.x, live_hi = next_live.y;
       next_live = info->live[min(i + 1, kMaxChunks - 1)];  // a chunk ahead: shared loads queue behind the producers' copies
 
-      if (!warp_wait(sm.bar(kSFull), chunk_count & 1, abort_flag)) return;
+      if (!warp_wait(sm.bar(kSFull0 + (chunk_count & 1)), (chunk_count >> 1) & 1, abort_flag)) { give_up(); anybody(true); return; }
       tc_fence_after_sync();
       // Of a head's two lanes the low one (0-15) holds the scores' sums over the even pairs of features, the
       // high one (16-31) those over the odd pairs. The two threads of a head share the softmax work: the low
@@ -956,20 +974,6 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
           if (!(live >> (2 * e + 1) & 1u)) raw[e].y = -INFINITY;
         }
       }
-      float2 prob[16];
-      float chunk_sum;
-      auto exponentials = [&]() {
-        const float2 scale = make_float2(p.scale_log2, p.scale_log2), reference = make_float2(-run_max, -run_max);
-        float2 sum_a = make_float2(0.f, 0.f), sum_b = sum_a;  // four partial sums
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          prob[e] = fma_pair(raw[e], scale, reference);
-          prob[e].x = exp2f(prob[e].x);
-          prob[e].y = exp2f(prob[e].y);
-          if (e & 1) sum_b = add_pair(sum_b, prob[e]); else sum_a = add_pair(sum_a, prob[e]);
-        }
-        chunk_sum = (sum_a.x + sum_a.y) + (sum_b.x + sum_b.y);
-      };
       float partial_max[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -985,31 +989,35 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       float alpha = 1.f;
       if (__any_sync(0xffffffffu, own_max > run_max + kReferenceRoom))
         alpha = move_reference(run_max, fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16)));
-      if (i > 0) {
-        // O holds earlier chunks. The factor of a head is known to the thread that has its scores;
-        // the head's accumulator rows are in other threads' lanes: hand the factors over.
-        // They are picked up after the exponentials, when everybody's have long been written.
-        if (half == 0) alpha_exchange[(chunk_count & 1) * kHeads + head] = alpha;
-      }
-      if (chunk_count > 0) step_arrive(chunk_count);
-      exponentials();
-      run_sum = run_sum * alpha + chunk_sum;
-      // There is one P tile: the previous chunk's PV must have finished reading it. (In step, that
-      // PV ran right behind the QK whose scores this chunk started from.)
-      if (chunk_count > 0 && !step_wait(chunk_count)) return;
-      const float o_alpha = i > 0 ? alpha_exchange[(chunk_count & 1) * kHeads + o_head] : 1.f;  // on its way while P is packed and stored
       // P to shared memory, one 128-byte row per head; this lane writes its 32 rows (64 bytes).
+      const float2 scale = make_float2(p.scale_log2, p.scale_log2), reference = make_float2(-run_max, -run_max);
+      float2 sum_a = make_float2(0.f, 0.f), sum_b = sum_a;  // four partial sums
+      unsigned char* p_tile = sm.ptr + kSmemP + (chunk_count & 1) * kPTileBytes;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        uint4 v;
-        v.x = pack_pair<kFormat>(prob[4 * u + 0].x, prob[4 * u + 0].y); v.y = pack_pair<kFormat>(prob[4 * u + 1].x, prob[4 * u + 1].y);
-        v.z = pack_pair<kFormat>(prob[4 * u + 2].x, prob[4 * u + 2].y); v.w = pack_pair<kFormat>(prob[4 * u + 3].x, prob[4 * u + 3].y);
-        *reinterpret_cast<uint4*>(sm.ptr + kSmemP + p_offset(head, half * 4 + u)) = v;
+        uint32_t words[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const int e = 4 * u + w;
+          float2 prob = fma_pair(raw[e], scale, reference);
+          prob.x = exp2f(prob.x);
+          prob.y = exp2f(prob.y);
+          if (e & 1) sum_b = add_pair(sum_b, prob); else sum_a = add_pair(sum_a, prob);
+          words[w] = pack_pair<kFormat>(prob.x, prob.y);
+        }
+        *reinterpret_cast<uint4*>(p_tile + p_offset(head, half * 4 + u)) = make_uint4(words[0], words[1], words[2], words[3]);
       }
-      if (__any_sync(0xffffffffu, o_alpha != 1.f)) {  // the previous PV has landed (wait above)
+      run_sum = run_sum * alpha + ((sum_a.x + sum_a.y) + (sum_b.x + sum_b.y));
+      // O holds earlier chunks (if any). The factor of a head is known to the thread that has its scores;
+      // the head's accumulator rows are in other threads' lanes: where some reference moves the factors are handed over.
+      if (anybody(i > 0 && alpha != 1.f)) {
+        if (*failed_word != 0) return;
+        if (half == 0) alpha_exchange[head] = alpha;
+        named_barrier_sync(4, 32 * kSoftmaxWarps);
+        const float o_alpha = alpha_exchange[o_head];
+        if (!warp_wait(sm.bar(kPvDone), (chunk_count - 1) & 1, abort_flag)) give_up();
         tc_fence_after_sync();
-        // 32 columns at a time: a round trip to tensor memory each (in 16s the pass took 1500 cycles, and a
-        // quarter of the chunks has one in some warp; prefill of 8K tokens, one call at a time, 896 -> 859 us).
+        // 32 columns at a time: a round trip to tensor memory each (in 16s the pass took 1500 cycles).
 #pragma unroll 1
         for (int c = 0; c < 256; c += 32) {
           uint32_t o[32];
@@ -1026,9 +1034,9 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       fence_proxy_async();  // the PV reads the tile through the async proxy
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(sm.bar(kPFull));
+      if (lane == 0) mbar_arrive(sm.bar(kPFull0 + (chunk_count & 1)));
       // The previous token's output, now that the MMA thread has this token's first P to go on with.
-      if (done_token >= 0 && !epilogue()) return;
+      if (done_token >= 0) epilogue(chunk_count);
     }
     done_token = token;
     done_count = token_count;
@@ -1036,7 +1044,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
     const float own_inverse = 1.f / (run_sum + __shfl_xor_sync(0xffffffffu, run_sum, 16));
     if (half == 0) inverse_exchange[(done_count & 1) * kHeads + head] = own_inverse;
   }
-  if (done_token >= 0 && !epilogue()) return;
+  anybody(false);  // of a warp that has given up since the last one
 }
 
 // ---- kernel and launch ------------------------------------------------------------------------
@@ -1054,10 +1062,13 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
 
   if (threadIdx.x == 0) {
     const int P = kProducerWarps, S = kSoftmaxWarps, T = kProducerThreads;
-    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, 1, 1, 1, S, S, T + S, T + S, T + S, S + 1, P + 2, P + 2};
+    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, 1, 1, 2, 2, S, S, S, T + S, T + S, T + S, 1, 1, P + 2, P + 2};
     for (int i = 0; i < kBarCount; ++i) mbar_init(sm.bar(i), counts[i]);
     mbar_fence_init();
+    mbar_arrive(sm.bar(kSFull0));  // the P tiles start out free
+    mbar_arrive(sm.bar(kSFull1));
     *sm.abort_flag() = 0;
+    *sm.softmax_failed() = 0;
   }
   if (warp == kMmaWarp) { tmem_alloc(smem_u32(tmem_slot), kTmemColumns); tmem_relinquish(); }
   tc_fence_before_sync();
