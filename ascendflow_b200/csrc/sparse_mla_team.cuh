@@ -78,7 +78,7 @@ __device__ __forceinline__ void follow_reference(const volatile float* maxima, f
   float reference = sink;
 #pragma unroll
   for (int i = 0; i < kMaxChunks; ++i) {
-    const float alpha = i < chunks ? move_reference(reference, chunk_max[i]) : 1.f;
+    const float alpha = i < chunks ? move_reference(reference, chunk_max[i], i == 0) : 1.f;
     visit(i, reference, alpha);
   }
 }

@@ -1,6 +1,6 @@
-"""The softmax's running reference moves when a chunk's best row is more than 15 binades above it, to 8 below that row.
-Sinks from level with the best row to 40 binades below it, on both sides of every line; the best row alone, or behind an
-earlier one that the reference may have moved for."""
+"""The softmax's running reference moves when a chunk's best row is more than 15 binades above it, to 8 below that row, and
+with a token's first chunk to a whole number of binades off that chunk's best row. Sinks from 70 binades above the best row to
+40 below it, on both sides of every line; the best row alone, or behind an earlier one that the reference may have moved for."""
 
 import numpy as np
 import pytest
@@ -31,7 +31,8 @@ def test_sinks_far_below_the_best_row(tokens, dtype, gap):
     q[:, :, 0] = 32.0 / (4.0 * SCALE_LOG2)
     q = q.to(storage)
     best = q[0, :, 0].double() * 4.0 * SCALE_LOG2
-    sinks = ((best - torch.linspace(-1.0, 40.0, heads)) / 1.4426950408889634).float()
+    below = torch.cat([torch.linspace(-70.0, -1.5, 16), torch.linspace(-1.0, 40.0, heads - 16)])
+    sinks = ((best - below) / 1.4426950408889634).float()
 
     i32 = lambda value: torch.tensor(np.ascontiguousarray(value), dtype=torch.int32, device="cuda")  # noqa: E731
     cache = rows.cuda().view(window // 128, 128, 1, 512)
@@ -48,5 +49,6 @@ def test_sinks_far_below_the_best_row(tokens, dtype, gap):
     expected = (weights * rows[:, 1].double()).sum(1) / (weights.sum(1) + torch.exp2(sinks.double() * 1.4426950408889634 - best))
     actual = out[:, :, 1].double().cpu()
     # P and the output are each rounded once, to 11 or 8 bits: an ulp in all. The rest is FP32 (exponents of up to 40:
-    # 2^-18). A half that overflowed would be infinite, a reference that was not followed a power of two off.
-    assert (actual / expected - 1).abs().max() <= 2.0 ** (-10 if dtype == "float16" else -7)
+    # 2^-18). A half that overflowed would be infinite, a reference that was not followed a power of two off. Below a sink far
+    # above the rows a half's steps are of 2^-24: half a step for the output and for either of two probabilities.
+    assert ((actual - expected).abs() <= expected * 2.0 ** (-10 if dtype == "float16" else -7) + 1.5 * 2.0**-24).all()
