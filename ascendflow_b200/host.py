@@ -72,9 +72,10 @@ _connected = False
 
 def set_fallback(function):
     """The front end's call for what the registered op refuses."""
-    global _fallback
+    global _fallback, _connected
     _fallback = function
     calls.configure(0, 0, 0, function)
+    _connected = False  # the neighbouring steps may have handed the entry points over before this was imported
 
 
 def connect():

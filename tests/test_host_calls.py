@@ -128,3 +128,21 @@ def test_host_library_is_identified_by_its_command_and_replaced_as_a_whole(tmp_p
     assert library.read_bytes() == b"built\n" and library.stat().st_ino != inode
     assert build.HOST_STAMP.read_text() == build._host_identity()
     assert sorted(path.name for path in tmp_path.iterdir()) == ["_host_calls.so", "_host_calls.stamp", "compiler"]
+
+
+def test_entry_points_are_handed_over_again_when_the_front_end_comes_last(monkeypatch):
+    """A program that selects or appends before it imports the operator: the operator's import clears the entry points, and
+    calls went through the Python front end for good, whose reports `ops.status()` does not read."""
+    class Recorder:
+        def configure(self, *given):
+            self.given = given
+
+    recorder, fallback = Recorder(), object()
+    monkeypatch.setattr(host, "calls", recorder)
+    monkeypatch.setattr(host, "_connected", False)
+    monkeypatch.setattr(host, "_fallback", None)
+    assert host.connect() and recorder.given[3] is None      # `neighbours` first
+    host.set_fallback(fallback)                              # then `ops`
+    assert recorder.given == (0, 0, 0, fallback)
+    assert host.connect() and all(recorder.given[:3]) and recorder.given[3] is fallback
+    assert not host.connect()
