@@ -93,10 +93,10 @@ constexpr int kSelectBins = 256;
 // The longest row. Loops over a row reach up to one of their steps past its end and count unsigned.
 constexpr int kMostSpan = INT32_MAX - 8192;
 
-// Shared memory of one selecting block.
-template <int kThreads, int kCapacity>
+// Shared memory of one selecting block. kWindow: row positions covered by the bitmap of winners at a time.
+template <int kThreads, int kCapacity, int kWindowSize>
 struct SelectShared {
-  static constexpr int kWindow = kThreads >= 256 ? 65536 : 256 * kThreads;  // row positions covered by the bitmap of winners at a time
+  static constexpr int kWindow = kWindowSize;
   uint2 list[kCapacity];               // candidates: row position, score
   __align__(16) unsigned bitmap[kWindow / 32];
   unsigned short place[kWindow / 32];  // winners before each word of the bitmap
@@ -484,9 +484,9 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
 // 768 x 65536 scores, against the radix select that read every row five times: constant 373 -> 55 us, zeros 383
 // -> 80, all but 300 masked 360 -> 142, correlated over 64 positions 326 -> 192 (a fifth of the rows);
 // 100 rows of the latter 114 -> 80. With that select as the way out they took 461, 433, 457, 283 and 127.
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
-  using Shared = SelectShared<kThreads, kCapacity>;
+  using Shared = SelectShared<kThreads, kCapacity, kWindowSize>;
   constexpr int kWindow = Shared::kWindow;
   extern __shared__ __align__(16) unsigned char select_smem[];
   Shared& s = *reinterpret_cast<Shared*>(select_smem);
@@ -667,10 +667,10 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads)>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight>;
-  constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity>));
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow>;
+  constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity, kWindow>));
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
   int device = 0;
@@ -711,16 +711,22 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // Two blocks of 512 threads to an SM are better before that, and where the buffer is wide but the rows are
   // not (600 x 200 K: 131 us against 154, 2000 rows of 2 K in a buffer of 140000: 68 against 120). No more tokens than SMs: a
   // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
-  // with thirty-two; of 65536: 11 us against 15). Otherwise
+  // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread where the row has several
+  // steps (16 x 64 K: 11.3 -> 10.8, 100 x 64 K: 11.7 -> 11.1; 16 x 4 K: 6.6 against 7.1, so not for short rows). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
   // more than a wave of them (8192 rows of 12-16 K scores: 120 us against 144 with eight warps, which
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
-  // 38) or where the row needs the larger sample. Eight loads in flight per thread need one block fewer per
-  // SM: better where a row has several steps (1800 x 32 K: 59.5 -> 54.0 us; 4000 x 4 K: 42.7 -> 43.4).
+  // 38) or where the row needs the larger sample. What such rows wait for is one step after the other: up to 16 K scores
+  // (a bitmap of one window) ten blocks of 48 registers per SM with four loads in flight are better than eight with eight loads (8192
+  // x 12-16 K: 119.9 -> 118.0 us, 16384 rows of a prompt of 10 K: 194.0 -> 176.0, 4096 x 8 K: 53.6 -> 49.9; rows
+  // that correlate 1 to 5 % faster, rows of nothing but equal scores, which are all streaming, 6 to 10 % slower). Longer rows are streaming for
+  // the most part: eight blocks, eight loads (1800 x 32 K: 59.5 -> 54.0 us). Eleven blocks leave a list of 1536 entries, which
+  // rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
+  if (T <= multiprocessors && SPAN > 16384) return launch_select<512, 4096, 1, 2, 8>(p, s);
   if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
-    return SPAN <= 8192 ? launch_select<128, 2048, 9, 4>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
+    return SPAN <= 16384 ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
   return launch_select<256, 2560, 6, 2>(p, s);
 }
 
