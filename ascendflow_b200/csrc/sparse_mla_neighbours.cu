@@ -468,7 +468,7 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
 //
 // Bound by memory for long rows (768 x 65536 scores: 45 us, 68 % of the copy bandwidth; the radix
 // select that read the row five times took 335 us) and by issue slots for many short ones (8192 x
-// 12-16 K: 120 us, 3.9 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
+// 12-16 K: 118 us, 4.0 TB/s; before 1003 us). The row is streamed once. A strided sample (one or
 // two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the
 // stream lists what reaches the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256

@@ -11,8 +11,8 @@
 //   producer warps   gather the token's rows with 16-byte cp.async into a three-stage ring of
 //                    128-byte-swizzled shared tiles (a row is fetched once and serves as K and
 //                    V), and move the token's Q from global to tensor memory through registers.
-//   MMA warp         one thread issues S = Q X^T (Q from tensor memory, X K-major from the tile)
-//                    and O += P X (P from a shared tile, X MN-major from the same tile; issued
+//   MMA warps        one thread issues S = Q X^T (Q from tensor memory, X K-major from the tile)
+//                    and another O += P X (P from a shared tile, X MN-major from the same tile; issued
 //                    as tcgen05.mma.ws so that M = 64 does not halve the rate).
 //   softmax warps    tcgen05.ld S, joint online softmax with the per-head sink
 //                    (examples/sparse_attention/attention.py:398-490: one maximum and one
@@ -34,7 +34,8 @@
 // the chunk; it loads both partial scores of each.
 //
 // Every wait on an mbarrier is bounded (tcgen05_ptx.cuh): on expiry the block records
-// kStatusWaitExpired, all roles leave their loops, tensor memory is released, the kernel returns.
+// kStatusWaitExpired, all roles leave their loops, tensor memory is released, the kernel returns. The softmax warps' named
+// barriers are passed by all four of them or by none (`softmax_role`).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -808,16 +809,16 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
   return d;
 }
 
-// What paces the kernel. Inside of a token a chunk takes 1.75 k cycles, and shared memory is what it takes them for: a tile
-// is written once (64 KiB), read by QK and by PV (64 each), and P is written and read (8 and 16): 216 KiB at 128 bytes
-// per cycle are 1.69 k. (The products' instructions, 704 and 640 cycles by themselves, take 920 each beside the copies.)
-// From scores to P handed over these warps need 1.35 k; nothing that is known a chunk earlier is fetched late, and additions
-// go two to an instruction. Between two tokens lie 4 to 5 k cycles more: the output leaves the SM at 32 bytes per cycle (2.05 k for
-// 64 KiB, by stores or bulk copies alike), and the conversion to 16 bits before it takes 1.7 k.
+// What paces the kernel. Inside of a token a chunk takes 1.75 k cycles: the instructions of QK and PV follow each other without a gap
+// and take about 900 cycles each (704 and 640 by themselves): their operands, 144 KiB, and the copies that write 64 KiB beside
+// them share the ports of one shared memory. From scores to P handed over these warps need 1.35 k; nothing that is known a
+// chunk earlier is fetched late, and additions go two to an instruction. Between two tokens lie 4 to 5 k cycles more, for
+// which no product runs: the output leaves the SM at 32 bytes per cycle (2.05 k for 64 KiB, by stores or bulk copies alike), and
+// the conversion to 16 bits in front of it takes 1.7 k.
 //
 // A second P tile takes the wait for the previous PV out of the chain, and flags by named barriers a word in shared memory and a
 // wait: 256 tokens at 4K 30.0 -> 28.5 us, 100 tokens 16.9 -> 15.9, 1000 tokens 106.7 -> 104.4, prefill of 8K tokens 840 -> 832.
-// In a steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides and not cycles.
+// In a steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides more than cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

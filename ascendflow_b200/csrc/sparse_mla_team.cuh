@@ -16,7 +16,7 @@
 // the output pass. Here the chunks' first product and softmax run side by side, and the output pass is a
 // quarter. Of the 19 k cycles that are left the token's resolution takes 3.7 k, gather, scores and maxima of up to
 // three chunks 6 k, the first P 1.1 k, the second product, in the order of the chunks, 6.6 k (and a thousand more for
-// every chunk at which a reference moves), output 1.7 k. A call of one token 15.3 -> 11.1 us, of 16 tokens 16.3 -> 11.4
+// every chunk at which a reference moves), output 1.7 k. A call of one token 15.3 -> 10.7 us, of 16 tokens 16.3 -> 11.0
 // (one warp resolving the token, all slices gathered behind a barrier of the cluster, products issued by a whole
 // warp before). Eight blocks had less for one token, nothing for eight; P written to the other blocks by
 // the softmax threads instead of bulk copies was slower by a fifth. Copies between blocks are of local shared
