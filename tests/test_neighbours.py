@@ -183,7 +183,7 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
 @pytest.mark.parametrize("tokens,visible", [
     (1790, [16384, 16383, 513, 9000]), (1790, [16388, 16384, 700]),   # many rows, one window of winners or more
     (1790, [8192, 1025, 8191]), (148, [16388, 512, 20000]), (148, [16384, 2049]),  # a row per SM, either number of loads
-    (149, [16388, 1]), (20, [131072, 16388, 65537]),
+    (149, [16388, 1]), (149, [16384, 16383, 2561]), (20, [131072, 16388, 65537]),
 ])
 def test_gpu_selection_at_the_lines_between_its_kernels(tokens, visible):
     test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible)
