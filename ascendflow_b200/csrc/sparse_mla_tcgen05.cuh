@@ -103,7 +103,7 @@ enum Bar {
   kTokenReady0 = 0, kTokenReady1, kTokenDone0, kTokenDone1, kQFull, kQFree,
   kKvFree0, kKvFree1, kKvFree2, kKvFree3, kKvFree4, kKvFree5,  // halves of the ring stages
   kSFull0, kSFull1, kPFull0, kPFull1, kOFree,
-  kKvFull0, kKvFull1, kKvFull2, kPvDone, kOutReady, kInfoRead0, kInfoRead1, kBarCount
+  kKvFull0, kKvFull1, kKvFull2, kOutReady, kInfoRead0, kInfoRead1, kBarCount
 };
 static_assert(kBarCount <= 32, "the barrier area holds 32 mbarriers");
 
@@ -742,7 +742,6 @@ __device__ void pv_role(const Params& p, const Shared& sm, uint32_t tmem) {
       tc_fence_after_sync();
       issue_pv<kFormat>(sm, tmem, stage, p_tile, i != 0);
       mma_commit(sm.bar(kSFull0 + p_tile));  // the P tile is free: half of what the softmax warps wait for at chunk c + 2
-      mma_commit(sm.bar(kPvDone));
       if (i + 1 == chunks) mma_commit(sm.bar(kOutReady));  // O is complete
     }
     ++working_tokens;
@@ -1026,7 +1025,9 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         if (half == 0) alpha_exchange[head] = alpha;
         named_barrier_sync(4, 32 * kSoftmaxWarps);
         const float o_alpha = alpha_exchange[o_head];
-        if (!warp_wait(sm.bar(kPvDone), (chunk_count - 1) & 1, abort_flag)) give_up();
+        // PV c - 1 has ended when its tile's second half is free. A parity tells that phase from the one before only, the end of
+        // PV c - 4, which is long past: the producers waited for it before they brought tile c - 1 into the stage.
+        if (!warp_wait(sm.bar(kKvFree0 + 2 * ((chunk_count - 1) % kStages) + 1), ((chunk_count - 1) / kStages) & 1, abort_flag)) give_up();
         tc_fence_after_sync();
         // 32 columns at a time: a round trip to tensor memory each (in 16s the pass took 1500 cycles).
 #pragma unroll 1
@@ -1073,7 +1074,7 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
 
   if (threadIdx.x == 0) {
     const int P = kProducerWarps, S = kSoftmaxWarps, T = kProducerThreads;
-    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, 1, 1, 2, 2, S, S, S, T + S, T + S, T + S, 1, 1, P + 2, P + 2};
+    const int counts[kBarCount] = {1, 1, S, S, P, 1, 1, 1, 1, 1, 1, 1, 2, 2, S, S, S, T + S, T + S, T + S, 1, P + 2, P + 2};
     for (int i = 0; i < kBarCount; ++i) mbar_init(sm.bar(i), counts[i]);
     mbar_fence_init();
     mbar_arrive(sm.bar(kSFull0));  // the P tiles start out free

@@ -38,6 +38,38 @@ def test_waits_for_other_blocks_acquire_at_cluster_scope():
     assert "mbarrier.try_wait.parity.acquire.cluster." in body[: body.index("\n}\n")]
 
 
+def test_a_rescale_tells_the_end_of_the_products_before_it_from_earlier_ones():
+    """A wait by parity passes on any phase that is not the present one, so whoever waits for the end of PV c - 1 has to know that the
+    barrier's phase before that has ended. Arrivals of different commits come in no particular order: known is what somebody
+    on the way to chunk c has waited for on the same barrier."""
+    source = (CSRC / "sparse_mla_tcgen05.cuh").read_text()
+    stages = int(re.search(r"constexpr int kStages = (\d+);", source).group(1))
+
+    def barrier(expression, **names):  # (name, number) of "kName" or "kName0 + number"
+        name, _, number = expression.partition("0 + ")
+        return name, eval(number or "0", {"kStages": stages}, names)
+
+    rescale = source[source.index("named_barrier_sync(4,"):]
+    waited, parity = re.search(r"warp_wait\(sm\.bar\((.+)\), (.+), abort_flag\)", rescale).groups()
+    issue = source[source.index("void issue_pv("):source.index("void qk_role(")]
+    commits = re.findall(r"mma_commit\(sm\.bar\((.+?)\)\);", issue.split("kPvSteps, false>")[-1])
+    role = source[source.index("void pv_role("):source.index("void softmax_role(")]
+    commits += re.findall(r"\n      mma_commit\(sm\.bar\((.+?)\)\);", role)
+    producers = source[source.index("void producer_role("):source.index("void qk_role(")]
+    gathered_behind = re.findall(r"use > 0 && !warp_wait\(sm\.bar\((.+?)\), \(use - 1\) & 1, abort_flag", producers)
+
+    for chunk in range(1, 40):
+        phase = eval(parity.replace("/", "//"), {"kStages": stages}, {"chunk_count": chunk})
+        wanted = barrier(waited, chunk_count=chunk)
+        ends = [k for k in range(chunk) if any(barrier(c, stage=k % stages, p_tile=k & 1) == wanted for c in commits)]
+        assert ends and ends[-1] == chunk - 1, (chunk, wanted)
+        # the producers brought tile k into its stage behind the end of PV k - kStages, and tiles 0 .. c have been multiplied
+        known = [k - stages for k in range(stages, chunk) if any(barrier(b, stage=k % stages) == wanted for b in gathered_behind)]
+        for phases in range(len(set(known) & set(ends)), len(ends)):
+            assert phases & 1 == phase, (chunk, phases)  # waits
+        assert len(ends) & 1 != phase  # passes
+
+
 def test_slots_are_resolved_by_one_routine():
     """The rule from slot to row stands once beside the tcgen05 kernels, and all forms of resolving a token run it."""
     source = (CSRC / "sparse_mla_tcgen05.cuh").read_text()
