@@ -461,6 +461,11 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
   }
 }
 
+template <int kCount>
+struct Loads {
+  static constexpr int value = kCount;
+};
+
 // One block per query token. Candidates are compressed rows [0, min(available, cutoff)): the rows
 // the attention kernel would accept for this token. The min(TopK, candidates) highest scores win,
 // ties going to the lower index; winners are written in ascending index order, the rest of the 512
@@ -484,7 +489,7 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
 // 768 x 65536 scores, against the radix select that read every row five times: constant 373 -> 55 us, zeros 383
 // -> 80, all but 300 masked 360 -> 142, correlated over 64 positions 326 -> 192 (a fifth of the rows);
 // 100 rows of the latter 114 -> 80. With that select as the way out they took 461, 433, 457, 283 and 127.
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
   using Shared = SelectShared<kThreads, kCapacity, kWindowSize>;
   constexpr int kWindow = Shared::kWindow;
@@ -509,9 +514,9 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   if (threadIdx.x == 0) { s.count = s.few_count = 0; s.mass = false; s.low = 0xffffffffu; s.high = 0; s.bin = kSelectBins; }
   __syncthreads();
 
-  // kInFlight: 16-byte loads in flight per thread of the pass over the row
+  // kInFlight: 16-byte loads in flight per thread of the pass over the row (four for rows of up to kShortRow scores)
   static_assert(kInFlight <= 8, "a word of signs");
-  constexpr unsigned kStep = kInFlight * 4 * kThreads, kAhead = kStep > 4096 ? kStep : 4096;
+  constexpr unsigned kHead = kInFlight * 4 * kThreads > 4096 ? kInFlight * 4 * kThreads : 4096;
   const unsigned end = unsigned(candidates);  // unsigned: a step may reach past INT32_MAX
 
   // ---- floor ----------------------------------------------------------------------------------
@@ -529,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     for (int q = 0; q < kMostQuads; ++q)
       if (q < quads) v[q] = __ldg(reinterpret_cast<const uint4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
     // The row's head on its way to L2 behind the sample, while the floor is found.
-    if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kAhead));
+    if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kHead));
     uint32_t key[4 * kMostQuads];
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q) {
@@ -589,45 +594,52 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   const bool normal = floor_key == 0 || (exponent != 0 && exponent != 0x7f800000u);
   const float floor_value = __uint_as_float(floor_bits);
   if (normal) {
-    // What lies kAhead scores (16 KiB) further on is on its way to L2 meanwhile: a block's own loads are
-    // not in flight while it looks at what they brought (768 x 65536 scores: 51.1 -> 45.0 us, 1800 x 65536:
-    // 105 -> 89; 12 and 32 KiB: 46.1, and 64 KiB at the row's head alone, 51.1).
-    for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
-      if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
-      uint4 v[kInFlight];
+    // What lies further on is on its way to L2 meanwhile, 16 KiB with 128 and 256 threads, a step with more: a block's own loads are
+    // not in flight while it looks at what they brought (768 x 65536 scores, 256 threads: 51.1 -> 45.0 us, 1800 x 65536:
+    // 105 -> 89; 12 and 32 KiB: 46.1, and 64 KiB at the row's head alone, 51.1. 512 threads with eight loads, 16 and 100 x 64 K:
+    // no difference between 16, 32 and 64 KiB).
+    auto list_row = [&](auto loads) {
+      constexpr int kLoads = decltype(loads)::value;
+      constexpr unsigned kStep = kLoads * 4 * kThreads, kAhead = kStep > 4096 ? kStep : 4096;
+      for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
+        if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
+        uint4 v[kLoads];
 #pragma unroll
-      for (int h = 0; h < kInFlight; ++h) {
-        const unsigned i = first + h * kThreads * 4;
-        v[h] = i < end ? __ldcs(reinterpret_cast<const uint4*>(row + i)) : make_uint4(0, 0, 0, 0);
-      }
-      // The sign of score - floor, shifted in: bit 4 (kInFlight - 1 - h) + 3 - e is clear where the score reaches it.
-      unsigned below = 0;
+        for (int h = 0; h < kLoads; ++h) {
+          const unsigned i = first + h * kThreads * 4;
+          v[h] = i < end ? __ldcs(reinterpret_cast<const uint4*>(row + i)) : make_uint4(0, 0, 0, 0);
+        }
+        // The sign of score - floor, shifted in: bit 4 (kLoads - 1 - h) + 3 - e is clear where the score reaches it.
+        unsigned below = 0;
 #pragma unroll
-      for (int h = 0; h < kInFlight; ++h) {
-        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].x) - floor_value), below, 1);
-        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].y) - floor_value), below, 1);
-        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].z) - floor_value), below, 1);
-        below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].w) - floor_value), below, 1);
-      }
-      unsigned hits = ~below & (0xffffffffu >> (32 - 4 * kInFlight));
-      if (first + (kInFlight - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
+        for (int h = 0; h < kLoads; ++h) {
+          below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].x) - floor_value), below, 1);
+          below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].y) - floor_value), below, 1);
+          below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].z) - floor_value), below, 1);
+          below = __funnelshift_l(__float_as_uint(__uint_as_float(v[h].w) - floor_value), below, 1);
+        }
+        unsigned hits = ~below & (0xffffffffu >> (32 - 4 * kLoads));
+        if (first + (kLoads - 1) * kThreads * 4 + 3 >= end) {  // the last step: drop what lies past the end
 #pragma unroll
-        for (int h = 0; h < kInFlight; ++h) {
-          const unsigned i = first + h * kThreads * 4, left = i < end ? min(end - i, 4u) : 0u;
-          hits &= ~((15u >> left) << (4 * (kInFlight - 1 - h)));
+          for (int h = 0; h < kLoads; ++h) {
+            const unsigned i = first + h * kThreads * 4, left = i < end ? min(end - i, 4u) : 0u;
+            hits &= ~((15u >> left) << (4 * (kLoads - 1 - h)));
+          }
+        }
+        if (hits == 0) continue;
+        unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+        if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
+#pragma unroll
+        for (int h = 0; h < kLoads; ++h) {
+          const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (hits >> (4 * (kLoads - 1 - h) + 3 - e) & 1) s.list[at++] = make_uint2(first + h * kThreads * 4 + e, values[e]);
         }
       }
-      if (hits == 0) continue;
-      unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
-      if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
-#pragma unroll
-      for (int h = 0; h < kInFlight; ++h) {
-        const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (hits >> (4 * (kInFlight - 1 - h) + 3 - e) & 1) s.list[at++] = make_uint2(first + h * kThreads * 4 + e, values[e]);
-      }
-    }
+    };
+    if (kShortRow > 0 && end <= unsigned(kShortRow)) list_row(Loads<4>{});
+    else list_row(Loads<kInFlight>{});
     __syncthreads();
     const int listed = int(s.count);
     if (listed >= kTopK && listed <= kCapacity && select_from_list<kThreads, kCapacity>(s, end, listed, floor_key, list)) return;
@@ -667,9 +679,9 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads)>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads), int kShortRow = 0>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow>;
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow>;
   constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity, kWindow>));
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
@@ -711,8 +723,9 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // Two blocks of 512 threads to an SM are better before that, and where the buffer is wide but the rows are
   // not (600 x 200 K: 131 us against 154, 2000 rows of 2 K in a buffer of 140000: 68 against 120). No more tokens than SMs: a
   // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
-  // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread where the row has several
-  // steps (16 x 64 K: 11.3 -> 10.8, 100 x 64 K: 11.7 -> 11.1; 16 x 4 K: 6.6 against 7.1, so not for short rows). Otherwise
+  // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread for rows of more than three steps of
+  // four. The kernel looks at the row for that: a buffer is as wide as the longest context (16 x 64 K: 10.8 with four loads, 10.3 with
+  // eight; 30000: 8.5, 8.3; 24000: 7.6, 8.0; 4 K in buffers of 32 to 128 K: 6.9, 7.35). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
   // more than a wave of them (8192 rows of 12-16 K scores: 120 us against 144 with eight warps, which
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
@@ -723,7 +736,7 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // the most part: eight blocks, eight loads (1800 x 32 K: 59.5 -> 54.0 us). Eleven blocks leave a list of 1536 entries, which
   // rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
-  if (T <= multiprocessors && SPAN > 16384) return launch_select<512, 4096, 1, 2, 8>(p, s);
+  if (T <= multiprocessors && SPAN > 24576) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
   if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
     return SPAN <= 16384 ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
