@@ -731,15 +731,18 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
   // 38) or where the row needs the larger sample. What such rows wait for is one step after the other: up to 16 K scores
   // (a bitmap of one window) ten blocks of 48 registers per SM with four loads in flight are better than eight with eight loads (8192
-  // x 12-16 K: 119.9 -> 118.0 us, 16384 rows of a prompt of 10 K: 194.0 -> 176.0, 4096 x 8 K: 53.6 -> 49.9; rows
-  // that correlate 1 to 5 % faster, rows of nothing but equal scores, which are all streaming, 6 to 10 % slower). Longer rows are streaming for
-  // the most part: eight blocks, eight loads (1800 x 32 K: 59.5 -> 54.0 us). Eleven blocks leave a list of 1536 entries, which
+  // x 12-16 K: 119.9 -> 118.0 us, 16384 rows of a prompt of 10 K: 194.0 -> 176.0, 4096 x 8 K: 54.8 -> 51.3), but beyond 10 K scores
+  // only where they make fewer waves: every block is slower for it (eight / ten blocks per SM, 1800 x 16 K: 34.0 / 36.7, 3300 x 16 K: 54.6 /
+  // 56.8, 2450 x 16 K: 44.1 / 42.0, 7400 x 16 K: 121.8 / 120.9; 2300 x 12 K: 36.5 / 38.1, 7400 x 12 K: 107.8 / 106.0; 3300 x 10 K:
+  // 49.8 / 49.3). Longer rows are streaming for the most part: eight blocks, eight loads (4096 x 17408: 74.3 / 76.9, 2000 x 20 K:
+  // 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536 entries, which
   // rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
   if (T <= multiprocessors && SPAN > 24576) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
   if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);
+  const bool fewer_waves = (T - 1) / (multiprocessors * 10) < (T - 1) / (multiprocessors * 8);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
-    return SPAN <= 16384 ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
+    return SPAN <= (fewer_waves ? 16384 : 10240) ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
   // A bitmap no larger than the row: what shared memory it does not take holds scores that are read again (860 x 16 K: 19.7 ->
   // 19.0 us, 150 such rows that correlate 39.1 -> 36.3; blocks of 512 threads: no change).
   return SPAN <= 16384 ? launch_select<256, 2560, 6, 2, 4, 16384>(p, s) : launch_select<256, 2560, 6, 2>(p, s);

@@ -184,6 +184,7 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     (1790, [16384, 16383, 513, 9000]), (1790, [16388, 16384, 700]),   # many rows, one window of winners or more
     (1790, [8192, 1025, 8191]), (148, [16388, 512, 20000]), (148, [16384, 2049]),  # a row per SM, either number of loads
     (149, [16388, 1]), (149, [16384, 16383, 2561]), (20, [131072, 16388, 65537]),
+    (2368, [16000, 9000, 12289]), (2369, [16384, 10241]), (1800, [10240, 700]), (1800, [10244, 10241, 10240]),  # waves of eight and of ten blocks
     (148, [24576, 24575, 4096]), (148, [24580, 24576, 24577, 24575, 2049, 700, 512]),  # the row's own length chooses it
 ])
 def test_gpu_selection_at_the_lines_between_its_kernels(tokens, visible):
@@ -282,7 +283,7 @@ def test_gpu_selection_over_the_longest_row():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tokens,span", [(1800, 14336), (320, 65536), (19, 16384), (19, 40000), (7, 150000)])  # 128, 256, 512, 512, 1024 threads
+@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (19, 16384), (19, 40000), (7, 150000)])  # 128, 128, 256, 512, 512, 1024 threads
 def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
     """NaNs above and below the infinities by their sign, masks of -inf and of the lowest finite value, more and
     fewer of them than are selected."""
