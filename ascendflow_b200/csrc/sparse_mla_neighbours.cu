@@ -395,6 +395,47 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
   return true;
 }
 
+// Lists what reaches the floor, by keys. For 128 threads: with 48 registers the loop in `select_by_keys` spills and waits for every
+// load, which took rows of zeros (8192 x 16 K, whose floor is subnormal) from 130 to 143 us when ten blocks came to share an SM.
+// The scores' order in place of their bits, a look at the highest of sixteen first, and 16 KiB on their way to L2: 111. (With 256
+// threads and 40 registers the whole kernel is slower for it, usual rows of 768 x 65536 scores 38.1 -> 43.2.)
+template <int kThreads, int kCapacity, typename Shared>
+__device__ __forceinline__ void list_by_order(Shared& s, const float* row, unsigned end, unsigned floor_key) {
+  constexpr unsigned kStep = 16 * kThreads, kAhead = kStep > 4096 ? kStep : 4096;
+  const auto order = [](uint32_t bits) { return int(bits ^ (uint32_t(int(bits) >> 31) & 0x7fffffffu)); };  // its own inverse
+  const int least = int(floor_key ^ 0x80000000u);
+  for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += kStep) {
+    if (threadIdx.x == 0 && first + kAhead < end) prefetch_l2(row + first + kAhead, 4u * min((end - first - kAhead + 3u) & ~3u, kStep));
+    int v[16];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const unsigned i = first + h * 4 * kThreads;
+      const uint4 w = i < end ? __ldcs(reinterpret_cast<const uint4*>(row + i)) : make_uint4(0, 0, 0, 0);
+      v[4 * h] = order(w.x); v[4 * h + 1] = order(w.y); v[4 * h + 2] = order(w.z); v[4 * h + 3] = order(w.w);
+    }
+    int best = v[0];
+#pragma unroll
+    for (int e = 1; e < 16; ++e) best = max(best, v[e]);
+    if (best < least) continue;
+    unsigned hits = 0;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) hits |= unsigned(v[e] >= least) << e;
+    if (first + 12 * kThreads + 3 >= end) {  // the last step: drop what lies past the end
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const unsigned i = first + h * 4 * kThreads, left = i < end ? min(end - i, 4u) : 0u;
+        hits &= ~((15u << left & 15u) << (4 * h));
+      }
+      if (hits == 0) continue;
+    }
+    unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+    if (at + unsigned(__popc(hits)) > kCapacity) continue;
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+      if (hits >> e & 1) s.list[at++] = make_uint2(first + (e >> 2) * 4 * kThreads + (e & 3), unsigned(order(unsigned(v[e]))));
+  }
+}
+
 // What is left of `topk_select_kernel` where the list of what reaches the floor is too short or too long, or has not
 // been made (`listed`), since the floor is zero, subnormal, infinite or a NaN. All by keys, and not inline: the
 // usual row's instructions stay together.
@@ -403,24 +444,28 @@ __device__ __noinline__ void select_by_keys(Shared& s, const float* row, unsigne
   bool fits = false;  // the floor has been found to
   while (true) {
     if (!listed) {
-      for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += 16 * kThreads) {
-        uint32_t key[4][4];
-        bool valid[4][4];
-        uint4 v[4];
+      if constexpr (kThreads == 128) {
+        list_by_order<kThreads, kCapacity>(s, row, end, floor_key);
+      } else {
+        for (unsigned first = threadIdx.x * 4; first < end + threadIdx.x * 4; first += 16 * kThreads) {
+          uint32_t key[4][4];
+          bool valid[4][4];
+          uint4 v[4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h) v[h] = load_keys(row, first + h * 4 * kThreads, end, key[h], valid[h]);
-        unsigned hits = 0;
+          for (int h = 0; h < 4; ++h) v[h] = load_keys(row, first + h * 4 * kThreads, end, key[h], valid[h]);
+          unsigned hits = 0;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) hits |= unsigned(valid[e >> 2][e & 3] && key[e >> 2][e & 3] >= floor_key) << e;
-        if (hits == 0) continue;
-        unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
-        if (at + unsigned(__popc(hits)) > kCapacity) continue;
+          for (int e = 0; e < 16; ++e) hits |= unsigned(valid[e >> 2][e & 3] && key[e >> 2][e & 3] >= floor_key) << e;
+          if (hits == 0) continue;
+          unsigned at = atomicAdd(&s.count, unsigned(__popc(hits)));
+          if (at + unsigned(__popc(hits)) > kCapacity) continue;
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+          for (int h = 0; h < 4; ++h) {
+            const unsigned values[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (hits >> (4 * h + e) & 1) s.list[at++] = make_uint2(first + h * 4 * kThreads + e, values[e]);
+            for (int e = 0; e < 4; ++e)
+              if (hits >> (4 * h + e) & 1) s.list[at++] = make_uint2(first + h * 4 * kThreads + e, values[e]);
+          }
         }
       }
       __syncthreads();
