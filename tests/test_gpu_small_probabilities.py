@@ -1,6 +1,6 @@
 """IEEE half keeps the precision of small probabilities: a row 2^-20 below the best one has a probability of
-2^-12 (a normal number) while the reference stays at the sink, eight binades below the best row, and of
-2^-20 (four bits) where the reference moves up although it need not."""
+2^-12 (a normal number) while the reference stays eight binades below the best row, next to the sink, and of
+2^-20 (four bits) where the reference moves up to that row although it need not."""
 
 import numpy as np
 import pytest
@@ -25,7 +25,7 @@ def test_probabilities_far_below_the_best_row_keep_their_bits(tokens):
     q = np.zeros((tokens, heads, 512), dtype=np.float16)
     q[:, :, 0] = 63.0 + np.arange(heads) / 32.0
     best = q[0, :, 0].astype(np.float64) * 4.0 * SCALE_LOG2
-    sinks = ((best - 7.75) / 1.4426950408889634).astype(np.float32)   # below the move at 8
+    sinks = ((best - 7.75) / 1.4426950408889634).astype(np.float32)   # the reference: eight below the best
 
     i32 = lambda value: torch.tensor(np.ascontiguousarray(value), dtype=torch.int32, device="cuda")  # noqa: E731
     cache = torch.from_numpy(rows).cuda().view(window // 128, 128, 1, 512)
