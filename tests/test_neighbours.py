@@ -138,9 +138,9 @@ def test_gpu_selection_over_long_rows(max_seq, ratio):
     (19, (512, 513, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 16384, 16385, 131071, 131072, 65537)),
     # 1024-thread blocks: listed whole (4096), the list (8192), one step (16384), more than a window of winners
     (7, (4096, 4097, 8193, 16385, 131073, 200001, 150000)),
-    # 128-thread blocks, rows of at most 8192 scores: the list and one step (2048)
+    # 128-thread blocks, ten per SM (rows of at most 10240 scores): the list and one step (2048)
     (1900, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 6143, 8191, 8192)),
-    # 128-thread blocks, longer rows: the list (2048), one step (4096), the window of winners (32768), the longest
+    # 128-thread blocks, eight per SM: the list (2048), one step (4096), the window of winners (32768), the longest
     (1800, (511, 512, 513, 2047, 2048, 2049, 3000, 4095, 4097, 8191, 16385, 32767, 32768)),
 ])
 def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
@@ -283,7 +283,7 @@ def test_gpu_selection_over_the_longest_row():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (19, 16384), (19, 40000), (7, 150000)])  # 128, 128, 256, 512, 512, 1024 threads
+@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (320, 14336), (19, 16384), (19, 40000), (7, 150000)])  # 128 (twice), 256, 512, 1024 threads
 def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
     """NaNs above and below the infinities by their sign, masks of -inf and of the lowest finite value, more and
     fewer of them than are selected."""
@@ -336,7 +336,7 @@ def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (19, 16384), (19, 40000), (7, 150000)])  # 128, 128, 256, 512, 512, 1024
+@pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (320, 14336), (19, 16384), (19, 40000), (7, 150000)])  # as above
 def test_gpu_selection_of_rows_that_a_sample_says_little_about(tokens, span):
     """Many equal scores at, above and below the threshold, at zero, among subnormals and at a mask; scores that
     change slowly along the row, in both directions of a missed floor; winners the sample has not seen."""
