@@ -779,9 +779,10 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // x 12-16 K: 119.9 -> 118.0 us, 16384 rows of a prompt of 10 K: 194.0 -> 176.0, 4096 x 8 K: 54.8 -> 51.3), but beyond 10 K scores
   // only where they make fewer waves: every block is slower for it (eight / ten blocks per SM, 1800 x 16 K: 34.0 / 36.7, 3300 x 16 K: 54.6 /
   // 56.8, 2450 x 16 K: 44.1 / 42.0, 7400 x 16 K: 121.8 / 120.9; 2300 x 12 K: 36.5 / 38.1, 7400 x 12 K: 107.8 / 106.0; 3300 x 10 K:
-  // 49.8 / 49.3). Longer rows are streaming for the most part: eight blocks, eight loads (4096 x 17408: 74.3 / 76.9, 2000 x 20 K:
-  // 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536 entries, which
-  // rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
+  // 49.8 / 49.3). Rows of one constant are all streaming and 3 to 7 % slower with ten (8192 x 12 K: 88.9 / 93.9; zeros 109.6 / 94.0 by
+  // `list_by_order`); nothing says so before the launch. Longer rows are streaming for the most part: eight blocks, eight
+  // loads (4096 x 17408: 74.3 / 76.9, 2000 x 20 K: 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536
+  // entries, which rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
   if (T <= multiprocessors && SPAN > 24576) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
   if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);

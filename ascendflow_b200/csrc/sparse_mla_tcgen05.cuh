@@ -671,9 +671,9 @@ __device__ __forceinline__ void issue_pv_steps(uint32_t o_tmem, uint64_t p_desc,
 //
 // The tile's rows are used up in order, both products of 16 rows after each other, and its first half is
 // given back when it has been: a tile stays in the ring from its copies' issue to the end of its PV, through QK, softmax and
-// PV, and the next tile of the stage can be 320 cycles on its way by that end. Decode 128 x 6 118.2 -> 115.3 us, 64 x 6 61.1 -> 59.8,
-// prefill of 8K tokens 864 -> 846, 23 mixed requests 170.6 -> 167.1. (Quarters: 115.7, 60.5 and 864: what a wait
-// and its commit cost is what they bring.)
+// PV, and the next tile of the stage can be 320 cycles on its way by that end. Two per cent of decode (128 x 6 and 64 x 6), of prefill
+// of 8K tokens and of 23 mixed requests. (Quarters: 2 and 1 % of decode, nothing of prefill: what a wait and its commit
+// cost is what they bring.)
 template <int kFormat>
 __device__ __forceinline__ void issue_pv(const Shared& sm, uint32_t tmem, int stage, int p_tile, bool accumulate) {
   const uint64_t x_desc = smem_desc_sw128(sm.base + kSmemKv + stage * kTileBytes, kBlockBytes, 1024);
@@ -770,17 +770,18 @@ __device__ __forceinline__ float max3(float a, float b, float c) {  // one instr
 // The running reference of a head (log2 domain; it starts at the sink) moves when a chunk's maximum exceeds it by more
 // than kReferenceRoom, and then to kReferenceStep below that maximum. All terms of a head share the reference, which
 // cancels in the final division; what it decides is how often the accumulator is rescaled (everybody waits for it) and
-// which probabilities fit the storage type. Probabilities reach 2^15 (IEEE half ends below 2^16, sums are FP32). A reference
+// which probabilities fit the storage type. Probabilities reach 2^15 (IEEE half ends below 2^16). Sums are FP32 and reach as much
+// further: 640 rows stay finite up to values of 1.6e31 in a bf16 cache (2e33 with a room of 8). A reference
 // that moved at 2^8 already, up to the maximum, rescaled in a tenth of all chunks where sinks are N(0, 1); now it takes a sink
 // seven standard deviations down. The step back keeps the reference at or below that one's in every chunk: the room is at
-// least a step wider, so whatever was a normal number in half still is. 8 x 2 tokens 11.63 -> 11.15 us, one token 10.81
-// -> 10.69, 23 mixed requests 172.4 -> 170.5, prefill of 8K tokens 872 -> 866.
+// least a step wider, so whatever was a normal number in half still is. Four per cent of 8 x 2 tokens, one of one
+// token, of 23 mixed requests and of prefill.
 //
 // With a token's first chunk, where there is nothing to rescale, it moves down to a whole number of binades below the maximum
 // (by less than one): the probability of the chunk's best row is then a power of two and not rounded. The error against
-// 64 bits falls by half a per cent for N(0, 1) inputs and by a tenth for scores three times as wide, where it had grown by 0.1 %
-// with the wider room (a reference that moved to a maximum had the same effect). Beyond kReferenceAligned binades
-// that row weighs nothing. Returns the factor of what has been accumulated.
+// 64 bits, relative by the 2-norm: 2.14e-3 in bf16 and 2.67e-4 in half for N(0, 1) inputs (2.15e-3 and 2.70e-4 without the step and
+// a room of 8), 7 to 10 % less than without it for scores three times as wide, 1 to 2 % less for six times. Beyond kReferenceAligned
+// binades that row weighs nothing. Returns the factor of what has been accumulated.
 constexpr float kReferenceRoom = 15.f, kReferenceStep = 8.f, kReferenceAligned = 64.f;
 __device__ __forceinline__ float move_reference(float& reference, float chunk_max, bool first) {
   const float above = chunk_max - reference;
@@ -816,8 +817,11 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // the conversion to 16 bits in front of it takes 1.7 k.
 //
 // A second P tile takes the wait for the previous PV out of the chain, and flags by named barriers a word in shared memory and a
-// wait: 256 tokens at 4K 30.0 -> 28.5 us, 100 tokens 16.9 -> 15.9, 1000 tokens 106.7 -> 104.4, prefill of 8K tokens 840 -> 832.
-// In a steady loop the large calls are at the board's power limit (1.6 GHz), where energy decides more than cycles.
+// wait: five per cent of 100 and of 256 tokens, two of 1000, one of prefill of 8K.
+//
+// Calls one after the other take 841 us for prefill of 8K tokens at 32K, 116 for decode 128 x 6 at 128K, 167 for 23 mixed requests, 31 for
+// 256 tokens at 4K. The first three are at the board's power limit (1000 W; 1.50 to 1.57 GHz while they run), where energy decides
+// more than cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
