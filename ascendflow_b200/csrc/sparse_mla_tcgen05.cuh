@@ -35,7 +35,7 @@
 //
 // Every wait on an mbarrier is bounded (tcgen05_ptx.cuh): on expiry the block records
 // kStatusWaitExpired, all roles leave their loops, tensor memory is released, the kernel returns. The softmax warps' named
-// barriers are passed by all four of them or by none (`softmax_role`).
+// barrier is passed by all four of them or by none (`softmax_role`).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -76,10 +76,10 @@ constexpr int kSmemRows = kSmemStore + kSoftmaxWarps * 2048;   // int[2][640]
 constexpr int kSmemInfo = kSmemRows + 2 * kSlots * 4;       // TokenInfo[2]
 constexpr int kSmemBars = kSmemInfo + 2 * 128;              // mbarriers
 constexpr int kSmemMisc = kSmemBars + 32 * 8;               // tmem slot, abort flag
-// Per-head factors handed between the softmax warps (float[64] and, double-buffered, float[2][64]): a
+// Per-head factors handed between the softmax warps (float[2][64] each, double-buffered): a
 // thread works out the softmax of one head but reads the accumulator of another (see below).
 constexpr int kSmemAlpha = kSmemMisc + 64;
-constexpr int kSmemInverse = kSmemAlpha + kHeads * 4;
+constexpr int kSmemInverse = kSmemAlpha + 2 * kHeads * 4;
 constexpr int kSmemEnd = kSmemInverse + 2 * kHeads * 4;
 constexpr int kSmemBytes = kSmemEnd + 1024;  // + slack for the 1024-byte alignment
 
@@ -138,9 +138,6 @@ struct Shared {
   }
   __device__ __forceinline__ volatile uint32_t* rescale_mask() const {  // (team kernel)
     return reinterpret_cast<volatile uint32_t*>(ptr + kSmemMisc + 8);
-  }
-  __device__ __forceinline__ volatile int* softmax_failed() const {  // a softmax warp's wait has given up
-    return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 12);
   }
   __device__ __forceinline__ volatile int* first_negative() const {  // one per softmax warp
     return reinterpret_cast<volatile int*>(ptr + kSmemMisc + 16);
@@ -846,19 +843,14 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   __syncwarp();
   // The score buffer starts out free (first chunk, stage 0), and the metadata is in place.
   if (lane == 0) mbar_arrive(sm.bar(kKvFull0));
-  // What the four warps tell each other goes through named barriers: P for chunk c needs no wait but that for the scores (its
-  // barrier counts the end of PV c - 2, which read the same P tile), and a barrier that reduces a flag costs
+  // What the four warps tell each other goes through a named barrier: P for chunk c needs no wait but that for the scores (its
+  // barrier counts the end of PV c - 2, which read the same P tile), and a barrier that counts flags costs
   // less than the round trips to shared memory, behind the producers' copies, that an mbarrier and a word would be.
-  // Nobody may be left waiting at one. A warp whose wait gives up says so at the next reduction, and all four leave
-  // behind it.
-  volatile int* failed_word = sm.softmax_failed();
+  // Nobody may be left waiting at it. A warp whose wait gives up says so the next time they meet, and all four leave
+  // behind that. It counts with all its threads, one whose references move with one thread.
   bool failed = false;
-  auto give_up = [&]() {
-    failed = true;
-    if (lane == 0) *failed_word = 1;
-    __syncwarp();
-  };
-  auto anybody = [&](bool flag) { return named_barrier_any(3, 32 * kSoftmaxWarps, flag || failed); };
+  constexpr uint32_t kGivenUp = 32;
+  auto meet = [&](bool flag) { return named_barrier_count(3, 32 * kSoftmaxWarps, failed || (flag && lane == 0)); };
 
   // A finished token waits for its epilogue until the first chunk of the next working token has
   // been through the softmax, so that the MMA thread has a P to go on with while O is written out.
@@ -871,7 +863,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   // writes four complete 128-byte lines.
   // `chunks_before`: chunks of the stream whose PV precedes. Everybody's reciprocal denominators are there (a reduction lies between).
   auto epilogue = [&](uint32_t chunks_before) {
-    if (!warp_wait(sm.bar(kOutReady), outputs & 1, abort_flag)) { give_up(); return; }
+    if (!warp_wait(sm.bar(kOutReady), outputs & 1, abort_flag)) { failed = true; return; }
     ++outputs;
     tc_fence_after_sync();
     const float inverse = inverse_exchange[(done_count & 1) * kHeads + o_head];
@@ -924,14 +916,14 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
     const TokenInfo* info = sm.info(token_count & 1);
     int chunks = 0;
     if (token >= 0) {
-      if (!warp_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) { give_up(); break; }
+      if (!warp_wait(sm.bar(kTokenReady0 + (token_count & 1)), (token_count >> 1) & 1, abort_flag)) { failed = true; break; }
       chunks = info->chunks;
     }
     if (chunks == 0) {
       // No chunk to put the finished token's output behind. (And the resolver needs the finished token's row buffer
       // back before it can publish the token after this one: no point in holding its epilogue any longer.)
       if (done_token >= 0) {
-        if (anybody(false)) return;
+        if (meet(false) != 0) return;
         epilogue(chunk_count);
       }
       if (token < 0) break;
@@ -950,7 +942,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       const unsigned live_lo = next_live.x, live_hi = next_live.y;
       next_live = info->live[min(i + 1, kMaxChunks - 1)];  // a chunk ahead: shared loads queue behind the producers' copies
 
-      if (!warp_wait(sm.bar(kSFull0 + (chunk_count & 1)), (chunk_count >> 1) & 1, abort_flag)) { give_up(); anybody(true); return; }
+      if (!warp_wait(sm.bar(kSFull0 + (chunk_count & 1)), (chunk_count >> 1) & 1, abort_flag)) { failed = true; meet(true); return; }
       tc_fence_after_sync();
       // Of a head's two lanes the low one (0-15) holds the scores' sums over the even pairs of features, the
       // high one (16-31) those over the odd pairs. The two threads of a head share the softmax work: the low
@@ -1001,8 +993,15 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
       // two lanes of a head exchange their maxima only in the rare case: a shuffle waits in the same queue as
       // the producers' copies, a vote does not.
       float alpha = 1.f;
-      if (__any_sync(0xffffffffu, own_max - run_max > (i == 0 ? -kReferenceAligned : kReferenceRoom)))
-        alpha = move_reference(run_max, fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16)), i == 0);
+      const bool look = __any_sync(0xffffffffu, own_max - run_max > (i == 0 ? -kReferenceAligned : kReferenceRoom));
+      if (look) alpha = move_reference(run_max, fmaxf(own_max, __shfl_xor_sync(0xffffffffu, own_max, 16)), i == 0);
+      const bool moves = look && i > 0;  // some head's, and O holds earlier chunks
+      // The factor of a head is known to the threads that have its scores; the head's accumulator rows are in other threads' lanes.
+      // It goes along with every chunk: written only where some reference moves, behind the meeting and with another one for itself, it made
+      // chunks that rescale slower (4000 tokens whose scores rise by twelve binades from chunk to chunk 474 -> 456 us without; prefill
+      // of 8K tokens, which hardly rescales, 832 -> 818, 23 mixed requests 163.8 -> 162.0).
+      float* factors = alpha_exchange + (chunk_count & 1) * kHeads;
+      if (half == 0) factors[head] = alpha;
       // P to shared memory, one 128-byte row per head; this lane writes its 32 rows (64 bytes).
       const float2 scale = make_float2(p.scale_log2, p.scale_log2), reference = make_float2(-run_max, -run_max);
       float2 sum_a = make_float2(0.f, 0.f), sum_b = sum_a;  // four partial sums
@@ -1022,16 +1021,13 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
         *reinterpret_cast<uint4*>(p_tile + p_offset(head, half * 4 + u)) = make_uint4(words[0], words[1], words[2], words[3]);
       }
       run_sum = run_sum * alpha + ((sum_a.x + sum_a.y) + (sum_b.x + sum_b.y));
-      // O holds earlier chunks (if any). The factor of a head is known to the thread that has its scores;
-      // the head's accumulator rows are in other threads' lanes: where some reference moves the factors are handed over.
-      if (anybody(i > 0 && alpha != 1.f)) {
-        if (*failed_word != 0) return;
-        if (half == 0) alpha_exchange[head] = alpha;
-        named_barrier_sync(4, 32 * kSoftmaxWarps);
-        const float o_alpha = alpha_exchange[o_head];
+      const uint32_t met = meet(moves);
+      if (met >= kGivenUp) return;
+      if (met != 0) {
+        const float o_alpha = factors[o_head];
         // PV c - 1 has ended when its tile's second half is free. A parity tells that phase from the one before only, the end of
         // PV c - 4, which is long past: the producers waited for it before they brought tile c - 1 into the stage.
-        if (!warp_wait(sm.bar(kKvFree0 + 2 * ((chunk_count - 1) % kStages) + 1), ((chunk_count - 1) / kStages) & 1, abort_flag)) give_up();
+        if (!warp_wait(sm.bar(kKvFree0 + 2 * ((chunk_count - 1) % kStages) + 1), ((chunk_count - 1) / kStages) & 1, abort_flag)) failed = true;
         tc_fence_after_sync();
         // 32 columns at a time: a round trip to tensor memory each (in 16s the pass took 1500 cycles).
 #pragma unroll 1
@@ -1060,7 +1056,7 @@ __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
     const float own_inverse = 1.f / (run_sum + __shfl_xor_sync(0xffffffffu, run_sum, 16));
     if (half == 0) inverse_exchange[(done_count & 1) * kHeads + head] = own_inverse;
   }
-  anybody(false);  // of a warp that has given up since the last one
+  meet(false);  // with a warp that has given up since the last time
 }
 
 // ---- kernel and launch ------------------------------------------------------------------------
@@ -1084,7 +1080,6 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
     mbar_arrive(sm.bar(kSFull0));  // the P tiles start out free
     mbar_arrive(sm.bar(kSFull1));
     *sm.abort_flag() = 0;
-    *sm.softmax_failed() = 0;
   }
   if (warp == kMmaWarp) { tmem_alloc(smem_u32(tmem_slot), kTmemColumns); tmem_relinquish(); }
   tc_fence_before_sync();

@@ -45,18 +45,17 @@ inline cudaError_t launch_overlapped(Kernel kernel, int grid, int threads, size_
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) { asm volatile("barrier.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void named_barrier_arrive(int id, int threads) { asm volatile("barrier.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
 
-// Whether `flag` is set in any of `threads` threads (whole warps), all of which come here.
-__device__ __forceinline__ bool named_barrier_any(int id, int threads, bool flag) {
-  uint32_t any;
+// In how many of `threads` threads (whole warps), all of which come here, `flag` is set.
+__device__ __forceinline__ uint32_t named_barrier_count(int id, int threads, bool flag) {
+  uint32_t count;
   asm volatile(
       "{\n"
-      ".reg .pred p, q;\n"
+      ".reg .pred p;\n"
       "setp.ne.u32 p, %1, 0;\n"
-      "barrier.red.or.pred q, %2, %3, p;\n"
-      "selp.u32 %0, 1, 0, q;\n"
+      "barrier.red.popc.u32 %0, %2, %3, p;\n"
       "}\n"
-      : "=r"(any) : "r"(uint32_t(flag)), "r"(id), "r"(threads) : "memory");
-  return any != 0;
+      : "=r"(count) : "r"(uint32_t(flag)), "r"(id), "r"(threads) : "memory");
+  return count;
 }
 
 // ---- mbarrier -----------------------------------------------------------------------------

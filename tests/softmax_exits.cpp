@@ -1,6 +1,6 @@
-// The softmax warps' control flow on the CPU: `softmax_role`, taken from the kernel's source as it stands (role.inc), with one thread
-// for a warp, data that nobody looks at, and waits that give up where a run says so. The named barriers have no limit: whoever
-// would be left behind at one is what this looks for. stdin: runs as lines
+// The softmax warps' control flow on the CPU: `softmax_role`, taken from the kernel's source (role.inc), with one thread
+// for a warp, data that nobody looks at, and waits that give up where a run says so. The named barrier has no limit: whoever
+// would be left behind at it is what this looks for. stdin: runs as lines
 //   mode tokens chunks... rescale-mask warp wait     (mode 0: this wait of this warp gives up; 1: and every later one of anybody;
 // 2: as 0, and later ones by the toss of a coin). Prints "ok", or "left behind" for the first run in which not all four leave.
 #include <algorithm>
@@ -35,26 +35,27 @@ struct TokenInfo { int chunks; uint2 live[kMaxChunks]; };
 
 struct Run { int mode; std::vector<int> chunks; uint32_t rescale; int warp, wait; } run;
 std::vector<TokenInfo> infos;
-int abort_word, failed_flag;
+int abort_word;
 alignas(16) unsigned char shared_bytes[kSmemEnd];
 
 struct Barrier {  // like the hardware's: arrivals of any warps, four to a generation
   int arrived = 0, generation = 0;
-  bool flag = false, result = false;
-} barriers[5];
+  uint32_t count = 0, result = 0;
+} barriers[4];
 std::mutex mutex;
 std::condition_variable changed;
 bool stuck;
 struct LeftBehind {};
-inline bool meet(int id, int threads, bool flag) {
+template <typename Flag>
+inline uint32_t named_barrier_count(int id, int threads, Flag flag) {  // flag: of a lane
   std::unique_lock<std::mutex> lock(mutex);
   Barrier& b = barriers[id];
-  b.flag |= flag;
+  for (int lane = 0; lane < 32; ++lane) b.count += flag(lane);
   const int generation = b.generation;
   if (++b.arrived == threads / 32) {
-    b.result = b.flag;
+    b.result = b.count;
     b.arrived = 0;
-    b.flag = false;
+    b.count = 0;
     ++b.generation;
     changed.notify_all();
     return b.result;
@@ -66,8 +67,6 @@ inline bool meet(int id, int threads, bool flag) {
   }
   return b.result;
 }
-inline bool named_barrier_any(int id, int threads, bool flag) { return meet(id, threads, flag); }
-inline void named_barrier_sync(int id, int threads) { meet(id, threads, false); }
 
 thread_local int waits;
 thread_local std::minstd_rand coin;
@@ -113,7 +112,6 @@ struct Shared {
   uint32_t bar(int which) const { return which; }
   TokenInfo* info(int buffer) const;
   volatile int* abort_flag() const { return &abort_word; }
-  volatile int* softmax_failed() const { return &failed_flag; }
 };
 thread_local int tokens_walked;  // next() has run this often
 inline TokenInfo* Shared::info(int) const { return &infos[min(std::max(tokens_walked - 1, 0), int(infos.size()) - 1)]; }
@@ -137,7 +135,7 @@ int main() {
       infos[t].chunks = run.chunks[t];
       for (auto& live : infos[t].live) live = {0xffffffffu, 0xffffffffu};
     }
-    abort_word = failed_flag = 0;
+    abort_word = 0;
     for (auto& b : barriers) b = Barrier();
     std::vector<uint16_t> out(size_t(std::max(tokens, 1)) * kHeads * kFeatures + 8);
     void* aligned = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(out.data()) + 15) & ~uintptr_t(15));

@@ -49,7 +49,7 @@ def test_a_rescale_tells_the_end_of_the_products_before_it_from_earlier_ones():
         name, _, number = expression.partition("0 + ")
         return name, eval(number or "0", {"kStages": stages}, names)
 
-    rescale = source[source.index("named_barrier_sync(4,"):]
+    rescale = source[source.index("const float o_alpha = "):]
     waited, parity = re.search(r"warp_wait\(sm\.bar\((.+)\), (.+), abort_flag\)", rescale).groups()
     issue = source[source.index("void issue_pv("):source.index("void qk_role(")]
     commits = re.findall(r"mma_commit\(sm\.bar\((.+?)\)\);", issue.split("kPvSteps, false>")[-1])

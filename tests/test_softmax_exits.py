@@ -1,6 +1,7 @@
-"""The softmax warps meet at named barriers, which have no limit. A warp whose bounded wait has given up leaves only behind one at
-which all four learn of it: with any wait of any warp giving up, alone or with others, none is left at a barrier."""
+"""The softmax warps meet at a named barrier, which has no limit. A warp whose bounded wait has given up leaves only behind a meeting at
+which all four learn of it: with any wait of any warp giving up, alone or with others, none is left at the barrier."""
 
+import re
 import shutil
 import subprocess
 from pathlib import Path
@@ -15,8 +16,11 @@ WALKS = [  # chunks of a block's tokens
 
 def role(source):
     start = source.index("template <int kFormat>\n__device__ void softmax_role(")
-    return source[source.index("enum Bar {"):source.index("};", source.index("enum Bar {")) + 2] + "\n" + \
-        source[start:source.index("// ---- kernel and launch", start)]
+    text = source[start:source.index("// ---- kernel and launch", start)]
+    # what a thread of a warp hands to the barrier, as a function of its lane
+    text, found = re.subn(r"named_barrier_count\((.*), (failed [^;]*)\); };", r"named_barrier_count(\1, [&](int lane) -> bool { return \2; }); };", text)
+    assert found == 1
+    return source[source.index("enum Bar {"):source.index("};", source.index("enum Bar {")) + 2] + "\n" + text
 
 
 @pytest.fixture(scope="module")
@@ -49,13 +53,13 @@ def test_no_warp_is_left_at_a_barrier_when_waits_give_up(program):
     assert result.stdout == "ok\n", result.stdout
 
 
-@pytest.mark.parametrize("line", ["give_up(); anybody(true); return;", "if (*failed_word != 0) return;", "  anybody(false);  // of a warp that"])
+@pytest.mark.parametrize("line", ["failed = true; meet(true); return;", "if (met >= kGivenUp) return;", "  meet(false);  // with a warp that"])
 def test_a_way_out_that_misses_a_barrier_is_found(program, line):
     """The same on a text of the role in which one of its exits forgets the others."""
     if shutil.which("g++") is None:
         pytest.skip("no C++ compiler")
     source = (ROOT / "ascendflow_b200/csrc/sparse_mla_tcgen05.cuh").read_text()
     assert source.count(line) == 1
-    broken = source.replace(line, {"g": "give_up(); return;", "i": ""}.get(line[0], "//"))
+    broken = source.replace(line, {"f": "failed = true; return;", "i": ""}.get(line[0], "//"))
     result = subprocess.run([program(broken)], input="".join(runs()), capture_output=True, text=True, timeout=300)
     assert result.stdout.startswith("left behind"), result.stdout
