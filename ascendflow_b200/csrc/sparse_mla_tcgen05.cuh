@@ -1097,10 +1097,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_kernel(const Params p) 
     publish_first_token<false>(p, sm, first, sm.bar(kTokenReady0));
     softmax_role<kFormat>(p, sm, tmem);
   } else if (warp == kMmaWarp) {
-    if ((threadIdx.x & 31) == 0) qk_role<kFormat>(p, sm, tmem);
+    if (elect_one()) qk_role<kFormat>(p, sm, tmem);
     __syncwarp();
   } else if (warp == kPvWarp) {
-    if ((threadIdx.x & 31) == 0) pv_role<kFormat>(p, sm, tmem);
+    if (elect_one()) pv_role<kFormat>(p, sm, tmem);
     __syncwarp();
   } else if (warp == kResolverWarp) {
     publish_first_token<true>(p, sm, first, sm.bar(kTokenReady0));

@@ -470,11 +470,11 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
     team_maxima(p, sm, tmem, rank);
     team_softmax<kFormat>(p, sm, tmem, token, rank, sink, other_sink);
   } else if (warp == kMmaWarp) {
-    if (lane == 0) team_qk<kFormat>(sm, tmem, rank);
+    if (elect_one()) team_qk<kFormat>(sm, tmem, rank);
     __syncwarp();
     team_mask(sm, sink, other_sink);
   } else if (warp == kPvWarp) {
-    if (lane == 0) team_pv<kFormat>(sm, tmem);
+    if (elect_one()) team_pv<kFormat>(sm, tmem);
   } else {
     team_gather(p, sm, tmem, token, rank);
     team_early_slices(p, sm, rank);

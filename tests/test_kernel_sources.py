@@ -75,3 +75,12 @@ def test_slots_are_resolved_by_one_routine():
     source = (CSRC / "sparse_mla_tcgen05.cuh").read_text()
     assert source.count("report(p, kStatusBadPage") == 1
     assert "kStatusBadPage" not in (CSRC / "sparse_mla_team.cuh").read_text()
+
+
+@pytest.mark.parametrize("name", ["sparse_mla_tcgen05.cuh", "sparse_mla_team.cuh"])
+def test_issuing_threads_are_elected(name):
+    """A role that issues products runs in the thread that `elect.sync` chose: behind a comparison of the thread index every operand
+    of every product is moved to a uniform register by itself."""
+    kernel = (CSRC / name).read_text().split("__global__ void __launch_bounds__")[-1]
+    calls = re.findall(r"if \((\w+\(\))\) (?:team_)?(?:qk|pv)\w*<kFormat>\(", kernel)
+    assert calls == ["elect_one()"] * 2
