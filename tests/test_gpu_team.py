@@ -82,3 +82,24 @@ def test_a_token_without_visible_rows_and_the_fp32_reference():
     actual = S.output_to_numpy(tensors["attention_out"], "bf16")
     S.assert_close(actual, S.sampled_reference(tensors, meta, policy, list(range(5))), "team")
     assert not actual[1].any()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+def test_an_output_that_starts_between_sectors(dtype):
+    """Whole sectors are stored where the output starts on one, halves of them otherwise: the same bits, and nothing beside them."""
+    import torch
+
+    from ascendflow_b200 import ops
+
+    tensors, _, _ = call(np.random.default_rng(5), [1500, 90, 0, 640], 2, dtype, 1.0)
+    ops.sparse_mla(*(tensors[name] for name in S.TENSOR_ORDER))
+    count = tensors["attention_out"].numel()
+    for offset in (8, 16, 24):  # elements of two bytes
+        room = torch.full((count + 48,), 7.0, dtype=tensors["attention_out"].dtype, device="cuda")
+        start = offset + (-room.data_ptr() // 2) % 16
+        moved = dict(tensors, attention_out=room[start : start + count].view(tensors["attention_out"].shape))
+        assert moved["attention_out"].data_ptr() % 32 == offset * 2 % 32
+        ops.sparse_mla(*(moved[name] for name in S.TENSOR_ORDER))
+        torch.cuda.synchronize()
+        assert torch.equal(moved["attention_out"].view(torch.int16), tensors["attention_out"].view(torch.int16)), offset
+        assert (room[:start] == 7).all() and (room[start + count :] == 7).all(), offset
