@@ -192,6 +192,17 @@ def test_gpu_selection_at_the_lines_between_its_kernels(tokens, visible):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tokens,visible", [
+    (1800, [1024, 1023, 1025, 896, 897, 641, 640, 513]),  # 128 threads: lists that fill their last round, all but fill it, begin one
+    (300, [1024, 1023, 1025, 769, 768, 513]),             # 256
+    (140, [2048, 2047, 2049, 1537, 1536, 1024, 513]),     # 512
+])
+def test_gpu_selection_from_lists_that_end_on_a_round_of_their_block(tokens, visible):
+    """Rows as short as these are listed in full: the list is as long as the row."""
+    test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible)
+
+
+@pytest.mark.gpu
 def test_gpu_selection_feeds_the_attention_call():
     """Scores -> indices on the device -> attention, against the oracle fed with the oracle's selection."""
     import torch
