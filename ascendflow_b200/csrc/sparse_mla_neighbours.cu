@@ -606,7 +606,7 @@ struct Loads {
 // 768 x 65536 scores, against the radix select that read every row five times: constant 373 -> 55 us, zeros 383
 // -> 80, all but 300 masked 360 -> 142, correlated over 64 positions 326 -> 192 (a fifth of the rows);
 // 100 rows of the latter 114 -> 80. With that select as the way out they took 461, 433, 457, 283 and 127.
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow, bool kCopyScores>
 __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
   using Shared = SelectShared<kThreads, kCapacity, kWindowSize>;
   constexpr int kWindow = Shared::kWindow;
@@ -644,6 +644,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     // An eighth of the row, or kMostQuads 16-byte quads per thread: eight threads share a 128-byte
     // segment, and the segments lie at equal distances.
     constexpr int kSegments = kThreads / 8;
+    // Where more quads than these are for long rows only, short ones step over them (8192 x 4 K scores 76 -> 73 us).
+    constexpr int kFewQuads = 2;
     const int quads = max(1, min(kMostQuads, candidates / (32 * kThreads))), sampled = quads * kThreads;
     const unsigned step = (unsigned(candidates) >> 2) / unsigned(quads * kSegments);  // at least eight quads
     uint4 v[kMostQuads];
@@ -652,9 +654,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
       if (q < quads) v[q] = __ldg(reinterpret_cast<const uint4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
     // The row's head on its way to L2 behind the sample, while the floor is found.
     if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kHead));
-    uint32_t key[4 * kMostQuads];
+    uint32_t key[4 * kMostQuads] = {};
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q) {
+      if (q == kFewQuads && quads <= kFewQuads) break;
       key[4 * q + 0] = q < quads ? score_key(v[q].x) : 0; key[4 * q + 1] = q < quads ? score_key(v[q].y) : 0;
       key[4 * q + 2] = q < quads ? score_key(v[q].z) : 0; key[4 * q + 3] = q < quads ? score_key(v[q].w) : 0;
     }
@@ -667,7 +670,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     // which lie about four G samples: G = all threads, or a quarter of them where that is enough.
     unsigned best = 0;
 #pragma unroll
-    for (int e = 0; e < 4 * kMostQuads; ++e) best = max(best, key[e]);
+    for (int e = 0; e < 4 * kMostQuads; ++e) {
+      if (e == 4 * kFewQuads && quads <= kFewQuads) break;
+      best = max(best, key[e]);
+    }
     if (wanted <= unsigned(kThreads / 4)) {
       best = max(best, __shfl_xor_sync(0xffffffffu, best, 1));
       best = max(best, __shfl_xor_sync(0xffffffffu, best, 2));
@@ -679,8 +685,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     while (true) {  // normally once; again inside a bin that holds too many (a sample of both signs, say)
       const int shift = max(0, 24 - __clz(int(upper - lower)));  // 256 bins over [lower, upper]
 #pragma unroll
-      for (int e = 0; e < 4 * kMostQuads; ++e)
+      for (int e = 0; e < 4 * kMostQuads; ++e) {
+        if (e == 4 * kFewQuads && quads <= kFewQuads) break;
         if (key[e] >= lower && key[e] <= upper) atomicAdd(&s.histogram[(upper - key[e]) >> shift], 1u);
+      }
       __syncthreads();
       find_bin(s, wanted);
       if (s.bin == kSelectBins) break;  // fewer samples than wanted: all of them
@@ -749,8 +757,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
         if (at + unsigned(__popc(hits)) > kCapacity) continue;  // noticed below: s.count says so
         // Few rows wait for what is issued for them, all of a step's scores as candidates for a place: a loop over the hits, which
         // copies the scores from where the load has just put them (16 x 16 K scores 6.56 -> 6.44 us, 100 x 64 K 10.7 -> 9.2). With many
-        // rows these copies wait for L2, or for memory where it has been given up (8192 x 12-16 K 116 -> 145, 768 x 64 K 38 -> 56).
-        if constexpr (kThreads >= 512) {
+        // rows these copies wait for L2, or for memory where it has been given up (8192 x 12-16 K 116 -> 145, 768 x 64 K 38 -> 56, 600 x 200 K 113 -> 117).
+        if constexpr (kCopyScores) {
           do {
             const unsigned which = __clz(hits), position = first + (which >> 2) * 4 * kThreads + (which & 3);
             s.list[at].x = position;
@@ -771,7 +779,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
     };
     if (kShortRow > 0 && end <= unsigned(kShortRow)) list_row(Loads<4>{});
     else list_row(Loads<kInFlight>{});
-    if constexpr (kThreads >= 512) asm volatile("cp.async.wait_all;\n" ::: "memory");
+    if constexpr (kCopyScores) asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     const int listed = int(s.count);
     if (listed >= kTopK && listed <= kCapacity) {
@@ -813,9 +821,10 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
   }
 }
 
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads), int kShortRow = 0>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads), int kShortRow = 0,
+          bool kCopyScores = (kThreads >= 512)>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow>;
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow, kCopyScores>;
   constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity, kWindow>));
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
@@ -859,28 +868,34 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
   // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread for rows of more than three steps of
   // four. The kernel looks at the row for that: a buffer is as wide as the longest context (16 x 64 K: 10.8 with four loads, 10.3 with
-  // eight; 30000: 8.5, 8.3; 24000: 7.6, 8.0; 4 K in buffers of 32 to 128 K: 6.9, 7.35). Otherwise
+  // eight; 30000: 8.5, 8.3; 24000: 7.6, 8.0; 4 K in buffers of 32 to 128 K: 6.9, 7.35). Two such blocks run on an SM: up to twice as
+  // many tokens in buffers beyond 32 K (sixteen / eight warps, 200 x 64 K: 13.3 / 16.8, 296 x 64 K: 14.3 / 18.5, 296 x 40000: 12.0 / 12.9,
+  // 200 x 32768: 10.9 / 11.4, 296 x 17000: 10.5 / 10.0, and rows of 4 K in a buffer of 64 K 9.6 / 9.1). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
-  // more than a wave of them (8192 rows of 12-16 K scores: 120 us against 144 with eight warps, which
-  // repeat the per-row steps twice as often), eight where there are fewer (1500 such rows: 33 us against
-  // 38) or where the row needs the larger sample. What such rows wait for is one step after the other: up to 16 K scores
-  // (a bitmap of one window) ten blocks of 48 registers per SM with four loads in flight are better than eight with eight loads (8192
-  // x 12-16 K: 119.9 -> 118.0 us, 16384 rows of a prompt of 10 K: 194.0 -> 176.0, 4096 x 8 K: 54.8 -> 51.3), but beyond 10 K scores
-  // only where they make fewer waves: every block is slower for it (eight / ten blocks per SM, 1800 x 16 K: 34.0 / 36.7, 3300 x 16 K: 54.6 /
-  // 56.8, 2450 x 16 K: 44.1 / 42.0, 7400 x 16 K: 121.8 / 120.9; 2300 x 12 K: 36.5 / 38.1, 7400 x 12 K: 107.8 / 106.0; 3300 x 10 K:
-  // 49.8 / 49.3). Rows of one constant are all streaming and 3 to 7 % slower with ten (8192 x 12 K: 88.9 / 93.9; zeros 109.6 / 94.0 by
-  // `list_by_order`); nothing says so before the launch. Longer rows are streaming for the most part: eight blocks, eight
+  // more than a wave of them (four / eight warps, 8192 x 13000: 115.6 / 130, 4096 x 8 K: 49.6 / 58, 1500 x 2000: 16.8 / 19.8, but 2300 x 12 K: 32.9
+  // / 37.8 beside 75 / 65 for scores that correlate), eight where there are fewer (1000 x 8 K: 14.9 / 19.0, but correlated 39.8 / 32.9: their
+  // lists miss more often the smaller the sample is) or where the row needs the larger sample. What such rows wait for is one step after the
+  // other: up to 16 K scores (a bitmap of one window) ten blocks of 48 registers per SM with four loads in flight against eight with
+  // eight loads: ten / eight, 8192 x 2000: 66.0 / 76.3, 4096 x 8 K: 49.6 / 50.9, 3300 x 10 K: 45.5 / 45.0; beyond 10 K scores
+  // only where they make fewer waves (2450 x 16 K: 39.9 / 40.9, 7400 x 12 K: 98.0 / 98.2, 7400 x 16 K: 111.1 / 107.6; where they do not, 1800 x
+  // 16 K: 34.4 / 30.4, 3300 x 16 K: 54.9 / 50.7). Longer rows are streaming for the most part: eight blocks, eight
   // loads (4096 x 17408: 74.3 / 76.9, 2000 x 20 K: 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536
   // entries, which rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
-  if (T <= multiprocessors && SPAN > 24576) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
-  if (T <= multiprocessors || SPAN > 131072) return launch_select<512, 4096, 2, 2>(p, s);
+  if (T <= multiprocessors && SPAN <= 24576) return launch_select<512, 4096, 2, 2>(p, s);
+  if (SPAN <= 131072 && (T <= multiprocessors || (T <= int64_t(multiprocessors) * 2 && SPAN > 32768))) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
+  if (SPAN > 131072)
+    return T <= int64_t(multiprocessors) * 2 ? launch_select<512, 4096, 2, 2>(p, s) : launch_select<512, 4096, 2, 2, 4, 65536, 0, false>(p, s);
   const bool fewer_waves = (T - 1) / (multiprocessors * 10) < (T - 1) / (multiprocessors * 8);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
     return SPAN <= (fewer_waves ? 16384 : 10240) ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
   // A bitmap no larger than the row: what shared memory it does not take holds scores that are read again (860 x 16 K: 19.7 ->
   // 19.0 us, 150 such rows that correlate 39.1 -> 36.3; blocks of 512 threads: no change).
-  return SPAN <= 16384 ? launch_select<256, 2560, 6, 2, 4, 16384>(p, s) : launch_select<256, 2560, 6, 2>(p, s);
+  if (SPAN <= 16384) return launch_select<256, 2560, 6, 2, 4, 16384>(p, s);
+  // Of 128 K scores a sample of 2048 leaves some fifteen hundred in the list, give or take three hundred, and room for 2560: every few
+  // thousand rows one is gone through again, which the call waits for. Twice the sample, 768 x 128 K: 82 us where it was 159 (500: 51 / 125, 3000: 252 / 332; calls
+  // without such a row, 320 x 128 K: 37.9 / 36.8). Up to 98304 scores the smaller one is enough (768 of them: 63.0, 65.3 with the larger).
+  return SPAN > 98304 ? launch_select<256, 2560, 6, 4>(p, s) : launch_select<256, 2560, 6, 2>(p, s);
 }
 
 int launch_sparse_mla_cache_append_flagged(void* stream, void* arg_new_rows, void* arg_cache, void* arg_block_table,

@@ -185,6 +185,9 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     (1790, [8192, 1025, 8191]), (148, [16388, 512, 20000]), (148, [16384, 2049]),  # a row per SM, either number of loads
     (149, [16388, 1]), (149, [16384, 16383, 2561]), (20, [131072, 16388, 65537]),
     (2368, [16000, 9000, 12289]), (2369, [16384, 10241]), (1800, [10240, 700]), (1800, [10244, 10241, 10240]),  # waves of eight and of ten blocks
+    (296, [32772, 32768, 700]), (296, [32768, 4097]), (297, [32772, 20000]),  # two rows per SM
+    (297, [98308, 98304, 1025]), (297, [98304, 30000]),  # the larger sample
+    (296, [131076, 513]), (297, [131076, 700]),  # scores copied or listed with their positions
     (148, [24576, 24575, 4096]), (148, [24580, 24576, 24577, 24575, 2049, 700, 512]),  # the row's own length chooses it
 ])
 def test_gpu_selection_at_the_lines_between_its_kernels(tokens, visible):
