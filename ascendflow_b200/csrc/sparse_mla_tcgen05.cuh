@@ -504,28 +504,21 @@ __device__ __forceinline__ void store_places(uint32_t places_tmem, int lane) {
   tmem_st16(places_tmem, columns);
 }
 
-// Copies of a chunk's rows into a tile, all 64 or one half of them, by the 256 producer threads.
+// Copies of a chunk's rows into a tile, all 64 or one half of them, by the 256 producer threads. A row is taken by eight threads, 128
+// bytes at a time: two rows and their addresses to a thread. (Sixteen threads with 256 bytes at a time make as many requests, but four rows
+// to a thread: 62.3 million instructions of a warp for 2072 tokens against 58.6, one token 9.09 -> 8.97 us, 256 tokens at 4K 28.3 -> 27.6.)
 template <int kHalf, int kHalves>
 __device__ __forceinline__ void gather_rows(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
-  constexpr int kRows = kChunkRows / (kProducerThreads / 16) / kHalves;  // of a thread
-  const int sub = tid & 15;  // sixteen threads per row: 256 bytes at a time
-  const char* source[kRows];
-  bool live[kRows];
+  constexpr int kAtOnce = kProducerThreads / 8, kRows = kChunkRows / kAtOnce / kHalves;  // rows side by side; of a thread
+  const int sub = tid & 7;  // eight threads per row: 128 bytes at a time
+  const char* base = static_cast<const char*>(chunk * kChunkRows < kWindow ? p.ori_kv : p.cmp_kv) + sub * 16;
 #pragma unroll
   for (int k = 0; k < kRows; ++k) {
-    const int slot = chunk * kChunkRows + (tid >> 4) + (kHalf * kRows + k) * (kProducerThreads / 16);
-    const int row = rows[slot];
-    live[k] = row >= 0;
-    source[k] = static_cast<const char*>(slot < kWindow ? p.ori_kv : p.cmp_kv) + (size_t)(row < 0 ? 0 : row) * kRowBytes;
-  }
+    const int r = (tid >> 3) + (kHalf * kRows + k) * kAtOnce, row = rows[chunk * kChunkRows + r];
+    const char* source = base + (size_t)max(row, 0) * kRowBytes;
+    const uint32_t target = tile + swizzled(r, sub);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int unit = q * 16 + sub;
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const int r = (tid >> 4) + (kHalf * kRows + k) * (kProducerThreads / 16);
-      cp_async16(tile + swizzled(r, unit), source[k] + unit * 16, live[k]);
-    }
+    for (int q = 0; q < 8; ++q) cp_async16(target + q * kBlockBytes, source + q * 128, row >= 0);
   }
 }
 

@@ -82,5 +82,5 @@ def test_issuing_threads_are_elected(name):
     """A role that issues products runs in the thread that `elect.sync` chose: behind a comparison of the thread index every operand
     of every product is moved to a uniform register by itself."""
     kernel = (CSRC / name).read_text().split("__global__ void __launch_bounds__")[-1]
-    calls = re.findall(r"if \((\w+\(\))\) (?:team_)?(?:qk|pv)\w*<kFormat>\(", kernel)
+    calls = re.findall(r"if \((\w+\(\))\) (?:team_)?(?:qk|pv)\w*<kFormat[^>]*>\(", kernel)
     assert calls == ["elect_one()"] * 2
