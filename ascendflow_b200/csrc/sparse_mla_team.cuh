@@ -381,11 +381,13 @@ __device__ __forceinline__ bool team_softmax(const Params& p, const Shared& sm, 
   }
   const volatile float* maxima = sm.maxima(kTeamMaxima);
   if (!warp_wait<true>(sm.bar(kMaxima), 0, abort_flag)) return false;  // all blocks' (and so all own scores have been read)
+  // The references of all own chunks at once: followed for every chunk it took 200 cycles of the way from scores to P (16 tokens 9.37 -> 9.26 us).
+  float references[kOwnItems] = {sink, sink, sink};
+  follow_reference(maxima + head, sink, chunks, [&](int i, float reference, float) { if (i % kBlocks == rank) references[i / kBlocks] = reference; });
+  tc_fence_after_sync();
   int own = 0;
   for (int item = rank; item < chunks; item += kBlocks, ++own) {
-    float run_max = sink;
-    follow_reference(maxima + head, sink, chunks, [&](int i, float reference, float) { if (i == item) run_max = reference; });
-    tc_fence_after_sync();
+    const float run_max = own == 0 ? references[0] : own == 1 ? references[1] : references[2];  // (no array by a variable index)
     float2 prob[16];
     team_scores(tmem, own, half ? info->live[item].y : info->live[item].x, prob);
     const float2 scale = make_float2(p.scale_log2, p.scale_log2), reference = make_float2(-run_max, -run_max);
