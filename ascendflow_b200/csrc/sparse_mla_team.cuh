@@ -53,6 +53,7 @@ constexpr int kTeamMaxima = kTeamSums + kMaxChunks * kSumBytes;  // float[10][64
 static_assert(kTeamMaxima + kMaxChunks * kHeads * 4 <= kSmemRows && kTeamMaxima >= kOwnItems * kTileBytes,
               "areas do not meet; maxima arrive while tiles are in use");
 static_assert(kMaxChunks - kSliceSlots == 2, "two late slices");
+static_assert(kTileBytes == kBlocks * kSliceBytes && kTeamSlices == kSmemKv && kSliceSlots == 2 * kBlocks, "slices of the first two own chunks lie in their tiles");
 __host__ __device__ constexpr uint32_t score_columns(int own) { return own == 0 ? 0 : own == 1 ? 128 : 384; }
 constexpr uint32_t kTeamO = kTmemQ;
 
@@ -139,6 +140,7 @@ __device__ __forceinline__ void gather_slices(const Params& p, const Shared& sm,
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
     if (item + i >= chunks) break;
+    if (item + i < kSliceSlots && (item + i) % kBlocks == rank) continue;  // in place
     const char* cache = static_cast<const char*>(chunk[i] * kChunkRows < kWindow ? p.ori_kv : p.cmp_kv) + rank * 256 + unit * 16;
     const uint32_t slice = sm.base + kTeamSlices + (item + i) % kSliceSlots * kSliceBytes + (unit >> 3) * kBlockBytes;
 #pragma unroll
@@ -150,7 +152,8 @@ __device__ __forceinline__ void gather_slices(const Params& p, const Shared& sm,
 }
 
 // Phase A, producer warps: the first eight chunks' slices. They fill the places of the own chunks' first two
-// tiles, four each, which are free when these have been multiplied.
+// tiles, four each, which are free when these have been multiplied. A block's slice of its own chunk is there already: in the tile's order of
+// features it lies just where the slice of that item has to be (one token 8.88 -> 8.80 us, 33 tokens 11.21 -> 11.11).
 __device__ void team_early_slices(const Params& p, const Shared& sm, int rank) {
   const int tid = threadIdx.x - kFirstProducerWarp * 32;
   volatile int* abort_flag = sm.abort_flag();
