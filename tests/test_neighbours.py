@@ -206,6 +206,37 @@ def test_gpu_selection_from_lists_that_end_on_a_round_of_their_block(tokens, vis
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tokens", [7, 140, 300, 1800])  # 512 threads twice, 256, 128
+def test_gpu_selection_with_every_number_of_scores_at_its_threshold(tokens):
+    """One to 34 equal scores, the threshold among them: up to 32 are ranked by one warp, eight at a time or one by one."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+
+    rng = np.random.default_rng(tokens)
+    span = 1000
+    policy = O.make_policy(tokens, tokens, ratio=1, max_seq=1024, blocks=8)
+    lengths = np.full(tokens, span, dtype=np.int32)
+    data = {
+        "cu_seqlens_q": np.arange(tokens + 1, dtype=np.int32),
+        "seqused_ori_kv": lengths, "seqused_cmp_kv": lengths,
+        "cmp_residual_kv": np.zeros(tokens, dtype=np.int32),
+    }
+    scores = np.empty((tokens, span), dtype=np.float32)
+    for token in range(tokens):
+        equal = 1 + token % 34 if tokens > 34 else (1, 8, 9, 16, 17, 32, 33)[token]
+        inside = int(rng.integers(1, equal + 1))                 # of them win
+        better = 512 - inside
+        row = np.concatenate([rng.uniform(2e4, 4e4, better), np.full(equal, 1e4), rng.uniform(0, 10, span - better - equal)])
+        scores[token] = rng.permutation(row)
+    expected = O.select_topk_indices(scores, data, policy)
+    device = {k: torch.from_numpy(v).cuda() for k, v in data.items()}
+    actual = neighbours.topk_indices(torch.from_numpy(scores).cuda(), device["cu_seqlens_q"], device["seqused_cmp_kv"],
+                                     device["cmp_residual_kv"], ratio=1)
+    assert np.array_equal(actual.cpu().numpy(), expected)
+
+
+@pytest.mark.gpu
 def test_gpu_selection_feeds_the_attention_call():
     """Scores -> indices on the device -> attention, against the oracle fed with the oracle's selection."""
     import torch
