@@ -809,9 +809,10 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // A second P tile takes the wait for the previous PV out of the chain, and flags by a named barrier a word in shared memory and a
 // wait: five per cent of 100 and of 256 tokens, two of 1000, one of prefill of 8K.
 //
-// Calls one after the other take 815 us for prefill of 8K tokens at 32K, 110 for decode 128 x 6 at 128K, 162 for 23 mixed requests, 30 for
-// 256 tokens at 4K. The first three are at the board's power limit (990 to 1000 W; 1.55 to 1.60 GHz while they run, 0.05 less and
-// three per cent more time on other boards), where energy decides more than cycles.
+// Calls one after the other take 815 us for prefill of 8K tokens at 32K (835 with sixteen threads to a gathered row and issuing threads that were not
+// elected, in turn on one board), 114 for decode 128 x 6 at 128K (116), 162 for 23 mixed requests (166), 27.5 for
+// 256 tokens at 4K (29.4). The first three are at the board's power limit (990 to 1000 W; 1.47 to 1.60 GHz while they run, by the board: three
+// per cent of time between two of them), where energy decides more than cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

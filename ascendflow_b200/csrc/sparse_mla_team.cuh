@@ -14,13 +14,13 @@
 //
 // Bound by latency. One token on one block takes 30 k cycles: 6 k until its first scores, 2 k per chunk, 3 k for
 // the output pass. Here the chunks' first product and softmax run side by side, and the output pass is a
-// quarter. Of the 19 k cycles that are left the token's resolution takes 3.7 k, gather, scores and maxima of up to
-// three chunks 6 k, the first P 1.1 k, the second product, in the order of the chunks, 6.6 k (and a thousand more for
-// every chunk at which a reference moves), output 1.7 k. A call of one token 15.3 -> 10.7 us, of 16 tokens 16.3 -> 11.0
-// (one warp resolving the token, all slices gathered behind a barrier of the cluster, products issued by a whole
-// warp before). Eight blocks had less for one token, nothing for eight; P written to the other blocks by
-// the softmax threads instead of bulk copies was slower by a fifth. Copies between blocks are of local shared
-// memory; nothing multicasts.
+// quarter. Of the 15 k cycles that are left the token's resolution takes 2.9 k, gather, scores and maxima of up to
+// three chunks 5.3 k, the first P 1 k, the second product, in the order of the chunks, 4.5 k (and a thousand more for
+// every chunk at which a reference moves), output 1.3 k. Between calls of one token 8.8 us pass, of 16 tokens 9.2, of 33 tokens
+// 11.2 (10.7, 11.0 and 12.9 before the issuing threads were elected and the softmax's way from maxima to P was cut short); 1.3 to 1.6 of
+// them lie between the end of one launch and the first instruction of the next that may read. Eight blocks: 9.19 against 9.18 for one token,
+// 10.3 against 9.3 for eight. P written to the other blocks by the softmax threads instead of bulk copies was slower by a fifth.
+// Copies between blocks are of local shared memory; nothing multicasts.
 //
 // Tensor memory: columns 0-63, 128-191 and 384-447 the scores of the own chunks, 256-383 Q and 448-463 its
 // metadata as in `attention_kernel`; once all scores are computed, 256-319 O (128 features).
@@ -254,8 +254,8 @@ __device__ __forceinline__ void issue_team_pv(uint32_t tmem, uint64_t p_desc, ui
 }
 
 // Phase B, one thread: O = P X over all chunks, this block's 128 features. Unrolled over the chunks: in a loop the
-// descriptors of every instruction are moved to uniform registers first, and a chunk's four instructions take
-// twice as long (one token 11.7 -> 11.0 us, 16 tokens 12.5 -> 11.7).
+// descriptors of every instruction are worked out on the way to it (one token 9.69 -> 8.83 us, 16 tokens 10.02 -> 9.20; two
+// chunks to a pass 9.14 and 9.46).
 template <int kFormat>
 __device__ void team_pv(const Shared& sm, uint32_t tmem) {
   volatile int* abort_flag = sm.abort_flag();
