@@ -47,14 +47,14 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # B16 x 6 queries at ctx 128K: 96 tokens). Other sizes of the same regime are scaled by token
 # count, since traffic is Q + O + gathered rows per token. Every figure belongs to the kernel
 # sources whose hash is recorded with it: a line measured with other sources says so.
-PROFILED_SOURCES = "e8cacc8f5123e0e93ee443255d83c84729468a7fc0b5033129b73282e9cab6b7"
+PROFILED_SOURCES = "1ff1d5fe86501ccc937439aeb2e28d8b8c7a7673eff8bce68d16bd20e045f5cd"
 FULL_SIZE_DECODE_SOURCES = "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3"
 MEASURED_TRAFFIC = {  # query tokens of the captured launches: bytes of a launch, sources
     "prefill": {"profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md",
-                "launches": {8192: (1077.67e6, PROFILED_SOURCES)}, "scaled_from": 8192},
+                "launches": {8192: (1077.29e6, PROFILED_SOURCES)}, "scaled_from": 8192},
     "decode": {"profile": "profiles/attention_kernel_decode_dram_traffic.md",
                "launches": {768: (500.34e6, FULL_SIZE_DECODE_SOURCES), 384: (242.30e6, FULL_SIZE_DECODE_SOURCES),
-                            96: (58.98e6, PROFILED_SOURCES)}, "scaled_from": 768},
+                            96: (59.72e6, PROFILED_SOURCES)}, "scaled_from": 768},
 }
 EXTRA_WORKLOADS = ("prefill_q32k_ctx32k", "decode_b64_q6_ctx128k", "decode_b128_q6_ctx128k")
 CONFIG_KEYS = {"heads": 64, "features": 512, "topk": 512, "window": 128, "ratio": 2, "values": "N(0,1)",
