@@ -35,6 +35,7 @@ struct SelectParams {
   const int32_t* residual;   // [B]
   int32_t* out;              // [T, 512]
   int32_t batches, tokens, ratio;
+  bool one_wave;             // no more rows than blocks of 256 threads run at once
   int64_t span;
 };
 
@@ -665,8 +666,11 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q)
       if (q < quads) v[q] = __ldg(reinterpret_cast<const uint4*>(row) + (q * kSegments + (threadIdx.x >> 3)) * step + (threadIdx.x & 7));
-    // The row's head on its way to L2 behind the sample, while the floor is found.
-    if (threadIdx.x == 0) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kHead));
+    // The row's head on its way to L2 behind the sample, while the floor is found. Not where all rows of a call start at once and are not
+    // long: the heads of those that are first stand in front of the others' samples (800 x 8 K 14.26 -> 13.60 us, 500 x 16 K 13.86 -> 13.38, 888 x
+    // 18000 19.4 -> 18.9, 300 x 16 K 11.6 -> 11.3; but 300 x 3000 8.03 -> 8.12, 300 x 18000 with little L1 12.7 -> 13.2, 1200 x 16 K 25.6 -> 26.9).
+    constexpr bool kMayWait = kThreads == 256 && kWindow <= 24576;
+    if (threadIdx.x == 0 && !(kMayWait && p.one_wave && end > kHead / 4 * 3)) prefetch_l2(row, 4u * min((end + 3u) & ~3u, kHead));
     uint32_t key[4 * kMostQuads] = {};
 #pragma unroll
     for (int q = 0; q < kMostQuads; ++q) {
@@ -873,6 +877,7 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   p.span = SPAN;
   int device = 0, multiprocessors = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
+  p.one_wave = T <= int64_t(multiprocessors) * 6;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // Rows so long that a small block's sample says too little: large blocks (16 x 1 M scores: 98 us against 398
   // with 512 threads, 300 x 1 M: 357 against 695, 16 x 200 K: 32.8 against 35.8), for many rows only beyond 256 K.
