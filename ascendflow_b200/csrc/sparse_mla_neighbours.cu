@@ -910,13 +910,15 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // A bitmap no larger than the row: what shared memory it does not take holds scores that are read again (860 x 16 K: 19.7 ->
   // 19.0 us, 150 such rows that correlate 39.1 -> 36.3; blocks of 512 threads: no change).
   if (SPAN <= 16384) return launch_select<256, 2560, 6, 2, 4, 16384>(p, s);
-  // The same beyond, where two more such steps lie: six blocks with a bitmap of 24 K leave 92 KiB of L1 on an SM, of 32 K 60, of 64 K
+  // The same beyond, where three more such steps lie: six blocks with a bitmap of 24 K leave 92 KiB of L1 on an SM, of 32 and 48 K 60, of 64 K
   // 28, and the sample's 48 KiB are read again in the pass (64 K / the smaller one: 600 x 18000 17.8 / 16.6, 888 x 24000 23.0 / 21.0, 1200
-  // x 18000 30.5 / 27.8, 300 x 20000 12.8 / 12.6). The step to 32 K is taken where the last wave is at least half full (600 x 30000
-  // 22.9 / 20.9, 888 x 32768 26.0 / 24.9, 1750 x 30000 50.0 / 46.3; where it is not, 300 x 32768 14.6 / 15.1, 1200 x 32768 35.4 / 35.8).
+  // x 18000 30.5 / 27.8, 300 x 20000 12.8 / 12.6). The steps to 32 and 48 K are taken where the last wave is at least half full (600 x 30000
+  // 22.9 / 20.9, 888 x 32768 26.0 / 24.9, 1750 x 30000 50.0 / 46.3, 600 x 45000 28.9 / 25.5, 888 x 48 K 35.4 / 34.0; where it is not, 300 x
+  // 32768 14.6 / 15.1, 1200 x 32768 35.4 / 35.8, 1000 x 48 K 43.2 / 44.8).
   // A smaller one for longer rows, in several rounds: 500 x 50000 27.5 / 26.2, but 300 x 64 K 21.8 / 24.4.
   if (SPAN <= 24576) return launch_select<256, 2560, 6, 2, 4, 24576>(p, s);
-  if (SPAN <= 32768 && (T - 1) % (int64_t(multiprocessors) * 6) >= int64_t(multiprocessors) * 3) return launch_select<256, 2560, 6, 2, 4, 32768>(p, s);
+  if (SPAN <= 49152 && (T - 1) % (int64_t(multiprocessors) * 6) >= int64_t(multiprocessors) * 3)
+    return SPAN <= 32768 ? launch_select<256, 2560, 6, 2, 4, 32768>(p, s) : launch_select<256, 2560, 6, 2, 4, 49152>(p, s);
   // Of 128 K scores a sample of 2048 leaves some fifteen hundred in the list, give or take three hundred, and room for 2560: every few
   // thousand rows one is gone through again, which the call waits for. Twice the sample, 768 x 128 K: 82 us where it was 159 (500: 51 / 125, 3000: 252 / 332; calls
   // without such a row, 320 x 128 K: 37.9 / 36.8). Up to 98304 scores the smaller one is enough (768 of them: 63.0, 65.3 with the larger).

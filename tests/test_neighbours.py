@@ -188,7 +188,8 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     (296, [32772, 32768, 700]), (296, [32768, 4097]), (297, [32772, 20000]),  # two rows per SM
     (297, [98308, 98304, 1025]), (297, [98304, 30000]),  # the larger sample
     (297, [16388, 16384, 513]), (297, [24576, 24575, 16385, 700]), (297, [24580, 24576]),  # bitmaps of 16, 24 and 64 K
-    (444, [32768, 24577]), (446, [24580, 24577, 1025]), (446, [32768, 32767, 30001, 2561]), (446, [32772, 32768]),  # or 32 K
+    (444, [32768, 24577]), (446, [24580, 24577, 1025]), (446, [32768, 32767, 30001, 2561]), (446, [32772, 32768]),
+    (446, [49152, 49151, 40001]), (446, [49156, 49152]), (444, [49152]),  # or 32 and 48 K
     (296, [131076, 513]), (297, [131076, 700]),  # scores copied or listed with their positions
     (148, [24576, 24575, 4096]), (148, [24580, 24576, 24577, 24575, 2049, 700, 512]),  # the row's own length chooses it
 ])
