@@ -308,7 +308,8 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
   };
   const bool sampled = floor_key != 0;
   int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
-  // The list is filled up to whole rounds of the block with entries that come last and win nothing: no loop over it looks for its end.
+  // The list is filled up to whole rounds of the block: no loop over it looks for its end. The filling's position is one that no row has (it is in
+  // no window and not before `end`), its key is 0: it reaches no sampled floor, which is at least 1, and lies above no key.
   const int rounds = (listed + kThreads - 1) / kThreads;
   static_assert(kCapacity % kThreads == 0, "whole rounds fit");
   if (listed + int(threadIdx.x) < rounds * kThreads) s.list[listed + threadIdx.x] = make_uint2(0xffffffffu, 0xffffffffu);
@@ -374,14 +375,16 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
   auto win_if = [&](bool wins, unsigned position) { shared_or_if(wins && position < kWindow, bitmap + (position >> 5) * 4, 1u << (position & 31)); };
   auto compare = [&](uint2 entry) { s.few[atomicAdd(&s.few_count, 1u)] = (unsigned long long)~entry.y << 32 | entry.x; };
   if (ties == 0xffffffffu) {
-    // Keys above `before` lie before the bin (whatever lies above the sample's highest among them), keys from `within` on in it.
+    // Keys above `before` lie before the bin (whatever lies above the sample's highest among them), keys from `within` on in it. A bin that
+    // reaches down to key 0 (rows listed whole, with masks or NaNs that have a sign at the threshold) has the filling's key in it, which a
+    // real entry may have too: there it is the position that tells them apart.
     const unsigned before = top - (prefix << shift), depth = prefix << shift | ((1u << shift) - 1);
     const unsigned within = max(floor_key, top - min(depth, top));
 #pragma unroll 4
     for (int r = 0; r < rounds; ++r) {
       const uint2 entry = s.list[r * kThreads + threadIdx.x];
       win_if(entry.y > before, entry.x);
-      if (entry.y <= before && entry.y >= within) compare(entry);
+      if (entry.y <= before && entry.y >= within && entry.x < end) compare(entry);
     }
   } else {
     const unsigned tie = top - ties;

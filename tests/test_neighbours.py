@@ -384,6 +384,26 @@ def test_gpu_selection_orders_what_is_not_finite_by_its_bits(tokens, span):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tokens,longest,width", [(1800, 1024, 1024), (320, 1024, 1024), (140, 2048, 2048), (280, 2048, 40000), (140, 4096, 140000)])  # 128, 256, 512 (twice), 1024 threads
+def test_gpu_selection_with_masks_at_the_threshold_of_rows_that_are_listed_whole(tokens, longest, width):
+    """Few masks, or NaNs with a sign, among which the threshold lies: the lowest bins, which reach down to the lowest key."""
+    import torch
+
+    from ascendflow_b200 import neighbours
+    from tests.test_select_block import best, masked_rows
+
+    lengths, bits = masked_rows(np.random.default_rng(tokens), longest)
+    lengths = np.resize(np.array(lengths, dtype=np.int32), tokens)
+    rows = np.full((tokens, width), 0xFFFFFFFF, dtype=np.uint32)
+    rows[:, :longest] = bits[np.arange(tokens) % len(bits)]
+    device = lambda array: torch.from_numpy(np.ascontiguousarray(array)).cuda()  # noqa: E731
+    actual = neighbours.topk_indices(device(rows.view(np.float32)), device(np.arange(tokens + 1, dtype=np.int32)), device(lengths),
+                                     device(np.zeros(tokens, dtype=np.int32)), ratio=1).cpu().numpy()[:, 0]
+    for token in range(tokens):
+        assert np.array_equal(actual[token], best(rows[token, :lengths[token]])), (token, lengths[token])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tokens,span", [(1800, 14336), (1800, 4096), (320, 65536), (320, 14336), (19, 16384), (19, 40000), (7, 150000)])  # as above
 def test_gpu_selection_of_rows_that_a_sample_says_little_about(tokens, span):
     """Many equal scores at, above and below the threshold, at zero, among subnormals and at a mask; scores that
