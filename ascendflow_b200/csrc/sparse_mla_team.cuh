@@ -524,8 +524,8 @@ __global__ void __launch_bounds__(kThreads, 1) team_kernel(const Params p) {
   tc_fence_before_sync();
   if (!arrived) cluster_arrive_relaxed();
   cluster_wait();
+  __syncthreads();  // (the softmax warps come here from their last wait; the cluster's barrier they have passed before it)
   if (threadIdx.x == 0 && *sm.abort_flag() != 0) report(p, kStatusWaitExpired, blockIdx.x, 0);
-  __syncthreads();
   if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemColumns);
 }
 

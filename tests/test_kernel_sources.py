@@ -84,3 +84,13 @@ def test_issuing_threads_are_elected(name):
     kernel = (CSRC / name).read_text().split("__global__ void __launch_bounds__")[-1]
     calls = re.findall(r"if \((\w+\(\))\) (?:team_)?(?:qk|pv)\w*<kFormat[^>]*>\(", kernel)
     assert calls == ["elect_one()"] * 2
+
+
+@pytest.mark.parametrize("name", ["sparse_mla_tcgen05.cuh", "sparse_mla_team.cuh"])
+def test_a_wait_that_gave_up_is_looked_for_behind_a_barrier_of_the_whole_block(name):
+    """Any role's last wait can give up after other warps have left theirs; the softmax warps of a cluster arrive at its last barrier
+    before such a wait. So the flag is read behind a barrier that every warp comes to with nothing left to wait for."""
+    kernel = (CSRC / name).read_text().split("__global__ void __launch_bounds__")[-1]
+    roles_end = max(kernel.index("producer_role(p") if "producer_role(p" in kernel else 0, kernel.find("team_slices(p"))
+    behind = kernel[roles_end:kernel.index("report(p, kStatusWaitExpired")]
+    assert behind.rfind("__syncthreads();") > behind.rfind("cluster_wait();")
