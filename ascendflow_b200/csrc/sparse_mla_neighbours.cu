@@ -95,6 +95,7 @@ __device__ __forceinline__ uint4 load_keys(const float* row, unsigned i, unsigne
 }
 
 constexpr int kSelectBins = 256;
+constexpr int kHalfCapacity = 2560;  // of the list of 256 threads
 // The longest row. Loops over a row reach up to one of their steps past its end and count unsigned.
 constexpr int kMostSpan = INT32_MAX - 8192;
 
@@ -622,25 +623,12 @@ struct Loads {
 // 768 x 65536 scores, against the radix select that read every row five times: constant 373 -> 55 us, zeros 383
 // -> 80, all but 300 masked 360 -> 142, correlated over 64 positions 326 -> 192 (a fifth of the rows);
 // 100 rows of the latter 114 -> 80. With that select as the way out they took 461, 433, 457, 283 and 127.
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow, bool kCopyScores>
-__global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
+template <int kThreads, int kCapacity, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow, bool kCopyScores>
+__device__ __forceinline__ void select_row(const SelectParams& p, unsigned char* shared, const float* row, int candidates, int32_t* list) {
   using Shared = SelectShared<kThreads, kCapacity, kWindowSize>;
   constexpr int kWindow = Shared::kWindow;
-  extern __shared__ __align__(16) unsigned char select_smem[];
-  Shared& s = *reinterpret_cast<Shared*>(select_smem);
+  Shared& s = *reinterpret_cast<Shared*>(shared);
   const int lane = threadIdx.x & 31;
-  const int token = blockIdx.x;
-  sm100::wait_for_predecessor();
-  // Many rows: blocks of the next launch come when these end. Waiting beside them they take the slots
-  // of SMs that got fewer rows, and so spread their own unevenly (600 x 16 K: 19.3 against 16.4 us).
-  if constexpr (kThreads >= 512) sm100::let_successor_start();
-  const int candidates = int(min((int64_t)visible_compressed_rows<(kThreads >= 512)>(p, token, lane), p.span));
-  int32_t* list = p.out + (size_t)token * kTopK;
-  const float* row = p.scores + (size_t)token * p.span;
-  if (candidates <= kTopK) {
-    for (int i = threadIdx.x; i < kTopK; i += kThreads) list[i] = i < candidates ? i : -1;
-    return;
-  }
   for (int i = threadIdx.x * 4; i < min(candidates + 31, kWindow) / 32; i += kThreads * 4)
     *reinterpret_cast<uint4*>(&s.bitmap[i]) = make_uint4(0, 0, 0, 0);
   for (int i = threadIdx.x; i < kSelectBins; i += kThreads) s.histogram[i] = 0;
@@ -809,6 +797,34 @@ __global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const Se
   select_by_keys<kThreads, kCapacity>(s, row, end, list, floor_key, normal);
 }
 
+// kHalfRow: rows of up to so many scores are left to the first half of the block, which does as a block of its size.
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindowSize, int kShortRow, bool kCopyScores, int kHalfRow>
+__global__ void __launch_bounds__(kThreads, kBlocks) topk_select_kernel(const SelectParams p) {
+  extern __shared__ __align__(16) unsigned char select_smem[];
+  const int token = blockIdx.x;
+  sm100::wait_for_predecessor();
+  // Many rows: blocks of the next launch come when these end. Waiting beside them they take the slots
+  // of SMs that got fewer rows, and so spread their own unevenly (600 x 16 K: 19.3 against 16.4 us; two rows per SM and less, 149 of 600 to 64 K
+  // scores 10.9 / 10.3).
+  constexpr bool kFewRows = kThreads >= 512 && kHalfRow == 0;
+  if constexpr (kFewRows) sm100::let_successor_start();
+  const int candidates = int(min((int64_t)visible_compressed_rows<kFewRows>(p, token, threadIdx.x & 31), p.span));
+  int32_t* list = p.out + (size_t)token * kTopK;
+  const float* row = p.scores + (size_t)token * p.span;
+  if (candidates <= kTopK) {
+    for (int i = threadIdx.x; i < kTopK; i += kThreads) list[i] = i < candidates ? i : -1;
+    return;
+  }
+  if constexpr (kHalfRow > 0) {
+    if (candidates <= kHalfRow) {
+      // (Barriers of the block are of the threads that have not left.)
+      if (threadIdx.x < kThreads / 2) select_row<kThreads / 2, kHalfCapacity, 2, 4, kHalfRow, 0, false>(p, select_smem, row, candidates, list);
+      return;
+    }
+  }
+  select_row<kThreads, kCapacity, kMostQuads, kInFlight, kWindowSize, kShortRow, kCopyScores>(p, select_smem, row, candidates, list);
+}
+
 // One warp per new row: token j of n of request b goes to logical position L_b - n + j of the raw
 // cache (L_b includes this call's tokens, as `seqused_ori_kv` does for the attention operator),
 // i.e. to row `position % rows_per_page` of page `table[b][position / rows_per_page]`.
@@ -842,10 +858,11 @@ __global__ void cache_append_kernel(const char* new_rows, char* cache, const int
 }
 
 template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads), int kShortRow = 0,
-          bool kCopyScores = (kThreads >= 512)>
+          bool kCopyScores = (kThreads >= 512), int kHalfRow = 0>
 int launch_select(const SelectParams& p, cudaStream_t stream) {
-  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow, kCopyScores>;
+  auto* kernel = topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow, kCopyScores, kHalfRow>;
   constexpr int bytes = int(sizeof(SelectShared<kThreads, kCapacity, kWindow>));
+  static_assert(kHalfRow == 0 || sizeof(SelectShared<kThreads / 2, kHalfCapacity, kHalfRow>) <= bytes, "the half's fits");
   // A per-device setting: plain words written with the same value by whoever gets there first.
   static bool configured[64] = {false};
   int device = 0;
@@ -890,8 +907,10 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread for rows of more than three steps of
   // four. The kernel looks at the row for that: a buffer is as wide as the longest context (16 x 64 K: 10.8 with four loads, 10.3 with
   // eight; 30000: 8.5, 8.3; 24000: 7.6, 8.0; 4 K in buffers of 32 to 128 K: 6.9, 7.35). Two such blocks run on an SM: up to twice as
-  // many tokens in buffers beyond 32 K (sixteen / eight warps, 200 x 64 K: 13.3 / 16.8, 296 x 64 K: 14.3 / 18.5, 296 x 40000: 12.0 / 12.9,
-  // 200 x 32768: 10.9 / 11.4, 296 x 17000: 10.5 / 10.0, and rows of 4 K in a buffer of 64 K 9.6 / 9.1). Otherwise
+  // many tokens in buffers beyond 32 K, where rows of up to 16 K scores are left to half of their block, since what is shorter waits for sixteen
+  // warps' barriers and not for memory (296 rows in a buffer of 64 K, eight warps / sixteen / sixteen or half of them: 64 K scores 19.9 / 19.0 / 18.6, 32000
+  // 13.1 / 12.4 / 11.9, 17000 10.9 / 10.8 / 10.1, 8000 8.3 / 9.5 / 8.5, 2000 7.3 / 10.1 / 7.3, 600 6.8 / 8.0 / 6.9, 600 to 64 K 17.0 / 12.8 / 12.2; in a
+  // buffer of 32772 the last 12.4 / 10.9 / 10.9). Otherwise
   // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
   // more than a wave of them (four / eight warps, 8192 x 13000: 115.6 / 130, 4096 x 8 K: 49.6 / 58, 1500 x 2000: 16.8 / 19.8, but 2300 x 12 K: 32.9
   // / 37.8 beside 75 / 65 for scores that correlate), eight where there are fewer (1000 x 8 K: 14.9 / 19.0, but correlated 39.8 / 32.9: their
@@ -904,7 +923,8 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   // entries, which rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
   if (T <= multiprocessors && SPAN <= 24576) return launch_select<512, 4096, 2, 2>(p, s);
-  if (SPAN <= 131072 && (T <= multiprocessors || (T <= int64_t(multiprocessors) * 2 && SPAN > 32768))) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
+  if (SPAN <= 131072 && T <= multiprocessors) return launch_select<512, 4096, 2, 2, 8, 65536, 24576>(p, s);
+  if (SPAN <= 131072 && T <= int64_t(multiprocessors) * 2 && SPAN > 32768) return launch_select<512, 4096, 2, 2, 8, 65536, 24576, true, 16384>(p, s);
   if (SPAN > 131072)
     return T <= int64_t(multiprocessors) * 2 ? launch_select<512, 4096, 2, 2>(p, s) : launch_select<512, 4096, 2, 2, 4, 65536, 0, false>(p, s);
   const bool fewer_waves = (T - 1) / (multiprocessors * 10) < (T - 1) / (multiprocessors * 8);

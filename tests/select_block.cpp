@@ -44,6 +44,7 @@ inline void yield() {
 void enter() {
   body();
   finished[threadIdx.x] = true;
+  if (block_arrived == --block_threads && block_arrived > 0) { block_arrived = 0; ++block_generation; }  // barriers are of those who have not left
   swapcontext(&fibers[threadIdx.x], &scheduler);
 }
 inline void __syncthreads() {
@@ -132,21 +133,21 @@ inline void prefetch_l2(const void*, unsigned) {}
 
 struct SelectParams;
 template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight = 4, int kWindow = (kThreads >= 256 ? 65536 : 256 * kThreads), int kShortRow = 0,
-          bool kCopyScores = (kThreads >= 512)>
+          bool kCopyScores = (kThreads >= 512), int kHalfRow = 0>
 int launch_select(const SelectParams& p, cudaStream_t);
 
 #include "select.inc"
 
 const char* fault;
 int looked_at;
-template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindow, int kShortRow, bool kCopyScores>
+template <int kThreads, int kCapacity, int kBlocks, int kMostQuads, int kInFlight, int kWindow, int kShortRow, bool kCopyScores, int kHalfRow>
 int launch_select(const SelectParams& p, cudaStream_t) {
   constexpr size_t bytes = sizeof(SelectShared<kThreads, kCapacity, kWindow>);
   static_assert(bytes <= 227 << 10, "a block's shared memory");
   for (int token = 0; token < looked_at && fault == nullptr; ++token) {
     memset(select_smem, 0xa5, sizeof(select_smem));
     blockIdx.x = unsigned(token);
-    body = [&] { topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow, kCopyScores>(p); };
+    body = [&] { topk_select_kernel<kThreads, kCapacity, kBlocks, kMostQuads, kInFlight, kWindow, kShortRow, kCopyScores, kHalfRow>(p); };
     if (!run_block(kThreads)) fault = "a thread waits for ever";
     for (size_t i = bytes; i < sizeof(select_smem); ++i)
       if (select_smem[i] != 0xa5) { fault = "written behind the block's shared memory"; break; }

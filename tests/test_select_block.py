@@ -71,10 +71,10 @@ def masked_rows(rng, longest):
     return lengths, np.array(rows)
 
 
-@pytest.mark.parametrize("rows,longest", [(2000, 1024), (300, 1024), (100, 2048), (101, 4096)])  # 128, 256, 512 threads, and 1024 by the width below
+@pytest.mark.parametrize("rows,longest", [(2000, 1024), (300, 1024), (280, 1030), (100, 2048), (101, 4096)])  # 128, 256, half of 512, 512 threads, and 1024 by the widths below
 def test_masks_at_the_threshold_of_rows_that_are_listed_whole(select, rows, longest):
     lengths, bits = masked_rows(np.random.default_rng(rows), longest)
-    width = 140000 if longest == 4096 else longest + 4
+    width = {4096: 140000, 1030: 33000}.get(longest, longest + 4)
     wide = np.zeros((len(bits), width), dtype=np.uint32)
     wide[:, :longest] = bits
     picked = select(rows, lengths, wide)
@@ -82,7 +82,7 @@ def test_masks_at_the_threshold_of_rows_that_are_listed_whole(select, rows, long
         assert np.array_equal(picked[row], best(bits[row, :length])), (row, length)
 
 
-@pytest.mark.parametrize("rows,span", [(2000, 6000), (300, 6000), (100, 9000), (101, 140000)])
+@pytest.mark.parametrize("rows,span", [(2000, 6000), (300, 6000), (280, 40000), (100, 9000), (101, 140000)])
 def test_rows_that_are_sampled(select, rows, span):
     """The usual way, and the one by keys behind lists that are too long or too short."""
     rng = np.random.default_rng(span)
