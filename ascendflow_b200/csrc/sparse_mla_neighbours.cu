@@ -651,7 +651,11 @@ __device__ __forceinline__ void select_row(const SelectParams& p, unsigned char*
     constexpr int kSegments = kThreads / 8;
     // Where more quads than these are for long rows only, short ones step over them (8192 x 4 K scores 76 -> 73 us).
     constexpr int kFewQuads = 2;
-    const int quads = max(1, min(kMostQuads, candidates / (32 * kThreads))), sampled = quads * kThreads;
+    // Larger blocks have more quads for rows beyond this many (see the launch): a buffer is as wide as the longest context (in one of 128 K scores
+    // 888 x 64 K 40.3 -> 38.8 us, 600 x 96 K 46.1 -> 45.1).
+    constexpr int kLargeSampleRow = 98304;
+    const int most = kThreads >= 256 && candidates <= kLargeSampleRow ? min(kMostQuads, kFewQuads) : kMostQuads;
+    const int quads = max(1, min(most, candidates / (32 * kThreads))), sampled = quads * kThreads;
     const unsigned step = (unsigned(candidates) >> 2) / unsigned(quads * kSegments);  // at least eight quads
     uint4 v[kMostQuads];
 #pragma unroll
@@ -943,8 +947,9 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   if (SPAN <= 49152 && (T - 1) % (int64_t(multiprocessors) * 6) >= int64_t(multiprocessors) * 3)
     return SPAN <= 32768 ? launch_select<256, 2560, 6, 2, 4, 32768>(p, s) : launch_select<256, 2560, 6, 2, 4, 49152>(p, s);
   // Of 128 K scores a sample of 2048 leaves some fifteen hundred in the list, give or take three hundred, and room for 2560: every few
-  // thousand rows one is gone through again, which the call waits for. Twice the sample, 768 x 128 K: 82 us where it was 159 (500: 51 / 125, 3000: 252 / 332; calls
-  // without such a row, 320 x 128 K: 37.9 / 36.8). Up to 98304 scores the smaller one is enough (768 of them: 63.0, 65.3 with the larger).
+  // thousand rows one is gone through again, which the call waits for. Twice the sample (scores from memory): 768 x 128 K 80.9 us where it was 166,
+  // 888: 85 / 168, 1500: 136 / 223. Calls without such a row pay up to one per cent for it (600 x 128 K 65.3 / 64.6);
+  // with one they take 80 us more. Rows of up to 98304 scores have the smaller sample.
   return SPAN > 98304 ? launch_select<256, 2560, 6, 4>(p, s) : launch_select<256, 2560, 6, 2>(p, s);
 }
 

@@ -187,7 +187,7 @@ def test_gpu_selection_at_the_edges_of_its_blocks(tokens, visible):
     (2368, [16000, 9000, 12289]), (2369, [16384, 10241]), (1800, [10240, 700]), (1800, [10244, 10241, 10240]),  # waves of eight and of ten blocks
     (296, [32772, 32768, 700]), (296, [32768, 4097]), (297, [32772, 20000]),  # two rows per SM
     (149, [40000, 16384, 16385, 16383, 1025, 1024, 513, 512]), (296, [65536, 16385, 2560, 2561, 1024, 1]),  # all of a block or half of it
-    (297, [98308, 98304, 1025]), (297, [98304, 30000]),  # the larger sample
+    (297, [98308, 98304, 1025]), (297, [98304, 30000]), (300, [131072, 98304, 98305, 40000, 8192, 1025]),  # the larger sample, of long rows
     (297, [16388, 16384, 513]), (297, [24576, 24575, 16385, 700]), (297, [24580, 24576]),  # bitmaps of 16, 24 and 64 K
     (444, [32768, 24577]), (446, [24580, 24577, 1025]), (446, [32768, 32767, 30001, 2561]), (446, [32772, 32768]),
     (446, [49152, 49151, 40001]), (446, [49156, 49152]), (444, [49152]),  # or 32 and 48 K
