@@ -20,7 +20,7 @@ def kernel_text(source):
         text, found = re.subn(rf"__device__ __forceinline__ void {name}\([^)]*\) {{\n  asm volatile\(.*\);\n}}\n", "", text)
         assert found == 1, name
     text, found = re.subn(r'asm volatile\("cp\.async\.wait_all;\\n" ::: "memory"\);', "wait_for_words();", text)
-    assert found == 1 and "asm" not in text
+    assert found == 2 and "asm" not in text
     rule = source[source.index("int launch_sparse_mla_topk_indices("):]
     return text + rule[:rule.index("\n}\n") + 3]
 
