@@ -282,7 +282,7 @@ __device__ __forceinline__ void copy_word(uint32_t to, const float* from) {
 // bound by what is issued, or wait for it: scores become keys once, behind the first digit an entry is compared with two keys, a
 // winner is known by its bit when it looks for its place, and loops have no ends to look for and no branches. 8192 rows of 12-16 K scores 118 ->
 // 110 us (94 -> 81 million instructions of a warp), of 4 K 85 -> 76, 1500 x 10 K 28.9 -> 25.8, 2000 x 20 K 40.4 -> 35.8, 16 x 16 K 6.85 -> 6.45.
-template <int kThreads, int kCapacity, typename Shared>
+template <int kThreads, int kCapacity, bool kKeysApart, typename Shared>
 __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int listed, unsigned floor_key, int32_t* list) {
   constexpr int kWindow = Shared::kWindow;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -293,11 +293,13 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
   // threshold turns out to lie there.
   unsigned top = s.high, bottom = floor_key;
   bool exact = false;
-  auto find_extremes = [&]() {
+  auto find_extremes = [&](bool scores) {
     unsigned low = 0xffffffffu, high = 0;
     for (int i = threadIdx.x; i < listed; i += kThreads) {
-      low = min(low, s.list[i].y);
-      high = max(high, s.list[i].y);
+      unsigned key = s.list[i].y;
+      if (scores) s.list[i].y = key = score_key(key);
+      low = min(low, key);
+      high = max(high, key);
     }
     low = __reduce_min_sync(0xffffffffu, low);
     high = __reduce_max_sync(0xffffffffu, high);
@@ -308,28 +310,28 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
     exact = true;
   };
   const bool sampled = floor_key != 0;
-  int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
   // The list is filled up to whole rounds of the block: no loop over it looks for its end. The filling's position is one that no row has (it is in
   // no window and not before `end`), its key is 0: it reaches no sampled floor, which is at least 1, and lies above no key.
   const int rounds = (listed + kThreads - 1) / kThreads;
   static_assert(kCapacity % kThreads == 0, "whole rounds fit");
-  if (listed + int(threadIdx.x) < rounds * kThreads) s.list[listed + threadIdx.x] = make_uint2(0xffffffffu, 0xffffffffu);
-  __syncthreads();
+  if (listed + int(threadIdx.x) < rounds * kThreads) s.list[listed + threadIdx.x] = make_uint2(0xffffffffu, kKeysApart || sampled ? 0xffffffffu : 0u);
   const uint32_t histogram = sm100::smem_u32(s.histogram);
-#pragma unroll 4
-  for (int r = 0; r < rounds; ++r) {
-    uint2& entry = s.list[r * kThreads + threadIdx.x];
-    const unsigned key = score_key(entry.y);
-    entry.y = key;
-    shared_add_if(sampled && key >= floor_key, histogram + ((top - min(key, top)) >> shift) * 4);
-  }
-  bool counted = sampled;  // the present digit
-  if (!sampled) {
+  // Rows listed whole have nothing counted yet: their keys are made on the way to the extremes (600 x 600 scores 9.45 -> 8.9 us, 888 x 600 10.9 ->
+  // 10.2, 8192 x 600 59.6 -> 56.8). kKeysApart: in the loop of the others, and gone through again.
+  if (kKeysApart || sampled) {
+    const int shift = max(0, 24 - __clz(int(top - bottom)));
     __syncthreads();
-    find_extremes();
-    above = 32 - __clz(int(top - bottom));
-    shift = max(0, above - 8);
+#pragma unroll 4
+    for (int r = 0; r < rounds; ++r) {
+      uint2& entry = s.list[r * kThreads + threadIdx.x];
+      const unsigned key = score_key(entry.y);
+      entry.y = key;
+      shared_add_if(sampled && key >= floor_key, histogram + ((top - min(key, top)) >> shift) * 4);
+    }
   }
+  if (!sampled) find_extremes(!kKeysApart);  // of the entries that this thread has made keys, or makes keys now
+  int above = 32 - __clz(int(top - bottom)), shift = max(0, above - 8);  // bits of the distance; bits below the digit
+  bool counted = sampled;  // the present digit
   unsigned wanted = kTopK;
   unsigned prefix = 0;  // leading bits found so far
   unsigned ties = 0xffffffffu;  // distance of the threshold, once the position decides
@@ -351,7 +353,7 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
     }
     prefix = prefix << (above - shift) | s.bin;
     if (prefix == 0 && !exact && ties == 0xffffffffu) {
-      find_extremes();
+      find_extremes(false);
       above = 32 - __clz(int(top - bottom));
       shift = max(0, above - 8);
       continue;
@@ -476,12 +478,12 @@ __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int li
 // 115 called, rows of one constant 112.5 and 106.8). Larger blocks have it inline (768 x 64 K 37.6, called 39.0).
 template <int kThreads, int kCapacity, typename Shared>
 __device__ __noinline__ bool select_from_list_apart(Shared& s, unsigned end, int listed, unsigned floor_key, int32_t* list) {
-  return select_from_list<kThreads, kCapacity>(s, end, listed, floor_key, list);
+  return select_from_list<kThreads, kCapacity, false>(s, end, listed, floor_key, list);
 }
-template <int kThreads, int kCapacity, typename Shared>
+template <int kThreads, int kCapacity, bool kKeysApart = false, typename Shared>
 __device__ __forceinline__ bool select_listed(Shared& s, unsigned end, int listed, unsigned floor_key, int32_t* list) {
   if constexpr (kThreads == 128) return select_from_list_apart<kThreads, kCapacity>(s, end, listed, floor_key, list);
-  else return select_from_list<kThreads, kCapacity>(s, end, listed, floor_key, list);
+  else return select_from_list<kThreads, kCapacity, kKeysApart>(s, end, listed, floor_key, list);
 }
 
 // Lists what reaches the floor, by keys. For 128 threads: with 48 registers the loop in `select_by_keys` spills and waits for every
@@ -796,8 +798,10 @@ __device__ __forceinline__ void select_row(const SelectParams& p, unsigned char*
     if constexpr (kCopyScores) asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     const int listed = int(s.count);
+    // (With the keys of whole rows made apart the pass over long rows is slower in this one form: 768 x 64 K 41.8 -> 43.0 us, 2000 x 64 K 90.6 -> 96.2.)
+    constexpr bool kKeysApart = kThreads == 256 && kWindow == 65536 && kMostQuads == 2;
     if (listed >= kTopK && listed <= kCapacity) {
-      if (select_listed<kThreads, kCapacity>(s, end, listed, floor_key, list)) return;
+      if (select_listed<kThreads, kCapacity, kKeysApart>(s, end, listed, floor_key, list)) return;
     }
   }
   select_by_keys<kThreads, kCapacity>(s, row, end, list, floor_key, normal);
@@ -950,7 +954,7 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
     return SPAN <= 32768 ? launch_select<256, 2560, 6, 2, 4, 32768>(p, s) : launch_select<256, 2560, 6, 2, 4, 49152>(p, s);
   // Of 128 K scores a sample of 2048 leaves some fifteen hundred in the list, give or take three hundred, and room for 2560: every few
   // thousand rows one is gone through again, which the call waits for. Twice the sample (scores from memory): 768 x 128 K 80.9 us where it was 166,
-  // 888: 85 / 168, 1500: 136 / 223. Calls without such a row pay up to one per cent for it (600 x 128 K 65.3 / 64.6);
+  // 888: 85 / 168, 1500: 136 / 223. Calls without such a row pay up to two per cent for it (600 x 128 K 65.3 / 64.2);
   // with one they take 80 us more. Rows of up to 98304 scores have the smaller sample.
   return SPAN > 98304 ? launch_select<256, 2560, 6, 4>(p, s) : launch_select<256, 2560, 6, 2>(p, s);
 }
