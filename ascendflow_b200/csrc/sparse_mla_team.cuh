@@ -253,8 +253,8 @@ __device__ __forceinline__ void issue_team_pv(uint32_t tmem, uint64_t p_desc, ui
   }
 }
 
-// Phase B, one thread: O = P X over all chunks, this block's 128 features. Unrolled over the chunks: in a loop the
-// descriptors of every instruction are worked out on the way to it (one token 9.69 -> 8.83 us, 16 tokens 10.02 -> 9.20; two
+// Phase B, one thread: O = P X over all chunks, this block's 128 features. Unrolled over the chunks, so that
+// descriptors are constants off two addresses (in a loop one token 9.69 us against 8.83, 16 tokens 10.02 against 9.20; two
 // chunks to a pass 9.14 and 9.46).
 template <int kFormat>
 __device__ void team_pv(const Shared& sm, uint32_t tmem) {

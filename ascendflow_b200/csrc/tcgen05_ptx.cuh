@@ -199,10 +199,9 @@ __host__ __device__ constexpr uint32_t idesc_f16(int m, int n, int format, int a
 
 // ---- MMA issue (one thread) ------------------------------------------------------------------
 
-// True in one thread of the warp, always the same one. Who issues products is chosen by this and not by a comparison of the thread index:
-// the compiler then knows that a single thread is running and computes descriptors in uniform registers, where the instructions
-// take them from. Behind a comparison every operand of every instruction was moved there by itself (one token 10.6 -> 9.3 us,
-// 16 tokens 11.0 -> 9.6, 256 tokens at 4K 30.6 -> 29.9, prefill of 8K tokens 824 -> 809, 23 mixed requests 163.9 -> 160.2).
+// True in one thread of the warp, always the same one. Who issues products is chosen by this and not by a comparison of the thread index, from
+// which the compiler cannot tell that a single thread runs. Measured against `lane == 0`: one token 10.6 -> 9.3 us,
+// 16 tokens 11.0 -> 9.6, 256 tokens at 4K 30.6 -> 29.9, prefill of 8K tokens 824 -> 809, 23 mixed requests 163.9 -> 160.2.
 __device__ __forceinline__ bool elect_one() {
   uint32_t elected;
   asm volatile(
