@@ -281,7 +281,7 @@ __device__ __forceinline__ void copy_word(uint32_t to, const float* from) {
 // Every instruction here is executed for each of the eight or nine hundred entries of every row, and rows are
 // bound by what is issued, or wait for it: scores become keys once, behind the first digit an entry is compared with two keys, a
 // winner is known by its bit when it looks for its place, and loops have no ends to look for and no branches. 8192 rows of 12-16 K scores 118 ->
-// 110 us (94 -> 81 million instructions of a warp), of 4 K 85 -> 76, 1500 x 10 K 28.9 -> 25.8, 2000 x 20 K 40.4 -> 35.8, 16 x 16 K 6.85 -> 6.45.
+// 110 us (93.5 -> 86.5 million instructions of a warp), of 4 K 85 -> 76, 1500 x 10 K 28.9 -> 25.8, 2000 x 20 K 40.4 -> 35.8, 16 x 16 K 6.85 -> 6.45.
 template <int kThreads, int kCapacity, bool kKeysApart, typename Shared>
 __device__ __forceinline__ bool select_from_list(Shared& s, unsigned end, int listed, unsigned floor_key, int32_t* list) {
   constexpr int kWindow = Shared::kWindow;
@@ -607,9 +607,9 @@ struct Loads {
 // ties going to the lower index; winners are written in ascending index order, the rest of the 512
 // entries is -1.
 //
-// Bound by memory for long rows (768 x 65536 scores: 44 us, 70 % of the copy bandwidth; the radix
+// Bound by memory for long rows (768 x 65536 scores: 44 us as called, 70 % of the copy bandwidth; the radix
 // select that read the row five times took 335 us) and by what is issued, instructions and shared memory's accesses, for many
-// short ones (8192 x 12-16 K: 110 us, 4.3 TB/s; issue slots 64 %, the pipe to shared memory and L1 71 %; before 1003 us). The row is streamed once. A strided sample (one or
+// short ones (8192 x 12-16 K: 110 us, 4.3 TB/s; issue slots 69 %; before 1003 us). The row is streamed once. A strided sample (one or
 // two thousand scores in 128-byte pieces) gives a floor that about twice TopK scores lie above; the
 // stream lists what reaches the floor (two instructions per score, next to nothing listed), and the exact selection runs on
 // that short list in shared memory: a histogram of the keys' distances from the highest, 256
@@ -909,27 +909,31 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device);
   p.one_wave = T <= int64_t(multiprocessors) * 6;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Rows so long that a small block's sample says too little: large blocks (16 x 1 M scores: 98 us against 398
-  // with 512 threads, 300 x 1 M: 357 against 695, 16 x 200 K: 32.8 against 35.8), for many rows only beyond 256 K.
-  // Two blocks of 512 threads to an SM are better before that, and where the buffer is wide but the rows are
-  // not (600 x 200 K: 131 us against 154, 2000 rows of 2 K in a buffer of 140000: 68 against 120). No more tokens than SMs: a
-  // row's latency counts, sixteen warps (16 tokens of 8192 scores: 7.6 us against 8.6 with eight and 13
-  // with thirty-two; of 65536: 11 us against 15), with eight loads in flight per thread for rows of more than three steps of
-  // four. The kernel looks at the row for that: a buffer is as wide as the longest context (16 x 64 K: 10.8 with four loads, 10.3 with
-  // eight; 30000: 8.5, 8.3; 24000: 7.6, 8.0; 4 K in buffers of 32 to 128 K: 6.9, 7.35). Two such blocks run on an SM: up to twice as
-  // many tokens in buffers beyond 32 K, where rows of up to 16 K scores are left to half of their block, since what is shorter waits for sixteen
+  // T x N below are T rows of N scores, in a buffer as wide unless its width is given; us per call, scores from memory, these kernels unless said otherwise.
+  //
+  // Rows so long that a smaller block's sample says too little: 1024 threads (1024 / 512: 16 x 1 M 89 / 318, 300 x 1 M 330 / 599, 148 x 300 K 44.3 / 46.7, 16 x 200 K
+  // 23.4 / 26.8), for more rows than SMs only beyond 256 K: two blocks of 512 threads to an SM are better before that (300 x 200 K 81.2 / 71.9, 600 x 200 K 137 /
+  // 114) and where the buffer is wide but the rows are not (2000 x 2000 in 140000 107 / 57). What loses by it: 600 x 300 K 186 / 162, 16 x 6000 in 140000 8.7 / 6.9.
+  //
+  // No more rows than SMs: a row's latency counts, 512 threads (1024 / 512 / 256: 16 x 16 K 8.1 / 6.7 / 7.6, 148 x 64 K 13.8 / 12.8 / 17.5, 148 x 128 K 21.4 / 19.8 / 30.0; what
+  // loses: 16 x 8 K 8.7 / 6.9 / 6.6, 16 x 2000 8.0 / 7.3 / 6.2), with eight loads in flight per thread for rows of more than three steps of
+  // four. The kernel looks at the row for that: a buffer is as wide as the longest context (four / eight in a buffer of 64 K, 16 x 64 K 9.7 / 8.8, 30000 7.9 / 7.6, 24000
+  // 7.4 / 7.5, 4096 6.8 / 7.0). Two such blocks run on an SM: up to twice as
+  // many rows in buffers beyond 32 K, where rows of up to 16 K scores are left to half of their block, since what is shorter waits for sixteen
   // warps' barriers and not for memory (296 rows in a buffer of 64 K, eight warps / sixteen / sixteen or half of them: 64 K scores 19.9 / 19.0 / 18.6, 32000
-  // 13.1 / 12.4 / 11.9, 17000 10.9 / 10.8 / 10.1, 8000 8.3 / 9.5 / 8.5, 2000 7.3 / 10.1 / 7.3, 600 6.8 / 8.0 / 6.9, 600 to 64 K 17.0 / 12.8 / 12.2; in a
-  // buffer of 32772 the last 12.4 / 10.9 / 10.9). Otherwise
-  // small blocks, several to an SM, whose phases overlap: four warps per row where there are rows for
-  // more than a wave of them (four / eight warps, 8192 x 13000: 115.6 / 130, 4096 x 8 K: 49.6 / 58, 1500 x 2000: 16.8 / 19.8, but 2300 x 12 K: 32.9
-  // / 37.8 beside 75 / 65 for scores that correlate), eight where there are fewer (1000 x 8 K: 14.9 / 19.0, but correlated 39.8 / 32.9: their
-  // lists miss more often the smaller the sample is) or where the row needs the larger sample. What such rows wait for is one step after the
-  // other: up to 16 K scores (a bitmap of one window) ten blocks of 48 registers per SM with four loads in flight against eight with
-  // eight loads: ten / eight, 8192 x 2000: 66.0 / 76.3, 4096 x 8 K: 49.6 / 50.9, 3300 x 10 K: 45.5 / 45.0; beyond 10 K scores
-  // only where they make fewer waves (2450 x 16 K: 39.9 / 40.9, 7400 x 12 K: 98.0 / 98.2, 7400 x 16 K: 111.1 / 107.6; where they do not, 1800 x
-  // 16 K: 34.4 / 30.4, 3300 x 16 K: 54.9 / 50.7). Longer rows are streaming for the most part: eight blocks, eight
-  // loads (4096 x 17408: 74.3 / 76.9, 2000 x 20 K: 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536
+  // 13.1 / 12.4 / 11.9, 17000 10.9 / 10.8 / 10.1, 8000 8.3 / 9.5 / 8.5, 2000 7.3 / 10.1 / 7.3, 600 6.8 / 8.0 / 6.5, 600 to 64 K 17.0 / 12.8 / 12.2; in a
+  // buffer of 32772 the last 12.4 / 10.9 / 10.9).
+  //
+  // More rows: small blocks, several to an SM, whose phases overlap. Four warps per row from twelve rows per SM on (four / eight, 8192 x 12 K 103 / 124, 4096 x 8 K 47.7 /
+  // 57.8, 2000 x 4 K 22.5 / 26.6, 4096 x 32 K 97.5 / 102). Fewer rows too would be faster with four (1184 x 8 K 16.0 / 21.2, 1500 x 4 K 19.1 / 20.7), but not where scores
+  // correlate: the list misses more often the smaller the sample is (1184 x 8 K 40.0 / 35.5, 1500 x 16 K 79 / 64, 888 x 16 K 69 / 55; beyond the line as well, 1776 x 16 K
+  // 83 / 69, 4096 x 16 K 124 / 114).
+  // Of these, rows of up to 16 K scores (a bitmap of one window) run ten blocks of 48 registers per SM with four loads in flight, or eight blocks with eight loads (ten /
+  // eight). Up to 10 K ten: 8192 x 2000 63.2 / 72.0, 8192 x 4 K 73.3 / 76.3, 4096 x 8 K 47.7 / 47.6, 4096 x 10 K 51.8 / 53.6. Beyond, ten where they make fewer waves: 2450 x
+  // 12 K 36.1 / 36.6, 4096 of 600 to 16 K 44.4 / 46.7, but 4096 x 16 K 65.1 / 63.0, 7400 x 16 K 108 / 106, 8192 of 12 to 16 K 109.8 / 107.8; where they do not, eight: 1776 x
+  // 12 K 31.3 / 27.2, 3300 x 16 K 55.5 / 51.1. With as many waves eight are better from 5 K on by now (1776 x 2000 18.5 / 19.2, 1776 x 4 K 21.3 / 20.8, 1800 of 7.5
+  // to 10 K 30.2 / 26.6, 3000 x 8 K 38.7 / 36.1): the line at 10 K is that of a slower ranking. Longer rows are streaming for the most part: eight blocks, eight
+  // loads (against ten, with that ranking: 4096 x 17408: 74.3 / 76.9, 2000 x 20 K: 39.2 / 43.9, 4096 x 32 K: 107.4 / 112.8). Eleven blocks leave a list of 1536
   // entries, which rows that correlate overflow (8192 x 16 K of zeros 130 -> 164).
   if (SPAN > 262144 || (SPAN > 131072 && T <= multiprocessors)) return launch_select<1024, 8192, 1, 2>(p, s);
   if (T <= multiprocessors && SPAN <= 24576) return launch_select<512, 4096, 2, 2>(p, s);
@@ -940,14 +944,14 @@ int launch_sparse_mla_topk_indices(void* stream, void* arg_scores, void* arg_cu_
   const bool fewer_waves = (T - 1) / (multiprocessors * 10) < (T - 1) / (multiprocessors * 8);
   if (T >= int64_t(multiprocessors) * 12 && SPAN <= 32768)
     return SPAN <= (fewer_waves ? 16384 : 10240) ? launch_select<128, 2048, 10, 4, 4, 16384>(p, s) : launch_select<128, 2048, 8, 4, 8>(p, s);
-  // A bitmap no larger than the row: what shared memory it does not take holds scores that are read again (860 x 16 K: 19.7 ->
-  // 19.0 us, 150 such rows that correlate 39.1 -> 36.3; blocks of 512 threads: no change).
+  // A bitmap no larger than the row: what shared memory it does not take holds scores that are read again (860 x 16 K 18.8 ->
+  // 17.2, such rows that correlate 54.5 -> 53.2; blocks of 512 threads: no change).
   if (SPAN <= 16384) return launch_select<256, 2560, 6, 2, 4, 16384>(p, s);
   // The same beyond, where three more such steps lie: six blocks with a bitmap of 24 K leave 92 KiB of L1 on an SM, of 32 and 48 K 60, of 64 K
-  // 28, and the sample's 48 KiB are read again in the pass (64 K / the smaller one: 600 x 18000 17.8 / 16.6, 888 x 24000 23.0 / 21.0, 1200
-  // x 18000 30.5 / 27.8, 300 x 20000 12.8 / 12.6). The steps to 32 and 48 K are taken where the last wave is at least half full (600 x 30000
-  // 22.9 / 20.9, 888 x 32768 26.0 / 24.9, 1750 x 30000 50.0 / 46.3, 600 x 45000 28.9 / 25.5, 888 x 48 K 35.4 / 34.0; where it is not, 300 x
-  // 32768 14.6 / 15.1, 1200 x 32768 35.4 / 35.8, 1000 x 48 K 43.2 / 44.8).
+  // 28, and the sample's 48 KiB are read again in the pass (64 K / the smaller one: 600 x 18000 17.8 / 16.2, 888 x 24000 23.0 / 20.9, 1200
+  // x 18000 30.7 / 28.1, 300 x 20000 12.2 / 12.0). The steps to 32 and 48 K are taken where the last wave is at least half full (600 x 30000
+  // 23.2 / 21.1, 888 x 32768 26.2 / 25.1, 1750 x 30000 50.2 / 46.8, 600 x 45000 28.5 / 25.2, 888 x 48 K 35.0 / 33.6; where it is not, 300 x
+  // 32768 14.8 / 15.2, 1200 x 32768 35.5 / 35.7, 1000 x 48 K 43.3 / 45.0).
   // A smaller one for longer rows, in several rounds: 500 x 50000 27.5 / 26.2, but 300 x 64 K 21.8 / 24.4.
   if (SPAN <= 24576) return launch_select<256, 2560, 6, 2, 4, 24576>(p, s);
   if (SPAN <= 49152 && (T - 1) % (int64_t(multiprocessors) * 6) >= int64_t(multiprocessors) * 3)

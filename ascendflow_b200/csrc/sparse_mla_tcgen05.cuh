@@ -506,7 +506,7 @@ __device__ __forceinline__ void store_places(uint32_t places_tmem, int lane) {
 
 // Copies of a chunk's rows into a tile, all 64 or one half of them, by the 256 producer threads. A row is taken by eight threads, 128
 // bytes at a time: two rows and their addresses to a thread. (Sixteen threads with 256 bytes at a time make as many requests, but four rows
-// to a thread: 62.3 million instructions of a warp for 2072 tokens against 58.6, one token 9.09 -> 8.97 us, 256 tokens at 4K 28.3 -> 27.6.)
+// to a thread: 62.3 million instructions of a warp for 2072 tokens against 58.6; loops over the launch alone, one token 9.09 -> 8.97 us, 256 tokens at 4K 28.3 -> 27.6.)
 template <int kHalf, int kHalves>
 __device__ __forceinline__ void gather_rows(const Params& p, const int* rows, int chunk, uint32_t tile, int tid) {
   constexpr int kAtOnce = kProducerThreads / 8, kRows = kChunkRows / kAtOnce / kHalves;  // rows side by side; of a thread
@@ -809,9 +809,9 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
 // A second P tile takes the wait for the previous PV out of the chain, and flags by a named barrier a word in shared memory and a
 // wait: five per cent of 100 and of 256 tokens, two of 1000, one of prefill of 8K.
 //
-// Calls one after the other take 815 us for prefill of 8K tokens at 32K (835 with sixteen threads to a gathered row and issuing threads that were not
-// elected, in turn on one board), 114 for decode 128 x 6 at 128K (116), 162 for 23 mixed requests (166), 27.5 for
-// 256 tokens at 4K (29.4). The first three are at the board's power limit (990 to 1000 W; 1.47 to 1.60 GHz while they run, by the board: three
+// Calls one after the other through the Python entry points take 822 us for prefill of 8K tokens at 32K (842 with sixteen threads to a gathered row and
+// issuing threads that were not elected, in turn on one board), 163 for 23 mixed requests (167), 29.9 for 256 tokens at 4K (31.0); decode
+// 128 x 6 at 128K 115 either way. The first two and the last are at the board's power limit (990 to 1000 W; 1.47 to 1.60 GHz while they run, by the board: three
 // per cent of time between two of them), where energy decides more than cycles.
 template <int kFormat>
 __device__ void softmax_role(const Params& p, const Shared& sm, uint32_t tmem) {
