@@ -47,14 +47,14 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # B16 x 6 queries at ctx 128K: 96 tokens). Other sizes of the same regime are scaled by token
 # count, since traffic is Q + O + gathered rows per token. Every figure belongs to the kernel
 # sources whose hash is recorded with it: a line measured with other sources says so.
-PROFILED_SOURCES = "1ff1d5fe86501ccc937439aeb2e28d8b8c7a7673eff8bce68d16bd20e045f5cd"
+PROFILED_SOURCES = "e1e3e10171251dba11c5c9261b82555f4af794b534ddfc9dc2ce7d16dba67627"
 FULL_SIZE_DECODE_SOURCES = "a052a0f1daaa0bb772d9b2730e66d14607c8ec27f78db0ebf7f42e0c5f4431b3"
 MEASURED_TRAFFIC = {  # query tokens of the captured launches: bytes of a launch, sources
     "prefill": {"profile": "profiles/attention_kernel_prefill_q8k_ctx32k.md",
-                "launches": {8192: (1077.29e6, PROFILED_SOURCES)}, "scaled_from": 8192},
+                "launches": {8192: (1076.44e6, PROFILED_SOURCES)}, "scaled_from": 8192},
     "decode": {"profile": "profiles/attention_kernel_decode_dram_traffic.md",
                "launches": {768: (500.34e6, FULL_SIZE_DECODE_SOURCES), 384: (242.30e6, FULL_SIZE_DECODE_SOURCES),
-                            96: (59.72e6, PROFILED_SOURCES)}, "scaled_from": 768},
+                            96: (58.70e6, PROFILED_SOURCES)}, "scaled_from": 768},
 }
 EXTRA_WORKLOADS = ("prefill_q32k_ctx32k", "decode_b64_q6_ctx128k", "decode_b128_q6_ctx128k")
 CONFIG_KEYS = {"heads": 64, "features": 512, "topk": 512, "window": 128, "ratio": 2, "values": "N(0,1)",
